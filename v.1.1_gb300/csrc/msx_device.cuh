@@ -1396,36 +1396,45 @@ __device__ __forceinline__ void stress_mixed(const MatParams &m, const float *H,
         return;
     }
     float D[9];
-    float a0 = t + I2, a1 = 1.0f + t;
+    const float a0 = t + I2, a1 = 1.0f + t;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             // (H^2)^T_ij = sum_k H_jk H_ki
-            float h2 = H[j * 3] * H[i] + H[j * 3 + 1] * H[3 + i] + H[j * 3 + 2] * H[6 + i];
-            D[i * 3 + j] = (i == j ? a0 : 0.0f) - a1 * H[j * 3 + i] + h2;
+            const float x = H[j * 3], X = H[i], y = H[j * 3 + 1], Y = H[3 + i], z = H[j * 3 + 2], Z = H[6 + i];
+            float h2;
+            if (i == 0 && j == 0) h2 = __fadd_rn(fmaf(x, X, __fmul_rn(y, Y)), __fmul_rn(z, Z));
+            else if (i == 1 && j == 1) h2 = __fadd_rn(fmaf(y, Y, __fmul_rn(x, X)), __fmul_rn(z, Z));
+            else if (i == 2 && j == 2) h2 = fmaf(z, Z, __fadd_rn(__fmul_rn(x, X), __fmul_rn(y, Y)));
+            else h2 = fmaf(z, Z, fmaf(x, X, __fmul_rn(y, Y)));
+            D[i * 3 + j] = __fadd_rn(i == j ? fmaf(-a1, H[j * 3 + i], a0) : -__fmul_rn(a1, H[j * 3 + i]), h2);
         }
-    float iJ = 1.0f / (1.0f + Jm1);
+    const float Jx = 1.0f + Jm1, iJ = 1.0f / Jx;
     if (m.law == 1) {
         // P = [mu (Jm1 I + (1+Jm1) H - D) + lambda lnJ (I + D)] / J
-        float lj = m.lambda_f * lnJ;
+        const float lj = __fmul_rn(m.lambda_f, lnJ);
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-            float dg = (k % 4 == 0) ? 1.0f : 0.0f;
-            P[k] = (m.mu_f * (Jm1 * dg + (1.0f + Jm1) * H[k] - D[k]) + lj * (dg + D[k])) * iJ;
+    // Products and sums are spelled out (fmaf, _rn) from here on: which product
+    // of a*b + c*d is fused is otherwise the compiler's choice, and differs
+    // between the instantiations of this body; a pooled solve has to give the
+    // bits of the solve run alone.
+            const float q = __fadd_rn(k % 4 == 0 ? fmaf(Jx, H[k], Jm1) : __fmul_rn(Jx, H[k]), -D[k]);
+            P[k] = __fmul_rn(fmaf(lj, k % 4 == 0 ? __fadd_rn(1.0f, D[k]) : D[k], __fmul_rn(m.mu_f, q)), iJ);
         }
     } else {
-        // P = mu J^-2/3 [(Jm1 - beta) I + (1+Jm1) H - (1+beta) D]/J + K Jm1 (I + D)
+        // P = mu J^-2/3 [(Jm1 - beta) I + (1+Jm1) H - (1+beta) D]/J + K Jm1 (I + D), beta = b3 / 3
         float hh = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 9; k++) hh += H[k] * H[k];
-        float beta = (2.0f * t + hh) * (1.0f / 3.0f);
-        float j23 = expf(-(2.0f / 3.0f) * lnJ) * m.mu_f * iJ;
-        float kj = m.K1_f * Jm1;
+        for (int k = 0; k < 9; k++) hh = fmaf(H[k], H[k], hh);
+        const float b3 = fmaf(2.0f, t, hh), b1 = fmaf(b3, 1.0f / 3.0f, 1.0f), Jb = fmaf(-b3, 1.0f / 3.0f, Jm1);
+        const float j23 = __fmul_rn(__fmul_rn(expf(__fmul_rn(-(2.0f / 3.0f), lnJ)), m.mu_f), iJ);
+        const float kj = __fmul_rn(m.K1_f, Jm1);
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-            float dg = (k % 4 == 0) ? 1.0f : 0.0f;
-            P[k] = j23 * ((Jm1 - beta) * dg + (1.0f + Jm1) * H[k] - (1.0f + beta) * D[k]) + kj * (dg + D[k]);
+            const float q = fmaf(-b1, D[k], k % 4 == 0 ? fmaf(Jx, H[k], Jb) : __fmul_rn(Jx, H[k]));
+            P[k] = fmaf(kj, k % 4 == 0 ? __fadd_rn(1.0f, D[k]) : D[k], __fmul_rn(j23, q));
         }
     }
 }
@@ -1458,7 +1467,8 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) H[i * 3 + j] = du[i] * G[j] + du[3 + i] * G[3 + j] + du[6 + i] * G[6 + j];
+            for (int j = 0; j < 3; j++)
+                H[i * 3 + j] = fmaf(du[6 + i], G[6 + j], fmaf(du[i], G[j], __fmul_rn(du[3 + i], G[3 + j])));
         // J - 1 = tr H + (I2(H) + det H).  The trace carries J - 1 and may
         // cancel (nearly isochoric motion), so it is summed without rounding,
         // as s + err by TwoSum; I2 and det H are O(|H|^2) and their FP32
@@ -1466,9 +1476,12 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
         // good to FP32 relative precision, and so is ln J = log1p(J - 1);
         // F = I + H is never formed or reduced.
         float tf = H[0] + H[4] + H[8];
-        float I2f = (H[0] * H[4] - H[1] * H[3]) + (H[4] * H[8] - H[5] * H[7]) + (H[0] * H[8] - H[2] * H[6]);
-        float I3f = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
-                    H[2] * (H[3] * H[7] - H[4] * H[6]);
+        // spelled out, as in stress_mixed
+        const float m48 = fmaf(H[4], H[8], -__fmul_rn(H[5], H[7])), m38 = fmaf(H[3], H[8], -__fmul_rn(H[5], H[6])),
+                    m37 = fmaf(H[3], H[7], -__fmul_rn(H[4], H[6]));
+        const float I2f = __fadd_rn(__fadd_rn(fmaf(H[0], H[4], -__fmul_rn(H[1], H[3])), m48),
+                                    fmaf(H[0], H[8], -__fmul_rn(H[2], H[6])));
+        const float I3f = fmaf(H[2], m37, fmaf(H[0], m48, -__fmul_rn(H[1], m38)));
         const float s1 = H[0] + H[4], s2 = s1 + H[8];
         const float terr = two_sum_err(H[0], H[4], s1) + two_sum_err(s1, H[8], s2);
         const float Jm1 = s2 + (terr + (I2f + I3f));
@@ -1503,8 +1516,8 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
         for (int a = 1; a < 4; a++)
 #pragma unroll
             for (int i = 0; i < 3; i++)
-                f[a * 3 + i] = P[i * 3] * G[(a - 1) * 3] + P[i * 3 + 1] * G[(a - 1) * 3 + 1] +
-                               P[i * 3 + 2] * G[(a - 1) * 3 + 2];
+                f[a * 3 + i] = fmaf(P[i * 3 + 2], G[(a - 1) * 3 + 2],
+                                    fmaf(P[i * 3], G[(a - 1) * 3], __fmul_rn(P[i * 3 + 1], G[(a - 1) * 3 + 1])));
 #pragma unroll
         for (int i = 0; i < 3; i++) f[i] = -(f[3 + i] + f[6 + i] + f[9 + i]);
         if (ACT && elem_dead(p, e, t))
@@ -2012,18 +2025,65 @@ __device__ __forceinline__ float block_min_bcast(float v)
 // and the same graph serves any admitted set.  Per-solve control, CFL slot
 // and NaN flag are those of the solve's Problem.
 // ---------------------------------------------------------------------------
-// Dynamic tile assignment.  sched = {tile count, claim counter, blocks done}.
-// Thread 0 claims the block's next tile while the block works on the current
+// Where the tiled kernels get their work.  PoolTiles: the pool's tile list and
+// descriptors in device memory.  SolveTiles: one solve, whose Problem is a
+// kernel argument (the constant bank: no load stands before the first use of
+// its pointers) and whose tiles are equal ranges of `size` of its n elements or
+// nodes, computed instead of loaded.
+struct PoolTiles {
+    const Problem *descs;
+    const Tile *tiles;
+    __device__ __forceinline__ Tile tile(int t) const { return tiles[t]; }
+    __device__ __forceinline__ const Problem &problem(const Tile &tl) const { return descs[tl.solve]; }
+};
+
+struct SolveTiles {
+    const Problem &p;
+    long long n;
+    int size;
+    __device__ __forceinline__ Tile tile(int t) const
+    {
+        const long long b = (long long)t * size, e = b + size;
+        return {0, (int)b, (int)(e < n ? e : n)};
+    }
+    __device__ __forceinline__ const Problem &problem(const Tile &) const { return p; }
+};
+
+// Tile assignment over n tiles; sched = {tile count, claim counter, blocks done}.
+// When the grid has a block for every tile, block b takes tile b and nothing
+// is claimed: the claims of a whole grid serialise on one address, 1.7 us of a
+// launch of 608 blocks (0.71 us for the launch alone).  Otherwise dynamic:
+// thread 0 claims the block's next tile while the block works on the current
 // one; every block makes exactly one claim past the end, and the last block to
 // run out puts both counters back to zero for the next launch.  Which block
 // runs a tile changes no result.
 struct TileQueue {
     int *sched;
     int n;
-    __device__ __forceinline__ int claim() { return atomicAdd(sched + 1, 1); }
+    bool fixed;
+    __device__ __forceinline__ TileQueue(int *sched_, int n_) : sched(sched_), n(n_), fixed(n_ <= (int)gridDim.x) {}
+    // the block's first tile, in every thread (s_tile: shared scratch)
+    __device__ __forceinline__ int first(int *s_tile)
+    {
+        if (fixed) return blockIdx.x;
+        if (threadIdx.x == 0) *s_tile = atomicAdd(sched + 1, 1);
+        __syncthreads();
+        return *s_tile;
+    }
+    // thread 0: claims the next tile (the others: ignored)
+    __device__ __forceinline__ int claim() { return fixed || threadIdx.x != 0 ? n : atomicAdd(sched + 1, 1); }
+    // the claimed tile, in every thread; a barrier either way
+    __device__ __forceinline__ int next(int claimed, int *s_tile)
+    {
+        __syncthreads();
+        if (fixed) return n;
+        if (threadIdx.x == 0) *s_tile = claimed;
+        __syncthreads();
+        return *s_tile;
+    }
     __device__ __forceinline__ void finish()
     {
-        if (threadIdx.x == 0 && atomicAdd(sched + 2, 1) == (int)gridDim.x - 1) {
+        if (!fixed && threadIdx.x == 0 && atomicAdd(sched + 2, 1) == (int)gridDim.x - 1) {
             atomicExch(sched + 1, 0);
             atomicExch(sched + 2, 0);
         }
@@ -2031,21 +2091,16 @@ struct TileQueue {
 };
 
 // Node kernel over tiles (node ranges of one solve), four lanes per node.
-template <int MODE>
-__global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
-                                 int *__restrict__ sched, int parity)
+template <int MODE, typename SRC>
+__device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int parity)
 {
     __shared__ int s_tile;
-    TileQueue q{sched, sched[0]};
-    if (threadIdx.x == 0) s_tile = q.claim();
-    __syncthreads();
-    int t = s_tile, cur = -1;
+    int t = q.first(&s_tile), cur = -1;
     NodeStep ns;
     while (t < q.n) {
-        int next = 0;
-        if (threadIdx.x == 0) next = q.claim();
-        const Tile tl = tiles[t];
-        const Problem &p = descs[tl.solve];
+        const int claimed = q.claim();
+        const Tile tl = src.tile(t);
+        const Problem &p = src.problem(tl);
         if (tl.solve != cur) {
             node_step<MODE>(p, parity, ns);
             cur = tl.solve;
@@ -2060,10 +2115,7 @@ __global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *
                 else node_quad_fp64(p, i, i < tl.end, ns);
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_tile = next;
-        __syncthreads();
-        t = s_tile;
+        t = q.next(claimed, &s_tile);
     }
     q.finish();
 }
@@ -2084,6 +2136,21 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
     const double idt = VISC ? 1.0 / p.ctrl[parity].dt : 0.0;   // the step's dt (bulk viscosity)
     const float idtf = (float)idt;
     long long e = tl.begin + threadIdx.x;
+template <int MODE>
+__global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
+                                 int *__restrict__ sched, int parity)
+{
+    node_tile_loop<MODE>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+}
+
+// One solve: tiles of `size` nodes
+template <int MODE>
+__global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
+                                                                  int *__restrict__ sched, int parity)
+{
+    node_tile_loop<MODE>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
+}
+
     int4 cn_next = make_int4(0, 0, 0, 0);
     if (MODE == MODE_MIXED || MODE == MODE_DW) {
         if (e < tl.end) cn_next = p.conn[e];
@@ -2110,14 +2177,14 @@ constexpr int kMixedPending = 2 * kStepThreads;  // deferred FP64 rechecks a mix
 // barrier): one warp per entry, its lanes over the posting thread's elements
 // of that tile (one each when the tile has at most 32 per thread), skipping
 // entries above 2^-8 of the solve's running screen minimum.
-static __device__ __noinline__ void mixed_flush(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
-                                          const int2 *pend, const float *pendv, int np, int parity)
+template <typename SRC>
+static __device__ __noinline__ void mixed_flush(const SRC src, const int2 *pend, const float *pendv, int np, int parity)
 {
     const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
     for (int j = threadIdx.x >> 5; j < np; j += nwarp) {
         const int2 pe = pend[j];
-        const Tile tl = tiles[pe.x];
-        const Problem &p = descs[tl.solve];
+        const Tile tl = src.tile(pe.x);
+        const Problem &p = src.problem(tl);
         const float mine = pendv[j];
         if (!(mine < 0.0f)) {
             const unsigned long long g = __ldcg(p.dtmin + 2 + (parity ^ 1));
@@ -2149,24 +2216,19 @@ static __device__ __noinline__ void mixed_flush(const Problem *__restrict__ desc
 // entry per thread, so the list is flushed at a tile boundary once it holds
 // more than kMixedPending - blockDim entries, and never overflows; the element
 // loop itself calls no FP64 code.
-template <bool ACT, bool VISC>
-__device__ __forceinline__ void mixed_tile_loop(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
-                                                TileQueue &q, int parity)
+template <bool ACT, bool VISC, typename SRC>
+__device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, int parity)
 {
     __shared__ int s_tile, s_npend;
     __shared__ int2 s_pend[kMixedPending];      // (tile, thread)
     __shared__ float s_pendv[kMixedPending];    // the thread's minimum, -1 for a sliver
-    if (threadIdx.x == 0) {
-        s_tile = q.claim();
-        s_npend = 0;
-    }
+    if (threadIdx.x == 0) s_npend = 0;
     __syncthreads();
-    int t = s_tile;
+    int t = q.first(&s_tile);
     while (t < q.n) {
-        int next = 0;
-        if (threadIdx.x == 0) next = q.claim();
-        const Tile tl = tiles[t];
-        const Problem &p = descs[tl.solve];
+        const int claimed = q.claim();
+        const Tile tl = src.tile(t);
+        const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
             const float mine = tile_elements<MODE_MIXED, ACT, VISC>(p, tl, parity, nullptr);
             const bool neg = mine < 0.0f;
@@ -2179,18 +2241,15 @@ __device__ __forceinline__ void mixed_tile_loop(const Problem *__restrict__ desc
                 s_pendv[k] = neg ? -1.0f : mine;
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_tile = next;
-        __syncthreads();
+        t = q.next(claimed, &s_tile);
         if (s_npend > kMixedPending - (int)blockDim.x) {   // the same value in every thread
-            mixed_flush(descs, tiles, s_pend, s_pendv, s_npend, parity);
+            mixed_flush(src, s_pend, s_pendv, s_npend, parity);
             __syncthreads();
             if (threadIdx.x == 0) s_npend = 0;
             __syncthreads();
         }
-        t = s_tile;
     }
-    mixed_flush(descs, tiles, s_pend, s_pendv, s_npend, parity);   // posted before the loop's last barrier
+    mixed_flush(src, s_pend, s_pendv, s_npend, parity);   // posted before the loop's last barrier
 }
 
 // Element kernel over tiles.  Each element's FP32 CFL screen value is
@@ -2205,29 +2264,23 @@ __device__ __forceinline__ void mixed_tile_loop(const Problem *__restrict__ desc
 // (mixed_tile_loop).  ACT: the instantiation with element birth (single
 // solves whose block has it on), VISC the one with artificial bulk viscosity;
 // the plain one carries no trace of either.
-template <int MODE, bool ACT = false, bool VISC = false>
-__global__ void __launch_bounds__(kStepThreads, MODE == MODE_MIXED ? 4 : (MODE == MODE_DW ? 3 : 2)) pool_elem_kernel(const Problem *__restrict__ descs,
-                                                                 const Tile *__restrict__ tiles,
-                                                                 int *__restrict__ sched, int parity)
+template <int MODE, bool ACT, bool VISC, typename SRC>
+__device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int parity)
 {
     __shared__ float sdt[MODE == MODE_MIXED ? 1 : kMaxTileElems];
     __shared__ unsigned short scand[MODE == MODE_MIXED ? 1 : kMaxTileElems];
     __shared__ int s_tile, s_ncand;
     __shared__ float s_thr;
-    TileQueue q{sched, sched[0]};
     if constexpr (MODE == MODE_MIXED) {
-        mixed_tile_loop<ACT, VISC>(descs, tiles, q, parity);
+        mixed_tile_loop<ACT, VISC>(src, q, parity);
         q.finish();
         return;
     }
-    if (threadIdx.x == 0) s_tile = q.claim();
-    __syncthreads();
-    int t = s_tile;
+    int t = q.first(&s_tile);
     while (t < q.n) {
-        int next = 0;
-        if (threadIdx.x == 0) next = q.claim();
-        const Tile tl = tiles[t];
-        const Problem &p = descs[tl.solve];
+        const int claimed = q.claim();
+        const Tile tl = src.tile(t);
+        const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
             if (MODE != MODE_MIXED && threadIdx.x == 0) s_ncand = 0;
             const float v32 = tile_elements<MODE, ACT, VISC>(p, tl, parity, sdt);
@@ -2277,10 +2330,7 @@ __global__ void __launch_bounds__(kStepThreads, MODE == MODE_MIXED ? 4 : (MODE =
                 }
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_tile = next;
-        __syncthreads();
-        t = s_tile;
+        t = q.next(claimed, &s_tile);
     }
     q.finish();
 }
@@ -2301,6 +2351,24 @@ __device__ __forceinline__ void ref_jacobian(const double *xyz, double *Jac)
 #pragma unroll
     for (int k = 0; k < 12; k++) finite &= isfinite(xyz[k]);
     if (finite) {
+// CTAs of kStepThreads an SM holds: the register caps of the element kernels
+constexpr int elem_ctas(int mode) { return mode == MODE_MIXED ? 4 : (mode == MODE_DW ? 3 : 2); }
+
+template <int MODE, bool ACT = false, bool VISC = false>
+__global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
+    pool_elem_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles, int *__restrict__ sched, int parity)
+{
+    elem_tile_loop<MODE, ACT, VISC>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+}
+
+// One solve: tiles of `size` elements
+template <int MODE, bool ACT = false, bool VISC = false>
+__global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
+    solve_elem_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
+{
+    elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+}
+
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const double y0 = 0.0 - xyz[i * 4];

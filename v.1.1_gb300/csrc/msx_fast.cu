@@ -1,6 +1,7 @@
 // msx_fast.cu -- FP64 (contracted, simplified algebra), double-word and
-// mixed-precision kernels.  The tiled step kernels are instantiated here only, so a single
-// solve (msx_run) and the pool execute the same machine code.
+// mixed-precision kernels.  The tiled step kernels of single solves (msx_run)
+// and of the pool are the same loops, instantiated here only, so a pooled solve
+// gives the bits of the solve run alone.
 #include "msx_device.cuh"
 
 namespace msx {
@@ -34,29 +35,49 @@ void launch_tiled_node(const Problem *descs, const Tile *ntiles, int *counts, in
         pool_node_kernel<MODE_FP64><<<grid, threads, 0, s>>>(descs, ntiles, counts + 3, parity);
 }
 
-template <int MODE>
-static void launch_elem_variant(const Problem *descs, const Tile *etiles, int *counts, int parity, int grid,
-                                int threads, size_t smem, cudaStream_t s, bool act, bool visc)
+void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, int mode, int parity, int grid,
+                       int threads, cudaStream_t s)
 {
-    // element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
-    if (act)
-        pool_elem_kernel<MODE, true><<<grid, threads, smem, s>>>(descs, etiles, counts, parity);
-    else if (visc)
-        pool_elem_kernel<MODE, false, true><<<grid, threads, smem, s>>>(descs, etiles, counts, parity);
+    if (mode == MODE_MIXED)
+        pool_elem_kernel<MODE_MIXED><<<grid, threads, 0, s>>>(descs, etiles, counts, parity);
+    else if (mode == MODE_DW)
+        pool_elem_kernel<MODE_DW><<<grid, threads, 0, s>>>(descs, etiles, counts, parity);
     else
-        pool_elem_kernel<MODE><<<grid, threads, smem, s>>>(descs, etiles, counts, parity);
+        pool_elem_kernel<MODE_FP64><<<grid, threads, 0, s>>>(descs, etiles, counts, parity);
 }
 
-void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, int mode, int parity, int grid,
-                       int threads, int tile_elems, cudaStream_t s, bool act, bool visc)
+void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
 {
-    (void)tile_elems;
+    const int n = (int)((p.nn + q.node_tile - 1) / q.node_tile), grid = n < q.node_grid ? n : q.node_grid;
     if (mode == MODE_MIXED)
-        launch_elem_variant<MODE_MIXED>(descs, etiles, counts, parity, grid, threads, 0, s, act, visc);
+        solve_node_kernel<MODE_MIXED><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
     else if (mode == MODE_DW)
-        launch_elem_variant<MODE_DW>(descs, etiles, counts, parity, grid, threads, 0, s, act, visc);
+        solve_node_kernel<MODE_DW><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
     else
-        launch_elem_variant<MODE_FP64>(descs, etiles, counts, parity, grid, threads, 0, s, act, visc);
+        solve_node_kernel<MODE_FP64><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
+}
+
+template <int MODE>
+static void launch_elem_variant(const Problem &p, const SolveSched &q, int *counts, int parity, cudaStream_t s)
+{
+    const int n = (int)((p.ne + q.elem_tile - 1) / q.elem_tile), grid = n < q.elem_grid ? n : q.elem_grid;
+    // element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
+    if (p.act_t)
+        solve_elem_kernel<MODE, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
+    else if (p.visc)
+        solve_elem_kernel<MODE, false, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
+    else
+        solve_elem_kernel<MODE><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
+}
+
+void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
+{
+    if (mode == MODE_MIXED)
+        launch_elem_variant<MODE_MIXED>(p, q, counts, parity, s);
+    else if (mode == MODE_DW)
+        launch_elem_variant<MODE_DW>(p, q, counts, parity, s);
+    else
+        launch_elem_variant<MODE_FP64>(p, q, counts, parity, s);
 }
 
 // a32: the mixed mode, whose acceleration is one FP32 per DOF (mixed_a32)
@@ -165,18 +186,18 @@ void launch_abs_range(const double *x, long long n, unsigned long long *mm, cuda
     abs_range_kernel<<<256, 256, 0, s>>>(x, n, mm);
 }
 
-int tiled_ctas_per_sm(int mode, int threads, bool node)
+int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool)
 {
+    const void *f[3][2][2] = {
+        {{(const void *)solve_elem_kernel<MODE_FP64>, (const void *)pool_elem_kernel<MODE_FP64>},
+         {(const void *)solve_node_kernel<MODE_FP64>, (const void *)pool_node_kernel<MODE_FP64>}},
+        {{(const void *)solve_elem_kernel<MODE_MIXED>, (const void *)pool_elem_kernel<MODE_MIXED>},
+         {(const void *)solve_node_kernel<MODE_MIXED>, (const void *)pool_node_kernel<MODE_MIXED>}},
+        {{(const void *)solve_elem_kernel<MODE_DW>, (const void *)pool_elem_kernel<MODE_DW>},
+         {(const void *)solve_node_kernel<MODE_DW>, (const void *)pool_node_kernel<MODE_DW>}}};
     int a = 0;
-    if (mode == MODE_MIXED)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, node ? (const void *)pool_node_kernel<MODE_MIXED>
-                                                               : (const void *)pool_elem_kernel<MODE_MIXED>, threads, 0);
-    else if (mode == MODE_DW)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, node ? (const void *)pool_node_kernel<MODE_DW>
-                                                               : (const void *)pool_elem_kernel<MODE_DW>, threads, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, node ? (const void *)pool_node_kernel<MODE_FP64>
-                                                               : (const void *)pool_elem_kernel<MODE_FP64>, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f[mode == MODE_MIXED ? 1 : (mode == MODE_DW ? 2 : 0)][node][pool],
+                                                  threads, 0);
     return a > 0 ? a : 1;
 }
 

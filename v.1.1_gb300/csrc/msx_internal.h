@@ -162,9 +162,8 @@ struct Problem {
     double sf, tf;
 };
 
-// A contiguous element (or node) range [begin, end) of one solve.  The step
-// kernels of the FP64 and mixed modes take tiles from a list, so one solve and
-// many pooled solves run the same kernels.
+// A contiguous element (or node) range [begin, end) of one solve, the unit of
+// work of the step kernels of the FP64, mixed and double-word modes.
 struct Tile {
     int solve;
     int begin, end;
@@ -173,20 +172,27 @@ struct Tile {
 constexpr int kStepThreads = 256;   // upper bound on the CTA size of the tiled step kernels
 constexpr int kMaxTileElems = 4096; // upper bound on the elements of one tile
 
-// Tiled step kernels (one instantiation in msx_fast.cu, used by msx_run and
-// the pool).  `counts` is kTileSched ints of device memory: element-tile
-// count, claim counter, blocks done, then the same three for the node tiles;
-// the counters start at zero and every launch leaves them at zero.
+// Tiled step kernels of the pool.  `counts` is kTileSched ints of device
+// memory: element-tile count, claim counter, blocks done, then the same three
+// for the node tiles; the counters start at zero and every launch leaves them
+// at zero.
 constexpr int kTileSched = 6;
 void launch_tiled_node(const Problem *descs, const Tile *ntiles, int *counts, int mode, int parity, int grid,
                        int threads, cudaStream_t s);
-// tile_elems: the largest tile of etiles (unused: every kernel's shared memory
-// is static); act: the instantiation with element birth
-// (Problem::act_t set); visc: the one with bulk viscosity (Problem::visc set)
 void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, int mode, int parity, int grid,
-                       int threads, int tile_elems, cudaStream_t s, bool act = false, bool visc = false);
-// CTAs of the tiled element kernel (node kernel when `node` is true) that fit on one SM
-int tiled_ctas_per_sm(int mode, int threads, bool node = false);
+                       int threads, cudaStream_t s);
+// The same kernels over one solve, whose Problem goes as a kernel argument:
+// CTA size, tile sizes and the largest grids (a launch takes no more CTAs than
+// it has tiles).  Problem::act_t selects the element kernel with element birth,
+// Problem::visc the one with bulk viscosity.
+struct SolveSched {
+    int threads = kStepThreads;
+    int elem_tile = 0, node_tile = 0, elem_grid = 0, node_grid = 0;
+};
+void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
+void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
+// CTAs of a tiled element kernel (node kernel when `node` is true) that fit on one SM
+int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false);
 // Mixed-mode state conversions: u, v, a (FP64) -> uhl, vhl, ahl, and back
 // (hi + lo, exact unless the pair spans more than 53 bits); minv -> minv2.
 void launch_state_split(const Problem &p, bool mixed, cudaStream_t s);

@@ -236,14 +236,13 @@ static msx_status build_pool_graph(msx_pool *p, int steps)
     }
     const int mode = pool_mode(p->opts.precision);
     const int threads = p->sched.threads, grid = p->sms * p->sched.ctas_per_sm;
-    const int node_grid = p->sms * tiled_ctas_per_sm(mode, threads, true);
+    const int node_grid = p->sms * tiled_ctas_per_sm(mode, threads, true, true);
     cudaGraph_t g;
     PCUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < steps; i++) {
         int parity = (i & 1) ? 0 : 1;
         launch_tiled_node(p->d_descs, p->d_ntiles, p->d_counts, mode, parity, node_grid, threads, p->stream);
-        launch_tiled_elem(p->d_descs, p->d_etiles, p->d_counts, mode, parity, grid, threads, p->sched.tile_elems,
-                          p->stream);
+        launch_tiled_elem(p->d_descs, p->d_etiles, p->d_counts, mode, parity, grid, threads, p->stream);
     }
     cudaError_t err = cudaStreamEndCapture(p->stream, &g);
     if (err != cudaSuccess) return pfail(MSX_ERR_CUDA, std::string("pool graph capture: ") + cudaGetErrorString(err));
@@ -382,7 +381,7 @@ static msx_status replay(msx_pool *p, float *ms)
 static msx_status autotune(msx_pool *p)
 {
     const int mode = pool_mode(p->opts.precision);
-    const int occ128 = tiled_ctas_per_sm(mode, 128), occ256 = tiled_ctas_per_sm(mode, 256);
+    const int occ128 = tiled_ctas_per_sm(mode, 128, false, true), occ256 = tiled_ctas_per_sm(mode, 256, false, true);
     const Sched cands[] = {{128, 512, occ128}, {128, 1024, occ128}, {256, 512, occ256}, {256, 1024, occ256},
                            {256, 2048, occ256}, {256, 4096, occ256}, {256, 1024, std::max(1, occ256 / 2)},
                            {128, 2048, occ128}};
@@ -479,18 +478,18 @@ extern "C" msx_status msx_pool_create(const msx_pool_opts *opts, msx_pool **out)
     p->spl = opts->steps_per_launch > 0 ? ((opts->steps_per_launch + 1) & ~1) : 32;
     const int pmode = pool_mode(opts->precision);
     p->sched.threads = kStepThreads;
-    p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, kStepThreads);
+    p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, kStepThreads, false, true);
     if (opts->elems_per_block > 0) {
         p->sched.threads = opts->elems_per_block >= 256 ? 256 : 128;
         p->sched.tile_elems = opts->elems_per_block;
-        p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, p->sched.threads);
+        p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, p->sched.threads, false, true);
         p->tuned = true;
     } else if (opts->tune_cache) {
         if (FILE *f = fopen(opts->tune_cache, "r")) {
             Sched s;
             if (fscanf(f, "%d %d %d", &s.threads, &s.tile_elems, &s.ctas_per_sm) == 3 && s.threads > 0 &&
                 s.threads <= kStepThreads && s.tile_elems > 0 && s.ctas_per_sm > 0 &&
-                s.ctas_per_sm <= tiled_ctas_per_sm(pmode, s.threads)) {
+                s.ctas_per_sm <= tiled_ctas_per_sm(pmode, s.threads, false, true)) {
                 p->sched = s;
                 p->tuned = true;
             }

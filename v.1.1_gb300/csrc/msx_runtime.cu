@@ -133,7 +133,6 @@ struct msx_handle {
     double dt_init = 0;
     launch_fn node = nullptr, elem = nullptr;   // reference-order kernels (exact mode)
     bool tiled = false;                          // FP64 / mixed: the shared tiled step kernels
-    DBuf<Problem> d_desc;
     DBuf<double> act;                    // activation times (element birth), when set
     bool act_enabled = false;
     // artificial viscosity (msx_set_viscosity): kind and parameters; the
@@ -142,10 +141,8 @@ struct msx_handle {
     double visc_c1 = 0, visc_cl = 0, visc_h = 0, visc_c0 = 0;
     DBuf<double> visc_f0;
     DBuf<float> visc_h0;
-    DBuf<Tile> d_etiles, d_ntiles;
-    int tile_elems = 0;                 // element-tile size of d_etiles
-    DBuf<int> d_counts;
-    int tgrid = 0, tgrid_node = 0, tthreads = kStepThreads;
+    DBuf<int> d_counts;                 // tile queues of the tiled kernels
+    SolveSched sched;
     // captured step chunks: `graph` holds spg steps; part[k] (k >= 1) holds 2^k
     // steps and runs a call's remainder, so a call replays at most one idle step
     cudaGraphExec_t graph = nullptr;
@@ -354,31 +351,40 @@ static bool pair_state(const msx_handle *h)
     return h->precision == MSX_PREC_MIXED || h->precision == MSX_PREC_DOUBLE_WORD;
 }
 
-// One step's kernels: the shared tiled pair for FP64 / mixed (the same
-// machine code the pool runs), the reference-order pair for exact mode.
-static void launch_step(msx_handle *h, int parity)
+static void launch_node_part(msx_handle *h, int parity)
 {
-    if (h->tiled)
-        launch_tiled_node(h->d_desc.p, h->d_ntiles.p, h->d_counts.p, tiled_mode(h), parity, h->tgrid_node,
-                          h->tthreads, h->stream);
-    else
-        h->node(h->P, parity, h->stream);
+    if (h->tiled) launch_solve_node(h->P, h->sched, h->d_counts.p, tiled_mode(h), parity, h->stream);
+    else h->node(h->P, parity, h->stream);
     if (h->nfaces) launch_face_loads(h->P, parity, pair_state(h), h->stream);
-    if (h->tiled)
-        launch_tiled_elem(h->d_desc.p, h->d_etiles.p, h->d_counts.p, tiled_mode(h), parity, h->tgrid, h->tthreads,
-                          h->tile_elems, h->stream, h->P.act_t != nullptr, h->P.visc != 0);
-    else
-        h->elem(h->P, parity, h->stream);
 }
 
-// Descriptor and one-solve tile list of the tiled kernels.
-static msx_status upload_tiled(msx_handle *h)
+static void launch_elem_part(msx_handle *h, int parity)
+{
+    if (h->tiled) launch_solve_elem(h->P, h->sched, h->d_counts.p, tiled_mode(h), parity, h->stream);
+    else h->elem(h->P, parity, h->stream);
+}
+
+// One step's kernels: the tiled pair (the pool's loops) for FP64, mixed and
+// double-word, the reference-order pair for exact mode.  All take the Problem
+// by value, so a captured step names the one it was captured with.
+static void launch_step(msx_handle *h, int parity)
+{
+    launch_node_part(h, parity);
+    launch_elem_part(h, parity);
+}
+
+// Schedule of the tiled kernels.
+static msx_status plan_tiled(msx_handle *h)
 {
     if (!h->tiled) return MSX_OK;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-    h->tgrid = sms * tiled_ctas_per_sm(tiled_mode(h), h->tthreads);
-    h->tgrid_node = sms * tiled_ctas_per_sm(tiled_mode(h), h->tthreads, true);
+    SolveSched q;
+    // CTAs of 128 threads while one warp per scheduler holds the whole mesh
+    // (sms * 128 elements): the elements then spread over all SMs.  256 above.
+    q.threads = h->P.ne <= 128LL * sms ? 128 : kStepThreads;
+    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads);
+    q.node_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true);
     // Element tiles of P whole CTA passes (P * threads elements).  Spread over
     // the grid, the busiest CTA runs ceil(tiles / grid) tiles; P minimises that
     // count times (P + 1/2), the half pass standing for a tile's close (the
@@ -386,40 +392,29 @@ static msx_status upload_tiled(msx_handle *h)
     // reductions), so the last wave of tiles fills the grid instead of
     // leaving most CTAs idle.  P is capped at 4096 elements for those two
     // kernels and at 1024 for the mixed one, whose tiles balance best small.
-    const int thr = h->tthreads;
+    const int thr = q.threads;
     const int pmax = (h->precision == MSX_PREC_MIXED ? 1024 : kMaxTileElems) / thr;
     const long long passes = (h->P.ne + thr - 1) / thr;
     int bestp = pmax;
     double best = 1e300;
     for (int P = pmax; P >= 1; P--) {
-        const long long rounds = ((passes + P - 1) / P + h->tgrid - 1) / h->tgrid;
+        const long long rounds = ((passes + P - 1) / P + q.elem_grid - 1) / q.elem_grid;
         const double cost = (double)rounds * (P + 0.5);
         if (cost < best) {
             best = cost;
             bestp = P;
         }
     }
-    const int te = bestp * thr;
-    const int tn = 128;
-    if (!h->d_desc.p || te != h->tile_elems) {
-        std::vector<Tile> et, nt;
-        for (long long b = 0; b < h->P.ne; b += te) et.push_back({0, (int)b, (int)std::min<long long>(h->P.ne, b + te)});
-        for (long long b = 0; b < h->P.nn; b += tn) nt.push_back({0, (int)b, (int)std::min<long long>(h->P.nn, b + tn)});
-        int counts[kTileSched] = {(int)et.size(), 0, 0, (int)nt.size(), 0, 0};
-        h->d_etiles.release();
-        h->d_ntiles.release();
-        if (!h->d_desc.p) MSX_CUDA(h->d_desc.alloc(1));
-        MSX_CUDA(h->d_etiles.alloc(et.size()));
-        MSX_CUDA(h->d_ntiles.alloc(nt.size()));
-        if (!h->d_counts.p) MSX_CUDA(h->d_counts.alloc(kTileSched));
-        MSX_CUDA(cudaMemcpyAsync(h->d_etiles.p, et.data(), sizeof(Tile) * et.size(), cudaMemcpyHostToDevice, h->stream));
-        MSX_CUDA(cudaMemcpyAsync(h->d_ntiles.p, nt.data(), sizeof(Tile) * nt.size(), cudaMemcpyHostToDevice, h->stream));
-        MSX_CUDA(cudaMemcpyAsync(h->d_counts.p, counts, sizeof(counts), cudaMemcpyHostToDevice, h->stream));
-        h->tile_elems = te;
-        drop_graphs(h);   // the captured launches name the old tile lists
+    q.elem_tile = bestp * thr;
+    // node tiles of two CTA passes (four lanes a node); one pass while that
+    // leaves no more tiles than the grid has CTAs
+    q.node_tile = (h->P.nn + thr / 4 - 1) / (thr / 4) <= q.node_grid ? thr / 4 : 128;
+    if (!h->d_counts.p) {
+        MSX_CUDA(h->d_counts.alloc(kTileSched));
+        MSX_CUDA(cudaMemsetAsync(h->d_counts.p, 0, sizeof(int) * kTileSched, h->stream));
     }
-    MSX_CUDA(cudaMemcpyAsync(h->d_desc.p, &h->P, sizeof(Problem), cudaMemcpyHostToDevice, h->stream));
-    MSX_CUDA(cudaStreamSynchronize(h->stream));
+    if (memcmp(&q, &h->sched, sizeof(q))) drop_graphs(h);   // the captured launches name the old schedule
+    h->sched = q;
     return MSX_OK;
 }
 
@@ -591,7 +586,7 @@ static msx_status set_opts(msx_handle *h, const msx_solver_opts *o)
 static msx_status init_block(msx_handle *h)
 {
     bind_problem(h);
-    msx_status tst = upload_tiled(h);
+    msx_status tst = plan_tiled(h);
     if (tst != MSX_OK) return tst;
     const Problem &P = h->P;
     // CFL minima (double bits) and the screen's running minima (FP32 bits)
@@ -626,8 +621,8 @@ static msx_status init_block(msx_handle *h)
     return MSX_OK;
 }
 
-// Destroys the captured step chunks (their launches name the tile lists, the
-// kernel instantiation and, in the exact mode, the Problem by value).
+// Destroys the captured step chunks (their launches name the schedule, the
+// kernel instantiation and the Problem by value).
 static void drop_graphs(msx_handle *h)
 {
     if (h->graph) cudaGraphExecDestroy(h->graph);
@@ -895,9 +890,6 @@ extern "C" msx_status msx_destroy(msx_handle *h)
     h->ext_term.release();
     h->nfs.release();
     h->faces.release();
-    h->d_desc.release();
-    h->d_etiles.release();
-    h->d_ntiles.release();
     h->d_counts.release();
     h->ctrl.release();
     h->dtmin.release();
@@ -1145,10 +1137,10 @@ extern "C" msx_status msx_set_load_blocks(msx_handle *h, const msx_load_block *b
         h->nfaces = (int)faces.size();
     }
     bind_problem(h);
-    msx_status st = upload_tiled(h);
+    msx_status st = plan_tiled(h);
     if (st != MSX_OK) return st;
     MSX_CUDA(cudaStreamSynchronize(h->stream));
-    drop_graphs(h);   // the step's kernel list (face kernel) and the exact mode's Problem changed
+    drop_graphs(h);   // the step's kernel list (face kernel) and the Problem changed
     return MSX_OK;
 }
 
@@ -1165,10 +1157,10 @@ extern "C" msx_status msx_set_activation(msx_handle *h, const double *activation
         return fail(MSX_ERR_STATE, "element birth and bulk viscosity together are not supported");
     h->act_enabled = enabled != 0;
     bind_problem(h);
-    msx_status st = upload_tiled(h);
+    msx_status st = plan_tiled(h);
     if (st != MSX_OK) return st;
     MSX_CUDA(cudaStreamSynchronize(h->stream));
-    drop_graphs(h);   // the exact mode's captured launches hold the Problem by value
+    drop_graphs(h);   // the captured launches hold the Problem by value
     return MSX_OK;
 }
 
@@ -1198,10 +1190,10 @@ extern "C" msx_status msx_set_viscosity(msx_handle *h, int32_t kind, double c1, 
         launch_visc_init(h->P, h->u.p, h->stream);
         MSX_CUDA(cudaGetLastError());
     }
-    msx_status st = upload_tiled(h);
+    msx_status st = plan_tiled(h);
     if (st != MSX_OK) return st;
     MSX_CUDA(cudaStreamSynchronize(h->stream));
-    drop_graphs(h);   // another element-kernel instantiation, and the exact mode's launches hold the Problem
+    drop_graphs(h);   // another element-kernel instantiation, and the captured launches hold the Problem
     return MSX_OK;
 }
 
@@ -1522,18 +1514,9 @@ extern "C" msx_status msx_profile(msx_handle *h, int64_t steps, msx_profile_repo
     for (long long i = 0; i < n; i++) {
         int parity = (i & 1) ? 0 : 1;
         cudaEventRecord(ev[3 * i], h->stream);
-        if (h->tiled)
-            launch_tiled_node(h->d_desc.p, h->d_ntiles.p, h->d_counts.p, tiled_mode(h), parity, h->tgrid_node,
-                              h->tthreads, h->stream);
-        else
-            h->node(h->P, parity, h->stream);
-        if (h->nfaces) launch_face_loads(h->P, parity, pair_state(h), h->stream);
+        launch_node_part(h, parity);
         cudaEventRecord(ev[3 * i + 1], h->stream);
-        if (h->tiled)
-            launch_tiled_elem(h->d_desc.p, h->d_etiles.p, h->d_counts.p, tiled_mode(h), parity, h->tgrid, h->tthreads,
-                              h->tile_elems, h->stream, h->P.act_t != nullptr, h->P.visc != 0);
-        else
-            h->elem(h->P, parity, h->stream);
+        launch_elem_part(h, parity);
         cudaEventRecord(ev[3 * i + 2], h->stream);
     }
     if (pair_state(h)) launch_state_merge(h->P, h->precision == MSX_PREC_MIXED, h->stream);
