@@ -1176,20 +1176,35 @@ __device__ __forceinline__ float cfl_screen(const Problem &p, long long e, const
     return cfl_screen_edges(p, e, e1, e2, e3, m);
 }
 
-// Plain FP64, compressible neo-Hookean, without forming F: with the deformed
-// edges e_b = E_b + (u_b - u_0) (b = 1..3, E_b the reference edges), the
-// corner force of node a = 1..3 is
-//   f_a = wJ P g_a = wJ mu F g_a + wJ (lambda ln J - mu) F^-T g_a,
-//   F g_a = sum_b M_ab e_b        (F = I + du G and E G = I give F = e G, and
-//                                  G g_a = (g_b . g_a)_b = M_a),
-//   F^-T g_a = (e_c x e_d) / det e   (the rows of e^-1: e2 x e3, e3 x e1, e1 x e2),
-//   J = det e / det E,
-// and f_0 = -(f_1 + f_2 + f_3): about 113 FP64 operations per element instead
-// of the cofactor form's 130.  The CFL screen takes the deformed edges
-// directly (truncated to FP32).
-template <bool ACT>
-__device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, double t,
-                                                    const MatParams &m, const int *nd)
+template <bool FORCE_ONLY, bool ACT, bool VISC>
+__device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
+                                                    const MatParams &m, const int *nd);
+
+// The cofactor form's corner forces of one element that fixed point leaves out.
+static __device__ __noinline__ void elem_cnh_general(const Problem &p, long long e, int parity)
+{
+    const int4 cn = p.conn[e];
+    const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
+    elem_cofactor_fp64<true, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd);
+}
+
+// x 2^k for an integer x: the exponent is added to the converted integer's
+// (|x| < 2^63 and -900 <= k <= 900, so the result is a normal number or zero)
+__device__ __forceinline__ double fixed_to_double(long long x, int k)
+{
+    const double d = __ll2double_rn(x);
+    const int hi = __double2hiint(d);
+    return __hiloint2double(hi ? hi + (k << 20) : 0, __double2loint(d));
+}
+
+// Plain FP64 mode, compressible neo-Hookean: the deformed edges
+// e_b = E_b + (u_b - u_0) in FP64, the corner forces from them in 64-bit fixed
+// point (msx_fixed.cuh), rounded to FP64 at the end.  FP64 arithmetic is left
+// with the 24 additions of the edges and of f_0 and nine conversions, against
+// 115 operations of the same formulas in FP64.  The CFL screen takes the deformed
+// edges directly (truncated to FP32).
+__device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
+                                                    const int *nd)
 {
     const long long ne = p.ne, nn = p.nn;
     double ua[4][3];
@@ -1219,44 +1234,38 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
         for (int k = 0; k < 9; k++) e32[k] = f32_trunc(ed[k]);
         scr = cfl_screen_edges(p, e, e32, e32 + 3, e32 + 6, m);
     }
-    const double *e1 = ed, *e2 = ed + 3, *e3 = ed + 6;
-    double cr[9];   // cr[(a-1)*3 + i] = det(e) (F^-T g_a)_i
-    cr[0] = e2[1] * e3[2] - e2[2] * e3[1];
-    cr[1] = e2[2] * e3[0] - e2[0] * e3[2];
-    cr[2] = e2[0] * e3[1] - e2[1] * e3[0];
-    cr[3] = e3[1] * e1[2] - e3[2] * e1[1];
-    cr[4] = e3[2] * e1[0] - e3[0] * e1[2];
-    cr[5] = e3[0] * e1[1] - e3[1] * e1[0];
-    cr[6] = e1[1] * e2[2] - e1[2] * e2[1];
-    cr[7] = e1[2] * e2[0] - e1[0] * e2[2];
-    cr[8] = e1[0] * e2[1] - e1[1] * e2[0];
-    const double dete = e1[0] * cr[0] + e1[1] * cr[1] + e1[2] * cr[2];
-    const double J = dete * __ldg(p.rdetE + e);
-    const double wJ = __ldg(p.wJ + e);
-    const double c1 = m.mu * wJ;
-    const double c2 = (m.lambda * log_near1(J) - m.mu) * (wJ / dete);
-    double Mv[6];
+    if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+    const int4 sl = __ldg(p.slot + e);
+    const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
+    const uint2 w = __ldg(p.fxw + e);
+    FixedElem q;
+    int64_t f[9];
+    bool ok = w.x != 0;
+    if (ok) {
+        fixed_unpack(w.x, w.y, q);
+        const longlong2 d = __ldg(p.fxD + e);
+        q.d0 = d.x;
+        q.rd = d.y;
 #pragma unroll
-    for (int k = 0; k < 6; k++) Mv[k] = __ldg(p.Mg + k * ne + e);
-    const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};   // M_ab at Mv[mi[(a-1)*3 + (b-1)]]
-    double f[12];
+        for (int k = 0; k < 6; k++) {
+            const int2 x = __ldg(p.fxS + k * ne + e);
+            q.S[k] = {x.x, x.y};
+        }
+        ok = fixed_forces(q, ed, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f);
+    }
+    if (!ok) {
+        elem_cnh_general(p, e, parity);
+        return scr;
+    }
+    double fa[3][3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const double Fg = e1[i] * Mv[mi[a * 3]] + e2[i] * Mv[mi[a * 3 + 1]] + e3[i] * Mv[mi[a * 3 + 2]];
-            f[(a + 1) * 3 + i] = c1 * Fg + c2 * cr[a * 3 + i];
-        }
+        for (int i = 0; i < 3; i++) fa[a][i] = fixed_to_double(f[a * 3 + i], q.x0 - q.lw[a]);
+    st_slot24(p.fe, ks[0], -(fa[0][0] + fa[1][0] + fa[2][0]), -(fa[0][1] + fa[1][1] + fa[2][1]),
+              -(fa[0][2] + fa[1][2] + fa[2][2]));
 #pragma unroll
-    for (int i = 0; i < 3; i++) f[i] = -(f[3 + i] + f[6 + i] + f[9 + i]);
-    if (ACT && elem_dead(p, e, t))
-#pragma unroll
-        for (int k = 0; k < 12; k++) f[k] = 0.0;
-    const int4 sl = __ldg(p.slot + e);
-    const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
-#pragma unroll
-    for (int a = 0; a < 4; a++) st_slot24(p.fe, ks[a], f[a * 3], f[a * 3 + 1], f[a * 3 + 2]);
-    if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+    for (int a = 0; a < 3; a++) st_slot24(p.fe, ks[a + 1], fa[a][0], fa[a][1], fa[a][2]);
     return scr;
 }
 
@@ -1265,15 +1274,11 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 // the 4th corner force as minus the sum of the other three.  Same algebra as
 // the reference, about half its FP64 operations.  Returns the FP32 CFL screen
 // value (see cfl_screen).
-template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
-__device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
-                                                double idt = 0.0)
+template <bool FORCE_ONLY, bool ACT, bool VISC>
+__device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
+                                                    const MatParams &m, const int *nd)
 {
     const long long ne = p.ne, nn = p.nn;
-    int4 cn = p.conn[e];
-    int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    const MatParams &m = mat_of(p, e);
-    if (!FORCE_ONLY && !VISC && p.Eref && m.law == 1) return elem_body_fp64_cnh<ACT>(p, e, parity, t, m, nd);
     double G[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) G[k] = __ldg(p.G + k * ne + e);
@@ -1344,6 +1349,17 @@ __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, i
     return scr;
 }
 
+template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
+__device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
+                                                double idt = 0.0)
+{
+    const int4 cn = p.conn[e];
+    const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
+    const MatParams &m = mat_of(p, e);
+    if (!FORCE_ONLY && !VISC && p.Eref && m.law == 1) return elem_body_fp64_cnh(p, e, parity, m, nd);   // never dead
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd);
+}
+
 // corner forces only (internal-force hook)
 static __global__ void __launch_bounds__(kElemBlock) elem_force_kernel_fp64(Problem p, int parity)
 {
@@ -1395,6 +1411,10 @@ __device__ __forceinline__ void stress_mixed(const MatParams &m, const float *H,
                 P[i * 3 + j] = S[i * 3 + j] + (H[i * 3] * S[j] + H[i * 3 + 1] * S[3 + j] + H[i * 3 + 2] * S[6 + j]);
         return;
     }
+    // Products and sums are spelled out (fmaf, _rn) from here on: which product
+    // of a*b + c*d is fused is otherwise the compiler's choice, and differs
+    // between the instantiations of this body; a pooled solve has to give the
+    // bits of the solve run alone.
     float D[9];
     const float a0 = t + I2, a1 = 1.0f + t;
 #pragma unroll
@@ -1416,10 +1436,6 @@ __device__ __forceinline__ void stress_mixed(const MatParams &m, const float *H,
         const float lj = __fmul_rn(m.lambda_f, lnJ);
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-    // Products and sums are spelled out (fmaf, _rn) from here on: which product
-    // of a*b + c*d is fused is otherwise the compiler's choice, and differs
-    // between the instantiations of this body; a pooled solve has to give the
-    // bits of the solve run alone.
             const float q = __fadd_rn(k % 4 == 0 ? fmaf(Jx, H[k], Jm1) : __fmul_rn(Jx, H[k]), -D[k]);
             P[k] = __fmul_rn(fmaf(lj, k % 4 == 0 ? __fadd_rn(1.0f, D[k]) : D[k], __fmul_rn(m.mu_f, q)), iJ);
         }
@@ -2120,6 +2136,21 @@ __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int 
     q.finish();
 }
 
+template <int MODE>
+__global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
+                                 int *__restrict__ sched, int parity)
+{
+    node_tile_loop<MODE>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+}
+
+// One solve: tiles of `size` nodes
+template <int MODE>
+__global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
+                                                                  int *__restrict__ sched, int parity)
+{
+    node_tile_loop<MODE>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
+}
+
 // The elements of one tile for the tiled element kernel: each thread's
 // elements in turn; returns the thread's FP32 minimum of the CFL screen.  The
 // FP64 and double-word kernels keep every screen value in sdt; the mixed one
@@ -2136,21 +2167,6 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
     const double idt = VISC ? 1.0 / p.ctrl[parity].dt : 0.0;   // the step's dt (bulk viscosity)
     const float idtf = (float)idt;
     long long e = tl.begin + threadIdx.x;
-template <int MODE>
-__global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
-                                 int *__restrict__ sched, int parity)
-{
-    node_tile_loop<MODE>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
-}
-
-// One solve: tiles of `size` nodes
-template <int MODE>
-__global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
-                                                                  int *__restrict__ sched, int parity)
-{
-    node_tile_loop<MODE>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
-}
-
     int4 cn_next = make_int4(0, 0, 0, 0);
     if (MODE == MODE_MIXED || MODE == MODE_DW) {
         if (e < tl.end) cn_next = p.conn[e];
@@ -2335,22 +2351,6 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
     q.finish();
 }
 
-// ---------------------------------------------------------------------------
-// Set-up kernels (reference operation order), built in the exact unit only
-// ---------------------------------------------------------------------------
-#ifdef MSX_SETUP_KERNELS
-// Reference Jacobian of a tet from xyz[i*4 + k] (coordinate i of corner k):
-// Jac_ij = 0 + sum_k x_ik natDev_kj in corner order, natDev's entries -1, 0
-// and 1 (classLinearTetrahedra.cpp:171-268).  For finite coordinates that sum
-// is (0 - x_i0) + x_i(j+1) bit for bit: 0 - x_i0 is never -0, and the products
-// with 0 add signed zeros to a partial sum that is never -0, which leaves it
-// unchanged.  A non-finite coordinate (x * 0 is NaN) takes the full sum.
-__device__ __forceinline__ void ref_jacobian(const double *xyz, double *Jac)
-{
-    bool finite = true;
-#pragma unroll
-    for (int k = 0; k < 12; k++) finite &= isfinite(xyz[k]);
-    if (finite) {
 // CTAs of kStepThreads an SM holds: the register caps of the element kernels
 constexpr int elem_ctas(int mode) { return mode == MODE_MIXED ? 4 : (mode == MODE_DW ? 3 : 2); }
 
@@ -2369,6 +2369,22 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 
+// ---------------------------------------------------------------------------
+// Set-up kernels (reference operation order), built in the exact unit only
+// ---------------------------------------------------------------------------
+#ifdef MSX_SETUP_KERNELS
+// Reference Jacobian of a tet from xyz[i*4 + k] (coordinate i of corner k):
+// Jac_ij = 0 + sum_k x_ik natDev_kj in corner order, natDev's entries -1, 0
+// and 1 (classLinearTetrahedra.cpp:171-268).  For finite coordinates that sum
+// is (0 - x_i0) + x_i(j+1) bit for bit: 0 - x_i0 is never -0, and the products
+// with 0 add signed zeros to a partial sum that is never -0, which leaves it
+// unchanged.  A non-finite coordinate (x * 0 is NaN) takes the full sum.
+__device__ __forceinline__ void ref_jacobian(const double *xyz, double *Jac)
+{
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < 12; k++) finite &= isfinite(xyz[k]);
+    if (finite) {
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const double y0 = 0.0 - xyz[i * 4];
@@ -2390,25 +2406,28 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
 }
 
 // The plain FP64 mode's compressible neo-Hookean element data of element e
-// (Problem::Eref, Mg, rdetE) from its corner coordinates pts[k*3 + i], the
-// stored gradients g (G's nine entries) and the reference Jacobian's
-// determinant.
-__device__ __forceinline__ void write_cnh_arrays(const Problem &p, long long e, const double *pts, const double *g,
-                                                 double Jref)
+// (Problem::Eref, fxS, fxD, fxw) from its corner coordinates pts[k*3 + i].
+__device__ __forceinline__ void write_cnh_arrays(const Problem &p, long long e, const double *pts)
 {
     const long long ne = p.ne;
-    double *Er = const_cast<double *>(p.Eref), *Mw = const_cast<double *>(p.Mg);
+    double *Er = const_cast<double *>(p.Eref), E[9];
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) Er[(b * 3 + i) * ne + e] = pts[(b + 1) * 3 + i] - pts[i];
-    int k = 0;
+        for (int i = 0; i < 3; i++) {
+            E[b * 3 + i] = pts[(b + 1) * 3 + i] - pts[i];
+            Er[(b * 3 + i) * ne + e] = E[b * 3 + i];
+        }
+    const MatParams &m = mat_of(p, e);
+    FixedElem q;
+    uint32_t w[2] = {0, 0};
+    if (m.law == 1 && fixed_setup(E, m.kq[0], m.ks, q)) {
+        fixed_pack(q, w);
 #pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = a; b < 3; b++, k++)
-            Mw[k * ne + e] = g[a * 3] * g[b * 3] + g[a * 3 + 1] * g[b * 3 + 1] + g[a * 3 + 2] * g[b * 3 + 2];
-    const_cast<double *>(p.rdetE)[e] = 1.0 / Jref;
+        for (int k = 0; k < 6; k++) const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2(q.S[k].h, q.S[k].l);
+        const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(q.d0, q.rd);
+    }
+    const_cast<uint2 *>(p.fxw)[e] = make_uint2(w[0], w[1]);
 }
 
 // classLinearTetrahedra.cpp:171-268 (Jacobian, inverse, dphi), classGPs.cpp:27
@@ -2438,11 +2457,9 @@ __global__ void setup_elements_kernel(Problem p, const double *X, double *G, dou
     ref_jacobian(xyz, Jac);
     double J = det3_ref(Jac);
     inv3_ref(Jac, iJ);
-    double gst[9];   // G as stored
 #pragma unroll
     for (int k = 0; k < 9; k++) {
         double g = 0.0 + iJ[k];
-        gst[k] = g;
         G[k * ne + e] = g;
         if (G32) G32[k * ne + e] = (float)g;
         if (p.G32lo) const_cast<float *>(p.G32lo)[k * ne + e] = (float)(g - (double)(float)g);
@@ -2454,7 +2471,7 @@ __global__ void setup_elements_kernel(Problem p, const double *X, double *G, dou
     double v6;   // 6V, signed: the edge determinant of the inscribed-sphere volume
     double L = char_length_ref(pts, &v6);
     Lref[e] = L;
-    if (p.Eref) write_cnh_arrays(p, e, pts, gst, J);
+    if (p.Eref) write_cnh_arrays(p, e, pts);
     // A reference sliver (6V below 0.063 |e1||e2||e3|) gets a negative FP32
     // length: the FP32 CFL screens then always recompute it in FP64 (the mixed
     // screen rebuilds the reference edges from G in FP32, which loses accuracy
@@ -2494,27 +2511,20 @@ __global__ void mode_arrays_kernel(Problem p, float *G32, float *wJ32, float *G3
     if (wJ32lo) wJ32lo[e] = (float)(w - (double)(float)w);
 }
 
-// Problem::Eref, Mg and rdetE of a handle whose FP64 block starts after its
-// set-up: the same operations as setup_elements_kernel, from X and the stored G.
+// Problem::Eref, fxS, fxD and fxw of a handle whose FP64 block starts after its
+// set-up: what setup_elements_kernel writes, from X.
 __global__ void cnh_arrays_kernel(Problem p)
 {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.ne) return;
-    const long long nn = p.nn, ne = p.ne;
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    double xyz[12], pts[12], g[9], Jac[9];
+    double pts[12];
 #pragma unroll
     for (int k = 0; k < 4; k++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            xyz[i * 4 + k] = p.X[i * nn + nd[k]];
-            pts[k * 3 + i] = p.X[i * nn + nd[k]];
-        }
-    ref_jacobian(xyz, Jac);
-#pragma unroll
-    for (int k = 0; k < 9; k++) g[k] = p.G[k * ne + e];
-    write_cnh_arrays(p, e, pts, g, det3_ref(Jac));
+        for (int i = 0; i < 3; i++) pts[k * 3 + i] = p.X[i * p.nn + nd[k]];
+    write_cnh_arrays(p, e, pts);
 }
 
 // Previous-step F diagonal for the bulk viscosity, from displacement u, in the

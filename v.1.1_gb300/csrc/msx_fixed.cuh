@@ -1,0 +1,333 @@
+// msx_fixed.cuh -- corner forces of a compressible neo-Hookean tet in 64-bit
+// fixed point.
+//
+// The FP64 pipe of this GPU issues one warp instruction per scheduler in 64-80
+// cycles, the integer pipes one in 1-2 (multiply-add of two 32-bit limbs into
+// 64 bits: 2.2), so a product of two 60-bit numbers in three limb products
+// costs a tenth of an FP64 product and carries more bits.  With e_b the
+// deformed edges, g_a the gradients of shape functions 1..3, J = det e / det E
+// and W = 0.166666666667 the quadrature weight, the corner forces are
+//     f_a = S_a1 e_1 + S_a2 e_2 + S_a3 e_3 + c2 (e_c x e_d),  f_0 = -(f_1 + f_2 + f_3),
+//     S_ab = W |det E| mu g_a.g_b,   c2 = -W (mu - lambda ln J) / J:
+// sums of products of numbers whose size the reference element tells.  Each
+// edge has its own power-of-two unit w_b, so accuracy does not depend on the
+// element's aspect ratio: with e_b = w_b n_b and row a scaled by w_a,
+//     f_a w_a = sum_b (S_ab w_a w_b) n_b + (c2 w_1 w_2 w_3) (n_c x n_d)
+// has one unit for the nine products of a kind.
+//
+// Sizes.  |E_b| < 2^57 w_b, components of n_b below 2^58 (a stretch of two at
+// least); cross products in units of 2^57, below 2^60; S below 2^57 and c2
+// below 2^59; sums of a force in units of 2^58, below 2^61.3.  Numbers are split into a high and a signed 29-bit low limb,
+// whose products fit 64-bit accumulators.  Products of two low limbs are left
+// out; with the final shifts that drops half a unit of 2^-55 to 2^-56 of the
+// products summed, less than the FP64 sum it replaces rounds.  An element that
+// leaves these sizes is left to the FP64 arithmetic of its caller.
+//
+// Integer C that also compiles for the host.
+#pragma once
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define MSX_HD __host__ __device__ __forceinline__
+#else
+#define MSX_HD inline
+#endif
+
+namespace msx {
+
+constexpr int kFixTerms = 16;   // coefficients of c2's series in 1 - J: |1 - J| < 2^-4
+constexpr int kFixShort = 9;    // those that |1 - J| < 2^-7 needs
+// A tet of det E >= kFixFlat |E_1||E_2||E_3| (0.41 for the six tets of a cube):
+// in flatter ones the truncations of the cross products grow towards FP64's
+// rounding.  Corner-force error against quad precision over that of the same
+// formulas in FP64, 5000 random tets a case, nu 0 to 0.49, strains to 3 %: 0.3
+// to 0.5 (0.05 undeformed) above 0.25, 0.4 to 0.8 around 0.15, 1.1 at 0.06.
+constexpr double kFixFlat = 0.12;
+
+struct Limbs {
+    int32_t h, l;   // h 2^29 + l, |l| <= 2^28
+};
+
+MSX_HD Limbs limbs(int64_t x)
+{
+    return {(int32_t)((x + (1 << 28)) >> 29), (int32_t)((uint32_t)x << 3) >> 3};
+}
+
+MSX_HD Limbs limbs_neg(Limbs a) { return {-a.h, -a.l}; }
+
+// a b = hh 2^58 + mid 2^29 + a.l b.l, summed without the last
+MSX_HD void mac(int64_t &hh, int64_t &mid, Limbs a, Limbs b)
+{
+    hh += (int64_t)a.h * b.h;
+    mid += (int64_t)a.h * b.l;
+    mid += (int64_t)a.l * b.h;
+}
+
+// hh 2^58 + mid 2^29 in units of 2^(58 - k), rounded to nearest when mid began
+// at mac_half(k)
+MSX_HD int64_t mac_sum(int64_t hh, int64_t mid, int k) { return (int64_t)((uint64_t)hh << k) + (mid >> (29 - k)); }
+MSX_HD int64_t mac_half(int k) { return 1 << (28 - k); }
+
+MSX_HD int64_t mulhi64(int64_t a, int64_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __mul64hi(a, b);
+#else
+    return (int64_t)(((__int128)a * b) >> 64);
+#endif
+}
+
+MSX_HD int top_bit(int64_t x)   // floor(log2 x), x > 0
+{
+#ifdef __CUDA_ARCH__
+    return 63 - __clzll(x);
+#else
+    return 63 - __builtin_clzll((unsigned long long)x);
+#endif
+}
+
+MSX_HD uint64_t double_bits(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    memcpy(&b, &x, 8);
+    return b;
+#endif
+}
+
+MSX_HD double pow2_double(int k)   // 2^k, -1022 <= k <= 1023
+{
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)(k + 1023) << 52);
+#else
+    return ldexp(1.0, k);
+#endif
+}
+
+MSX_HD uint64_t shr64(uint64_t x, int s)   // zero for s < 0 and s > 63
+{
+#ifdef __CUDA_ARCH__
+    uint64_t r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+#else
+    return (unsigned)s > 63 ? 0 : x >> s;
+#endif
+}
+
+// A double, given as its words, in units of 2^lw, truncated toward zero.  room
+// becomes negative for |x| >= 2^58 2^lw, infinities and NaN, else stays.
+MSX_HD int64_t fixed_from(uint32_t hi, uint32_t lo, int lw, int &room)
+{
+    const int ex = (int)((hi >> 20) & 0x7FFu);
+    const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 5;   // below 2^58
+    const int s = lw + (1075 + 5) - ex;
+    room = room < s ? room : s;
+    const int64_t sg = (int64_t)((int32_t)hi >> 31);
+    return ((int64_t)shr64(m, s) ^ sg) - sg;
+}
+
+// c = n_a x n_b in units of 2^57
+MSX_HD void fixed_cross(const Limbs *a, const Limbs *b, int64_t *c)
+{
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        int64_t hh = 0, mid = mac_half(1);
+        mac(hh, mid, a[j], b[k]);
+        mac(hh, mid, limbs_neg(a[k]), b[j]);
+        c[i] = mac_sum(hh, mid, 1);
+    }
+}
+
+// n_1 . (n_2 x n_3) in units of 2^(57 + 57); cr: the limbs of the cross product
+MSX_HD int64_t fixed_det(const Limbs *n1, const Limbs *cr)
+{
+    int64_t hh = 0, mid = mac_half(1);
+#pragma unroll
+    for (int i = 0; i < 3; i++) mac(hh, mid, n1[i], cr[i]);
+    return mac_sum(hh, mid, 1);
+}
+
+// The element's static data beside its reference edges: S_ab w_a w_b 2^t (in the
+// order 11 12 13 22 23 33), det E as fixed_det gives it, 2^(62 + ds) / det E
+// for ds = floor(log2 det E), and exponents.
+struct FixedElem {
+    Limbs S[6];
+    int64_t d0, rd;
+    int32_t lw[3];   // log2 w_b
+    int32_t x0;      // log2 of f_a's unit = x0 - lw_a
+    int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t)
+    int32_t ds;
+};
+
+// The exponents as two words in device memory.  A zero first word (ds is at
+// least 40) sends the element to FP64.
+MSX_HD void fixed_pack(const FixedElem &q, uint32_t *w)
+{
+    w[0] = (uint32_t)q.ds | (uint32_t)(q.cs + 32) << 6 | (uint32_t)(q.lw[0] + 2048) << 12;
+    w[1] = (uint32_t)(q.lw[1] - q.lw[0] + 64) | (uint32_t)(q.lw[2] - q.lw[0] + 64) << 7 | (uint32_t)(q.x0 + 4096) << 14;
+}
+
+MSX_HD void fixed_unpack(uint32_t w0, uint32_t w1, FixedElem &q)
+{
+    q.ds = (int)(w0 & 63u);
+    q.cs = (int)((w0 >> 6) & 63u) - 32;
+    q.lw[0] = (int)(w0 >> 12) - 2048;
+    q.lw[1] = q.lw[0] + (int)(w1 & 127u) - 64;
+    q.lw[2] = q.lw[0] + (int)((w1 >> 7) & 127u) - 64;
+    q.x0 = (int)(w1 >> 14) - 4096;
+}
+
+// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of
+// 2^(x0 - lw_a); false when the element leaves the sizes above.  e: the deformed
+// edges' nine components; kq: c2's series.  scalar(J) gives -c2 in kq's units
+// for |1 - J| >= 2^-4, in FP64.  f_0 = -(f_1 + f_2 + f_3) is left to the caller,
+// in FP64: its rounding to nearest has no preferred sign (a sum of shifted
+// integers has, and pushes the whole body).
+template <typename SCALAR>
+MSX_HD bool fixed_forces(const FixedElem &q, const double *e, const int64_t *kq, SCALAR scalar, int64_t *f)
+{
+    int room = 63;
+    Limbs n[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const uint64_t b = double_bits(e[k]);
+        n[k] = limbs(fixed_from((uint32_t)(b >> 32), (uint32_t)b, q.lw[k / 3], room));
+    }
+    if (room < 0) return false;
+    Limbs cr[9];   // cr_1 = n_2 x n_3, cr_2 = n_3 x n_1, cr_3 = n_1 x n_2
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        int64_t c[3];
+        fixed_cross(n + 3 * ((a + 1) % 3), n + 3 * ((a + 2) % 3), c);
+#pragma unroll
+        for (int i = 0; i < 3; i++) cr[3 * a + i] = limbs(c[i]);
+    }
+    const int64_t D = fixed_det(n, cr);
+    const int64_t y = q.d0 - D;   // d0 (1 - J)
+    int64_t c2;
+    if (y < (q.d0 >> 4) && y > -(q.d0 >> 4)) {
+        const int64_t yq = mulhi64((int64_t)((uint64_t)y << (66 - q.ds)), q.rd);   // (1 - J) 2^64
+        const bool near1 = yq < (1LL << 57) && yq > -(1LL << 57);
+        c2 = near1 ? kq[kFixShort - 1] : kq[kFixTerms - 1];
+        if (!near1)
+#pragma unroll
+            for (int k = kFixTerms - 2; k >= kFixShort - 1; k--) c2 = kq[k] + mulhi64(yq, c2);
+#pragma unroll
+        for (int k = kFixShort - 2; k >= 0; k--) c2 = kq[k] + mulhi64(yq, c2);
+    } else {
+        c2 = scalar(1.0 - (double)y / (double)q.d0);
+    }
+    const int64_t most = q.cs >= 0 ? (1LL << 59) >> q.cs : (q.cs > -3 ? (1LL << 59) << -q.cs : INT64_MAX);
+    if (c2 >= most || c2 <= -most) return false;
+    c2 = q.cs >= 0 ? (int64_t)((uint64_t)c2 << q.cs) : c2 >> -q.cs;
+    const Limbs lc = limbs(-c2);
+    const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            int64_t hh = 0, mid = mac_half(0);
+            mac(hh, mid, lc, cr[3 * a + i]);
+#pragma unroll
+            for (int b = 0; b < 3; b++) mac(hh, mid, q.S[mi[a * 3 + b]], n[3 * b + i]);
+            f[3 * a + i] = mac_sum(hh, mid, 0);
+        }
+    return true;
+}
+
+// The static data from the reference edges E (E[3(b-1) + i]), the law's c2
+// series' first coefficient kq0 and exponent ks (fixed_series).  With the
+// integers of the reference element itself, n_a x n_b as c_a and det E as d0,
+//     S_ab w_a w_b = W mu w_1 w_2 w_3 (c_a . c_b) / d0,
+// so S and c2 carry the same truncations of the cross products and cancel to
+// the last bits in the undeformed state.  false: the element is left to FP64 (a
+// non-positive volume, too flat an element, numbers near the ends of the FP64
+// range).
+MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
+{
+    Limbs n[9], cl[9];
+    int64_t c[9], v[6], vm = 0;
+    int room = 63, sum = 0;
+    double vol = kFixFlat * kFixFlat;
+    for (int b = 0; b < 3; b++) {
+        const double l2 = E[3 * b] * E[3 * b] + E[3 * b + 1] * E[3 * b + 1] + E[3 * b + 2] * E[3 * b + 2];
+        if (!(l2 < 1e100) || !(l2 > 1e-100)) return false;
+        const int ex2 = (int)(double_bits(l2) >> 52) - 1023;
+        q.lw[b] = (ex2 >> 1) + 1 - 57;   // floor(log2 |E_b|) + 1 - 57
+        sum += q.lw[b];
+        vol *= l2 * pow2_double(-2 * q.lw[b]);
+        for (int i = 0; i < 3; i++) {
+            const uint64_t w = double_bits(E[3 * b + i]);
+            n[3 * b + i] = limbs(fixed_from((uint32_t)(w >> 32), (uint32_t)w, q.lw[b], room));
+        }
+    }
+    const int d1 = q.lw[1] - q.lw[0], d2 = q.lw[2] - q.lw[0];
+    if (d1 < -20 || d1 > 20 || d2 < -20 || d2 > 20) return false;
+    for (int a = 0; a < 3; a++) {
+        fixed_cross(n + 3 * ((a + 1) % 3), n + 3 * ((a + 2) % 3), c + 3 * a);
+        for (int i = 0; i < 3; i++) cl[3 * a + i] = limbs(c[3 * a + i]);
+    }
+    q.d0 = fixed_det(n, cl);
+    const double det = (double)q.d0 * 0x1p114;
+    if (q.d0 < (1LL << 48) || q.d0 >= (1LL << 62) || !(det * det >= vol)) return false;
+    q.ds = top_bit(q.d0);
+    // 2^(62 + ds) / d0: the FP64 quotient, corrected once
+    q.rd = (int64_t)(0x1p62 / ((double)q.d0 * pow2_double(-q.ds)));
+    const __int128 res = ((__int128)1 << (62 + q.ds)) - (__int128)q.rd * q.d0;   // below 2^66
+    q.rd += mulhi64((int64_t)(res >> 8), q.rd) >> (q.ds - 10);
+    __int128 dot[6], dm = 0;
+    int k = 0;
+    for (int a = 0; a < 3; a++)
+        for (int b = a; b < 3; b++, k++) {
+            dot[k] = (__int128)c[3 * a] * c[3 * b] + (__int128)c[3 * a + 1] * c[3 * b + 1] +
+                     (__int128)c[3 * a + 2] * c[3 * b + 2];
+            if (a == b && dot[k] > dm) dm = dot[k];   // the largest is on the diagonal
+        }
+    const int64_t dh = (int64_t)(dm >> 56);   // below 2^62
+    if (dh < 1) return false;
+    const int cs = 56 + top_bit(dh) - 61;   // dot >> cs below 2^62
+    for (k = 0; k < 6; k++) {
+        v[k] = mulhi64((int64_t)(dot[k] >> cs), q.rd);   // (c_a . c_b / 2^cs) / d0 2^(ds - 2)
+        const int64_t m = v[k] < 0 ? -v[k] : v[k];
+        vm = vm > m ? vm : m;
+    }
+    if (kq0 < (1LL << 32) || vm < (1LL << 32)) return false;
+    if (vm >= (1LL << 62)) return false;
+    const int z = 61 - top_bit(kq0), kv = 61 - top_bit(vm), kc = kv - cs + 56;   // kq0 and the largest v to [2^61, 2^62)
+    // S_ab w_a w_b 2^t = mulhi(kq0 << z, v << kv) >> sh, below 2^57, and
+    // kq0 << cs = c2 w_1 w_2 w_3 2^(57 + t) at J = 1, below 2^57 too
+    const int64_t top = mulhi64(kq0 << z, vm << kv);   // below 2^60
+    int sh = top >= (1LL << 59) ? 3 : (top >= (1LL << 58) ? 2 : 1);
+    if (q.ds + kc - 60 > sh) sh = q.ds + kc - 60;
+    const int t = ks + z - sum - 122 + q.ds + kc - sh;
+    for (k = 0; k < 6; k++)
+        q.S[k] = limbs((mulhi64(kq0 << z, (int64_t)((uint64_t)v[k] << kv)) + (1LL << (sh - 1))) >> sh);
+    q.x0 = 58 - t;
+    q.cs = -ks + sum + 57 + t;
+    if (sh > 20 || q.cs < -31 || q.cs > 20) return false;
+    const int lmax = q.lw[0] + (d1 > d2 ? (d1 > 0 ? d1 : 0) : (d2 > 0 ? d2 : 0));
+    const int lmin = q.lw[0] + (d1 < d2 ? (d1 < 0 ? d1 : 0) : (d2 < 0 ? d2 : 0));
+    return q.x0 - lmin <= 900 && q.x0 - lmax >= -900;   // forces stay normal FP64 numbers
+}
+
+// kq and ks of a material: (mu + lambda H_n) W 2^ks, n = 0..15 (H_n the harmonic
+// numbers), as integers below 2^61.
+inline void fixed_series(double lambda, double mu, int64_t *kq, int *ks)
+{
+    double c[kFixTerms], H = 0, big = 0;
+    for (int n = 0; n < kFixTerms; n++) {
+        if (n) H += 1.0 / n;
+        c[n] = (mu + lambda * H) * 0.166666666667;
+        if (std::fabs(c[n]) > big) big = std::fabs(c[n]);
+    }
+    *ks = 60 - std::ilogb(big);
+    for (int n = 0; n < kFixTerms; n++) kq[n] = (int64_t)std::rint(std::ldexp(c[n], *ks));
+}
+
+}  // namespace msx

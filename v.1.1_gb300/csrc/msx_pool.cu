@@ -158,8 +158,9 @@ static bool pair_state(int precision) { return precision == MSX_PREC_MIXED || pr
 static size_t footprint(long long nn, long long ne, long long nbc, int precision, bool cnh)
 {
     size_t b = 0;
-    if (cnh)   // plain FP64, compressible neo-Hookean: Eref, Mg, rdetE
-        b += align256(sizeof(double) * 9 * ne) + align256(sizeof(double) * 6 * ne) + align256(sizeof(double) * ne);
+    if (cnh)   // plain FP64, compressible neo-Hookean: Eref, fxS, fxD, fxw
+        b += align256(sizeof(double) * 9 * ne) + align256(sizeof(int2) * 6 * ne) + align256(sizeof(longlong2) * ne) +
+             align256(sizeof(uint2) * ne);
     b += align256(sizeof(int4) * ne) + align256(sizeof(double) * 9 * ne);           // conn, G
     b += 2 * align256(sizeof(double) * ne);                                         // wJ, Lref
     b += align256(sizeof(float) * 9 * ne) + 2 * align256(sizeof(float) * ne);        // G32, wJ32, Lref32
@@ -572,7 +573,7 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
             if (!dw_in_range(mesh->X[i]))
                 return pfail(MSX_ERR_ARG, "double-word pool: a nonzero coordinate lies outside [2^-100, 2^100]");
     }
-    const bool cnh = prec == MSX_PREC_FP64 && mp.law == 1;   // the FP64 element kernel's F-free path
+    const bool cnh = prec == MSX_PREC_FP64 && mp.law == 1;   // the FP64 element kernel's fixed-point path
     const size_t bytes = footprint(nn, ne, num_bcs, prec, cnh);
     {   // cheap early refusal; the slot is taken below, after the host tables
         std::lock_guard<std::mutex> lk(p->mu);
@@ -650,8 +651,9 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         if (prec == MSX_PREC_FP64) P.u4 = (double *)carve(sizeof(double) * 4 * nn);
         if (cnh) {   // written by the element set-up, as for a single solve
             P.Eref = (double *)carve(sizeof(double) * 9 * ne);
-            P.Mg = (double *)carve(sizeof(double) * 6 * ne);
-            P.rdetE = (double *)carve(sizeof(double) * ne);
+            P.fxS = (int2 *)carve(sizeof(int2) * 6 * ne);
+            P.fxD = (longlong2 *)carve(sizeof(longlong2) * ne);
+            P.fxw = (uint2 *)carve(sizeof(uint2) * ne);
         }
         float2 *minv2 = nullptr;
         if (pair_state(prec)) {

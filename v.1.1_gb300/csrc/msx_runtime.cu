@@ -102,8 +102,11 @@ struct msx_handle {
     DBuf<float2> uhl, vhl, ahl, minv2;
     DBuf<double> u4;   // plain FP64 mode: node-major copy of u (Problem::u4)
     // plain FP64 mode with a compressible neo-Hookean material: reference
-    // edges, gradient metric and 1/det of the reference Jacobian (Problem::Eref, Mg, rdetE)
-    DBuf<double> Eref, Mg, rdetE;
+    // edges and fixed-point data (Problem::Eref, fxS, fxD, fxw)
+    DBuf<double> Eref;
+    DBuf<int2> fxS;
+    DBuf<longlong2> fxD;
+    DBuf<uint2> fxw;
     DBuf<unsigned char> mat;
     DBuf<int> node_ptr, node_inc, node_bc;
     DBuf<int2> bc_nodes;   // (node, record) of the nodes with Dirichlet entries
@@ -190,6 +193,11 @@ bool msx::material_params(const msx_material &m, MatParams &o)
     o.mu2_w = dw(o.mu2);
     o.lam_stvk_w = dw(o.lam_stvk);
     o.mu3_w = dw(o.mu / 3.0);
+    o.ksw = 0;
+    if (m.law == 1) {
+        fixed_series(o.lambda, o.mu, o.kq, &o.ks);
+        o.ksw = 0.166666666667 * std::ldexp(1.0, o.ks);
+    }
     return true;
 }
 
@@ -299,8 +307,9 @@ static void bind_problem(msx_handle *h)
     P.uhl = h->uhl.p;
     P.u4 = h->precision == MSX_PREC_FP64 ? h->u4.p : nullptr;
     P.Eref = h->precision == MSX_PREC_FP64 ? h->Eref.p : nullptr;
-    P.Mg = h->precision == MSX_PREC_FP64 ? h->Mg.p : nullptr;
-    P.rdetE = h->precision == MSX_PREC_FP64 ? h->rdetE.p : nullptr;
+    P.fxS = P.Eref ? h->fxS.p : nullptr;
+    P.fxD = P.Eref ? h->fxD.p : nullptr;
+    P.fxw = P.Eref ? h->fxw.p : nullptr;
     P.vhl = h->vhl.p;
     P.ahl = h->ahl.p;
     P.minv2 = h->minv2.p;
@@ -468,7 +477,7 @@ static msx_status upload_bcs(msx_handle *h, const msx_bc *bcs, long long nbc)
 // are converted from the FP64 set-up data (a later block in a new mode); at
 // msx_create the set-up kernels fill them.
 // A material of the compressible neo-Hookean law (the plain FP64 mode's
-// F-free element path).
+// fixed-point element path).
 static bool has_cnh(const msx_handle *h)
 {
     for (int k = 0; k < h->P.nmat; k++)
@@ -510,8 +519,9 @@ static msx_status mode_buffers(msx_handle *h, int precision, bool fill, cudaStre
     bool cnh = false;
     if (precision == MSX_PREC_FP64 && has_cnh(h) && !h->Eref.p) {
         MSX_CUDA(h->Eref.alloc(9 * ne));
-        MSX_CUDA(h->Mg.alloc(6 * ne));
-        MSX_CUDA(h->rdetE.alloc(ne));
+        MSX_CUDA(h->fxS.alloc(6 * ne));
+        MSX_CUDA(h->fxD.alloc(ne));
+        MSX_CUDA(h->fxw.alloc(ne));
         cnh = true;
     }
     if (!mixed && !h->fe.p) {
@@ -797,14 +807,19 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
                 }
                 if (h->precision == MSX_PREC_FP64 && has_cnh(h)) {
                     ALLOC(h->Eref, 9 * ne);
-                    ALLOC(h->Mg, 6 * ne);
-                    ALLOC(h->rdetE, ne);
+                    ALLOC(h->fxS, 6 * ne);
+                    ALLOC(h->fxD, ne);
+                    ALLOC(h->fxw, ne);
                 }
                 bind_problem(h);
             }
             if (cudaStreamWaitEvent(s, side.chunk[c], 0) != cudaSuccess)
                 return bail(fail(MSX_ERR_CUDA, "stream ordering failed"));
-            launch_setup_elements(h->P, h->X.p, s, e0, e1);
+            // the fixed-point data need the materials: with several, they follow the
+            // material ids' upload
+            Problem P = h->P;
+            if (mesh->elem_material && num_mats > 1) P.Eref = nullptr;
+            launch_setup_elements(P, h->X.p, s, e0, e1);
         }
     }
     if (cudaMallocHost((void **)&h->h_ctrl, 2 * sizeof(Ctrl)) != cudaSuccess)
@@ -853,6 +868,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
 #undef UP
     if (cudaEventRecord(side.lists, side.s) != cudaSuccess || cudaStreamWaitEvent(s, side.lists, 0) != cudaSuccess)
         return bail(fail(MSX_ERR_CUDA, "stream ordering failed"));
+    if (h->P.mat && h->P.Eref) launch_cnh_arrays(h->P, s);
     launch_setup_mass(h->P, h->mass.p, h->minv.p, s);
     if (h->minv2.p) launch_minv_split(h->minv.p, h->minv2.p, nn, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
@@ -874,7 +890,10 @@ extern "C" msx_status msx_destroy(msx_handle *h)
     for (auto *b : {&h->G32, &h->wJ32, &h->Lref32, &h->fe32, &h->G32lo, &h->wJ32lo}) b->release();
     for (auto *b : {&h->uhl, &h->vhl, &h->ahl, &h->minv2}) b->release();
     h->u4.release();
-    for (auto *b : {&h->Eref, &h->Mg, &h->rdetE}) b->release();
+    h->Eref.release();
+    h->fxS.release();
+    h->fxD.release();
+    h->fxw.release();
     h->mat.release();
     for (auto *b : {&h->node_ptr, &h->node_inc, &h->node_bc, &h->flags}) b->release();
     h->bc_rec.release();
