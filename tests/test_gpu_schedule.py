@@ -35,3 +35,35 @@ def test_sizes(n, precision, tol):
     pu, pv, pa = P.fetch(t)
     P.close()
     assert np.array_equal(u, pu) and np.array_equal(v, pv) and np.array_equal(a, pa)
+
+
+DEFORMATIONS = {
+    "rest": lambda x, h: 0 * x,
+    "small": lambda x, h: 1e-3 * np.sin(3 * x[[1, 2, 0]]) * x[2],
+    "sheared": lambda x, h: np.stack([0.3 * x[2], 0 * x[0], 0 * x[0]]),
+    "one node pushed into its elements": lambda x, h: np.where(
+        np.arange(x.shape[1]) == np.argmin(((x - 0.5) ** 2).sum(0)), 0.45 * h, 0.0) * np.array([[1.0], [0.3], [-0.2]]),
+    "rotated by 90 degrees": lambda x, h: np.stack([-x[1], x[0], x[2]]) - x,
+    "moved": lambda x, h: 0 * x + np.array([[40.0], [-7.0], [3.0]]) * h,
+    "shrunk": lambda x, h: -0.3 * x,
+    "swollen": lambda x, h: 0.4 * x,
+}
+
+
+@pytest.mark.parametrize("jitter", [0.0, 0.1])
+@pytest.mark.parametrize("name", list(DEFORMATIONS))
+@pytest.mark.parametrize("precision", [msx.FP64, msx.FP64_EXACT, msx.MIXED, msx.DOUBLE_WORD])
+def test_time_step_is_the_minimum(name, jitter, precision):
+    """The step's dt, found by the gated screen in the element kernel, against the block's first dt, which an FP64
+    pass over every element gives: from rest the displacement of both steps is the initial one."""
+    n = 7
+    X, conn = msx.mesh_cube(n, 9, jitter)
+    u = DEFORMATIONS[name](X, 1.0 / n)
+    for law in (msx.COMPRESSIBLE_NH, msx.STVK):
+        S = msx.Solver(X, conn, [(law, 1e6, 0.3, 1000.0)], [], 0.0, 1e30, 0.5, precision=precision)
+        S.set_state(u.ravel())
+        first, second = S.run(1).dt, S.run(1).dt
+        S.close()
+        # 60 roundings of FP64, and u's own 2^-48 in the pair-state modes
+        tol = 60 * 2.0 ** -53 * 4 + (2.0 ** -46 * np.abs(u).max() * n if precision in (msx.MIXED, msx.DOUBLE_WORD) else 0)
+        assert abs(second - first) <= tol * first

@@ -11,8 +11,6 @@
 namespace msx {
 
 #define MSX_INF_BITS 0x7FF0000000000000ULL
-// FP32 +infinity as the running minimum of the CFL screen (dtmin[2..3])
-constexpr unsigned long long kScreenInfBits = 0x7F800000ULL;
 
 // ---------------------------------------------------------------------------
 // Reference-order arithmetic (src/mathematics/maths.cpp, geometry.cpp and the
@@ -775,7 +773,7 @@ __device__ __forceinline__ void publish_step(const Problem &p, const StepDecisio
 {
     p.ctrl[parity] = d.next;
     p.dtmin[parity ^ 1] = MSX_INF_BITS;
-    p.dtmin[2 + (parity ^ 1)] = kScreenInfBits;
+    p.dtmin[2 + (parity ^ 1)] = p.dtmin[4];   // the undeformed CFL minimum bounds every step's
     p.flags[parity ^ 1] = 0;
 }
 
@@ -796,6 +794,7 @@ __global__ void __launch_bounds__(kNodeBlock) node_kernel(Problem p, int parity)
 
 // Reference operation order (used with contraction off).
 __device__ __forceinline__ float f32_trunc(double x);
+__device__ __forceinline__ float gate_moved(float Lr, float d, float inv_c);
 __device__ __forceinline__ float cfl_screen(const Problem &p, long long e, const float *g, const float *du,
                                             const MatParams &m);
 
@@ -823,7 +822,7 @@ __device__ __forceinline__ double cfl_exact_ref(const Problem &p, long long e)
 // SCREEN: return the FP32 screen value of the CFL (cfl_screen) instead of the
 // exact one; the caller rechecks the elements near its block's minimum.
 template <bool FORCE_ONLY, bool SCREEN = false, bool VISC = false>
-__device__ __forceinline__ double elem_body_exact(const Problem &p, long long e, int parity)
+__device__ __forceinline__ double elem_body_exact(const Problem &p, long long e, int parity, float gmin = 0.0f)
 {
     const long long ne = p.ne, nn = p.nn;
     double vmin = INFINITY;
@@ -909,6 +908,27 @@ __device__ __forceinline__ double elem_body_exact(const Problem &p, long long e,
                 fe[a * 3 + i] = dead ? 0.0 : f;
             }
         if (!FORCE_ONLY && SCREEN) {
+            if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+            // the gate takes FP32 differences of the truncated displacements: off by 2^-22 |u|
+            float u32[12], d2 = 0.0f, um = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 12; k++) {
+                u32[k] = f32_trunc(ue[k]);
+                um = fmaxf(um, fabsf(u32[k]));
+            }
+#pragma unroll
+            for (int a = 1; a < 4; a++) {
+                float q = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const float w = u32[a * 3 + i] - u32[i];
+                    q += w * w;
+                }
+                d2 = fmaxf(d2, q);
+            }
+            float dm;
+            asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(dm) : "f"(d2));
+            if (gate_moved(__ldg(p.Lref32 + e), dm + 0x1p-20f * um, m.inv_c_f) > gmin) return INFINITY;
             float du32[9];
 #pragma unroll
             for (int a = 1; a < 4; a++)
@@ -918,7 +938,6 @@ __device__ __forceinline__ double elem_body_exact(const Problem &p, long long e,
 #pragma unroll
             for (int k = 0; k < 9; k++) g32[k] = f32_trunc(dphi[3 + k]);
             vmin = (double)cfl_screen(p, e, g32, du32, m);
-            if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
         } else if (!FORCE_ONLY) {
             // solvers.cpp:304-317: deformed inscribed sphere
             double x[12];
@@ -1128,6 +1147,41 @@ __device__ __forceinline__ float f32_trunc(double x)
     return __uint_as_float(r);
 }
 
+// The gate before the CFL screen.  An element whose nodes moved by at most d
+// relative to its first node keeps an inscribed sphere of diameter
+// L_ref - 2 d: ||F - I|| <= sum_b |u_b - u_0| / h_b <= max_b |u_b - u_0| / r
+// (heights h_b, 1/r = sum of the four 1/h), and the reference sphere of radius
+// r goes to an ellipsoid with half axes of at least (1 - ||F - I||) r inside
+// the tet.  gate = that bound with ||F - I||_F at hand, or with max |u_b - u_0|,
+// over the sound speed.  Elements above (1 + 2^-8) times the solve's running
+// minimum cannot hold the step's minimum and skip the screen: about 200 FP32
+// instructions an element, for 12 to 30.  A reference sliver (negative Lref32)
+// and NaN never pass.  Element kernels with and without: mixed, 6M tets 0.164
+// and 0.185 ms; reference order, 384 K tets 0.208 and 0.247; FP64, 6M tets 0.621
+// and 0.647; double-word, 1.57M tets 0.1165 and 0.1214.  (On a mesh of equal
+// elements everything is near the minimum and passes to the screen as before.)
+__device__ __forceinline__ float gate_frobenius(float Lr, float hh, float inv_c)
+{
+    float s;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(hh));
+    return Lr * (0.9995f - s) * inv_c;   // the margin covers sqrt.approx and the rounding of H
+}
+
+__device__ __forceinline__ float gate_moved(float Lr, float d, float inv_c) { return (Lr - 2.002f * d) * inv_c; }
+
+// An upper bound of max_k |x_k| of FP64 values from their high words; infinite
+// (or NaN) when it leaves FP32's range.
+template <int N>
+__device__ __forceinline__ float abs_bound(const double *x)
+{
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) m = max(m, __double2hiint(x[k]) & 0x7FFFFFFF);
+    // high word: 11 exponent bits biased by 1023, 20 of the mantissa's; modulo 2^32
+    const unsigned f = ((unsigned)(m + 1) << 3) - ((unsigned)(1023 - 127) << 23);
+    return m >= ((1023 + 100) << 20) ? INFINITY : (m <= ((1023 - 100) << 20) ? 0x1p-99f : __uint_as_float(f));
+}
+
 // FP32 estimate of an element's CFL value: the reference edges X_b - X_0 are
 // the columns of G^-1 (g: the rows of G, the gradients of shape functions
 // 1-3, in FP32), cof(G)^T / det G, plus the displacement differences du.  Its
@@ -1178,14 +1232,14 @@ __device__ __forceinline__ float cfl_screen(const Problem &p, long long e, const
 
 template <bool FORCE_ONLY, bool ACT, bool VISC>
 __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
-                                                    const MatParams &m, const int *nd);
+                                                    const MatParams &m, const int *nd, float gmin);
 
 // The cofactor form's corner forces of one element that fixed point leaves out.
 static __device__ __noinline__ void elem_cnh_general(const Problem &p, long long e, int parity)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    elem_cofactor_fp64<true, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd);
+    elem_cofactor_fp64<true, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, 0.0f);
 }
 
 // x 2^k for an integer x: the exponent is added to the converted integer's
@@ -1204,7 +1258,7 @@ __device__ __forceinline__ double fixed_to_double(long long x, int k)
 // 115 operations of the same formulas in FP64.  The CFL screen takes the deformed
 // edges directly (truncated to FP32).
 __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
-                                                    const int *nd)
+                                                    const int *nd, float gmin)
 {
     const long long ne = p.ne, nn = p.nn;
     double ua[4][3];
@@ -1222,13 +1276,16 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 #pragma unroll
             for (int i = 0; i < 3; i++) ua[a][i] = p.u[nd[a] + i * nn];
     }
-    double ed[9];   // ed[(b-1)*3 + i]: component i of the deformed edge e_b
+    double du[9], ed[9];   // ed[(b-1)*3 + i]: component i of the deformed edge e_b
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) ed[b * 3 + i] = __ldg(p.Eref + (b * 3 + i) * ne + e) + (ua[b + 1][i] - ua[0][i]);
-    float scr;
-    {
+        for (int i = 0; i < 3; i++) {
+            du[b * 3 + i] = ua[b + 1][i] - ua[0][i];
+            ed[b * 3 + i] = __ldg(p.Eref + (b * 3 + i) * ne + e) + du[b * 3 + i];
+        }
+    float scr = INFINITY;
+    if (!(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound<9>(du), m.inv_c_f) > gmin)) {
         float e32[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) e32[k] = f32_trunc(ed[k]);
@@ -1276,7 +1333,7 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 // value (see cfl_screen).
 template <bool FORCE_ONLY, bool ACT, bool VISC>
 __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
-                                                    const MatParams &m, const int *nd)
+                                                    const MatParams &m, const int *nd, float gmin)
 {
     const long long ne = p.ne, nn = p.nn;
     double G[9];
@@ -1312,8 +1369,9 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
             // the identity enters the FMA chain (no separate 0 + x or 1 + x)
             F[i * 3 + j] = fma(du[i], G[j], fma(du[3 + i], G[3 + j], i == j ? fma(du[6 + i], G[6 + j], 1.0)
                                                                              : du[6 + i] * G[6 + j]));
-    float scr = 0.0f;
-    if (!FORCE_ONLY) {   // the CFL screen first, so du dies before the stress
+    float scr = INFINITY;
+    // the CFL screen first, so du dies before the stress
+    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound<9>(du), m.inv_c_f) > gmin)) {
         float du32[9], g32[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) {
@@ -1351,13 +1409,13 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
 
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
 __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
-                                                double idt = 0.0)
+                                                double idt = 0.0, float gmin = 0.0f)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
-    if (!FORCE_ONLY && !VISC && p.Eref && m.law == 1) return elem_body_fp64_cnh(p, e, parity, m, nd);   // never dead
-    return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd);
+    if (!FORCE_ONLY && !VISC && p.Eref && m.law == 1) return elem_body_fp64_cnh(p, e, parity, m, nd, gmin);   // never dead
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
 }
 
 // corner forces only (internal-force hook)
@@ -1457,7 +1515,7 @@ __device__ __forceinline__ void stress_mixed(const MatParams &m, const float *H,
 
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
 __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, int parity, int4 cn, double t = 0.0,
-                                                 float idtf = 0.0f)
+                                                 float idtf = 0.0f, float gmin = 0.0f)
 {
     const long long ne = p.ne, nn = p.nn;
     float vmin = INFINITY;
@@ -1491,6 +1549,9 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
         // rounding lies far below the FP32 precision of J - 1.  So J - 1 is
         // good to FP32 relative precision, and so is ln J = log1p(J - 1);
         // F = I + H is never formed or reduced.
+        float hh = 0.0f;   // ||H||_F^2, for the CFL gate
+#pragma unroll
+        for (int k = 0; k < 9; k++) hh = fmaf(H[k], H[k], hh);
         float tf = H[0] + H[4] + H[8];
         // spelled out, as in stress_mixed
         const float m48 = fmaf(H[4], H[8], -__fmul_rn(H[5], H[7])), m38 = fmaf(H[3], H[8], -__fmul_rn(H[5], H[6])),
@@ -1546,7 +1607,8 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
         fe[sl.y] = make_float4(f[3], f[4], f[5], 0.f);
         fe[sl.z] = make_float4(f[6], f[7], f[8], 0.f);
         fe[sl.w] = make_float4(f[9], f[10], f[11], 0.f);
-        if (!FORCE_ONLY) {
+        if (!FORCE_ONLY && e == 0 && !isfinite(p.uhl[1].x)) atomicOr(p.flags + (parity ^ 1), 1);
+        if (!FORCE_ONLY && !(gate_frobenius(__ldg(p.Lref32 + e), hh, m.inv_c_f) > gmin)) {
             // reference edges X_b - X_0 = columns of G^-1 (G's rows are the
             // gradients of shape functions 1-3): cof(G)^T / det G in FP32,
             // instead of streaming them; only the CFL value uses them
@@ -1582,7 +1644,6 @@ __device__ __forceinline__ float elem_body_mixed(const Problem &p, long long e, 
             float Lr = __ldg(p.Lref32 + e);
             vmin = ((dist < Lr) ? dist : Lr) * m.inv_c_f;
             if (!(v6 * v6 >= 4e-3f * l1 * l2 * l3) || !(vmin > 0.0f)) vmin = -1.0f;
-            if (e == 0 && !isfinite(p.uhl[1].x)) atomicOr(p.flags + (parity ^ 1), 1);
         }
     }
     return vmin;
@@ -1836,7 +1897,7 @@ static __device__ __noinline__ double cfl_dw(const Problem &p, long long e)
 
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
 __device__ __forceinline__ float elem_body_dw(const Problem &p, long long e, int parity, int4 cn, double t = 0.0,
-                                              double idt = 0.0)
+                                              double idt = 0.0, float gmin = 0.0f)
 {
     const long long ne = p.ne, nn = p.nn;
     int nd[4] = {cn.x, cn.y, cn.z, cn.w};
@@ -1857,6 +1918,12 @@ __device__ __forceinline__ float elem_body_dw(const Problem &p, long long e, int
         for (int j = 0; j < 3; j++)
             F[i * 3 + j] = dw_dot3(du[i], G[j], du[3 + i], G[3 + j], du[6 + i], G[6 + j], i == j ? 1.0f : 0.0f);
     const MatParams &m = mat_of(p, e);
+    float hh = 0.0f;   // ||F - I||_F^2, for the CFL gate
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const float h = k % 4 == 0 ? F[k].x - 1.0f : F[k].x;
+        hh = fmaf(h, h, hh);
+    }
     stress_dw(m, F, make_float2(__ldg(p.wJ32 + e), __ldg(p.wJ32lo + e)), P);
     if (VISC && !FORCE_ONLY) {
         // bulk viscosity in FP64 from the double-word F (exact as doubles), added as double-words
@@ -1891,6 +1958,7 @@ __device__ __forceinline__ float elem_body_dw(const Problem &p, long long e, int
     }
     if (FORCE_ONLY) return 0.0f;
     if (e == 0 && !isfinite(p.uhl[1].x)) atomicOr(p.flags + (parity ^ 1), 1);
+    if (gate_frobenius(__ldg(p.Lref32 + e), hh, m.inv_c_f) > gmin) return INFINITY;
     float du32[9], g32[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) {
@@ -2005,17 +2073,22 @@ __device__ __forceinline__ float block_min_bcast(float v);
 
 // Reference-order element kernel with the FP32 CFL screen: forces in the
 // reference's order for every element, the exact reference-order CFL value only
-// for the elements of the block within 2^-8 of its FP32 minimum (and slivers),
-// a set that always holds the block's exact minimum, so dt is the reference's.
+// for the elements within 2^-8 of the solve's running FP32 minimum (and slivers),
+// a set that always holds the exact minimum, so dt is the reference's.  A block
+// without any returns at once.
 template <bool VISC>
 __global__ void __launch_bounds__(kElemBlock) elem_kernel_exact_screened(Problem p, int parity)
 {
     if (!p.ctrl[parity].ran) return;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const float d = e < p.ne ? (float)elem_body_exact<false, true, VISC>(p, e, parity) : INFINITY;
+    const float gmin = __uint_as_float((unsigned)__ldcg(p.dtmin + 2 + (parity ^ 1))) * (1.0f + 1.0f / 256.0f);
+    const float d = e < p.ne ? (float)elem_body_exact<false, true, VISC>(p, e, parity, gmin) : INFINITY;
+    if (!__syncthreads_or(!(d > gmin))) return;
     const float bmin = block_min_bcast(d >= 0.0f ? d : INFINITY);
+    if (threadIdx.x == 0 && bmin < gmin)
+        atomicMin(p.dtmin + 2 + (parity ^ 1), (unsigned long long)__float_as_uint(bmin));
     double v = INFINITY;
-    if (e < p.ne && (d < 0.0f || d <= bmin * (1.0f + 1.0f / 256.0f))) v = cfl_exact_ref(p, e);
+    if (e < p.ne && !(d > fminf(gmin, bmin * (1.0f + 1.0f / 256.0f)))) v = cfl_exact_ref(p, e);
     block_min_to(v, p.dtmin + (parity ^ 1));
 }
 
@@ -2152,15 +2225,19 @@ __global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_c
 }
 
 // The elements of one tile for the tiled element kernel: each thread's
-// elements in turn; returns the thread's FP32 minimum of the CFL screen.  The
-// FP64 and double-word kernels keep every screen value in sdt; the mixed one
-// keeps none and returns -1 once one of its elements was a sliver (a negative
-// screen value), so no other register stays live.  The mixed and double-word bodies take the element's
-// connectivity loaded one element ahead, so their node gathers wait for one
-// memory latency instead of two (connectivity, then the nodes).  ACT: element
-// birth is on, and the step's time decides which elements are dead.
+// elements in turn; returns the thread's FP32 minimum of the CFL screen
+// (infinite when the gate let none through).  gmin: (1 + 2^-8) times the
+// solve's running minimum as the tile began.  The FP64 and double-word kernels
+// list every element whose screen value is not above it (slivers, with -1,
+// included) in sval and scand; the mixed one lists none and returns -1 once one
+// of its elements was a sliver, so no other register stays live.  The mixed and
+// double-word bodies take the element's connectivity loaded one element ahead,
+// so their node gathers wait for one memory latency instead of two
+// (connectivity, then the nodes).  ACT: element birth is on, and the step's time
+// decides which elements are dead.
 template <int MODE, bool ACT, bool VISC>
-__device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl, int parity, float *sdt)
+__device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
+                                               unsigned short *scand, int *ncand)
 {
     float v32 = INFINITY;
     const double t = ACT ? p.ctrl[parity].t : 0.0;
@@ -2174,17 +2251,26 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
     for (; e < tl.end; e += blockDim.x) {
         const int4 cn = cn_next;
         if ((MODE == MODE_MIXED || MODE == MODE_DW) && e + blockDim.x < tl.end) cn_next = p.conn[e + blockDim.x];
-        float d = MODE == MODE_MIXED ? elem_body_mixed<false, ACT, VISC>(p, e, parity, cn, t, idtf)
-                                     : (MODE == MODE_DW ? elem_body_dw<false, ACT, VISC>(p, e, parity, cn, t, idt)
-                                                        : elem_body_fp64<false, ACT, VISC>(p, e, parity, t, idt));
+        float d = MODE == MODE_MIXED ? elem_body_mixed<false, ACT, VISC>(p, e, parity, cn, t, idtf, gmin)
+                                     : (MODE == MODE_DW ? elem_body_dw<false, ACT, VISC>(p, e, parity, cn, t, idt, gmin)
+                                                        : elem_body_fp64<false, ACT, VISC>(p, e, parity, t, idt, gmin));
         if (MODE == MODE_MIXED) {
             v32 = d < 0.0f ? -1.0f : fminf(v32, d);   // -1 sticks: fminf(-1, d) = -1 for d >= 0
-        } else {
-            sdt[e - tl.begin] = d;
+        } else if (!(d > gmin)) {
+            const int k = atomicAdd(ncand, 1);
+            sval[k] = d;
+            scand[k] = (unsigned short)(e - tl.begin);
             if (d >= 0.0f) v32 = fminf(v32, d);
         }
     }
     return v32;
+}
+
+// The solve's running FP32 minimum of the CFL screen for the step in progress:
+// the undeformed minimum at first (publish_step), lowered by the tiles.
+__device__ __forceinline__ float running_min(const Problem &p, int parity)
+{
+    return __uint_as_float((unsigned)__ldcg(p.dtmin + 2 + (parity ^ 1)));
 }
 
 constexpr int kMixedPending = 2 * kStepThreads;  // deferred FP64 rechecks a mixed CTA can hold
@@ -2202,10 +2288,7 @@ static __device__ __noinline__ void mixed_flush(const SRC src, const int2 *pend,
         const Tile tl = src.tile(pe.x);
         const Problem &p = src.problem(tl);
         const float mine = pendv[j];
-        if (!(mine < 0.0f)) {
-            const unsigned long long g = __ldcg(p.dtmin + 2 + (parity ^ 1));
-            if (g < kScreenInfBits && mine > __uint_as_float((unsigned)g) * (1.0f + 1.0f / 256.0f)) continue;
-        }
+        if (!(mine < 0.0f) && mine > running_min(p, parity) * (1.0f + 1.0f / 256.0f)) continue;
         double v = INFINITY;
         for (long long e = tl.begin + pe.y + (long long)lane * blockDim.x; e < tl.end; e += 32LL * blockDim.x)
             v = fmin(v, cfl_dw(p, e));
@@ -2216,22 +2299,20 @@ static __device__ __noinline__ void mixed_flush(const SRC src, const int2 *pend,
     }
 }
 
-// The mixed kernel's tile loop.  Each tile's FP32 screen minimum (over the
-// threads that met no sliver) goes to the solve's running minimum (an integer
-// atomicMin on its bit pattern, nothing waited for); a thread whose own
-// minimum lies within 2^-8 of the tile's, or that met a sliver, posts (tile,
-// thread, own minimum) to a per-CTA list.  Once
-// the CTA has run out of tiles, every entry whose minimum is still within
-// 2^-8 of the solve's running minimum -- by then nearly the step's FP32
-// minimum m -- has that thread's elements of that tile recomputed in FP64 by
-// one warp of the CTA.  An element x near the exact minimum has
-// d(x) <= m (1 + 2^-8) <= (tile minimum) (1 + 2^-8) (the tile minimum, taken
-// over part of the elements, is >= m), so its thread posted unless it met a
-// sliver, and then it posted anyway; the entry's minimum is <= d(x) <=
-// (running minimum) (1 + 2^-8), so it is rechecked.  A tile adds at most one
-// entry per thread, so the list is flushed at a tile boundary once it holds
-// more than kMixedPending - blockDim entries, and never overflows; the element
-// loop itself calls no FP64 code.
+// The mixed kernel's tile loop.  A thread whose own screen minimum lies within
+// 2^-8 of the solve's running minimum as its tile began, or that met a sliver,
+// posts (tile, thread, own minimum) to a per-CTA list; a warp that went clearly
+// below lowers the running minimum by an integer atomicMin on its bit pattern
+// (nothing waited for).  Once the CTA has run out of tiles, every entry whose
+// minimum is still within 2^-8 of the running minimum -- by then nearly the
+// step's FP32 minimum m -- has that thread's elements of that tile recomputed
+// in FP64 by one warp of the CTA.  The running minimum g is never below m, and
+// an element x near the exact minimum has d(x) <= m (1 + 2^-8) <= g (1 + 2^-8)
+// whenever g is read, so its thread posted (unless it met a sliver, and then it
+// posted anyway) and its entry, whose minimum is <= d(x), is rechecked.  A tile
+// adds at most one entry per thread, so the list is flushed at a tile boundary
+// once it holds more than kMixedPending - blockDim entries, and never
+// overflows; the element loop itself calls no FP64 code.
 template <bool ACT, bool VISC, typename SRC>
 __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, int parity)
 {
@@ -2246,15 +2327,19 @@ __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, in
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
-            const float mine = tile_elements<MODE_MIXED, ACT, VISC>(p, tl, parity, nullptr);
-            const bool neg = mine < 0.0f;
-            const float bmin = block_min_bcast(neg ? INFINITY : mine);
-            if (threadIdx.x == 0 && bmin < INFINITY)
-                atomicMin(p.dtmin + 2 + (parity ^ 1), (unsigned long long)__float_as_uint(bmin));
-            if (neg || (mine < INFINITY && mine <= bmin * (1.0f + 1.0f / 256.0f))) {
+            const float g = running_min(p, parity), gmin = g * (1.0f + 1.0f / 256.0f);
+            const float mine = tile_elements<MODE_MIXED, ACT, VISC>(p, tl, parity, gmin, nullptr, nullptr, nullptr);
+            if (!(mine > gmin)) {
                 const int k = atomicAdd(&s_npend, 1);   // < kMixedPending: flushed below in time
                 s_pend[k] = make_int2(t, (int)threadIdx.x);
-                s_pendv[k] = neg ? -1.0f : mine;
+                s_pendv[k] = mine;
+            }
+            float w = mine < 0.0f ? INFINITY : mine;
+            if (__any_sync(0xffffffffu, w < g * (1.0f - 1.0f / 1024.0f))) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) w = fminf(w, __shfl_xor_sync(0xffffffffu, w, o));
+                if ((threadIdx.x & 31) == 0)
+                    atomicMin(p.dtmin + 2 + (parity ^ 1), (unsigned long long)__float_as_uint(w));
             }
         }
         t = q.next(claimed, &s_tile);
@@ -2268,22 +2353,24 @@ __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, in
     mixed_flush(src, s_pend, s_pendv, s_npend, parity);   // posted before the loop's last barrier
 }
 
-// Element kernel over tiles.  Each element's FP32 CFL screen value is
-// compared with the solve's running FP32 minimum of the screen (a per-step
-// slot that every tile lowers by an integer atomicMin on its bit pattern):
-// elements within 2^-8 of it, and slivers, recompute the exact FP64 value,
-// whose minimum goes to the solve's CFL slot.  The screen's error stays far
-// below 2^-9 outside slivers, so that set always holds the step's exact
-// minimum.  FP64 and double-word keep the tile's screen values in shared
-// memory, list the candidates and recompute them by consecutive threads; the
-// mixed kernel defers its few rechecks to the end of the CTA's tiles
-// (mixed_tile_loop).  ACT: the instantiation with element birth (single
-// solves whose block has it on), VISC the one with artificial bulk viscosity;
-// the plain one carries no trace of either.
+// Element kernel over tiles.  The solve's running FP32 minimum of the CFL screen
+// (a per-step slot that starts from the undeformed minimum, an upper bound of
+// every step's, and that tiles lower by an integer atomicMin on its bit
+// pattern) decides which elements recompute the exact FP64 value, whose minimum
+// goes to the solve's CFL slot: those within 2^-8 of it, and slivers.  The
+// screen's error stays far below 2^-9 outside slivers, so that set always holds
+// the step's exact minimum.  FP64 and double-word list a tile's candidates in
+// shared memory as they come and recompute those that remain at its end by
+// consecutive threads, so a few candidates take one warp; a tile without any
+// (nearly every tile) closes with one barrier.  The mixed kernel defers its few
+// rechecks to the end of the CTA's tiles (mixed_tile_loop).  ACT: the
+// instantiation with element birth (single solves whose block has it on), VISC
+// the one with artificial bulk viscosity; the plain one carries no trace of
+// either.
 template <int MODE, bool ACT, bool VISC, typename SRC>
 __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int parity)
 {
-    __shared__ float sdt[MODE == MODE_MIXED ? 1 : kMaxTileElems];
+    __shared__ float sval[MODE == MODE_MIXED ? 1 : kMaxTileElems];
     __shared__ unsigned short scand[MODE == MODE_MIXED ? 1 : kMaxTileElems];
     __shared__ int s_tile, s_ncand;
     __shared__ float s_thr;
@@ -2292,58 +2379,38 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
         q.finish();
         return;
     }
+    if (threadIdx.x == 0) s_ncand = 0;
+    __syncthreads();
     int t = q.first(&s_tile);
     while (t < q.n) {
         const int claimed = q.claim();
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
-            if (MODE != MODE_MIXED && threadIdx.x == 0) s_ncand = 0;
-            const float v32 = tile_elements<MODE, ACT, VISC>(p, tl, parity, sdt);
-            const float bmin = block_min_bcast(v32);   // also orders the sdt writes before the reads below
-            if (threadIdx.x == 0) {
-                // g: the solve's smallest FP32 screen value over the tiles closed
-                // so far in this step, this one included.  g >= the step's FP32
-                // minimum m, and the exact minimum's screen value is <= m (1 + 2^-8)
-                // (screen error below 2^-9 outside slivers), so elements above
-                // g (1 + 2^-8) are never the exact minimum: most tiles skip the
-                // FP64 recheck, whichever order they close in.
-                float g = bmin;
-                if (bmin < INFINITY) {
-                    const unsigned long long old =
-                        atomicMin(p.dtmin + 2 + (parity ^ 1), (unsigned long long)__float_as_uint(bmin));
-                    g = old >= kScreenInfBits ? bmin : fminf(__uint_as_float((unsigned)old), bmin);
-                }
-                s_thr = g * (1.0f + 1.0f / 256.0f);
-            }
+            const float v32 = tile_elements<MODE, ACT, VISC>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
+                                                             sval, scand, &s_ncand);
             __syncthreads();
-            const float thr = s_thr;
-            if (MODE == MODE_MIXED) {
-                // a thread reads back only the entries it wrote itself
-                double v = INFINITY;
-                for (long long e = tl.begin + threadIdx.x; e < tl.end; e += blockDim.x) {
-                    const float d = sdt[e - tl.begin];
-                    if (d < 0.0f || d <= thr) v = fmin(v, cfl_dw(p, e));
-                }
-                if (v >= 0.0 && v < INFINITY)
-                    atomicMin(p.dtmin + (parity ^ 1), (unsigned long long)__double_as_longlong(v));
-            } else {
-                // the tile's candidates are listed first and then recomputed by
-                // consecutive threads, so a few candidates take one warp, not several
-                for (long long e = tl.begin + threadIdx.x; e < tl.end; e += blockDim.x) {
-                    float d = sdt[e - tl.begin];
-                    if (d < 0.0f || d <= thr) scand[atomicAdd(&s_ncand, 1)] = (unsigned short)(e - tl.begin);
+            const int nc = s_ncand;
+            if (nc > 0) {   // uniform across the block
+                const float bmin = block_min_bcast(v32);
+                if (threadIdx.x == 0) {
+                    s_ncand = 0;
+                    // g: the smallest screen value any tile has reported so far in this
+                    // step, this one included, or the undeformed minimum
+                    unsigned old = (unsigned)__ldcg(p.dtmin + 2 + (parity ^ 1));
+                    if (bmin < __uint_as_float(old))
+                        old = (unsigned)atomicMin(p.dtmin + 2 + (parity ^ 1), (unsigned long long)__float_as_uint(bmin));
+                    s_thr = fminf(__uint_as_float(old), bmin) * (1.0f + 1.0f / 256.0f);
                 }
                 __syncthreads();
-                const int nc = s_ncand;
-                if (nc > 0) {   // uniform across the block
-                    double v = INFINITY;
-                    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-                        const long long e = tl.begin + scand[c];
-                        v = fmin(v, MODE == MODE_DW ? cfl_dw(p, e) : cfl_fp64(p, e));
-                    }
-                    block_min_to(v, p.dtmin + (parity ^ 1));
+                const float thr = s_thr;
+                double v = INFINITY;
+                for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+                    if (sval[c] > thr) continue;
+                    const long long e = tl.begin + scand[c];
+                    v = fmin(v, MODE == MODE_DW ? cfl_dw(p, e) : cfl_fp64(p, e));
                 }
+                block_min_to(v, p.dtmin + (parity ^ 1));
             }
         }
         t = q.next(claimed, &s_tile);

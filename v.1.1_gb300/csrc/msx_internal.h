@@ -162,9 +162,10 @@ struct Problem {
     float visc_hf, visc_c1sq_hf, visc_clc0f;   // h, c1^2 h and cl c0 in FP32 (mixed mode)
     // control
     Ctrl *ctrl;                       // [2]
-    unsigned long long *dtmin;        // [4]: [0..1] bit patterns of positive doubles (the CFL
+    unsigned long long *dtmin;        // [5]: [0..1] bit patterns of positive doubles (the CFL
                                       // minimum by step parity); [2..3] FP32 bit patterns of the
-                                      // running minimum of the elements' FP32 CFL screen
+                                      // running minimum of the elements' FP32 CFL screen; [4] the
+                                      // undeformed minimum as FP32, rounded up, where [2..3] start
     int *flags;                       // [2] NaN flag raised by the element kernel
     double sf, tf;
 };

@@ -43,6 +43,7 @@ __global__ void init_block_kernel(Problem p, double t0, long long limit)
 {
     // solverExplicit.cpp:165-166: initial dt from the undeformed lengths
     double dt0 = __longlong_as_double((long long)p.dtmin[0]);
+    p.dtmin[4] = __float_as_uint(__double2float_ru(dt0));
     dt0 = dt0 * p.sf;
     Ctrl c;
     c.t = t0;
@@ -599,8 +600,8 @@ static msx_status init_block(msx_handle *h)
     msx_status tst = plan_tiled(h);
     if (tst != MSX_OK) return tst;
     const Problem &P = h->P;
-    // CFL minima (double bits) and the screen's running minima (FP32 bits)
-    unsigned long long inf[4] = {0x7FF0000000000000ULL, 0x7FF0000000000000ULL, 0x7F800000ULL, 0x7F800000ULL};
+    // CFL minima (double bits); the screen's minima follow from the undeformed one (init_block_kernel)
+    unsigned long long inf[2] = {0x7FF0000000000000ULL, 0x7FF0000000000000ULL};
     MSX_CUDA(cudaMemcpyAsync(h->dtmin.p, inf, sizeof(inf), cudaMemcpyHostToDevice, h->stream));
     launch_initial_cfl(P, nullptr, 0, h->stream);
     if (h->t0 < 1E-12 && !h->u_zero) {
@@ -833,7 +834,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
     ALLOC(h->node_ptr, nn + 1);
     ALLOC(h->node_inc, 4 * ne);
     ALLOC(h->ctrl, 2);
-    ALLOC(h->dtmin, 4);
+    ALLOC(h->dtmin, 5);
     ALLOC(h->flags, 2);
     if (mesh->elem_material && num_mats > 1) ALLOC(h->mat, ne);
 #undef ALLOC
