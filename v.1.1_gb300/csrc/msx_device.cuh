@@ -1234,12 +1234,18 @@ template <bool FORCE_ONLY, bool ACT, bool VISC>
 __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
                                                     const MatParams &m, const int *nd, float gmin);
 
-// The cofactor form's corner forces of one element that fixed point leaves out.
-static __device__ __noinline__ void elem_cnh_general(const Problem &p, long long e, int parity)
+// The cofactor form for an element that fixed point leaves out.
+static __device__ __noinline__ float elem_cnh_general(const Problem &p, long long e, int parity, float gmin)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    elem_cofactor_fp64<true, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, 0.0f);
+    return elem_cofactor_fp64<false, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, gmin);
+}
+
+// 2^k in FP32, infinite outside its normal range
+__device__ __forceinline__ float pow2f_or_inf(int k)
+{
+    return k >= -126 && k <= 127 ? __int_as_float((k + 127) << 23) : INFINITY;
 }
 
 // x 2^k for an integer x: the exponent is added to the converted integer's
@@ -1252,11 +1258,12 @@ __device__ __forceinline__ double fixed_to_double(long long x, int k)
 }
 
 // Plain FP64 mode, compressible neo-Hookean: the deformed edges
-// e_b = E_b + (u_b - u_0) in FP64, the corner forces from them in 64-bit fixed
-// point (msx_fixed.cuh), rounded to FP64 at the end.  FP64 arithmetic is left
-// with the 24 additions of the edges and of f_0 and nine conversions, against
-// 115 operations of the same formulas in FP64.  The CFL screen takes the deformed
-// edges directly (truncated to FP32).
+// e_b = E_b + (u_b - u_0) and the corner forces from them in 64-bit fixed point
+// (msx_fixed.cuh), rounded to FP64 at the end; nine conversions and the six
+// additions of f_0 are left to the FP64 pipe, against 115 operations of the same
+// formulas in FP64.
+// Per warp of 32 elements on the 6M-tet cube (ncu): 115 FP64 instructions and
+// 1020 others took 1.290 ms, FP64 pipe 86 % busy.
 __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
                                                     const int *nd, float gmin)
 {
@@ -1276,44 +1283,36 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 #pragma unroll
             for (int i = 0; i < 3; i++) ua[a][i] = p.u[nd[a] + i * nn];
     }
-    double du[9], ed[9];   // ed[(b-1)*3 + i]: component i of the deformed edge e_b
+    const uint2 w = __ldg(p.fxw + e);
+    if (w.x == 0) return elem_cnh_general(p, e, parity, gmin);
+    FixedElem q;
+    fixed_unpack(w.x, w.y, q);
 #pragma unroll
-    for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            du[b * 3 + i] = ua[b + 1][i] - ua[0][i];
-            ed[b * 3 + i] = __ldg(p.Eref + (b * 3 + i) * ne + e) + du[b * 3 + i];
-        }
+    for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
+    Limbs n[9];
+    int moved;
+    if (!fixed_edges(q, ua, n, moved)) return elem_cnh_general(p, e, parity, gmin);
     float scr = INFINITY;
-    if (!(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound<9>(du), m.inv_c_f) > gmin)) {
+    if (!(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(fixed_lw_min(q) + 32)), m.inv_c_f) > gmin)) {
         float e32[9];
 #pragma unroll
-        for (int k = 0; k < 9; k++) e32[k] = f32_trunc(ed[k]);
+        for (int k = 0; k < 9; k++) e32[k] = (float)n[k].h * pow2f_or_inf(q.lw[k / 3] + 29);
         scr = cfl_screen_edges(p, e, e32, e32 + 3, e32 + 6, m);
     }
+    const longlong2 dd = __ldg(p.fxD + e);
+    q.d0 = dd.x;
+    q.rd = dd.y;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const int2 x = __ldg(p.fxS + k * ne + e);
+        q.S[k] = {x.x, x.y};
+    }
+    int64_t f[9];
+    if (!fixed_forces(q, n, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f))
+        return elem_cnh_general(p, e, parity, gmin);
     if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
     const int4 sl = __ldg(p.slot + e);
     const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
-    const uint2 w = __ldg(p.fxw + e);
-    FixedElem q;
-    int64_t f[9];
-    bool ok = w.x != 0;
-    if (ok) {
-        fixed_unpack(w.x, w.y, q);
-        const longlong2 d = __ldg(p.fxD + e);
-        q.d0 = d.x;
-        q.rd = d.y;
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            const int2 x = __ldg(p.fxS + k * ne + e);
-            q.S[k] = {x.x, x.y};
-        }
-        ok = fixed_forces(q, ed, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f);
-    }
-    if (!ok) {
-        elem_cnh_general(p, e, parity);
-        return scr;
-    }
     double fa[3][3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
@@ -1407,14 +1406,14 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
     return scr;
 }
 
-template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
+template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, bool CNH = false>
 __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
                                                 double idt = 0.0, float gmin = 0.0f)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
-    if (!FORCE_ONLY && !VISC && p.Eref && m.law == 1) return elem_body_fp64_cnh(p, e, parity, m, nd, gmin);   // never dead
+    if (CNH || (!FORCE_ONLY && !VISC && p.fxE && m.law == 1)) return elem_body_fp64_cnh(p, e, parity, m, nd, gmin);   // never dead
     return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
 }
 
@@ -2235,7 +2234,7 @@ __global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_c
 // so their node gathers wait for one memory latency instead of two
 // (connectivity, then the nodes).  ACT: element birth is on, and the step's time
 // decides which elements are dead.
-template <int MODE, bool ACT, bool VISC>
+template <int MODE, bool ACT, bool VISC, bool CNH = false>
 __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
                                                unsigned short *scand, int *ncand)
 {
@@ -2253,7 +2252,7 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
         if ((MODE == MODE_MIXED || MODE == MODE_DW) && e + blockDim.x < tl.end) cn_next = p.conn[e + blockDim.x];
         float d = MODE == MODE_MIXED ? elem_body_mixed<false, ACT, VISC>(p, e, parity, cn, t, idtf, gmin)
                                      : (MODE == MODE_DW ? elem_body_dw<false, ACT, VISC>(p, e, parity, cn, t, idt, gmin)
-                                                        : elem_body_fp64<false, ACT, VISC>(p, e, parity, t, idt, gmin));
+                                                        : elem_body_fp64<false, ACT, VISC, CNH>(p, e, parity, t, idt, gmin));
         if (MODE == MODE_MIXED) {
             v32 = d < 0.0f ? -1.0f : fminf(v32, d);   // -1 sticks: fminf(-1, d) = -1 for d >= 0
         } else if (!(d > gmin)) {
@@ -2367,7 +2366,7 @@ __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, in
 // instantiation with element birth (single solves whose block has it on), VISC
 // the one with artificial bulk viscosity; the plain one carries no trace of
 // either.
-template <int MODE, bool ACT, bool VISC, typename SRC>
+template <int MODE, bool ACT, bool VISC, bool CNH = false, typename SRC>
 __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int parity)
 {
     __shared__ float sval[MODE == MODE_MIXED ? 1 : kMaxTileElems];
@@ -2387,7 +2386,7 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
-            const float v32 = tile_elements<MODE, ACT, VISC>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
+            const float v32 = tile_elements<MODE, ACT, VISC, CNH>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
                                                              sval, scand, &s_ncand);
             __syncthreads();
             const int nc = s_ncand;
@@ -2436,6 +2435,16 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 
+// One solve in FP64 whose every material is compressible neo-Hookean
+#ifndef CNHB
+#define CNHB 2
+#endif
+static __global__ void __launch_bounds__(kStepThreads, CNHB)
+    solve_elem_cnh_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
+{
+    elem_tile_loop<MODE_FP64, false, false, true>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+}
+
 // ---------------------------------------------------------------------------
 // Set-up kernels (reference operation order), built in the exact unit only
 // ---------------------------------------------------------------------------
@@ -2473,23 +2482,22 @@ __device__ __forceinline__ void ref_jacobian(const double *xyz, double *Jac)
 }
 
 // The plain FP64 mode's compressible neo-Hookean element data of element e
-// (Problem::Eref, fxS, fxD, fxw) from its corner coordinates pts[k*3 + i].
+// (Problem::fxE, fxS, fxD, fxw) from its corner coordinates pts[k*3 + i].
 __device__ __forceinline__ void write_cnh_arrays(const Problem &p, long long e, const double *pts)
 {
     const long long ne = p.ne;
-    double *Er = const_cast<double *>(p.Eref), E[9];
+    double E[9];
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            E[b * 3 + i] = pts[(b + 1) * 3 + i] - pts[i];
-            Er[(b * 3 + i) * ne + e] = E[b * 3 + i];
-        }
+        for (int i = 0; i < 3; i++) E[b * 3 + i] = pts[(b + 1) * 3 + i] - pts[i];
     const MatParams &m = mat_of(p, e);
     FixedElem q;
     uint32_t w[2] = {0, 0};
     if (m.law == 1 && fixed_setup(E, m.kq[0], m.ks, q)) {
         fixed_pack(q, w);
+#pragma unroll
+        for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = q.E[k];
 #pragma unroll
         for (int k = 0; k < 6; k++) const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2(q.S[k].h, q.S[k].l);
         const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(q.d0, q.rd);
@@ -2538,7 +2546,7 @@ __global__ void setup_elements_kernel(Problem p, const double *X, double *G, dou
     double v6;   // 6V, signed: the edge determinant of the inscribed-sphere volume
     double L = char_length_ref(pts, &v6);
     Lref[e] = L;
-    if (p.Eref) write_cnh_arrays(p, e, pts);
+    if (p.fxE) write_cnh_arrays(p, e, pts);
     // A reference sliver (6V below 0.063 |e1||e2||e3|) gets a negative FP32
     // length: the FP32 CFL screens then always recompute it in FP64 (the mixed
     // screen rebuilds the reference edges from G in FP32, which loses accuracy
@@ -2578,7 +2586,7 @@ __global__ void mode_arrays_kernel(Problem p, float *G32, float *wJ32, float *G3
     if (wJ32lo) wJ32lo[e] = (float)(w - (double)(float)w);
 }
 
-// Problem::Eref, fxS, fxD and fxw of a handle whose FP64 block starts after its
+// Problem::fxE, fxS, fxD and fxw of a handle whose FP64 block starts after its
 // set-up: what setup_elements_kernel writes, from X.
 __global__ void cnh_arrays_kernel(Problem p)
 {

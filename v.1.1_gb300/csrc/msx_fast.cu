@@ -64,6 +64,8 @@ static void launch_elem_variant(const Problem &p, const SolveSched &q, int *coun
     // element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
     if (p.act_t)
         solve_elem_kernel<MODE, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
+    else if (MODE == MODE_FP64 && q.cnh)
+        solve_elem_cnh_kernel<<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
     else if (p.visc)
         solve_elem_kernel<MODE, false, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
     else
@@ -186,7 +188,7 @@ void launch_abs_range(const double *x, long long n, unsigned long long *mm, cuda
     abs_range_kernel<<<256, 256, 0, s>>>(x, n, mm);
 }
 
-int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool)
+int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, bool cnh)
 {
     const void *f[3][2][2] = {
         {{(const void *)solve_elem_kernel<MODE_FP64>, (const void *)pool_elem_kernel<MODE_FP64>},
@@ -196,6 +198,7 @@ int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool)
         {{(const void *)solve_elem_kernel<MODE_DW>, (const void *)pool_elem_kernel<MODE_DW>},
          {(const void *)solve_node_kernel<MODE_DW>, (const void *)pool_node_kernel<MODE_DW>}}};
     int a = 0;
+    if (cnh) f[0][0][0] = (const void *)solve_elem_cnh_kernel;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f[mode == MODE_MIXED ? 1 : (mode == MODE_DW ? 2 : 0)][node][pool],
                                                   threads, 0);
     return a > 0 ? a : 1;

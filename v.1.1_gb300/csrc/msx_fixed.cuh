@@ -58,11 +58,22 @@ MSX_HD Limbs limbs(int64_t x)
 MSX_HD Limbs limbs_neg(Limbs a) { return {-a.h, -a.l}; }
 
 // a b = hh 2^58 + mid 2^29 + a.l b.l, summed without the last
+MSX_HD int64_t mad_wide(int32_t a, int32_t b, int64_t c)
+{
+#ifdef __CUDA_ARCH__
+    int64_t r;   // spelled out: from C the compiler splits many of these into a product and an addition
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+#else
+    return (int64_t)a * b + c;
+#endif
+}
+
 MSX_HD void mac(int64_t &hh, int64_t &mid, Limbs a, Limbs b)
 {
-    hh += (int64_t)a.h * b.h;
-    mid += (int64_t)a.h * b.l;
-    mid += (int64_t)a.l * b.h;
+    hh = mad_wide(a.h, b.h, hh);
+    mid = mad_wide(a.h, b.l, mid);
+    mid = mad_wide(a.l, b.h, mid);
 }
 
 // hh 2^58 + mid 2^29 in units of 2^(58 - k), rounded to nearest when mid began
@@ -77,6 +88,14 @@ MSX_HD int64_t mulhi64(int64_t a, int64_t b)
 #else
     return (int64_t)(((__int128)a * b) >> 64);
 #endif
+}
+
+// a b 2^-64 to two units, for the series (a = h 2^32 + 2 l with l >= 0, h = a >> 32)
+MSX_HD int64_t mulhi_near(int32_t h, int32_t l, int64_t b)
+{
+    const int32_t bh = (int32_t)(b >> 32), bl = (int32_t)((uint32_t)b >> 1);
+    const int64_t t = mad_wide(l, bh, mad_wide(h, bl, 0));
+    return mad_wide(h, bh, t >> 31);
 }
 
 MSX_HD int top_bit(int64_t x)   // floor(log2 x), x > 0
@@ -119,16 +138,16 @@ MSX_HD uint64_t shr64(uint64_t x, int s)   // zero for s < 0 and s > 63
 #endif
 }
 
-// A double, given as its words, in units of 2^lw, truncated toward zero.  room
-// becomes negative for |x| >= 2^58 2^lw, infinities and NaN, else stays.
-MSX_HD int64_t fixed_from(uint32_t hi, uint32_t lo, int lw, int &room)
+// The fixed-point value of x in units of 2^lw, truncated toward zero: |x| < 2^62
+// 2^lw.
+MSX_HD int64_t fixed_from(double x, int lw)
 {
+    const uint64_t v = double_bits(x);
+    const uint32_t hi = (uint32_t)(v >> 32);
     const int ex = (int)((hi >> 20) & 0x7FFu);
-    const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 5;   // below 2^58
-    const int s = lw + (1075 + 5) - ex;
-    room = room < s ? room : s;
+    const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | (uint32_t)v) << 9;   // below 2^62
     const int64_t sg = (int64_t)((int32_t)hi >> 31);
-    return ((int64_t)shr64(m, s) ^ sg) - sg;
+    return ((int64_t)shr64(m, lw + (1075 + 9) - ex) ^ sg) - sg;
 }
 
 // c = n_a x n_b in units of 2^57
@@ -153,10 +172,12 @@ MSX_HD int64_t fixed_det(const Limbs *n1, const Limbs *cr)
     return mac_sum(hh, mid, 1);
 }
 
-// The element's static data beside its reference edges: S_ab w_a w_b 2^t (in the
-// order 11 12 13 22 23 33), det E as fixed_det gives it, 2^(62 + ds) / det E
-// for ds = floor(log2 det E), and exponents.
+// The element's static data: the reference edges E_b in units of the smallest
+// w (with half a unit of w_b added, so that the shift to w_b rounds to nearest);
+// S_ab w_a w_b 2^t (in the order 11 12 13 22 23 33); det E as fixed_det gives
+// it; 2^(62 + ds) / det E for ds = floor(log2 det E); exponents.
 struct FixedElem {
+    int64_t E[9];
     Limbs S[6];
     int64_t d0, rd;
     int32_t lw[3];   // log2 w_b
@@ -164,6 +185,12 @@ struct FixedElem {
     int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t)
     int32_t ds;
 };
+
+MSX_HD int fixed_lw_min(const FixedElem &q)
+{
+    const int a = q.lw[0] < q.lw[1] ? q.lw[0] : q.lw[1];
+    return a < q.lw[2] ? a : q.lw[2];
+}
 
 // The exponents as two words in device memory.  A zero first word (ds is at
 // least 40) sends the element to FP64.
@@ -183,23 +210,73 @@ MSX_HD void fixed_unpack(uint32_t w0, uint32_t w1, FixedElem &q)
     q.x0 = (int)(w1 >> 14) - 4096;
 }
 
-// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of
-// 2^(x0 - lw_a); false when the element leaves the sizes above.  e: the deformed
-// edges' nine components; kq: c2's series.  scalar(J) gives -c2 in kq's units
-// for |1 - J| >= 2^-4, in FP64.  f_0 = -(f_1 + f_2 + f_3) is left to the caller,
-// in FP64: its rounding to nearest has no preferred sign (a sum of shifted
-// integers has, and pushes the whole body).
-template <typename SCALAR>
-MSX_HD bool fixed_forces(const FixedElem &q, const double *e, const int64_t *kq, SCALAR scalar, int64_t *f)
+// The deformed edges n_b = (E_b + u_b - u_0) / w_b in limbs, exact up to the
+// final rounding and the bits of u below the smallest w; false for a component
+// beyond 2^58, infinities and NaN.  Displacements beyond 2^62 of the smallest w
+// (32 edge lengths at least) are taken in a unit 2^k times larger, whose lost
+// bits lie 2^-9 below u's own last one.  moved: an upper bound of
+// max |u_b - u_0| component by component, in units of 2^32 of the smallest w.
+MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int &moved)
 {
-    int room = 63;
-    Limbs n[9];
+    const int lw = fixed_lw_min(q);
+    int emax = 0;
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-        const uint64_t b = double_bits(e[k]);
-        n[k] = limbs(fixed_from((uint32_t)(b >> 32), (uint32_t)b, q.lw[k / 3], room));
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int ex = (int)((double_bits(u[a][i]) >> 52) & 0x7FF);
+            emax = emax > ex ? emax : ex;
+        }
+    int k = emax - (lw + 1075 + 9);   // 2^k 2^lw is the unit of u
+    k = k > 0 ? k : 0;
+    if (k > 40) return false;
+    int64_t U[4][3];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) U[a][i] = fixed_from(u[a][i], lw + k);
+    if (k > 0) {   // back to units of 2^lw, as differences (the common part of a far motion is gone)
+        bool far = false;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+#pragma unroll
+            for (int b = 1; b < 4; b++) {
+                const int64_t d = U[b][i] - U[0][i];
+                far = far || d >= (1LL << (60 - k)) || d <= -(1LL << (60 - k));
+                U[b][i] = (int64_t)((uint64_t)d << k);
+            }
+            U[0][i] = 0;
+        }
+        if (far) return false;
     }
-    if (room < 0) return false;
+    uint32_t out = 0;
+    int m = 0;
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int d = q.lw[b] - lw;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int64_t du = U[b + 1][i] - U[0][i];
+            const int dh = (int)(du >> 32);
+            const int da = dh ^ (dh >> 31);
+            m = m > da ? m : da;
+            n[3 * b + i] = limbs((q.E[3 * b + i] + du) >> d);
+            out |= (uint32_t)(n[3 * b + i].h + (1 << 29));
+        }
+    }
+    moved = m + 1;
+    return out < (1u << 30);
+}
+
+// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of
+// 2^(x0 - lw_a); false when the element leaves the sizes above.  n: the deformed
+// edges (fixed_edges); kq: c2's series.  scalar(J) gives -c2 in kq's units for
+// |1 - J| >= 2^-4, in FP64.  f_0 = -(f_1 + f_2 + f_3) is left to the caller, in
+// FP64: its rounding to nearest has no preferred sign (a sum of shifted integers
+// has, and pushes the whole body).
+template <typename SCALAR>
+MSX_HD bool fixed_forces(const FixedElem &q, const Limbs *n, const int64_t *kq, SCALAR scalar, int64_t *f)
+{
     Limbs cr[9];   // cr_1 = n_2 x n_3, cr_2 = n_3 x n_1, cr_3 = n_1 x n_2
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -212,14 +289,16 @@ MSX_HD bool fixed_forces(const FixedElem &q, const double *e, const int64_t *kq,
     const int64_t y = q.d0 - D;   // d0 (1 - J)
     int64_t c2;
     if (y < (q.d0 >> 4) && y > -(q.d0 >> 4)) {
-        const int64_t yq = mulhi64((int64_t)((uint64_t)y << (66 - q.ds)), q.rd);   // (1 - J) 2^64
+        const int64_t ys = (int64_t)((uint64_t)y << (66 - q.ds));
+        const int64_t yq = mulhi_near((int32_t)(ys >> 32), (int32_t)((uint32_t)ys >> 1), q.rd);   // (1 - J) 2^64
+        const int32_t yh = (int32_t)(yq >> 32), yl = (int32_t)((uint32_t)yq >> 1);
         const bool near1 = yq < (1LL << 57) && yq > -(1LL << 57);
         c2 = near1 ? kq[kFixShort - 1] : kq[kFixTerms - 1];
         if (!near1)
 #pragma unroll
-            for (int k = kFixTerms - 2; k >= kFixShort - 1; k--) c2 = kq[k] + mulhi64(yq, c2);
+            for (int k = kFixTerms - 2; k >= kFixShort - 1; k--) c2 = kq[k] + mulhi_near(yh, yl, c2);
 #pragma unroll
-        for (int k = kFixShort - 2; k >= 0; k--) c2 = kq[k] + mulhi64(yq, c2);
+        for (int k = kFixShort - 2; k >= 0; k--) c2 = kq[k] + mulhi_near(yh, yl, c2);
     } else {
         c2 = scalar(1.0 - (double)y / (double)q.d0);
     }
@@ -253,7 +332,7 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
 {
     Limbs n[9], cl[9];
     int64_t c[9], v[6], vm = 0;
-    int room = 63, sum = 0;
+    int sum = 0;
     double vol = kFixFlat * kFixFlat;
     for (int b = 0; b < 3; b++) {
         const double l2 = E[3 * b] * E[3 * b] + E[3 * b + 1] * E[3 * b + 1] + E[3 * b + 2] * E[3 * b + 2];
@@ -262,13 +341,16 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
         q.lw[b] = (ex2 >> 1) + 1 - 57;   // floor(log2 |E_b|) + 1 - 57
         sum += q.lw[b];
         vol *= l2 * pow2_double(-2 * q.lw[b]);
-        for (int i = 0; i < 3; i++) {
-            const uint64_t w = double_bits(E[3 * b + i]);
-            n[3 * b + i] = limbs(fixed_from((uint32_t)(w >> 32), (uint32_t)w, q.lw[b], room));
-        }
     }
     const int d1 = q.lw[1] - q.lw[0], d2 = q.lw[2] - q.lw[0];
-    if (d1 < -20 || d1 > 20 || d2 < -20 || d2 > 20) return false;
+    if (d1 < -4 || d1 > 4 || d2 < -4 || d2 > 4 || d2 - d1 < -4 || d2 - d1 > 4) return false;   // E fits 2^61 of the smallest w
+    const int lw = fixed_lw_min(q);
+    for (int b = 0; b < 3; b++)
+        for (int i = 0; i < 3; i++) {
+            const int d = q.lw[b] - lw;
+            q.E[3 * b + i] = fixed_from(E[3 * b + i], lw) + (d ? 1LL << (d - 1) : 0);
+            n[3 * b + i] = limbs(q.E[3 * b + i] >> d);
+        }
     for (int a = 0; a < 3; a++) {
         fixed_cross(n + 3 * ((a + 1) % 3), n + 3 * ((a + 2) % 3), c + 3 * a);
         for (int i = 0; i < 3; i++) cl[3 * a + i] = limbs(c[3 * a + i]);

@@ -104,12 +104,12 @@ struct Problem {
     // kernel gathers a node with two loads of one sector instead of three
     // 8-byte loads from three rows.  Null in the other modes.
     double *u4;
-    // plain FP64 mode, compressible neo-Hookean elements: the reference edges
-    // X_b - X_0 (9*ne: Eref[(3(b-1) + i)*ne + e], b = 1..3) and the fixed-point
-    // data of msx_fixed.cuh: S's limbs (6*ne: fxS[k*ne + e]), (d0, rd) and the
-    // packed exponents (a zero word: the element takes the FP64 cofactor form).
-    // Null in the other modes.
-    const double *Eref;
+    // plain FP64 mode, compressible neo-Hookean elements: the fixed-point data of
+    // msx_fixed.cuh: the reference edges (9*ne: fxE[(3(b-1) + i)*ne + e],
+    // b = 1..3), S's limbs (6*ne: fxS[k*ne + e]), (d0, rd) and the packed
+    // exponents (a zero word: the element takes the FP64 cofactor form).  Null in
+    // the other modes.
+    const long long *fxE;
     const int2 *fxS;
     const longlong2 *fxD;
     const uint2 *fxw;
@@ -196,11 +196,12 @@ void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, in
 struct SolveSched {
     int threads = kStepThreads;
     int elem_tile = 0, node_tile = 0, elem_grid = 0, node_grid = 0;
+    int cnh = 0;   // plain FP64, every material compressible neo-Hookean, no viscosity
 };
 void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 // CTAs of a tiled element kernel (node kernel when `node` is true) that fit on one SM
-int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false);
+int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, bool cnh = false);
 // Mixed-mode state conversions: u, v, a (FP64) -> uhl, vhl, ahl, and back
 // (hi + lo, exact unless the pair spans more than 53 bits); minv -> minv2.
 void launch_state_split(const Problem &p, bool mixed, cudaStream_t s);
@@ -222,7 +223,7 @@ void launch_setup_elements(const Problem &p, const double *X, cudaStream_t s, lo
 void launch_setup_mass(const Problem &p, double *mass, double *minv, cudaStream_t s);
 // a precision mode's FP32 element arrays (any pointer may be null) from G, wJ and X
 void launch_mode_arrays(const Problem &p, float *G32, float *wJ32, float *G32lo, float *wJ32lo, cudaStream_t s);
-// Problem::Eref, fxS, fxD and fxw from X (the same values the set-up writes)
+// Problem::fxE, fxS, fxD and fxw from X (the same values the set-up writes)
 void launch_cnh_arrays(const Problem &p, cudaStream_t s);
 // bulk viscosity: the elements' previous-step F diagonal from displacement u
 void launch_visc_init(const Problem &p, const double *u, cudaStream_t s);

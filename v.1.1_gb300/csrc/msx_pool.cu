@@ -160,7 +160,7 @@ static bool pair_state(int precision) { return precision == MSX_PREC_MIXED || pr
 static size_t footprint(long long nn, long long ne, long long nbc, int precision, bool cnh)
 {
     size_t b = 0;
-    if (cnh)   // plain FP64, compressible neo-Hookean: Eref, fxS, fxD, fxw
+    if (cnh)   // plain FP64, compressible neo-Hookean: fxE, fxS, fxD, fxw
         b += align256(sizeof(double) * 9 * ne) + align256(sizeof(int2) * 6 * ne) + align256(sizeof(longlong2) * ne) +
              align256(sizeof(uint2) * ne);
     b += align256(sizeof(int4) * ne) + align256(sizeof(double) * 9 * ne);           // conn, G
@@ -652,7 +652,7 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         P.uhl = (float2 *)carve(sizeof(float2) * 3 * nn);
         if (prec == MSX_PREC_FP64) P.u4 = (double *)carve(sizeof(double) * 4 * nn);
         if (cnh) {   // written by the element set-up, as for a single solve
-            P.Eref = (double *)carve(sizeof(double) * 9 * ne);
+            P.fxE = (long long *)carve(sizeof(long long) * 9 * ne);
             P.fxS = (int2 *)carve(sizeof(int2) * 6 * ne);
             P.fxD = (longlong2 *)carve(sizeof(longlong2) * ne);
             P.fxw = (uint2 *)carve(sizeof(uint2) * ne);

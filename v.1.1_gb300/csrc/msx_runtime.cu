@@ -102,9 +102,8 @@ struct msx_handle {
     DBuf<float> G32, wJ32, Lref32, fe32, G32lo, wJ32lo;
     DBuf<float2> uhl, vhl, ahl, minv2;
     DBuf<double> u4;   // plain FP64 mode: node-major copy of u (Problem::u4)
-    // plain FP64 mode with a compressible neo-Hookean material: reference
-    // edges and fixed-point data (Problem::Eref, fxS, fxD, fxw)
-    DBuf<double> Eref;
+    // plain FP64 mode with a compressible neo-Hookean material: fixed-point data (Problem::fxE, fxS, fxD, fxw)
+    DBuf<long long> fxE;
     DBuf<int2> fxS;
     DBuf<longlong2> fxD;
     DBuf<uint2> fxw;
@@ -307,10 +306,10 @@ static void bind_problem(msx_handle *h)
     P.minv = h->minv.p;
     P.uhl = h->uhl.p;
     P.u4 = h->precision == MSX_PREC_FP64 ? h->u4.p : nullptr;
-    P.Eref = h->precision == MSX_PREC_FP64 ? h->Eref.p : nullptr;
-    P.fxS = P.Eref ? h->fxS.p : nullptr;
-    P.fxD = P.Eref ? h->fxD.p : nullptr;
-    P.fxw = P.Eref ? h->fxw.p : nullptr;
+    P.fxE = h->precision == MSX_PREC_FP64 ? h->fxE.p : nullptr;
+    P.fxS = P.fxE ? h->fxS.p : nullptr;
+    P.fxD = P.fxE ? h->fxD.p : nullptr;
+    P.fxw = P.fxE ? h->fxw.p : nullptr;
     P.vhl = h->vhl.p;
     P.ahl = h->ahl.p;
     P.minv2 = h->minv2.p;
@@ -393,7 +392,9 @@ static msx_status plan_tiled(msx_handle *h)
     // CTAs of 128 threads while one warp per scheduler holds the whole mesh
     // (sms * 128 elements): the elements then spread over all SMs.  256 above.
     q.threads = h->P.ne <= 128LL * sms ? 128 : kStepThreads;
-    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads);
+    q.cnh = h->P.fxE && !h->P.visc && !h->P.act_t;
+    for (int k = 0; k < h->P.nmat; k++) q.cnh = q.cnh && h->P.mats[k].law == 1;
+    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, false, false, q.cnh);
     q.node_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true);
     // Element tiles of P whole CTA passes (P * threads elements).  Spread over
     // the grid, the busiest CTA runs ceil(tiles / grid) tiles; P minimises that
@@ -518,8 +519,8 @@ static msx_status mode_buffers(msx_handle *h, int precision, bool fill, cudaStre
     }
     if (precision == MSX_PREC_FP64 && !h->u4.p) MSX_CUDA(h->u4.alloc(4 * nn));   // filled at each block start
     bool cnh = false;
-    if (precision == MSX_PREC_FP64 && has_cnh(h) && !h->Eref.p) {
-        MSX_CUDA(h->Eref.alloc(9 * ne));
+    if (precision == MSX_PREC_FP64 && has_cnh(h) && !h->fxE.p) {
+        MSX_CUDA(h->fxE.alloc(9 * ne));
         MSX_CUDA(h->fxS.alloc(6 * ne));
         MSX_CUDA(h->fxD.alloc(ne));
         MSX_CUDA(h->fxw.alloc(ne));
@@ -807,7 +808,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
                     ALLOC(h->wJ32lo, ne);
                 }
                 if (h->precision == MSX_PREC_FP64 && has_cnh(h)) {
-                    ALLOC(h->Eref, 9 * ne);
+                    ALLOC(h->fxE, 9 * ne);
                     ALLOC(h->fxS, 6 * ne);
                     ALLOC(h->fxD, ne);
                     ALLOC(h->fxw, ne);
@@ -819,7 +820,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
             // the fixed-point data need the materials: with several, they follow the
             // material ids' upload
             Problem P = h->P;
-            if (mesh->elem_material && num_mats > 1) P.Eref = nullptr;
+            if (mesh->elem_material && num_mats > 1) P.fxE = nullptr;
             launch_setup_elements(P, h->X.p, s, e0, e1);
         }
     }
@@ -869,7 +870,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
 #undef UP
     if (cudaEventRecord(side.lists, side.s) != cudaSuccess || cudaStreamWaitEvent(s, side.lists, 0) != cudaSuccess)
         return bail(fail(MSX_ERR_CUDA, "stream ordering failed"));
-    if (h->P.mat && h->P.Eref) launch_cnh_arrays(h->P, s);
+    if (h->P.mat && h->P.fxE) launch_cnh_arrays(h->P, s);
     launch_setup_mass(h->P, h->mass.p, h->minv.p, s);
     if (h->minv2.p) launch_minv_split(h->minv.p, h->minv2.p, nn, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
@@ -891,7 +892,7 @@ extern "C" msx_status msx_destroy(msx_handle *h)
     for (auto *b : {&h->G32, &h->wJ32, &h->Lref32, &h->fe32, &h->G32lo, &h->wJ32lo}) b->release();
     for (auto *b : {&h->uhl, &h->vhl, &h->ahl, &h->minv2}) b->release();
     h->u4.release();
-    h->Eref.release();
+    h->fxE.release();
     h->fxS.release();
     h->fxD.release();
     h->fxw.release();
