@@ -1408,9 +1408,9 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
 
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, bool CNH = false>
 __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
-                                                double idt = 0.0, float gmin = 0.0f)
+                                                double idt = 0.0, float gmin = 0.0f, int4 cn_ahead = make_int4(0, 0, 0, 0))
 {
-    const int4 cn = p.conn[e];
+    const int4 cn = CNH ? cn_ahead : p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
     if (CNH || (!FORCE_ONLY && !VISC && p.fxE && m.law == 1)) return elem_body_fp64_cnh(p, e, parity, m, nd, gmin);   // never dead
@@ -2223,6 +2223,30 @@ __global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_c
     node_tile_loop<MODE>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
 }
 
+// The compressible neo-Hookean FP64 kernel's streamed element data of the pass
+// of blockDim elements that begins at b, into L2: one or two lines a thread
+// instead of a DRAM latency before the next pass's arithmetic (6M tets: element
+// kernel 0.497 -> 0.476 ms; 0.473 -> 0.448 with the connectivity one pass ahead).
+__device__ __forceinline__ void prefetch_line(const char *r, bool in)
+{
+    if (in) asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
+}
+
+__device__ __forceinline__ void prefetch_pass(const Problem &p, long long b, long long end)
+{
+    // 16 rows of 8-byte entries, blockDim / 16 lines each, then two of 16 and one of
+    // 4 bytes; no line that begins past the tile's last element
+    const int sh = blockDim.x >= 256 ? 4 : 3, row = threadIdx.x >> sh, t = threadIdx.x;
+    const long long left = end - b;   // elements from b on
+    const int l = t - (row << sh);
+    const char *r = row < 9 ? (const char *)(p.fxE + row * p.ne + b)
+                            : (row < 15 ? (const char *)(p.fxS + (row - 9) * p.ne + b) : (const char *)(p.fxw + b));
+    prefetch_line(r + l * 128, l * 16 < left);
+    const int l2 = row < 2 ? t : (row < 4 ? t - (2 << sh) : t - (4 << sh)), per = row < 4 ? 8 : 32;
+    r = row < 2 ? (const char *)(p.fxD + b) : (row < 4 ? (const char *)(p.slot + b) : (const char *)(p.Lref32 + b));
+    prefetch_line(r + l2 * 128, t < (9 << sh) / 2 && l2 * per < left);
+}
+
 // The elements of one tile for the tiled element kernel: each thread's
 // elements in turn; returns the thread's FP32 minimum of the CFL screen
 // (infinite when the gate let none through).  gmin: (1 + 2^-8) times the
@@ -2244,15 +2268,17 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
     const float idtf = (float)idt;
     long long e = tl.begin + threadIdx.x;
     int4 cn_next = make_int4(0, 0, 0, 0);
-    if (MODE == MODE_MIXED || MODE == MODE_DW) {
+    constexpr bool ahead = MODE == MODE_MIXED || MODE == MODE_DW || CNH;
+    if (ahead) {
         if (e < tl.end) cn_next = p.conn[e];
     }
     for (; e < tl.end; e += blockDim.x) {
         const int4 cn = cn_next;
-        if ((MODE == MODE_MIXED || MODE == MODE_DW) && e + blockDim.x < tl.end) cn_next = p.conn[e + blockDim.x];
+        if (ahead && e + blockDim.x < tl.end) cn_next = p.conn[e + blockDim.x];
+        if (CNH) prefetch_pass(p, e - threadIdx.x + blockDim.x, tl.end);
         float d = MODE == MODE_MIXED ? elem_body_mixed<false, ACT, VISC>(p, e, parity, cn, t, idtf, gmin)
                                      : (MODE == MODE_DW ? elem_body_dw<false, ACT, VISC>(p, e, parity, cn, t, idt, gmin)
-                                                        : elem_body_fp64<false, ACT, VISC, CNH>(p, e, parity, t, idt, gmin));
+                                                        : elem_body_fp64<false, ACT, VISC, CNH>(p, e, parity, t, idt, gmin, cn));
         if (MODE == MODE_MIXED) {
             v32 = d < 0.0f ? -1.0f : fminf(v32, d);   // -1 sticks: fminf(-1, d) = -1 for d >= 0
         } else if (!(d > gmin)) {
@@ -2435,11 +2461,11 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 
-// One solve in FP64 whose every material is compressible neo-Hookean
-#ifndef CNHB
-#define CNHB 2
-#endif
-static __global__ void __launch_bounds__(kStepThreads, CNHB)
+// One solve in FP64 whose every material is compressible neo-Hookean.  128
+// registers and two CTAs an SM: three CTAs (80 registers, spills) 0.482 ms
+// against 0.497 without the prefetches and 0.509 against 0.448 with them; five
+// CTAs of 128 threads (96 registers) 0.469 against 0.452.
+static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
     solve_elem_cnh_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
 {
     elem_tile_loop<MODE_FP64, false, false, true>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
