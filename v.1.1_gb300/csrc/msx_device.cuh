@@ -1113,25 +1113,59 @@ __device__ __forceinline__ T char_length_edges(const T *e1, const T *e2, const T
     return T(2) * v6 / s;
 }
 
-// Exact FP64 CFL value of one element, min(L_ref, L(X+u)) / c, for the
-// elements the FP32 screen keeps (solvers.cpp:296-320).
-static __device__ __noinline__ double cfl_fp64(const Problem &p, long long e)
+// Exact FP64 CFL value of one element, min(L_ref, L(X+u)) / c, for the elements
+// the FP32 screen keeps (solvers.cpp:296-320), by four lanes of a warp (q = lane
+// & 3, all four with the same e): lane q loads node q and takes one face, so
+// the chain of FP64 instructions -- 68 cycles each, whatever the number of
+// active lanes -- is half that of one lane doing the four faces.  All 32 lanes
+// call this together; `pairs`: u as (hi, lo) pairs.  Every lane gets the value.
+__device__ __forceinline__ double cfl_quad(const Problem &p, long long e, bool pairs)
 {
     const long long nn = p.nn;
-    int4 cn = p.conn[e];
-    int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    double x0[3], e1[3], e2[3], e3[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) x0[k] = p.X[k * nn + nd[0]] + p.u[k * nn + nd[0]];
+    const int q = threadIdx.x & 3;
+    const int4 cn = p.conn[e];
+    const int nd = q == 0 ? cn.x : (q == 1 ? cn.y : (q == 2 ? cn.z : cn.w));
+    const double Lr = p.Lref[e], c = mat_of(p, e).c;
+    double x[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        e1[k] = (p.X[k * nn + nd[1]] + p.u[k * nn + nd[1]]) - x0[k];
-        e2[k] = (p.X[k * nn + nd[2]] + p.u[k * nn + nd[2]]) - x0[k];
-        e3[k] = (p.X[k * nn + nd[3]] + p.u[k * nn + nd[3]]) - x0[k];
+        double u;
+        if (pairs) {
+            const float2 w = p.uhl[k * nn + nd];
+            u = (double)w.x + (double)w.y;
+        } else {
+            u = p.u[k * nn + nd];
+        }
+        x[k] = p.X[k * nn + nd] + u;
     }
-    double dist = char_length_edges<double>(e1, e2, e3);
-    double Lr = p.Lref[e];
-    return ((dist < Lr) ? dist : Lr) / mat_of(p, e).c;
+    // lanes 0-2: e1 x e2, e1 x e3, e2 x e3; lane 3 the fourth face, (e2 - e1) x
+    // (e3 - e1) as their sum e2 x e3 + e1 x e2 - e1 x e3 (char_length_edges, with
+    // its products and sums spelled out so that every caller gets the same bits)
+    const int ia = q < 2 ? 1 : 2, ib = q == 0 ? 2 : 3;
+    double a[3], b[3], d[3], f[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double e0 = __shfl_sync(0xffffffffu, x[k], 0, 4), w = x[k] - e0;   // edge q
+        a[k] = __shfl_sync(0xffffffffu, w, ia, 4);
+        b[k] = __shfl_sync(0xffffffffu, w, ib, 4);
+        d[k] = __shfl_sync(0xffffffffu, w, 1, 4);
+    }
+    f[0] = fma(a[1], b[2], -__dmul_rn(a[2], b[1]));
+    f[1] = fma(a[2], b[0], -__dmul_rn(a[0], b[2]));
+    f[2] = fma(a[0], b[1], -__dmul_rn(a[1], b[0]));
+    const double v6 = __shfl_sync(0xffffffffu, fabs(fma(d[2], f[2], fma(d[0], f[0], __dmul_rn(d[1], f[1])))), 2, 4);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double A = __shfl_sync(0xffffffffu, f[k], 0, 4), B = __shfl_sync(0xffffffffu, f[k], 1, 4),
+                     C = __shfl_sync(0xffffffffu, f[k], 2, 4);
+        if (q == 3) f[k] = __dadd_rn(__dadd_rn(C, A), -B);
+    }
+    const double r = sqrt(fma(f[2], f[2], fma(f[0], f[0], __dmul_rn(f[1], f[1]))));
+    double s = __dadd_rn(__shfl_sync(0xffffffffu, r, 0, 4), __shfl_sync(0xffffffffu, r, 1, 4));
+    s = __dadd_rn(s, __shfl_sync(0xffffffffu, r, 2, 4));
+    s = __dadd_rn(s, __shfl_sync(0xffffffffu, r, 3, 4));
+    const double dist = __dmul_rn(2.0, v6) / s;
+    return ((dist < Lr) ? dist : Lr) / c;
 }
 
 // x rounded toward zero to FP32 with integer operations only (the FP64->FP32
@@ -1429,7 +1463,7 @@ static __global__ void __launch_bounds__(kElemBlock) elem_force_kernel_fp64(Prob
 // displacement gradient H = F - I (no 1 - 1 cancellation in FP32); J - 1 and
 // ln J in FP32 with an exactly summed trace; FP32 corner forces; an FP32
 // screen of the CFL values whose near-minimum elements are recomputed in FP64
-// (cfl_dw), so the stable dt is the FP64 minimum.
+// (cfl_quad), so the stable dt is the FP64 minimum.
 // cof(I + H) = I + D with D = (tr H + I2) I - (1 + tr H) H^T + (H^2)^T.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void stress_mixed(const MatParams &m, const float *H, float Jm1, float lnJ,
@@ -1868,32 +1902,6 @@ __device__ __forceinline__ void stress_dw(const MatParams &m, const float2 *F, f
     for (int k = 0; k < 9; k++) P[k] = dw_dot2(a1, F[k], g, K[k]);
 }
 
-// Exact FP64 CFL value of one element from the double-word displacement.
-static __device__ __noinline__ double cfl_dw(const Problem &p, long long e)
-{
-    const long long nn = p.nn;
-    int4 cn = p.conn[e];
-    int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    double x[4][3];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const float2 w = p.uhl[k * nn + nd[a]];
-            x[a][k] = p.X[k * nn + nd[a]] + ((double)w.x + (double)w.y);
-        }
-    double e1[3], e2[3], e3[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        e1[k] = x[1][k] - x[0][k];
-        e2[k] = x[2][k] - x[0][k];
-        e3[k] = x[3][k] - x[0][k];
-    }
-    double dist = char_length_edges<double>(e1, e2, e3);
-    double Lr = p.Lref[e];
-    return ((dist < Lr) ? dist : Lr) / mat_of(p, e).c;
-}
-
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false>
 __device__ __forceinline__ float elem_body_dw(const Problem &p, long long e, int parity, int4 cn, double t = 0.0,
                                               double idt = 0.0, float gmin = 0.0f)
@@ -2301,9 +2309,9 @@ __device__ __forceinline__ float running_min(const Problem &p, int parity)
 constexpr int kMixedPending = 2 * kStepThreads;  // deferred FP64 rechecks a mixed CTA can hold
 
 // The pending entries of a mixed CTA (all posted before the caller's last
-// barrier): one warp per entry, its lanes over the posting thread's elements
-// of that tile (one each when the tile has at most 32 per thread), skipping
-// entries above 2^-8 of the solve's running screen minimum.
+// barrier): one warp per entry, four lanes an element of the posting thread's of
+// that tile (at most eight), skipping entries above 2^-8 of the solve's running
+// screen minimum.
 template <typename SRC>
 static __device__ __noinline__ void mixed_flush(const SRC src, const int2 *pend, const float *pendv, int np, int parity)
 {
@@ -2315,10 +2323,12 @@ static __device__ __noinline__ void mixed_flush(const SRC src, const int2 *pend,
         const float mine = pendv[j];
         if (!(mine < 0.0f) && mine > running_min(p, parity) * (1.0f + 1.0f / 256.0f)) continue;
         double v = INFINITY;
-        for (long long e = tl.begin + pe.y + (long long)lane * blockDim.x; e < tl.end; e += 32LL * blockDim.x)
-            v = fmin(v, cfl_dw(p, e));
+        for (long long e0 = tl.begin + pe.y; e0 < tl.end; e0 += 8LL * blockDim.x) {   // the same in every lane
+            const long long e = e0 + (long long)(lane >> 2) * blockDim.x;
+            v = fmin(v, cfl_quad(p, e < tl.end ? e : e0, true));
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+        for (int o = 16; o > 2; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
         if (lane == 0 && v >= 0.0 && v < INFINITY)
             atomicMin(p.dtmin + (parity ^ 1), (unsigned long long)__double_as_longlong(v));
     }
@@ -2430,10 +2440,13 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
                 __syncthreads();
                 const float thr = s_thr;
                 double v = INFINITY;
-                for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-                    if (sval[c] > thr) continue;
-                    const long long e = tl.begin + scand[c];
-                    v = fmin(v, MODE == MODE_DW ? cfl_dw(p, e) : cfl_fp64(p, e));
+                const int quads = blockDim.x >> 2;
+                for (int c0 = 0; c0 < nc; c0 += quads) {   // four lanes a candidate
+                    const int c = c0 + (threadIdx.x >> 2);
+                    const bool mine = c < nc && !(sval[c] > thr);
+                    if (!__any_sync(0xffffffffu, mine)) continue;
+                    const double d = cfl_quad(p, tl.begin + (mine ? scand[c] : 0), MODE == MODE_DW);
+                    if (mine) v = fmin(v, d);
                 }
                 block_min_to(v, p.dtmin + (parity ^ 1));
             }
