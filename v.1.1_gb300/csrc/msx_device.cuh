@@ -233,8 +233,10 @@ __device__ __forceinline__ StepDecision decide_step(const Problem &p, const Ctrl
     d.next = cp;
     d.next.ran = 0;
     d.run = false;
+    const unsigned long long dtmin = p.dtmin[parity];   // with the flag and the slot: one latency
+    const int flag = p.flags[parity];
     if (cp.stop) return d;
-    if (cp.ran && p.flags[parity]) {        // uK[1] not finite after the last step
+    if (cp.ran && flag) {        // uK[1] not finite after the last step
         d.next.status = 4;
         d.next.stop = 1;
         return d;
@@ -247,7 +249,7 @@ __device__ __forceinline__ StepDecision decide_step(const Problem &p, const Ctrl
         } else {
             t += dt;
         }
-        double dtn = __longlong_as_double((long long)p.dtmin[parity]);
+        double dtn = __longlong_as_double((long long)dtmin);
         dtn = dtn * p.sf;
         d.next.t = t;
         if (dtn < 1E-20) {
@@ -264,7 +266,7 @@ __device__ __forceinline__ StepDecision decide_step(const Problem &p, const Ctrl
         // stopped at tf or at the step limit: keep the CFL min of the next step
         // so that a later call can resume the block where it left off
         d.next.stop = 1;
-        d.next.pending = p.dtmin[parity];
+        d.next.pending = dtmin;
     }
     return d;
 }
@@ -465,6 +467,15 @@ __device__ __forceinline__ float2 df_from(double x)
     return make_float2(hi, (float)(x - (double)hi));
 }
 
+// Writes the new control slot and clears the slots the element kernel fills.
+__device__ __forceinline__ void publish_step(const Problem &p, const StepDecision &d, int parity)
+{
+    p.ctrl[parity] = d.next;
+    p.dtmin[parity ^ 1] = MSX_INF_BITS;
+    p.dtmin[2 + (parity ^ 1)] = p.dtmin[4];   // the undeformed CFL minimum bounds every step's
+    p.flags[parity ^ 1] = 0;
+}
+
 // Per-solve quantities of the node kernel, derived once per block and solve
 // from the solve's control slot (not once per tile).
 struct NodeStep {
@@ -476,10 +487,11 @@ struct NodeStep {
 };
 
 template <int MODE>
-__device__ __forceinline__ void node_step(const Problem &p, int parity, NodeStep &ns)
+__device__ __forceinline__ void node_step(const Problem &p, int parity, bool publish, NodeStep &ns)
 {
     const Ctrl cp = p.ctrl[parity ^ 1];
     const StepDecision d = decide_step(p, cp, parity);
+    if (publish) publish_step(p, d, parity);
     ns.ran = cp.ran;
     ns.run = d.run;
     ns.step = d.next.step;
@@ -564,6 +576,12 @@ __device__ __forceinline__ void st_slot24(double *base, long long k, double x, d
     s[odd ? 0 : 2] = odd ? x : z;
 }
 
+// A node's first 4 kBatch corner-force slots go to registers in one batch when
+// BATCH (kernels whose grid has a block for every tile): few warps are resident
+// then, and slot after slot costs a memory latency each.
+constexpr int kBatch = 8;
+
+template <bool BATCH>
 __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bool valid, const NodeStep &ns)
 {
     const int q = threadIdx.x & 3;
@@ -595,7 +613,22 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
     // their warp), add in FP64.
     const int n = k1 - k0;   // the same for the node's four lanes
     int e0 = 0, e1 = 0, e2 = 0;
-    for (int k = k0 + q; k < k1; k += 4) {
+    constexpr int NB = BATCH ? kBatch : 0;
+    double g[3 * NB + 1];
+    if (BATCH) {
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            g[3 * j] = g[3 * j + 1] = g[3 * j + 2] = 0.0;
+            if (k0 + q + 4 * j < k1) ld_slot24(p.fe, k0 + q + 4 * j, g[3 * j], g[3 * j + 1], g[3 * j + 2]);
+        }
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            e0 = max(e0, dexp_field(g[3 * j]));
+            e1 = max(e1, dexp_field(g[3 * j + 1]));
+            e2 = max(e2, dexp_field(g[3 * j + 2]));
+        }
+    }
+    for (int k = k0 + q + 4 * NB; k < k1; k += 4) {
         double f0, f1, f2;
         ld_slot24(p.fe, k, f0, f1, f2);
         e0 = max(e0, dexp_field(f0));
@@ -615,7 +648,15 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
     double s;
     if (fixed) {
         long long a0 = 0, a1 = 0, a2 = 0;
-        for (int k = k0 + q; k < k1; k += 4) {
+        if (BATCH) {
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                a0 += dfixed(g[3 * j], e0, H);
+                a1 += dfixed(g[3 * j + 1], e1, H);
+                a2 += dfixed(g[3 * j + 2], e2, H);
+            }
+        }
+        for (int k = k0 + q + 4 * NB; k < k1; k += 4) {
             double f0, f1, f2;
             ld_slot24(p.fe, k, f0, f1, f2);
             a0 += dfixed(f0, e0, H);
@@ -686,6 +727,7 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
 // FP32 holds all it carries; u and v, the accumulated state, stay double-words.
 __device__ __forceinline__ float *mixed_a32(const Problem &p) { return reinterpret_cast<float *>(p.ahl); }
 
+template <bool BATCH>
 __device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, bool valid, const NodeStep &ns)
 {
     const int q = threadIdx.x & 3;
@@ -710,7 +752,27 @@ __device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, b
     const float4 *fe = reinterpret_cast<const float4 *>(p.fe32);
     float h0 = 0.f, h1 = 0.f, h2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
     int k = k0 + q;
-    if (k < k1) {
+    constexpr int NB = BATCH ? kBatch : 0;
+    float4 g[NB + 1];
+    if (BATCH) {
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+            if (k + 4 * j < k1) g[j] = fe[k + 4 * j];
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            if (k >= k1) break;
+            if (j == 0) {
+                h0 = g[0].x;
+                h1 = g[0].y;
+                h2 = g[0].z;
+            } else {
+                neumaier_merge(h0, c0, g[j].x, 0.0f);
+                neumaier_merge(h1, c1, g[j].y, 0.0f);
+                neumaier_merge(h2, c2, g[j].z, 0.0f);
+            }
+            k += 4;
+        }
+    } else if (k < k1) {
         const float4 f = fe[k];
         h0 = f.x;
         h1 = f.y;
@@ -766,15 +828,6 @@ __device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, b
         p.vhl[dof] = vq;
         mixed_a32(p)[dof] = aq.x;
     }
-}
-
-// Writes the new control slot and clears the slots the element kernel fills.
-__device__ __forceinline__ void publish_step(const Problem &p, const StepDecision &d, int parity)
-{
-    p.ctrl[parity] = d.next;
-    p.dtmin[parity ^ 1] = MSX_INF_BITS;
-    p.dtmin[2 + (parity ^ 1)] = p.dtmin[4];   // the undeformed CFL minimum bounds every step's
-    p.flags[parity ^ 1] = 0;
 }
 
 template <int MODE>
@@ -1992,6 +2045,7 @@ __device__ __forceinline__ void dw_sum_merge(float &s, float &c, float s2, float
     s = t;
 }
 
+template <bool BATCH>
 __device__ __forceinline__ void node_quad_dw(const Problem &p, long long i, bool valid, const NodeStep &ns)
 {
     const int q = threadIdx.x & 3;
@@ -2015,7 +2069,33 @@ __device__ __forceinline__ void node_quad_dw(const Problem &p, long long i, bool
     const float2 *fe = reinterpret_cast<const float2 *>(p.fe);
     float h0 = 0.f, h1 = 0.f, h2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
     int k = k0 + q;
-    if (k < k1) {
+    constexpr int NB = BATCH ? kBatch : 0;
+    float2 g[3 * NB + 1];
+    if (BATCH) {
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+            if (k + 4 * j < k1) {
+                const float2 *f = fe + (long long)(k + 4 * j) * 3;
+                g[3 * j] = f[0];
+                g[3 * j + 1] = f[1];
+                g[3 * j + 2] = f[2];
+            }
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            if (k >= k1) break;
+            const float2 f0 = g[3 * j], f1 = g[3 * j + 1], f2 = g[3 * j + 2];
+            if (j == 0) {
+                h0 = f0.x, c0 = f0.y;
+                h1 = f1.x, c1 = f1.y;
+                h2 = f2.x, c2 = f2.y;
+            } else {
+                dw_sum_merge(h0, c0, f0.x, f0.y);
+                dw_sum_merge(h1, c1, f1.x, f1.y);
+                dw_sum_merge(h2, c2, f2.x, f2.y);
+            }
+            k += 4;
+        }
+    } else if (k < k1) {
         const float2 *f = fe + (long long)k * 3;
         const float2 f0 = f[0], f1 = f[1], f2 = f[2];
         h0 = f0.x, c0 = f0.y;
@@ -2186,8 +2266,66 @@ struct TileQueue {
     }
 };
 
+// Programmatic dependent launch, used for single solves of small grids
+// (SolveSched::pdl): the next kernel of the step chain may start
+// once every block of this one has called pdl_release, and does its launch and
+// the loads of data no step writes (pull_*) while this one runs; pdl_wait
+// returns when the kernel before has completed and its writes are visible.  A
+// kernel releases only after its own wait, so no more than two are under way and
+// what a kernel reads before its wait was complete two kernels earlier.  Without
+// the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Loads the line at x into L1 (and drops the value).
+template <typename T>
+__device__ __forceinline__ void pull(const T *x)
+{
+    unsigned v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(x));
+}
+
+__device__ __forceinline__ void pull_node(const Problem &p, long long i)
+{
+    if (i >= p.nn) return;
+    pull(p.node_ptr + i);
+    pull(p.node_bc + i);
+    if (p.minv2) pull(p.minv2 + i);
+    else pull(p.minv + i);
+}
+
+template <int MODE>
+__device__ __forceinline__ void pull_element(const Problem &p, long long e)
+{
+    if (e >= p.ne) return;
+    pull(p.conn + e);
+    pull(p.slot + e);
+    pull(p.Lref32 + e);
+    if (MODE == MODE_FP64 && p.fxE) {
+        pull(p.fxw + e);
+        pull(p.fxD + e);
+#pragma unroll
+        for (int k = 0; k < 9; k++) pull(p.fxE + k * p.ne + e);
+#pragma unroll
+        for (int k = 0; k < 6; k++) pull(p.fxS + k * p.ne + e);
+    } else if (MODE == MODE_FP64) {
+        pull(p.wJ + e);
+#pragma unroll
+        for (int k = 0; k < 9; k++) pull(p.G + k * p.ne + e);
+    } else {
+        pull(p.wJ32 + e);
+#pragma unroll
+        for (int k = 0; k < 9; k++) pull(p.G32 + k * p.ne + e);
+        if (MODE == MODE_DW) {
+            pull(p.wJ32lo + e);
+#pragma unroll
+            for (int k = 0; k < 9; k++) pull(p.G32lo + k * p.ne + e);
+        }
+    }
+}
+
 // Node kernel over tiles (node ranges of one solve), four lanes per node.
-template <int MODE, typename SRC>
+template <int MODE, bool BATCH, typename SRC>
 __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int parity)
 {
     __shared__ int s_tile;
@@ -2197,18 +2335,17 @@ __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int 
         const int claimed = q.claim();
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
-        if (tl.solve != cur) {
-            node_step<MODE>(p, parity, ns);
+        if (tl.solve != cur) {   // a solve's first tile (begin 0) is the first of its tiles a block meets
+            node_step<MODE>(p, parity, tl.begin == 0 && threadIdx.x == 0, ns);
             cur = tl.solve;
         }
-        if (tl.begin == 0 && threadIdx.x == 0) publish_step(p, decide_step(p, p.ctrl[parity ^ 1], parity), parity);
         if (ns.ran || ns.run) {
             const int per = blockDim.x >> 2;   // every lane runs the same number of passes
             for (long long b = tl.begin; b < tl.end; b += per) {
                 long long i = b + (threadIdx.x >> 2);
-                if (MODE == MODE_MIXED) node_quad_mixed(p, i, i < tl.end, ns);
-                else if (MODE == MODE_DW) node_quad_dw(p, i, i < tl.end, ns);
-                else node_quad_fp64(p, i, i < tl.end, ns);
+                if (MODE == MODE_MIXED) node_quad_mixed<BATCH>(p, i, i < tl.end, ns);
+                else if (MODE == MODE_DW) node_quad_dw<BATCH>(p, i, i < tl.end, ns);
+                else node_quad_fp64<BATCH>(p, i, i < tl.end, ns);
             }
         }
         t = q.next(claimed, &s_tile);
@@ -2216,19 +2353,26 @@ __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int 
     q.finish();
 }
 
+// CTAs of kStepThreads an SM holds at the least: the register caps of the node
+// kernels (mixed, 6M tets: 0.120 ms with 48 registers, 0.137 with 58)
+constexpr int node_ctas(int mode, bool batch) { return batch ? (mode == MODE_MIXED ? 3 : 2) : (mode == MODE_MIXED ? 5 : 4); }
+
 template <int MODE>
-__global__ void __launch_bounds__(kStepThreads) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
+__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, false)) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
                                  int *__restrict__ sched, int parity)
 {
-    node_tile_loop<MODE>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+    node_tile_loop<MODE, false>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
 }
 
 // One solve: tiles of `size` nodes
-template <int MODE>
-__global__ void __launch_bounds__(kStepThreads) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
+template <int MODE, bool BATCH>
+__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH)) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
                                                                   int *__restrict__ sched, int parity)
 {
-    node_tile_loop<MODE>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
+    if (ntiles <= (int)gridDim.x) pull_node(p, (long long)blockIdx.x * size + (threadIdx.x >> 2));
+    pdl_wait();
+    pdl_release();
+    node_tile_loop<MODE, BATCH>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
 }
 
 // The compressible neo-Hookean FP64 kernel's streamed element data of the pass
@@ -2471,6 +2615,9 @@ template <int MODE, bool ACT = false, bool VISC = false>
 __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     solve_elem_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
 {
+    if (ntiles <= (int)gridDim.x) pull_element<MODE>(p, (long long)blockIdx.x * size + threadIdx.x);
+    pdl_wait();
+    pdl_release();
     elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 
@@ -2481,6 +2628,9 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
 static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
     solve_elem_cnh_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
 {
+    if (ntiles <= (int)gridDim.x) pull_element<MODE_FP64>(p, (long long)blockIdx.x * size + threadIdx.x);
+    pdl_wait();
+    pdl_release();
     elem_tile_loop<MODE_FP64, false, false, true>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 

@@ -46,40 +46,52 @@ void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, in
         pool_elem_kernel<MODE_FP64><<<grid, threads, 0, s>>>(descs, etiles, counts, parity);
 }
 
-void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
+// A step kernel of one solve over n tiles, with programmatic dependent launch
+// for small grids (SolveSched::pdl).
+typedef void (*solve_kernel)(const Problem, int, int, int *, int);
+
+static void launch_solve(solve_kernel f, const Problem &p, const SolveSched &q, int size, int n, int most, int *sched,
+                         int parity, cudaStream_t s)
 {
-    const int n = (int)((p.nn + q.node_tile - 1) / q.node_tile), grid = n < q.node_grid ? n : q.node_grid;
-    if (mode == MODE_MIXED)
-        solve_node_kernel<MODE_MIXED><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
-    else if (mode == MODE_DW)
-        solve_node_kernel<MODE_DW><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
-    else
-        solve_node_kernel<MODE_FP64><<<grid, q.threads, 0, s>>>(p, q.node_tile, n, counts + 3, parity);
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(n < most ? n : most);
+    c.blockDim = dim3(q.threads);
+    c.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = n <= q.pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, f, p, size, n, sched, parity);
 }
 
-template <int MODE>
-static void launch_elem_variant(const Problem &p, const SolveSched &q, int *counts, int parity, cudaStream_t s)
+void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
 {
-    const int n = (int)((p.ne + q.elem_tile - 1) / q.elem_tile), grid = n < q.elem_grid ? n : q.elem_grid;
-    // element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
-    if (p.act_t)
-        solve_elem_kernel<MODE, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
-    else if (MODE == MODE_FP64 && q.cnh)
-        solve_elem_cnh_kernel<<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
-    else if (p.visc)
-        solve_elem_kernel<MODE, false, true><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
-    else
-        solve_elem_kernel<MODE><<<grid, q.threads, 0, s>>>(p, q.elem_tile, n, counts, parity);
+    const int n = (int)((p.nn + q.node_tile - 1) / q.node_tile);
+    const bool b = q.node_batch;
+    solve_kernel f;
+    if (mode == MODE_MIXED) f = b ? solve_node_kernel<MODE_MIXED, true> : solve_node_kernel<MODE_MIXED, false>;
+    else if (mode == MODE_DW) f = b ? solve_node_kernel<MODE_DW, true> : solve_node_kernel<MODE_DW, false>;
+    else f = b ? solve_node_kernel<MODE_FP64, true> : solve_node_kernel<MODE_FP64, false>;
+    launch_solve(f, p, q, q.node_tile, n, q.node_grid, counts + 3, parity, s);
+}
+
+// element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
+template <int MODE>
+static solve_kernel solve_elem_variant(const Problem &p, const SolveSched &q)
+{
+    if (p.act_t) return solve_elem_kernel<MODE, true>;
+    if (MODE == MODE_FP64 && q.cnh) return solve_elem_cnh_kernel;
+    return p.visc ? solve_elem_kernel<MODE, false, true> : solve_elem_kernel<MODE>;
 }
 
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
 {
-    if (mode == MODE_MIXED)
-        launch_elem_variant<MODE_MIXED>(p, q, counts, parity, s);
-    else if (mode == MODE_DW)
-        launch_elem_variant<MODE_DW>(p, q, counts, parity, s);
-    else
-        launch_elem_variant<MODE_FP64>(p, q, counts, parity, s);
+    const int n = (int)((p.ne + q.elem_tile - 1) / q.elem_tile);
+    const solve_kernel f = mode == MODE_MIXED ? solve_elem_variant<MODE_MIXED>(p, q)
+                                              : (mode == MODE_DW ? solve_elem_variant<MODE_DW>(p, q)
+                                                                 : solve_elem_variant<MODE_FP64>(p, q));
+    launch_solve(f, p, q, q.elem_tile, n, q.elem_grid, counts, parity, s);
 }
 
 // a32: the mixed mode, whose acceleration is one FP32 per DOF (mixed_a32)
@@ -188,17 +200,22 @@ void launch_abs_range(const double *x, long long n, unsigned long long *mm, cuda
     abs_range_kernel<<<256, 256, 0, s>>>(x, n, mm);
 }
 
-int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, bool cnh)
+int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, bool cnh, bool batch)
 {
     const void *f[3][2][2] = {
         {{(const void *)solve_elem_kernel<MODE_FP64>, (const void *)pool_elem_kernel<MODE_FP64>},
-         {(const void *)solve_node_kernel<MODE_FP64>, (const void *)pool_node_kernel<MODE_FP64>}},
+         {(const void *)solve_node_kernel<MODE_FP64, false>, (const void *)pool_node_kernel<MODE_FP64>}},
         {{(const void *)solve_elem_kernel<MODE_MIXED>, (const void *)pool_elem_kernel<MODE_MIXED>},
-         {(const void *)solve_node_kernel<MODE_MIXED>, (const void *)pool_node_kernel<MODE_MIXED>}},
+         {(const void *)solve_node_kernel<MODE_MIXED, false>, (const void *)pool_node_kernel<MODE_MIXED>}},
         {{(const void *)solve_elem_kernel<MODE_DW>, (const void *)pool_elem_kernel<MODE_DW>},
-         {(const void *)solve_node_kernel<MODE_DW>, (const void *)pool_node_kernel<MODE_DW>}}};
+         {(const void *)solve_node_kernel<MODE_DW, false>, (const void *)pool_node_kernel<MODE_DW>}}};
     int a = 0;
     if (cnh) f[0][0][0] = (const void *)solve_elem_cnh_kernel;
+    if (batch) {
+        f[0][1][0] = (const void *)solve_node_kernel<MODE_FP64, true>;
+        f[1][1][0] = (const void *)solve_node_kernel<MODE_MIXED, true>;
+        f[2][1][0] = (const void *)solve_node_kernel<MODE_DW, true>;
+    }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f[mode == MODE_MIXED ? 1 : (mode == MODE_DW ? 2 : 0)][node][pool],
                                                   threads, 0);
     return a > 0 ? a : 1;

@@ -196,12 +196,15 @@ void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, in
 struct SolveSched {
     int threads = kStepThreads;
     int elem_tile = 0, node_tile = 0, elem_grid = 0, node_grid = 0;
+    int node_batch = 0;   // the node kernel with batched gathers (a block for every tile)
+    int pdl = 0;   // grids of up to this many CTAs are launched with programmatic dependent launch
     int cnh = 0;   // plain FP64, every material compressible neo-Hookean, no viscosity
 };
 void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 // CTAs of a tiled element kernel (node kernel when `node` is true) that fit on one SM
-int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, bool cnh = false);
+// of the pool, or of a single solve: for compressible neo-Hookean FP64 solves (cnh), with batched gathers
+int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, bool cnh = false, bool batch = false);
 // Mixed-mode state conversions: u, v, a (FP64) -> uhl, vhl, ahl, and back
 // (hi + lo, exact unless the pair spans more than 53 bits); minv -> minv2.
 void launch_state_split(const Problem &p, bool mixed, cudaStream_t s);
