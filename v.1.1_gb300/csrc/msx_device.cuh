@@ -3194,7 +3194,10 @@ __global__ void element_values_kernel(Problem p, int q, const int *elems, long l
 // grid-stride share in index order and fold it in a shared-memory tree into
 // part[2b] (the weighted sum, or the extreme) and part[2b+1] (the sum of dV);
 // one block then folds the partials the same way.
-constexpr int kReduceBlocks = 512, kReduceThreads = 256;
+// Blocks of 64 threads: on meshes of less than kReduceBlocks x kReduceThreads
+// elements the FP64 work of an element spreads evenly over the SMs' pipes (48,000
+// elements: 750 blocks of two warps against 188 of eight, 152 SMs).
+constexpr int kReduceBlocks = 2048, kReduceThreads = 64, kFinishThreads = 256;
 
 __device__ __forceinline__ void fold_pair(int op, double &s, double &w, double s2, double w2)
 {
@@ -3204,13 +3207,14 @@ __device__ __forceinline__ void fold_pair(int op, double &s, double &w, double s
     w += w2;
 }
 
+template <int THREADS>
 __device__ __forceinline__ void block_fold(int op, double &s, double &w)
 {
-    __shared__ double ss[kReduceThreads], ws[kReduceThreads];
+    __shared__ double ss[THREADS], ws[THREADS];
     ss[threadIdx.x] = s;
     ws[threadIdx.x] = w;
     __syncthreads();
-    for (int h = kReduceThreads / 2; h > 0; h >>= 1) {
+    for (int h = THREADS / 2; h > 0; h >>= 1) {
         if ((int)threadIdx.x < h) {
             double a = ss[threadIdx.x], b = ws[threadIdx.x];
             fold_pair(op, a, b, ss[threadIdx.x + h], ws[threadIdx.x + h]);
@@ -3244,19 +3248,19 @@ __global__ void __launch_bounds__(kReduceThreads) element_reduce_kernel(Problem 
         const double v = element_quantity_ref(p, q, e, t), dV = p.wJ[e];
         fold_pair(op, s, w, q == MSX_ELEM_VOLUME || op == MSX_OP_MAX || op == MSX_OP_MIN ? v : v * dV, dV);
     }
-    block_fold(op, s, w);
+    block_fold<kReduceThreads>(op, s, w);
     if (threadIdx.x == 0) {
         part[2 * blockIdx.x] = s;
         part[2 * blockIdx.x + 1] = w;
     }
 }
 
-__global__ void __launch_bounds__(kReduceThreads) element_reduce_finish_kernel(int q, int op, const double *part,
+__global__ void __launch_bounds__(kFinishThreads) element_reduce_finish_kernel(int q, int op, const double *part,
                                                                                double *out)
 {
     double s = reduce_identity(op), w = 0.0;
     for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) fold_pair(op, s, w, part[2 * b], part[2 * b + 1]);
-    block_fold(op, s, w);
+    block_fold<kFinishThreads>(op, s, w);
     if (threadIdx.x == 0) *out = op == MSX_OP_MEAN ? s / w : s;
 }
 

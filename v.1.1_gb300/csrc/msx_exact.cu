@@ -93,7 +93,7 @@ void launch_element_reduce(const Problem &p, int quantity, int op, const int *el
                            double *part, double *out, cudaStream_t s)
 {
     element_reduce_kernel<<<kReduceBlocks, kReduceThreads, 0, s>>>(p, quantity, op, elems, n, t, part);
-    element_reduce_finish_kernel<<<1, kReduceThreads, 0, s>>>(quantity, op, part, out);
+    element_reduce_finish_kernel<<<1, kFinishThreads, 0, s>>>(quantity, op, part, out);
 }
 
 long long element_reduce_scratch() { return 2LL * kReduceBlocks + 1; }

@@ -145,6 +145,10 @@ struct msx_handle {
     DBuf<double> visc_f0;
     DBuf<float> visc_h0;
     DBuf<int> d_counts;                 // tile queues of the tiled kernels
+    // scratch of the calls that compute and copy out (node and element values,
+    // reductions, internal force), kept between calls up to kScratchKept bytes
+    DBuf<unsigned char> scratch;
+    bool ctrl_known = false;            // h_ctrl[0] is the device's control slot 0
     SolveSched sched;
     // captured step chunks: `graph` holds spg steps; part[k] (k >= 1) holds 2^k
     // steps and runs a call's remainder, so a call replays at most one idle step
@@ -156,6 +160,47 @@ struct msx_handle {
 };
 
 static void drop_graphs(msx_handle *h);
+
+// Device scratch of one call, carved from the handle's buffer (a cudaMalloc and
+// its cudaFree cost 8-20 us a call, and the free waits for the device); a call
+// that needs more than kScratchKept bytes has its own allocation, freed with
+// this object.  The calls of a handle come from one thread and synchronise its
+// stream before they return, so one buffer serves them all.
+constexpr size_t kScratchKept = size_t(64) << 20;
+
+struct Scratch {
+    unsigned char *p = nullptr, *own = nullptr;
+    size_t used = 0;
+    ~Scratch()
+    {
+        if (own) cudaFree(own);
+    }
+    static size_t round(size_t b) { return (b + 255) & ~size_t(255); }
+    bool reserve(msx_handle *h, size_t bytes)
+    {
+        if (bytes > kScratchKept) {
+            if (cudaMalloc((void **)&own, bytes) != cudaSuccess) return false;
+            p = own;
+            return true;
+        }
+        if (h->scratch.n < bytes) {
+            h->scratch.release();
+            if (h->scratch.alloc(std::min(kScratchKept, std::max<size_t>(2 * bytes, 1 << 16))) != cudaSuccess) {
+                h->scratch = DBuf<unsigned char>();
+                return false;
+            }
+        }
+        p = h->scratch.p;
+        return true;
+    }
+    template <typename T>
+    T *take(size_t n)
+    {
+        T *r = reinterpret_cast<T *>(p + used);
+        used += round(sizeof(T) * n);
+        return r;
+    }
+};
 
 // ------------------------------------------------------------------ host helpers
 // Law parameters of one material (shared by single solves and the pool);
@@ -639,6 +684,7 @@ static msx_status init_block(msx_handle *h)
     MSX_CUDA(cudaStreamSynchronize(h->stream));
     h->dt_init = h->h_ctrl[0].dt;
     h->block_ready = true;
+    h->ctrl_known = true;
     return MSX_OK;
 }
 
@@ -676,8 +722,11 @@ static msx_status build_graph(msx_handle *h, int steps, cudaGraphExec_t *out)
 // block that an earlier cap stopped (tf and errors stay final).
 static msx_status arm_block(msx_handle *h, long long max_steps, long long *start_steps)
 {
-    MSX_CUDA(cudaMemcpyAsync(h->h_ctrl, h->ctrl.p, 2 * sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
-    MSX_CUDA(cudaStreamSynchronize(h->stream));
+    if (!h->ctrl_known) {
+        MSX_CUDA(cudaMemcpyAsync(h->h_ctrl, h->ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+        MSX_CUDA(cudaStreamSynchronize(h->stream));
+    }
+    h->ctrl_known = false;   // until this call has read the slot its last step wrote
     Ctrl latest = h->h_ctrl[0];   // replays start on parity 1 and read slot 0
     *start_steps = latest.step;
     long long limit = h->max_steps > 0 ? h->max_steps : (1LL << 62);
@@ -693,8 +742,8 @@ static msx_status arm_block(msx_handle *h, long long max_steps, long long *start
             MSX_CUDA(cudaMemcpyAsync(h->dtmin.p + 1, &slot1, sizeof(slot1), cudaMemcpyHostToDevice, h->stream));
             MSX_CUDA(cudaMemcpyAsync(h->flags.p + 1, &zero, sizeof(zero), cudaMemcpyHostToDevice, h->stream));
         }
+        // (pageable sources of these sizes are staged before the calls return)
         MSX_CUDA(cudaMemcpyAsync(h->ctrl.p, &latest, sizeof(Ctrl), cudaMemcpyHostToDevice, h->stream));
-        MSX_CUDA(cudaStreamSynchronize(h->stream));
         h->h_ctrl[0] = latest;
     }
     return MSX_OK;
@@ -921,6 +970,7 @@ extern "C" msx_status msx_destroy(msx_handle *h)
     h->nfs.release();
     h->faces.release();
     h->d_counts.release();
+    h->scratch.release();
     h->ctrl.release();
     h->dtmin.release();
     if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
@@ -1306,6 +1356,8 @@ extern "C" msx_status msx_run(msx_handle *h, int64_t max_steps, msx_run_report *
     MSX_CUDA(cudaEventRecord(h->ev1, h->stream));
     MSX_CUDA(cudaStreamSynchronize(h->stream));
     Ctrl fin = h->h_ctrl[k & 1];
+    h->h_ctrl[0] = fin;   // every replay ends on slot 0, copied after the last one
+    h->ctrl_known = true;
     float ms = 0;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     h->block_steps = fin.step;
@@ -1335,28 +1387,24 @@ extern "C" msx_status msx_node_values(msx_handle *h, int32_t field, int32_t comp
     for (int64_t k = 0; k < n; k++)
         if (nodes[k] < 0 || nodes[k] >= h->P.nn) return fail(MSX_ERR_ARG, "node index out of range");
     if (n == 0) return MSX_OK;
-    DBuf<int> dn;
-    DBuf<double> dv;
-    if (dn.alloc(n) != cudaSuccess || dv.alloc(n) != cudaSuccess) {
-        dn.release();
-        dv.release();
+    Scratch sc;
+    if (!sc.reserve(h, Scratch::round(sizeof(int) * n) + Scratch::round(sizeof(double) * n)))
         return fail(MSX_ERR_OOM, "node value scratch");
-    }
+    int *dn = sc.take<int>(n);
+    double *dv = sc.take<double>(n);
     bind_problem(h);
     const int mode = h->precision == MSX_PREC_FP64_EXACT ? MODE_EXACT : tiled_mode(h);
-    cudaMemcpyAsync(dn.p, nodes, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream);
-    launch_node_values(h->P, mode, field, comp, dn.p, n, h->last_t, dv.p, h->stream);
-    cudaMemcpyAsync(out, dv.p, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
+    cudaMemcpyAsync(dn, nodes, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream);
+    launch_node_values(h->P, mode, field, comp, dn, n, h->last_t, dv, h->stream);
+    cudaMemcpyAsync(out, dv, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t err = cudaStreamSynchronize(h->stream);
-    dn.release();
-    dv.release();
     if (err != cudaSuccess) return fail(MSX_ERR_CUDA, cudaGetErrorString(err));
     return MSX_OK;
 }
 
-// Shared checks of the element-extraction calls: the quantity, and the element
-// list (NULL = all) copied to the device; n becomes the number of entries.
-static msx_status element_list(msx_handle *h, int32_t quantity, const int32_t *elems, int64_t &n, DBuf<int> &de)
+// Shared checks of the element-extraction calls: the quantity and the element
+// list (NULL = all); n becomes the number of entries.
+static msx_status element_list(msx_handle *h, int32_t quantity, const int32_t *elems, int64_t &n)
 {
     if (quantity < MSX_ELEM_FXX || quantity > MSX_ELEM_VOLUME)
         return fail(MSX_ERR_ARG, "quantity must be a msx_element_quantity");
@@ -1367,9 +1415,6 @@ static msx_status element_list(msx_handle *h, int32_t quantity, const int32_t *e
     if (n < 0) return fail(MSX_ERR_ARG, "negative element count");
     for (int64_t k = 0; k < n; k++)
         if (elems[k] < 0 || elems[k] >= h->P.ne) return fail(MSX_ERR_ARG, "element index out of range");
-    if (n == 0) return MSX_OK;
-    if (de.alloc(n) != cudaSuccess) return fail(MSX_ERR_OOM, "element list scratch");
-    cudaMemcpyAsync(de.p, elems, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream);
     return MSX_OK;
 }
 
@@ -1377,23 +1422,18 @@ extern "C" msx_status msx_element_values(msx_handle *h, int32_t quantity, const 
 {
     if (!h || !out) return fail(MSX_ERR_ARG, "bad element value arguments");
     if (quantity == MSX_ELEM_EXTERNAL_ENERGY) return fail(MSX_ERR_ARG, "EXTERNAL_ENERGY has no per-element value");
-    DBuf<int> de;
-    DBuf<double> dv;
-    msx_status st = element_list(h, quantity, elems, n, de);
-    if (st != MSX_OK || n == 0) {
-        de.release();
-        return st;
-    }
-    if (dv.alloc(n) != cudaSuccess) {
-        de.release();
+    msx_status st = element_list(h, quantity, elems, n);
+    if (st != MSX_OK || n == 0) return st;
+    Scratch sc;
+    if (!sc.reserve(h, (elems ? Scratch::round(sizeof(int) * n) : 0) + Scratch::round(sizeof(double) * n)))
         return fail(MSX_ERR_OOM, "element value scratch");
-    }
+    int *de = elems ? sc.take<int>(n) : nullptr;
+    double *dv = sc.take<double>(n);
+    if (elems) cudaMemcpyAsync(de, elems, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream);
     bind_problem(h);
-    launch_element_values(h->P, quantity, elems ? de.p : nullptr, n, h->last_t, dv.p, h->stream);
-    cudaMemcpyAsync(out, dv.p, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
+    launch_element_values(h->P, quantity, de, n, h->last_t, dv, h->stream);
+    cudaMemcpyAsync(out, dv, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t err = cudaStreamSynchronize(h->stream);
-    de.release();
-    dv.release();
     if (err != cudaSuccess) return fail(MSX_ERR_CUDA, cudaGetErrorString(err));
     return MSX_OK;
 }
@@ -1414,28 +1454,23 @@ extern "C" msx_status msx_element_reduce(msx_handle *h, int32_t quantity, int32_
         set.erase(std::unique(set.begin(), set.end()), set.end());
         n = (int64_t)set.size();
     }
-    DBuf<int> de;
-    DBuf<double> scratch;
-    msx_status st = element_list(h, quantity, elems ? set.data() : nullptr, n, de);
-    if (st != MSX_OK) {
-        de.release();
-        return st;
-    }
+    msx_status st = element_list(h, quantity, elems ? set.data() : nullptr, n);
+    if (st != MSX_OK) return st;
+    const size_t nlist = elems ? (size_t)n : 0;
     if (quantity == MSX_ELEM_EXTERNAL_ENERGY) {   // u . f_ext over every DOF, whatever the operation
         n = 3 * h->P.nn;
         op = MSX_OP_SUM;
     }
-    if (scratch.alloc(element_reduce_scratch()) != cudaSuccess) {
-        de.release();
+    Scratch sc;
+    if (!sc.reserve(h, Scratch::round(sizeof(int) * nlist) + Scratch::round(sizeof(double) * element_reduce_scratch())))
         return fail(MSX_ERR_OOM, "element reduce scratch");
-    }
+    double *part = sc.take<double>(element_reduce_scratch()), *out = part + element_reduce_scratch() - 1;
+    int *de = elems ? sc.take<int>(nlist) : nullptr;
+    if (nlist) cudaMemcpyAsync(de, set.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, h->stream);
     bind_problem(h);
-    double *out = scratch.p + element_reduce_scratch() - 1;
-    launch_element_reduce(h->P, quantity, op, elems ? de.p : nullptr, n, h->last_t, scratch.p, out, h->stream);
+    launch_element_reduce(h->P, quantity, op, de, n, h->last_t, part, out, h->stream);
     cudaMemcpyAsync(value, out, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t err = cudaStreamSynchronize(h->stream);
-    de.release();
-    scratch.release();
     if (err != cudaSuccess) return fail(MSX_ERR_CUDA, cudaGetErrorString(err));
     return MSX_OK;
 }
@@ -1482,37 +1517,25 @@ extern "C" msx_status msx_next_solver(msx_handle *h, const msx_bc *bcs, int64_t 
 extern "C" msx_status msx_internal_force(msx_handle *h, const double *u, double *fint)
 {
     if (!h || !u || !fint) return fail(MSX_ERR_ARG, "NULL argument");
-    size_t bytes = sizeof(double) * 3 * h->P.nn;
-    DBuf<double> du, df;
-    if (du.alloc(3 * h->P.nn) != cudaSuccess || df.alloc(3 * h->P.nn) != cudaSuccess) {
-        du.release();
-        df.release();
-        return fail(MSX_ERR_OOM, "scratch for internal force");
-    }
+    const size_t n3 = 3 * (size_t)h->P.nn, bytes = sizeof(double) * n3;
+    const bool pairs = pair_state(h);
+    Scratch sc;
+    if (!sc.reserve(h, (pairs ? 3 : 2) * Scratch::round(bytes))) return fail(MSX_ERR_OOM, "scratch for internal force");
+    double *du = sc.take<double>(n3), *df = sc.take<double>(n3);
     bind_problem(h);
     Problem P = h->P;
-    P.u = du.p;
-    cudaMemcpyAsync(du.p, u, bytes, cudaMemcpyHostToDevice, h->stream);
-    DBuf<float2> uh;   // the mixed and double-word kernels read u as (hi, lo) pairs; the block's own stay untouched
-    if (pair_state(h)) {
-        if (uh.alloc(3 * h->P.nn) != cudaSuccess) {
-            du.release();
-            df.release();
-            return fail(MSX_ERR_OOM, "scratch for internal force");
-        }
-        long long n = 3 * P.nn;
-        P.uhl = uh.p;
-        split_kernel<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(du.p, P.uhl, n);
+    P.u = du;
+    cudaMemcpyAsync(du, u, bytes, cudaMemcpyHostToDevice, h->stream);
+    if (pairs) {   // the mixed and double-word kernels read u as (hi, lo) pairs; the block's own stay untouched
+        P.uhl = sc.take<float2>(n3);
+        split_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, h->stream>>>(du, P.uhl, (long long)n3);
     }
-    if (h->precision == MSX_PREC_FP64_EXACT) launch_internal_force_exact(P, df.p, h->stream);
-    else if (h->precision == MSX_PREC_MIXED) launch_internal_force_mixed(P, df.p, h->stream);
-    else if (h->precision == MSX_PREC_DOUBLE_WORD) launch_internal_force_dw(P, df.p, h->stream);
-    else launch_internal_force_fp64(P, df.p, h->stream);
-    cudaMemcpyAsync(fint, df.p, bytes, cudaMemcpyDeviceToHost, h->stream);
-    cudaError_t err = cudaStreamSynchronize(h->stream);
-    du.release();
-    df.release();
-    uh.release();
+    if (h->precision == MSX_PREC_FP64_EXACT) launch_internal_force_exact(P, df, h->stream);
+    else if (h->precision == MSX_PREC_MIXED) launch_internal_force_mixed(P, df, h->stream);
+    else if (h->precision == MSX_PREC_DOUBLE_WORD) launch_internal_force_dw(P, df, h->stream);
+    else launch_internal_force_fp64(P, df, h->stream);
+    cudaMemcpyAsync(fint, df, bytes, cudaMemcpyDeviceToHost, h->stream);
+    const cudaError_t err = cudaStreamSynchronize(h->stream);
     if (err != cudaSuccess) return fail(MSX_ERR_CUDA, cudaGetErrorString(err));
     return MSX_OK;
 }
@@ -1562,6 +1585,7 @@ extern "C" msx_status msx_profile(msx_handle *h, int64_t steps, msx_profile_repo
     for (auto &e : ev) cudaEventDestroy(e);
     if (err != cudaSuccess) return fail(MSX_ERR_CUDA, cudaGetErrorString(err));
     MSX_CUDA(cudaMemcpy(h->h_ctrl, h->ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost));
+    h->ctrl_known = true;
     h->block_steps = h->h_ctrl[0].step;
     const double ne = (double)h->P.ne, nn = (double)h->P.nn;
     rep->element_ms = te / n;
