@@ -1322,11 +1322,12 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
                                                     const MatParams &m, const int *nd, float gmin);
 
 // The cofactor form for an element that fixed point leaves out.
+template <bool FORCE_ONLY>
 static __device__ __noinline__ float elem_cnh_general(const Problem &p, long long e, int parity, float gmin)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    return elem_cofactor_fp64<false, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, gmin);
+    return elem_cofactor_fp64<FORCE_ONLY, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, gmin);
 }
 
 // 2^k in FP32, infinite outside its normal range
@@ -1351,12 +1352,13 @@ __device__ __forceinline__ double fixed_to_double(long long x, int k)
 // formulas in FP64.
 // Per warp of 32 elements on the 6M-tet cube (ncu): 115 FP64 instructions and
 // 1020 others took 1.290 ms, FP64 pipe 86 % busy.
+template <bool FORCE_ONLY>
 __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
                                                     const int *nd, float gmin)
 {
     const long long ne = p.ne, nn = p.nn;
     double ua[4][3];
-    if (p.u4) {
+    if (!FORCE_ONLY && p.u4) {
 #pragma unroll
         for (int a = 0; a < 4; a++) {
             const double2 xy = __ldg(reinterpret_cast<const double2 *>(p.u4) + 2LL * nd[a]);
@@ -1371,16 +1373,16 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
             for (int i = 0; i < 3; i++) ua[a][i] = p.u[nd[a] + i * nn];
     }
     const uint2 w = __ldg(p.fxw + e);
-    if (w.x == 0) return elem_cnh_general(p, e, parity, gmin);
+    if (w.x == 0) return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
     FixedElem q;
     fixed_unpack(w.x, w.y, q);
 #pragma unroll
     for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
     Limbs n[9];
     int moved;
-    if (!fixed_edges(q, ua, n, moved)) return elem_cnh_general(p, e, parity, gmin);
+    if (!fixed_edges(q, ua, n, moved)) return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
     float scr = INFINITY;
-    if (!(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(fixed_lw_min(q) + 32)), m.inv_c_f) > gmin)) {
+    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(fixed_lw_min(q) + 32)), m.inv_c_f) > gmin)) {
         float e32[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) e32[k] = (float)n[k].h * pow2f_or_inf(q.lw[k / 3] + 29);
@@ -1396,8 +1398,8 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
     }
     int64_t f[9];
     if (!fixed_forces(q, n, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f))
-        return elem_cnh_general(p, e, parity, gmin);
-    if (e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+        return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
+    if (!FORCE_ONLY && e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
     const int4 sl = __ldg(p.slot + e);
     const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
     double fa[3][3];
@@ -1500,7 +1502,7 @@ __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, i
     const int4 cn = CNH ? cn_ahead : p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
-    if (CNH || (!FORCE_ONLY && !VISC && p.fxE && m.law == 1)) return elem_body_fp64_cnh(p, e, parity, m, nd, gmin);   // never dead
+    if (CNH || (!VISC && p.fxE && m.law == 1)) return elem_body_fp64_cnh<FORCE_ONLY>(p, e, parity, m, nd, gmin);   // never dead
     return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
 }
 
@@ -3266,30 +3268,40 @@ __global__ void __launch_bounds__(kFinishThreads) element_reduce_finish_kernel(i
 
 #endif  // MSX_SETUP_KERNELS
 
-// f_int gather for the test hook: fint[node + c*nn] in element order
+// f_int gather for the internal-force hook: fint[node + c*nn] in element order,
+// a thread a node and component, its terms loaded eight at a time before they
+// are added (one after another they cost a memory latency each; 39,304 nodes in
+// FP64: 10 us)
 template <int MODE>
 __global__ void gather_kernel(Problem p, double *fint)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / 3;
+    const int c = (int)(t - 3 * i);
     if (i >= p.nn) return;
-    double s[3] = {0, 0, 0};
-    for (int k = p.node_ptr[i]; k < p.node_ptr[i + 1]; k++) {
-        // reference-order corner forces are in element order, the others in CSR slots
-        long long inc = MODE == MODE_EXACT ? p.node_inc[k] : k;
+    double s = 0;
+    const int k1 = p.node_ptr[i + 1];
+    for (int k0 = p.node_ptr[i]; k0 < k1; k0 += 8) {
+        double f[8];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
+        for (int j = 0; j < 8; j++) {
+            f[j] = 0.0;
+            if (k0 + j >= k1) continue;
+            // reference-order corner forces are in element order, the others in CSR slots
+            const long long inc = MODE == MODE_EXACT ? p.node_inc[k0 + j] : k0 + j;
             if (MODE == MODE_MIXED) {
-                s[c] += (double)p.fe32[inc * 4 + c];
+                f[j] = (double)p.fe32[inc * 4 + c];
             } else if (MODE == MODE_DW) {
                 const float2 w = reinterpret_cast<const float2 *>(p.fe)[inc * 3 + c];
-                s[c] += (double)w.x + (double)w.y;
+                f[j] = (double)w.x + (double)w.y;
             } else {
-                s[c] += p.fe[inc * 3 + c];
+                f[j] = p.fe[inc * 3 + c];
             }
         }
-    }
 #pragma unroll
-    for (int c = 0; c < 3; c++) fint[i + c * p.nn] = s[c];
+        for (int j = 0; j < 8; j++)
+            if (k0 + j < k1) s += f[j];
+    }
+    fint[i + c * p.nn] = s;
 }
 
 inline unsigned grid_for(long long n, int block) { return (unsigned)((n + block - 1) / block); }

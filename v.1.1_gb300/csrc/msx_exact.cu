@@ -58,7 +58,7 @@ void launch_initial_cfl(const Problem &p, const double *uK, int slot, cudaStream
 void launch_internal_force_exact(const Problem &p, double *fint, cudaStream_t s)
 {
     elem_kernel_exact<true><<<grid_for(p.ne, kElemBlock), kElemBlock, 0, s>>>(p, 0);
-    gather_kernel<MODE_EXACT><<<grid_for(p.nn, 256), 256, 0, s>>>(p, fint);
+    gather_kernel<MODE_EXACT><<<grid_for(3 * p.nn, 256), 256, 0, s>>>(p, fint);
 }
 
 void launch_node_values(const Problem &p, int mode, int field, int comp, const int *nodes, long long n, double t,

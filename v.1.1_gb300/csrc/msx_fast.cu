@@ -9,19 +9,19 @@ namespace msx {
 void launch_internal_force_fp64(const Problem &p, double *fint, cudaStream_t s)
 {
     elem_force_kernel_fp64<<<grid_for(p.ne, kElemBlock), kElemBlock, 0, s>>>(p, 0);
-    gather_kernel<MODE_FP64><<<grid_for(p.nn, 256), 256, 0, s>>>(p, fint);
+    gather_kernel<MODE_FP64><<<grid_for(3 * p.nn, 256), 256, 0, s>>>(p, fint);
 }
 
 void launch_internal_force_mixed(const Problem &p, double *fint, cudaStream_t s)
 {
     elem_force_kernel_mixed<<<grid_for(p.ne, kElemBlock), kElemBlock, 0, s>>>(p, 0);
-    gather_kernel<MODE_MIXED><<<grid_for(p.nn, 256), 256, 0, s>>>(p, fint);
+    gather_kernel<MODE_MIXED><<<grid_for(3 * p.nn, 256), 256, 0, s>>>(p, fint);
 }
 
 void launch_internal_force_dw(const Problem &p, double *fint, cudaStream_t s)
 {
     elem_force_kernel_dw<<<grid_for(p.ne, kElemBlock), kElemBlock, 0, s>>>(p, 0);
-    gather_kernel<MODE_DW><<<grid_for(p.nn, 256), 256, 0, s>>>(p, fint);
+    gather_kernel<MODE_DW><<<grid_for(3 * p.nn, 256), 256, 0, s>>>(p, fint);
 }
 
 void launch_tiled_node(const Problem *descs, const Tile *ntiles, int *counts, int mode, int parity, int grid,
