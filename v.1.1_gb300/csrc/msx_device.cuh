@@ -1322,12 +1322,12 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
                                                     const MatParams &m, const int *nd, float gmin);
 
 // The cofactor form for an element that fixed point leaves out.
-template <bool FORCE_ONLY>
-static __device__ __noinline__ float elem_cnh_general(const Problem &p, long long e, int parity, float gmin)
+template <bool FORCE_ONLY, bool ACT>
+static __device__ __noinline__ float elem_fp64_general(const Problem &p, long long e, int parity, double t, float gmin)
 {
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    return elem_cofactor_fp64<FORCE_ONLY, false, false>(p, e, parity, 0.0, 0.0, mat_of(p, e), nd, gmin);
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, false>(p, e, parity, t, 0.0, mat_of(p, e), nd, gmin);
 }
 
 // 2^k in FP32, infinite outside its normal range
@@ -1345,19 +1345,10 @@ __device__ __forceinline__ double fixed_to_double(long long x, int k)
     return __hiloint2double(hi ? hi + (k << 20) : 0, __double2loint(d));
 }
 
-// Plain FP64 mode, compressible neo-Hookean: the deformed edges
-// e_b = E_b + (u_b - u_0) and the corner forces from them in 64-bit fixed point
-// (msx_fixed.cuh), rounded to FP64 at the end; nine conversions and the six
-// additions of f_0 are left to the FP64 pipe, against 115 operations of the same
-// formulas in FP64.
-// Per warp of 32 elements on the 6M-tet cube (ncu): 115 FP64 instructions and
-// 1020 others took 1.290 ms, FP64 pipe 86 % busy.
+// The displacements of an element's four nodes.
 template <bool FORCE_ONLY>
-__device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
-                                                    const int *nd, float gmin)
+__device__ __forceinline__ void gather_u(const Problem &p, const int *nd, double (*ua)[3])
 {
-    const long long ne = p.ne, nn = p.nn;
-    double ua[4][3];
     if (!FORCE_ONLY && p.u4) {
 #pragma unroll
         for (int a = 0; a < 4; a++) {
@@ -1370,17 +1361,53 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 #pragma unroll
         for (int a = 0; a < 4; a++)
 #pragma unroll
-            for (int i = 0; i < 3; i++) ua[a][i] = p.u[nd[a] + i * nn];
+            for (int i = 0; i < 3; i++) ua[a][i] = p.u[nd[a] + i * p.nn];
     }
+}
+
+// The corner forces of fixed-point sums f[3(a-1) + i], a = 1..3, in units of
+// 2^(x0 - lw_a); f_0 = -(f_1 + f_2 + f_3) in FP64.
+template <bool FORCE_ONLY>
+__device__ __forceinline__ void store_fixed_forces(const Problem &p, long long e, int parity, const FixedElem &q,
+                                                   const int64_t *f)
+{
+    if (!FORCE_ONLY && e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+    const int4 sl = __ldg(p.slot + e);
+    const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
+    double fa[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) fa[a][i] = fixed_to_double(f[a * 3 + i], q.x0 - q.lw[a]);
+    st_slot24(p.fe, ks[0], -(fa[0][0] + fa[1][0] + fa[2][0]), -(fa[0][1] + fa[1][1] + fa[2][1]),
+              -(fa[0][2] + fa[1][2] + fa[2][2]));
+#pragma unroll
+    for (int a = 0; a < 3; a++) st_slot24(p.fe, ks[a + 1], fa[a][0], fa[a][1], fa[a][2]);
+}
+
+// Plain FP64 mode, compressible neo-Hookean: the deformed edges
+// e_b = E_b + (u_b - u_0) and the corner forces from them in 64-bit fixed point
+// (msx_fixed.cuh), rounded to FP64 at the end; nine conversions and the six
+// additions of f_0 are left to the FP64 pipe, against 115 operations of the same
+// formulas in FP64.
+// Per warp of 32 elements on the 6M-tet cube (ncu): 115 FP64 instructions and
+// 1020 others took 1.290 ms, FP64 pipe 86 % busy.
+template <bool FORCE_ONLY>
+__device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
+                                                    const int *nd, float gmin)
+{
+    const long long ne = p.ne;
+    double ua[4][3];
+    gather_u<FORCE_ONLY>(p, nd, ua);
     const uint2 w = __ldg(p.fxw + e);
-    if (w.x == 0) return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
+    if (w.x == 0) return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
     FixedElem q;
     fixed_unpack(w.x, w.y, q);
 #pragma unroll
     for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
     Limbs n[9];
     int moved;
-    if (!fixed_edges(q, ua, n, moved)) return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
+    if (!fixed_edges(q, ua, n, moved)) return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
     float scr = INFINITY;
     if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(fixed_lw_min(q) + 32)), m.inv_c_f) > gmin)) {
         float e32[9];
@@ -1398,19 +1425,51 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
     }
     int64_t f[9];
     if (!fixed_forces(q, n, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f))
-        return elem_cnh_general<FORCE_ONLY>(p, e, parity, gmin);
-    if (!FORCE_ONLY && e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
-    const int4 sl = __ldg(p.slot + e);
-    const int ks[4] = {sl.x, sl.y, sl.z, sl.w};
-    double fa[3][3];
+        return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
+    store_fixed_forces<FORCE_ONLY>(p, e, parity, q, f);
+    return scr;
+}
+
+// Plain FP64 mode, St-Venant-Kirchhoff and linear elasticity: the node
+// differences, the displacement gradient and the stress in 64-bit fixed point
+// (msx_fixed.cuh); 99 products of limb pairs in place of about 190 FP64
+// operations.  264,000 shuffled tets, StVK: 86 us in FP64, the FP64 pipe its
+// bound, 42 us now, bound by the integer pipes and the scattered slot writes.
+// ACT: element birth, whose dead elements have no force.
+template <bool FORCE_ONLY, bool ACT>
+__device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long e, int parity, double t,
+                                                    const MatParams &m, const int *nd, float gmin)
+{
+    const long long ne = p.ne;
+    double ua[4][3];
+    gather_u<FORCE_ONLY>(p, nd, ua);
+    const uint2 w = __ldg(p.fxw + e);
+    if (w.x == 0) return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    FixedElem q;
+    fixed_unpack(w.x, w.y, q);
 #pragma unroll
-    for (int a = 0; a < 3; a++)
+    for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
+    q.S[0] = limbs_unpack(__ldg(&p.fxD[e].x));
+    Limbs du[9];
+    int moved;
+    if (!fixed_edges<true>(q, ua, du, moved)) return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    float scr = INFINITY;
+    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(q.lw[0] + 32)), m.inv_c_f) > gmin)) {
+        float du32[9], g32[9];
 #pragma unroll
-        for (int i = 0; i < 3; i++) fa[a][i] = fixed_to_double(f[a * 3 + i], q.x0 - q.lw[a]);
-    st_slot24(p.fe, ks[0], -(fa[0][0] + fa[1][0] + fa[2][0]), -(fa[0][1] + fa[1][1] + fa[2][1]),
-              -(fa[0][2] + fa[1][2] + fa[2][2]));
+        for (int k = 0; k < 9; k++) {
+            du32[k] = (float)du[k].h * pow2f_or_inf(q.lw[0] + 29);
+            g32[k] = (float)limbs_unpack(q.E[k]).h * pow2f_or_inf(29 - 111 - q.lw[0]);
+        }
+        scr = cfl_screen(p, e, g32, du32, m);
+    }
+    int64_t f[9];
+    if (!fixed_forces_svk(q, du, m.law == 3, m.kq[0], m.ks, f))
+        return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    if (ACT && elem_dead(p, e, t))
 #pragma unroll
-    for (int a = 0; a < 3; a++) st_slot24(p.fe, ks[a + 1], fa[a][0], fa[a][1], fa[a][2]);
+        for (int k = 0; k < 9; k++) f[k] = 0;
+    store_fixed_forces<FORCE_ONLY>(p, e, parity, q, f);
     return scr;
 }
 
@@ -1495,14 +1554,17 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
     return scr;
 }
 
-template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, bool CNH = false>
+template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, int FIXED = FIXED_NONE>
 __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
                                                 double idt = 0.0, float gmin = 0.0f, int4 cn_ahead = make_int4(0, 0, 0, 0))
 {
-    const int4 cn = CNH ? cn_ahead : p.conn[e];
+    const int4 cn = FIXED ? cn_ahead : p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
-    if (CNH || (!VISC && p.fxE && m.law == 1)) return elem_body_fp64_cnh<FORCE_ONLY>(p, e, parity, m, nd, gmin);   // never dead
+    if (FIXED == FIXED_CNH || (!FIXED && !VISC && p.fxE && m.law == 1))   // never dead
+        return elem_body_fp64_cnh<FORCE_ONLY>(p, e, parity, m, nd, gmin);
+    if (FIXED == FIXED_SVK || (!VISC && p.fxE && m.law >= 2))
+        return elem_body_fp64_svk<FORCE_ONLY, ACT>(p, e, parity, t, m, nd, gmin);
     return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
 }
 
@@ -2308,8 +2370,9 @@ __device__ __forceinline__ void pull_element(const Problem &p, long long e)
         pull(p.fxD + e);
 #pragma unroll
         for (int k = 0; k < 9; k++) pull(p.fxE + k * p.ne + e);
+        if (p.fxS)
 #pragma unroll
-        for (int k = 0; k < 6; k++) pull(p.fxS + k * p.ne + e);
+            for (int k = 0; k < 6; k++) pull(p.fxS + k * p.ne + e);
     } else if (MODE == MODE_FP64) {
         pull(p.wJ + e);
 #pragma unroll
@@ -2377,7 +2440,7 @@ __global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH)) solve_no
     node_tile_loop<MODE, BATCH>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
 }
 
-// The compressible neo-Hookean FP64 kernel's streamed element data of the pass
+// The fixed-point FP64 kernels' streamed element data of the pass
 // of blockDim elements that begins at b, into L2: one or two lines a thread
 // instead of a DRAM latency before the next pass's arithmetic (6M tets: element
 // kernel 0.497 -> 0.476 ms; 0.473 -> 0.448 with the connectivity one pass ahead).
@@ -2386,16 +2449,17 @@ __device__ __forceinline__ void prefetch_line(const char *r, bool in)
     if (in) asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
 }
 
+template <int FIXED>
 __device__ __forceinline__ void prefetch_pass(const Problem &p, long long b, long long end)
 {
-    // 16 rows of 8-byte entries, blockDim / 16 lines each, then two of 16 and one of
+    // 16 rows (without fxS 10) of 8-byte entries, blockDim / 16 lines each, then two of 16 and one of
     // 4 bytes; no line that begins past the tile's last element
     const int sh = blockDim.x >= 256 ? 4 : 3, row = threadIdx.x >> sh, t = threadIdx.x;
     const long long left = end - b;   // elements from b on
     const int l = t - (row << sh);
     const char *r = row < 9 ? (const char *)(p.fxE + row * p.ne + b)
                             : (row < 15 ? (const char *)(p.fxS + (row - 9) * p.ne + b) : (const char *)(p.fxw + b));
-    prefetch_line(r + l * 128, l * 16 < left);
+    prefetch_line(r + l * 128, l * 16 < left && (FIXED == FIXED_CNH || row < 9 || row == 15));
     const int l2 = row < 2 ? t : (row < 4 ? t - (2 << sh) : t - (4 << sh)), per = row < 4 ? 8 : 32;
     r = row < 2 ? (const char *)(p.fxD + b) : (row < 4 ? (const char *)(p.slot + b) : (const char *)(p.Lref32 + b));
     prefetch_line(r + l2 * 128, t < (9 << sh) / 2 && l2 * per < left);
@@ -2412,7 +2476,7 @@ __device__ __forceinline__ void prefetch_pass(const Problem &p, long long b, lon
 // so their node gathers wait for one memory latency instead of two
 // (connectivity, then the nodes).  ACT: element birth is on, and the step's time
 // decides which elements are dead.
-template <int MODE, bool ACT, bool VISC, bool CNH = false>
+template <int MODE, bool ACT, bool VISC, int FIXED = FIXED_NONE>
 __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
                                                unsigned short *scand, int *ncand)
 {
@@ -2422,17 +2486,17 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
     const float idtf = (float)idt;
     long long e = tl.begin + threadIdx.x;
     int4 cn_next = make_int4(0, 0, 0, 0);
-    constexpr bool ahead = MODE == MODE_MIXED || MODE == MODE_DW || CNH;
+    constexpr bool ahead = MODE == MODE_MIXED || MODE == MODE_DW || FIXED;
     if (ahead) {
         if (e < tl.end) cn_next = p.conn[e];
     }
     for (; e < tl.end; e += blockDim.x) {
         const int4 cn = cn_next;
         if (ahead && e + blockDim.x < tl.end) cn_next = p.conn[e + blockDim.x];
-        if (CNH) prefetch_pass(p, e - threadIdx.x + blockDim.x, tl.end);
+        if constexpr (FIXED != FIXED_NONE) prefetch_pass<FIXED>(p, e - threadIdx.x + blockDim.x, tl.end);
         float d = MODE == MODE_MIXED ? elem_body_mixed<false, ACT, VISC>(p, e, parity, cn, t, idtf, gmin)
                                      : (MODE == MODE_DW ? elem_body_dw<false, ACT, VISC>(p, e, parity, cn, t, idt, gmin)
-                                                        : elem_body_fp64<false, ACT, VISC, CNH>(p, e, parity, t, idt, gmin, cn));
+                                                        : elem_body_fp64<false, ACT, VISC, FIXED>(p, e, parity, t, idt, gmin, cn));
         if (MODE == MODE_MIXED) {
             v32 = d < 0.0f ? -1.0f : fminf(v32, d);   // -1 sticks: fminf(-1, d) = -1 for d >= 0
         } else if (!(d > gmin)) {
@@ -2548,7 +2612,7 @@ __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, in
 // instantiation with element birth (single solves whose block has it on), VISC
 // the one with artificial bulk viscosity; the plain one carries no trace of
 // either.
-template <int MODE, bool ACT, bool VISC, bool CNH = false, typename SRC>
+template <int MODE, bool ACT, bool VISC, int FIXED = FIXED_NONE, typename SRC>
 __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int parity)
 {
     __shared__ float sval[MODE == MODE_MIXED ? 1 : kMaxTileElems];
@@ -2568,7 +2632,7 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
-            const float v32 = tile_elements<MODE, ACT, VISC, CNH>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
+            const float v32 = tile_elements<MODE, ACT, VISC, FIXED>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
                                                              sval, scand, &s_ncand);
             __syncthreads();
             const int nc = s_ncand;
@@ -2633,7 +2697,17 @@ static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
     if (ntiles <= (int)gridDim.x) pull_element<MODE_FP64>(p, (long long)blockIdx.x * size + threadIdx.x);
     pdl_wait();
     pdl_release();
-    elem_tile_loop<MODE_FP64, false, false, true>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+    elem_tile_loop<MODE_FP64, false, false, FIXED_CNH>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+}
+
+// One solve in FP64 whose every material is St-Venant-Kirchhoff or linear elastic.
+static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
+    solve_elem_svk_kernel(const __grid_constant__ Problem p, int size, int ntiles, int *__restrict__ sched, int parity)
+{
+    if (ntiles <= (int)gridDim.x) pull_element<MODE_FP64>(p, (long long)blockIdx.x * size + threadIdx.x);
+    pdl_wait();
+    pdl_release();
+    elem_tile_loop<MODE_FP64, false, false, FIXED_SVK>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
 }
 
 // ---------------------------------------------------------------------------
@@ -2672,9 +2746,9 @@ __device__ __forceinline__ void ref_jacobian(const double *xyz, double *Jac)
     }
 }
 
-// The plain FP64 mode's compressible neo-Hookean element data of element e
+// The plain FP64 mode's fixed-point data of element e
 // (Problem::fxE, fxS, fxD, fxw) from its corner coordinates pts[k*3 + i].
-__device__ __forceinline__ void write_cnh_arrays(const Problem &p, long long e, const double *pts)
+__device__ __forceinline__ void write_fixed_arrays(const Problem &p, long long e, const double *pts)
 {
     const long long ne = p.ne;
     double E[9];
@@ -2692,6 +2766,11 @@ __device__ __forceinline__ void write_cnh_arrays(const Problem &p, long long e, 
 #pragma unroll
         for (int k = 0; k < 6; k++) const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2(q.S[k].h, q.S[k].l);
         const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(q.d0, q.rd);
+    } else if (m.law >= 2 && fixed_setup_svk(E, 0.5 * m.mu2, m.ks, q)) {
+        fixed_pack(q, w);
+#pragma unroll
+        for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = q.E[k];
+        const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(limbs_pack(q.S[0]), 0);
     }
     const_cast<uint2 *>(p.fxw)[e] = make_uint2(w[0], w[1]);
 }
@@ -2737,7 +2816,7 @@ __global__ void setup_elements_kernel(Problem p, const double *X, double *G, dou
     double v6;   // 6V, signed: the edge determinant of the inscribed-sphere volume
     double L = char_length_ref(pts, &v6);
     Lref[e] = L;
-    if (p.fxE) write_cnh_arrays(p, e, pts);
+    if (p.fxE) write_fixed_arrays(p, e, pts);
     // A reference sliver (6V below 0.063 |e1||e2||e3|) gets a negative FP32
     // length: the FP32 CFL screens then always recompute it in FP64 (the mixed
     // screen rebuilds the reference edges from G in FP32, which loses accuracy
@@ -2779,7 +2858,7 @@ __global__ void mode_arrays_kernel(Problem p, float *G32, float *wJ32, float *G3
 
 // Problem::fxE, fxS, fxD and fxw of a handle whose FP64 block starts after its
 // set-up: what setup_elements_kernel writes, from X.
-__global__ void cnh_arrays_kernel(Problem p)
+__global__ void fixed_arrays_kernel(Problem p)
 {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.ne) return;
@@ -2790,7 +2869,7 @@ __global__ void cnh_arrays_kernel(Problem p)
     for (int k = 0; k < 4; k++)
 #pragma unroll
         for (int i = 0; i < 3; i++) pts[k * 3 + i] = p.X[i * p.nn + nd[k]];
-    write_cnh_arrays(p, e, pts);
+    write_fixed_arrays(p, e, pts);
 }
 
 // Previous-step F diagonal for the bulk viscosity, from displacement u, in the

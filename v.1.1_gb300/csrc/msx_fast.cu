@@ -81,7 +81,7 @@ template <int MODE>
 static solve_kernel solve_elem_variant(const Problem &p, const SolveSched &q)
 {
     if (p.act_t) return solve_elem_kernel<MODE, true>;
-    if (MODE == MODE_FP64 && q.cnh) return solve_elem_cnh_kernel;
+    if (MODE == MODE_FP64 && q.fixed) return q.fixed == FIXED_CNH ? solve_elem_cnh_kernel : solve_elem_svk_kernel;
     return p.visc ? solve_elem_kernel<MODE, false, true> : solve_elem_kernel<MODE>;
 }
 
@@ -200,7 +200,7 @@ void launch_abs_range(const double *x, long long n, unsigned long long *mm, cuda
     abs_range_kernel<<<256, 256, 0, s>>>(x, n, mm);
 }
 
-int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, bool cnh, bool batch)
+int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, int fixed, bool batch)
 {
     const void *f[3][2][2] = {
         {{(const void *)solve_elem_kernel<MODE_FP64>, (const void *)pool_elem_kernel<MODE_FP64>},
@@ -210,7 +210,7 @@ int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, bool cnh, boo
         {{(const void *)solve_elem_kernel<MODE_DW>, (const void *)pool_elem_kernel<MODE_DW>},
          {(const void *)solve_node_kernel<MODE_DW, false>, (const void *)pool_node_kernel<MODE_DW>}}};
     int a = 0;
-    if (cnh) f[0][0][0] = (const void *)solve_elem_cnh_kernel;
+    if (fixed) f[0][0][0] = fixed == FIXED_CNH ? (const void *)solve_elem_cnh_kernel : (const void *)solve_elem_svk_kernel;
     if (batch) {
         f[0][1][0] = (const void *)solve_node_kernel<MODE_FP64, true>;
         f[1][1][0] = (const void *)solve_node_kernel<MODE_MIXED, true>;

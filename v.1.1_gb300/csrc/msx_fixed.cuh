@@ -216,9 +216,11 @@ MSX_HD void fixed_unpack(uint32_t w0, uint32_t w1, FixedElem &q)
 // (32 edge lengths at least) are taken in a unit 2^k times larger, whose lost
 // bits lie 2^-9 below u's own last one.  moved: an upper bound of
 // max |u_b - u_0| component by component, in units of 2^32 of the smallest w.
+// MOTION: without E_b (all w_b equal), the differences of displacement alone.
+template <bool MOTION = false>
 MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int &moved)
 {
-    const int lw = fixed_lw_min(q);
+    const int lw = MOTION ? q.lw[0] : fixed_lw_min(q);
     int emax = 0;
 #pragma unroll
     for (int a = 0; a < 4; a++)
@@ -253,14 +255,14 @@ MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int 
     int m = 0;
 #pragma unroll
     for (int b = 0; b < 3; b++) {
-        const int d = q.lw[b] - lw;
+        const int d = MOTION ? 0 : q.lw[b] - lw;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const int64_t du = U[b + 1][i] - U[0][i];
             const int dh = (int)(du >> 32);
             const int da = dh ^ (dh >> 31);
             m = m > da ? m : da;
-            n[3 * b + i] = limbs((q.E[3 * b + i] + du) >> d);
+            n[3 * b + i] = limbs(MOTION ? du : (q.E[3 * b + i] + du) >> d);
             out |= (uint32_t)(n[3 * b + i].h + (1 << 29));
         }
     }
@@ -320,6 +322,15 @@ MSX_HD bool fixed_forces(const FixedElem &q, const Limbs *n, const int64_t *kq, 
     return true;
 }
 
+// ds and rd = 2^(62 + ds) / d0: the FP64 quotient, corrected once
+MSX_HD void fixed_reciprocal(FixedElem &q)
+{
+    q.ds = top_bit(q.d0);
+    q.rd = (int64_t)(0x1p62 / ((double)q.d0 * pow2_double(-q.ds)));
+    const __int128 res = ((__int128)1 << (62 + q.ds)) - (__int128)q.rd * q.d0;   // below 2^66
+    q.rd += mulhi64((int64_t)(res >> 8), q.rd) >> (q.ds - 10);
+}
+
 // The static data from the reference edges E (E[3(b-1) + i]), the law's c2
 // series' first coefficient kq0 and exponent ks (fixed_series).  With the
 // integers of the reference element itself, n_a x n_b as c_a and det E as d0,
@@ -358,11 +369,7 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
     q.d0 = fixed_det(n, cl);
     const double det = (double)q.d0 * 0x1p114;
     if (q.d0 < (1LL << 48) || q.d0 >= (1LL << 62) || !(det * det >= vol)) return false;
-    q.ds = top_bit(q.d0);
-    // 2^(62 + ds) / d0: the FP64 quotient, corrected once
-    q.rd = (int64_t)(0x1p62 / ((double)q.d0 * pow2_double(-q.ds)));
-    const __int128 res = ((__int128)1 << (62 + q.ds)) - (__int128)q.rd * q.d0;   // below 2^66
-    q.rd += mulhi64((int64_t)(res >> 8), q.rd) >> (q.ds - 10);
+    fixed_reciprocal(q);
     __int128 dot[6], dm = 0;
     int k = 0;
     for (int a = 0; a < 3; a++)
@@ -396,6 +403,154 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
     const int lmax = q.lw[0] + (d1 > d2 ? (d1 > 0 ? d1 : 0) : (d2 > 0 ? d2 : 0));
     const int lmin = q.lw[0] + (d1 < d2 ? (d1 < 0 ? d1 : 0) : (d2 < 0 ? d2 : 0));
     return q.x0 - lmin <= 900 && q.x0 - lmax >= -900;   // forces stay normal FP64 numbers
+}
+
+// St-Venant-Kirchhoff and linear elasticity: the displacement gradient and the
+// stress in the axes of space, as in FP64 (products of the edges would lose
+// accuracy with the square of an element's flatness).  With the shape
+// functions' gradients g_a, one unit w for all three edges and
+// du_b = (u_b - u_0) / w, f_a = f_a' |det E| W mu / w:
+//     H = sum_b du_b (w g_b),  G = H + H^T + H^T H (linear: without H^T H),
+//     S = scale (G + kappa tr(G) I),  kappa = lambda / (2 mu),
+//     P = (I + H) S (linear: S),  f_a' = P (w g_a),
+// where scale 2^x0 w = |det E| W mu, 1/2 <= scale < 1.  Units: du 2^-57, w g
+// 2^-111, H to P 2^-55, scale 2^-57; every one of them below 2^57.  An error of
+// one unit in H, S or P is 2^-55, against 2^-53 for F itself in FP64.  E holds
+// w g in limbs, S[0] the scale.
+MSX_HD int64_t limbs_pack(Limbs x) { return (int64_t)((uint64_t)(uint32_t)x.h << 32 | (uint32_t)x.l); }
+MSX_HD Limbs limbs_unpack(int64_t x) { return {(int32_t)(x >> 32), (int32_t)x}; }
+
+// kappa as kq 2^(ks - 61) with |kappa| < 2^ks; ks < 0 where there is none
+inline void fixed_kappa(double mu2, double lambda, int64_t *kq, int *ks)
+{
+    const double kappa = lambda / mu2;
+    *kq = 0;
+    *ks = -1;
+    if (!(mu2 > 0) || !(std::fabs(kappa) < 0x1p20)) return;
+    *ks = 0;
+    while (std::fabs(kappa) >= std::ldexp(1.0, *ks)) ++*ks;
+    *kq = (int64_t)std::rint(std::ldexp(kappa, 61 - *ks));
+}
+
+// false: the element is left to FP64 (see fixed_setup; w g beyond 4 to 8)
+MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
+{
+    Limbs n[9], cl[9];
+    int64_t c[9];
+    double l2 = 0;
+    for (int b = 0; b < 3; b++) {
+        const double x = E[3 * b] * E[3 * b] + E[3 * b + 1] * E[3 * b + 1] + E[3 * b + 2] * E[3 * b + 2];
+        if (!(x < 1e100) || !(x > 1e-100)) return false;
+        l2 = l2 > x ? l2 : x;
+    }
+    const int lw = (((int)(double_bits(l2) >> 52) - 1023) >> 1) + 1 - 57;
+    q.lw[0] = q.lw[1] = q.lw[2] = lw;
+    for (int k = 0; k < 9; k++) n[k] = limbs(fixed_from(E[k], lw));
+    for (int a = 0; a < 3; a++) {
+        fixed_cross(n + 3 * ((a + 1) % 3), n + 3 * ((a + 2) % 3), c + 3 * a);
+        for (int i = 0; i < 3; i++) cl[3 * a + i] = limbs(c[3 * a + i]);
+    }
+    q.d0 = fixed_det(n, cl);
+    if (q.d0 < (1LL << 50) || q.d0 >= (1LL << 62)) return false;
+    fixed_reciprocal(q);
+    for (int k = 0; k < 9; k++) {
+        const int64_t x = mulhi64((int64_t)((uint64_t)c[k] << 5), q.rd);   // c / d0 2^(ds + 3)
+        const int sh = q.ds - 51;
+        const int64_t g = sh > 0 ? (x + (1LL << (sh - 1))) >> sh : (int64_t)((uint64_t)x << -sh);
+        if (g >= (1LL << 57) || g <= -(1LL << 57)) return false;
+        q.E[k] = limbs_pack(limbs(g));
+    }
+    const double s = 0.166666666667 * ((double)q.d0 * pow2_double(-q.ds)) * mu;   // |det E| W mu = s 2^(ds + 114 + 3 lw)
+    if (ks < 0 || !(s < 1e100) || !(s > 1e-100)) return false;
+    const int x = (int)(double_bits(s) >> 52) - 1022;
+    q.S[0] = limbs((int64_t)(s * pow2_double(57 - x)));
+    q.cs = 0;
+    q.x0 = x + q.ds + 114 + 3 * lw - 109;
+    return q.x0 - lw <= 900 && q.x0 - lw >= -900;
+}
+
+// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of 2^(x0 - lw);
+// du: fixed_edges<true>; kq, ks: fixed_kappa.  false: beyond the sizes above.
+MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, int64_t kq, int ks, int64_t *f)
+{
+    Limbs g[9], H[9], S[6];
+    uint32_t out = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) g[k] = limbs_unpack(q.E[k]);
+    int64_t h[9], G[6];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            int64_t hh = 0, mid = mac_half(2);
+#pragma unroll
+            for (int b = 0; b < 3; b++) mac(hh, mid, du[3 * b + i], g[3 * b + j]);
+            h[3 * i + j] = mac_sum(hh, mid, 2);
+            H[3 * i + j] = limbs(h[3 * i + j]);
+            out |= (uint32_t)(H[3 * i + j].h + (1 << 28));
+        }
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) G[k++] = h[3 * i + j] + h[3 * j + i];
+    if (!linear) {
+        k = 0;
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = i; j < 3; j++) {
+                int64_t hh = 0, mid = mac_half(3);
+#pragma unroll
+                for (int r = 0; r < 3; r++) mac(hh, mid, H[3 * r + i], H[3 * r + j]);
+                G[k++] += mac_sum(hh, mid, 3);
+            }
+    }
+    const int64_t tr = G[0] + G[3] + G[5], most = 1LL << (57 - ks);
+    if (out >= (1u << 29) || tr >= most || tr <= -most) return false;
+    const int64_t ts = (int64_t)((uint64_t)tr << (3 + ks));
+    const int64_t kt = mulhi_near((int32_t)(ts >> 32), (int32_t)((uint32_t)ts >> 1), kq);
+    G[0] += kt;
+    G[3] += kt;
+    G[5] += kt;
+#pragma unroll
+    for (k = 0; k < 6; k++) {
+        const Limbs x = limbs(G[k]);
+        out |= (uint32_t)(x.h + (1 << 28));
+        int64_t hh = 0, mid = mac_half(1);
+        mac(hh, mid, x, q.S[0]);
+        S[k] = limbs(mac_sum(hh, mid, 1));
+    }
+    const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+    Limbs P[9];
+    if (linear) {
+#pragma unroll
+        for (k = 0; k < 9; k++) P[k] = S[mi[k]];
+    } else {
+#pragma unroll
+        for (k = 0; k < 3; k++) H[4 * k].h += 1 << 26;   // I + H
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                int64_t hh = 0, mid = mac_half(3);
+#pragma unroll
+                for (int r = 0; r < 3; r++) mac(hh, mid, H[3 * i + r], S[mi[3 * r + j]]);
+                P[3 * i + j] = limbs(mac_sum(hh, mid, 3));
+                out |= (uint32_t)(P[3 * i + j].h + (1 << 28));
+            }
+    }
+    if (out >= (1u << 29)) return false;
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            int64_t hh = 0, mid = mac_half(1);
+#pragma unroll
+            for (int j = 0; j < 3; j++) mac(hh, mid, P[3 * i + j], g[3 * a + j]);
+            f[3 * a + i] = mac_sum(hh, mid, 1);
+        }
+    return true;
 }
 
 // kq and ks of a material: (mu + lambda H_n) W 2^ks, n = 0..15 (H_n the harmonic

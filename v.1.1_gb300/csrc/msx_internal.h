@@ -104,11 +104,13 @@ struct Problem {
     // kernel gathers a node with two loads of one sector instead of three
     // 8-byte loads from three rows.  Null in the other modes.
     double *u4;
-    // plain FP64 mode, compressible neo-Hookean elements: the fixed-point data of
-    // msx_fixed.cuh: the reference edges (9*ne: fxE[(3(b-1) + i)*ne + e],
-    // b = 1..3), S's limbs (6*ne: fxS[k*ne + e]), (d0, rd) and the packed
-    // exponents (a zero word: the element takes the FP64 cofactor form).  Null in
-    // the other modes.
+    // plain FP64 mode: the fixed-point data of msx_fixed.cuh and the packed
+    // exponents fxw (a zero word: the element takes the FP64 cofactor form).
+    // Compressible neo-Hookean elements: the reference edges (9*ne:
+    // fxE[(3(b-1) + i)*ne + e], b = 1..3), S's limbs (6*ne: fxS[k*ne + e]) and
+    // (d0, rd).  St-Venant-Kirchhoff and linear elastic ones: the limbs of w g
+    // (fxE, the same order) and the scale's (fxD.x).  Null in the other modes;
+    // fxS only with a compressible neo-Hookean material.
     const long long *fxE;
     const int2 *fxS;
     const longlong2 *fxD;
@@ -193,18 +195,21 @@ void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, in
 // CTA size, tile sizes and the largest grids (a launch takes no more CTAs than
 // it has tiles).  Problem::act_t selects the element kernel with element birth,
 // Problem::visc the one with bulk viscosity.
+// Fixed-point forms of the plain FP64 mode (msx_fixed.cuh) by law
+enum : int { FIXED_NONE = 0, FIXED_CNH = 1, FIXED_SVK = 2 };
+__host__ __device__ inline int fixed_form(int law) { return law == 1 ? FIXED_CNH : (law >= 2 ? FIXED_SVK : FIXED_NONE); }
 struct SolveSched {
     int threads = kStepThreads;
     int elem_tile = 0, node_tile = 0, elem_grid = 0, node_grid = 0;
     int node_batch = 0;   // the node kernel with batched gathers (a block for every tile)
     int pdl = 0;   // grids of up to this many CTAs are launched with programmatic dependent launch
-    int cnh = 0;   // plain FP64, every material compressible neo-Hookean, no viscosity
+    int fixed = FIXED_NONE;   // plain FP64: the fixed-point form of every element
 };
 void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
 // CTAs of a tiled element kernel (node kernel when `node` is true) that fit on one SM
-// of the pool, or of a single solve: for compressible neo-Hookean FP64 solves (cnh), with batched gathers
-int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, bool cnh = false, bool batch = false);
+// of the pool, or of a single solve: of one fixed-point form (SolveSched::fixed), with batched gathers
+int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, int fixed = FIXED_NONE, bool batch = false);
 // Mixed-mode state conversions: u, v, a (FP64) -> uhl, vhl, ahl, and back
 // (hi + lo, exact unless the pair spans more than 53 bits); minv -> minv2.
 void launch_state_split(const Problem &p, bool mixed, cudaStream_t s);
@@ -227,7 +232,7 @@ void launch_setup_mass(const Problem &p, double *mass, double *minv, cudaStream_
 // a precision mode's FP32 element arrays (any pointer may be null) from G, wJ and X
 void launch_mode_arrays(const Problem &p, float *G32, float *wJ32, float *G32lo, float *wJ32lo, cudaStream_t s);
 // Problem::fxE, fxS, fxD and fxw from X (the same values the set-up writes)
-void launch_cnh_arrays(const Problem &p, cudaStream_t s);
+void launch_fixed_arrays(const Problem &p, cudaStream_t s);
 // bulk viscosity: the elements' previous-step F diagonal from displacement u
 void launch_visc_init(const Problem &p, const double *u, cudaStream_t s);
 // min over elements of Lref/c (undeformed) or min(Lref, L(X+u))/c, into dtmin[slot]

@@ -158,12 +158,12 @@ static int pool_mode(int precision)
 // modes whose running state is the (hi, lo) FP32 pairs uhl, vhl, ahl
 static bool pair_state(int precision) { return precision == MSX_PREC_MIXED || precision == MSX_PREC_DOUBLE_WORD; }
 
-static size_t footprint(long long nn, long long ne, long long nbc, int precision, bool cnh)
+static size_t footprint(long long nn, long long ne, long long nbc, int precision, int fixed)
 {
     size_t b = 0;
-    if (cnh)   // plain FP64, compressible neo-Hookean: fxE, fxS, fxD, fxw
-        b += align256(sizeof(double) * 9 * ne) + align256(sizeof(int2) * 6 * ne) + align256(sizeof(longlong2) * ne) +
-             align256(sizeof(uint2) * ne);
+    if (fixed)   // fixed-point data: fxE, fxD, fxw, fxS
+        b += align256(sizeof(double) * 9 * ne) + align256(sizeof(longlong2) * ne) + align256(sizeof(uint2) * ne);
+    if (fixed == FIXED_CNH) b += align256(sizeof(int2) * 6 * ne);
     b += align256(sizeof(int4) * ne) + align256(sizeof(double) * 9 * ne);           // conn, G
     b += 2 * align256(sizeof(double) * ne);                                         // wJ, Lref
     b += align256(sizeof(float) * 9 * ne) + 2 * align256(sizeof(float) * ne);        // G32, wJ32, Lref32
@@ -594,8 +594,8 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
             if (!dw_in_range(mesh->X[i]))
                 return pfail(MSX_ERR_ARG, "double-word pool: a nonzero coordinate lies outside [2^-100, 2^100]");
     }
-    const bool cnh = prec == MSX_PREC_FP64 && mp.law == 1;   // the FP64 element kernel's fixed-point path
-    const size_t bytes = footprint(nn, ne, num_bcs, prec, cnh);
+    const int fixed = prec == MSX_PREC_FP64 ? fixed_form(mp.law) : FIXED_NONE;
+    const size_t bytes = footprint(nn, ne, num_bcs, prec, fixed);
     {   // cheap early refusal; the slot is taken below, after the host tables
         std::lock_guard<std::mutex> lk(p->mu);
         bool free_slot = false;
@@ -670,9 +670,9 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         P.minv = minv;
         P.uhl = (float2 *)carve(sizeof(float2) * 3 * nn);
         if (prec == MSX_PREC_FP64) P.u4 = (double *)carve(sizeof(double) * 4 * nn);
-        if (cnh) {   // written by the element set-up, as for a single solve
+        if (fixed) {   // written by the element set-up, as for a single solve
             P.fxE = (long long *)carve(sizeof(long long) * 9 * ne);
-            P.fxS = (int2 *)carve(sizeof(int2) * 6 * ne);
+            if (fixed == FIXED_CNH) P.fxS = (int2 *)carve(sizeof(int2) * 6 * ne);
             P.fxD = (longlong2 *)carve(sizeof(longlong2) * ne);
             P.fxw = (uint2 *)carve(sizeof(uint2) * ne);
         }

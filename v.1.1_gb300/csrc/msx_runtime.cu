@@ -102,7 +102,7 @@ struct msx_handle {
     DBuf<float> G32, wJ32, Lref32, fe32, G32lo, wJ32lo;
     DBuf<float2> uhl, vhl, ahl, minv2;
     DBuf<double> u4;   // plain FP64 mode: node-major copy of u (Problem::u4)
-    // plain FP64 mode with a compressible neo-Hookean material: fixed-point data (Problem::fxE, fxS, fxD, fxw)
+    // plain FP64 mode, every law but neo-Hookean: fixed-point data (Problem::fxE, fxS, fxD, fxw)
     DBuf<long long> fxE;
     DBuf<int2> fxS;
     DBuf<longlong2> fxD;
@@ -242,6 +242,8 @@ bool msx::material_params(const msx_material &m, MatParams &o)
     if (m.law == 1) {
         fixed_series(o.lambda, o.mu, o.kq, &o.ks);
         o.ksw = 0.166666666667 * std::ldexp(1.0, o.ks);
+    } else if (m.law >= 2) {
+        fixed_kappa(o.mu2, o.lam_stvk, o.kq, &o.ks);
     }
     return true;
 }
@@ -442,9 +444,10 @@ static msx_status plan_tiled(msx_handle *h)
     // 11.9 -> 10.9); above, its CTAs take room and bandwidth from the one running
     // (35,000 tets FP64 17.6 -> 18.9, 115,000 mixed 17.6 -> 20.0).
     q.pdl = sms / 2;
-    q.cnh = h->P.fxE && !h->P.visc && !h->P.act_t;
-    for (int k = 0; k < h->P.nmat; k++) q.cnh = q.cnh && h->P.mats[k].law == 1;
-    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, false, false, q.cnh);
+    q.fixed = h->P.fxE && !h->P.visc && !h->P.act_t ? fixed_form(h->P.mats[0].law) : FIXED_NONE;
+    for (int k = 1; k < h->P.nmat; k++)
+        if (fixed_form(h->P.mats[k].law) != q.fixed) q.fixed = FIXED_NONE;
+    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, false, false, q.fixed);
     q.node_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true);
     // Element tiles of P whole CTA passes (P * threads elements).  Spread over
     // the grid, the busiest CTA runs ceil(tiles / grid) tiles; P minimises that
@@ -470,7 +473,7 @@ static msx_status plan_tiled(msx_handle *h)
     // node tiles of two CTA passes (four lanes a node); one pass, with batched
     // gathers, while all those tiles' CTAs are resident at once (115,506 tets in
     // mixed mode: 17.6 -> 16.4 us a step)
-    const int batch_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true, false, false, true);
+    const int batch_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true, false, FIXED_NONE, true);
     q.node_batch = (h->P.nn + thr / 4 - 1) / (thr / 4) <= batch_grid;
     q.node_tile = q.node_batch ? thr / 4 : 128;
     if (q.node_batch) q.node_grid = batch_grid;
@@ -532,12 +535,13 @@ static msx_status upload_bcs(msx_handle *h, const msx_bc *bcs, long long nbc)
 // double-word) or FP32 slots.  With `fill`, derived arrays
 // are converted from the FP64 set-up data (a later block in a new mode); at
 // msx_create the set-up kernels fill them.
-// A material of the compressible neo-Hookean law (the plain FP64 mode's
-// fixed-point element path).
-static bool has_cnh(const msx_handle *h)
+// A material of this fixed-point form, or of any (the plain FP64 mode).
+static bool has_fixed(const msx_handle *h, int form = FIXED_NONE)
 {
-    for (int k = 0; k < h->P.nmat; k++)
-        if (h->P.mats[k].law == 1) return true;
+    for (int k = 0; k < h->P.nmat; k++) {
+        const int f = fixed_form(h->P.mats[k].law);
+        if (form == FIXED_NONE ? f != FIXED_NONE : f == form) return true;
+    }
     return false;
 }
 
@@ -572,13 +576,13 @@ static msx_status mode_buffers(msx_handle *h, int precision, bool fill, cudaStre
         MSX_CUDA(cudaMemsetAsync(h->fe32.p, 0, sizeof(float) * 16 * ne, strm));
     }
     if (precision == MSX_PREC_FP64 && !h->u4.p) MSX_CUDA(h->u4.alloc(4 * nn));   // filled at each block start
-    bool cnh = false;
-    if (precision == MSX_PREC_FP64 && has_cnh(h) && !h->fxE.p) {
+    bool fixed = false;
+    if (precision == MSX_PREC_FP64 && has_fixed(h) && !h->fxE.p) {
         MSX_CUDA(h->fxE.alloc(9 * ne));
-        MSX_CUDA(h->fxS.alloc(6 * ne));
+        if (has_fixed(h, FIXED_CNH)) MSX_CUDA(h->fxS.alloc(6 * ne));
         MSX_CUDA(h->fxD.alloc(ne));
         MSX_CUDA(h->fxw.alloc(ne));
-        cnh = true;
+        fixed = true;
     }
     if (!mixed && !h->fe.p) {
         MSX_CUDA(h->fe.alloc(12 * ne));
@@ -587,7 +591,7 @@ static msx_status mode_buffers(msx_handle *h, int precision, bool fill, cudaStre
     bind_problem(h);
     if (fill) {
         if (G32 || G32lo) launch_mode_arrays(h->P, G32, wJ32, G32lo, wJ32lo, h->stream);
-        if (cnh) launch_cnh_arrays(h->P, h->stream);
+        if (fixed) launch_fixed_arrays(h->P, h->stream);
         if (minv2) launch_minv_split(h->minv.p, h->minv2.p, nn, h->stream);
         MSX_CUDA(cudaGetLastError());
         MSX_CUDA(cudaStreamSynchronize(h->stream));
@@ -865,9 +869,9 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
                     ALLOC(h->G32lo, 9 * ne);
                     ALLOC(h->wJ32lo, ne);
                 }
-                if (h->precision == MSX_PREC_FP64 && has_cnh(h)) {
+                if (h->precision == MSX_PREC_FP64 && has_fixed(h)) {
                     ALLOC(h->fxE, 9 * ne);
-                    ALLOC(h->fxS, 6 * ne);
+                    if (has_fixed(h, FIXED_CNH)) ALLOC(h->fxS, 6 * ne);
                     ALLOC(h->fxD, ne);
                     ALLOC(h->fxw, ne);
                 }
@@ -928,7 +932,7 @@ extern "C" msx_status msx_create(const msx_mesh *mesh, const msx_material *mats,
 #undef UP
     if (cudaEventRecord(side.lists, side.s) != cudaSuccess || cudaStreamWaitEvent(s, side.lists, 0) != cudaSuccess)
         return bail(fail(MSX_ERR_CUDA, "stream ordering failed"));
-    if (h->P.mat && h->P.fxE) launch_cnh_arrays(h->P, s);
+    if (h->P.mat && h->P.fxE) launch_fixed_arrays(h->P, s);
     launch_setup_mass(h->P, h->mass.p, h->minv.p, s);
     if (h->minv2.p) launch_minv_split(h->minv.p, h->minv2.p, nn, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
