@@ -526,20 +526,26 @@ __device__ __forceinline__ double node_fext(const Problem &p, long long i, int q
     return ext_force_dof(p, i + (long long)q * p.nn, ns.t);
 }
 
-// Biased exponent field of a double (0: zero or subnormal, 0x7FF: Inf or NaN).
-__device__ __forceinline__ int dexp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+// The high word of |x|: ordered as |x| to its first 20 mantissa bits.
+__device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7FFFFFFF; }
 
-// x as an integer multiple of 2^(max(E,1) - 1075 - H), truncated toward zero;
-// E is at least x's exponent field and not 0x7FF, 0 <= H <= 10.
-__device__ __forceinline__ long long dfixed(double x, int E, int H)
+// Adds x as an integer multiple of 2^(E - 1075 - H), truncated toward zero, to
+// a, for R = E + 10 - H, 0 <= H <= 10, and E >= kFixedLeast at least x's exponent
+// field and not 0x7FF.  Zeros and subnormals, which take the implicit bit too,
+// lie 2^64 below E's unit and shift out.
+constexpr int kFixedLeast = 75;
+__device__ __forceinline__ void add_fixed(long long &a, double x, int R)
 {
-    const long long b = __double_as_longlong(x);
-    const int ex = (int)((b >> 52) & 0x7FF);
-    unsigned long long m = (unsigned long long)b & 0xFFFFFFFFFFFFFull;
-    if (ex) m |= 1ull << 52;
-    const int d = max(E, 1) - max(ex, 1);
-    const unsigned long long t = d > 63 ? 0ull : (m << H) >> d;
-    return b < 0 ? -(long long)t : (long long)t;
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned h = (__funnelshift_l(xl, xh, 10) & 0x3FFFFFFFu) | 0x40000000u;   // the significand's 53 bits << 10
+    unsigned long long t = (unsigned long long)h << 32 | (xl << 10);
+    asm("{\n\t.reg .pred p;\n\t"
+        "shr.u64 %1, %1, %2;\n\t"   // beyond 63: zero
+        "setp.lt.s32 p, %3, 0;\n\t"
+        "@p sub.s64 %0, %0, %1;\n\t"
+        "@!p add.s64 %0, %0, %1;\n\t}"
+        : "+l"(a), "+l"(t)
+        : "r"(R - (int)((xh & 0x7FFFFFFFu) >> 20)), "r"((int)xh));
 }
 
 // x * 2^k for an integer-valued x (|x| < 2^63) and -1085 <= k <= 971: exact
@@ -558,16 +564,6 @@ __device__ __forceinline__ double pow2_scale(double x, int k)
 // aligned for even k) in one 16-byte and one 8-byte access instead of three
 // 8-byte ones: the 16-byte half holds values 0-1 of an even slot, 1-2 of an
 // odd one.  The selects keep the warp on one path.
-__device__ __forceinline__ void ld_slot24(const double *base, long long k, double &x, double &y, double &z)
-{
-    const bool odd = k & 1;
-    const double *s = base + 3 * k;
-    const double2 v = __ldg(reinterpret_cast<const double2 *>(s + (odd ? 1 : 0)));
-    const double w = __ldg(s + (odd ? 0 : 2));
-    x = odd ? w : v.x;
-    y = odd ? v.x : v.y;
-    z = odd ? v.y : w;
-}
 __device__ __forceinline__ void st_slot24(double *base, long long k, double x, double y, double z)
 {
     const bool odd = k & 1;
@@ -609,60 +605,78 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
     // n terms, H = 10 - ceil(log2 n) keeps the sum below 2^63; bits below the
     // guard bits are truncated (at most one unit of 2^(E - 1075 - H) per term).
     // The sum does not depend on the order of the terms.  Nodes with an
-    // infinite or NaN term, or too many terms for H >= 0 (and the other nodes of
-    // their warp), add in FP64.
+    // infinite or NaN term, a component whose largest term is below 2^-948 but
+    // not 0 (subnormals below 2^-1042 count as 0), or too many terms for H >= 0
+    // (and the other nodes of their warp), add in FP64.
+    // A lane's slots are all even or all odd, so it adds the three values in
+    // the order they lie in its two loads (xyz, or yzx) and turns the sums, not
+    // the values: 6M tets, node kernel 181 -> 174 us with this and add_fixed (the ALU
+    // pipe was 63 % busy); 6000 tets 14.8 -> 13.2 us a step.
     const int n = k1 - k0;   // the same for the node's four lanes
-    int e0 = 0, e1 = 0, e2 = 0;
+    const bool turned = (k0 + q) & 1;
+    const double *at = p.fe + 3LL * (k0 + q), *at2 = at + (turned ? 1 : 0), *at1 = at + (turned ? 0 : 2);
+    int zx = 0, zy = 0, zw = 0;
     constexpr int NB = BATCH ? kBatch : 0;
-    double g[3 * NB + 1];
+    double2 g2[NB + 1];
+    double g1[NB + 1];
     if (BATCH) {
 #pragma unroll
         for (int j = 0; j < NB; j++) {
-            g[3 * j] = g[3 * j + 1] = g[3 * j + 2] = 0.0;
-            if (k0 + q + 4 * j < k1) ld_slot24(p.fe, k0 + q + 4 * j, g[3 * j], g[3 * j + 1], g[3 * j + 2]);
+            g2[j] = make_double2(0.0, 0.0);
+            g1[j] = 0.0;
+            if (k0 + q + 4 * j < k1) {
+                g2[j] = __ldg(reinterpret_cast<const double2 *>(at2 + 12 * j));
+                g1[j] = __ldg(at1 + 12 * j);
+            }
         }
 #pragma unroll
         for (int j = 0; j < NB; j++) {
-            e0 = max(e0, dexp_field(g[3 * j]));
-            e1 = max(e1, dexp_field(g[3 * j + 1]));
-            e2 = max(e2, dexp_field(g[3 * j + 2]));
+            zx = max(zx, abs_hi(g2[j].x));
+            zy = max(zy, abs_hi(g2[j].y));
+            zw = max(zw, abs_hi(g1[j]));
         }
     }
-    for (int k = k0 + q + 4 * NB; k < k1; k += 4) {
-        double f0, f1, f2;
-        ld_slot24(p.fe, k, f0, f1, f2);
-        e0 = max(e0, dexp_field(f0));
-        e1 = max(e1, dexp_field(f1));
-        e2 = max(e2, dexp_field(f2));
+    for (int k = k0 + q + 4 * NB, o = 12 * NB; k < k1; k += 4, o += 12) {
+        const double2 f = __ldg(reinterpret_cast<const double2 *>(at2 + o));
+        zx = max(zx, abs_hi(f.x));
+        zy = max(zy, abs_hi(f.y));
+        zw = max(zw, abs_hi(__ldg(at1 + o)));
     }
+    int z0 = turned ? zw : zx, z1 = turned ? zx : zy, z2 = turned ? zy : zw;
 #pragma unroll
     for (int o = 1; o <= 2; o <<= 1) {
-        e0 = max(e0, __shfl_xor_sync(0xffffffffu, e0, o));
-        e1 = max(e1, __shfl_xor_sync(0xffffffffu, e1, o));
-        e2 = max(e2, __shfl_xor_sync(0xffffffffu, e2, o));
+        z0 = max(z0, __shfl_xor_sync(0xffffffffu, z0, o));
+        z1 = max(z1, __shfl_xor_sync(0xffffffffu, z1, o));
+        z2 = max(z2, __shfl_xor_sync(0xffffffffu, z2, o));
     }
     const int H = 10 - (n > 1 ? 32 - __clz(n - 1) : 0);
+    const auto in_range = [](int z) { return z == 0 || (z >= kFixedLeast << 20 && z < 0x7FF << 20); };
     // one path for the whole warp: both use shuffles over all 32 lanes (lanes
     // past the tile's end have no terms and vote for the integer path)
-    const bool fixed = __all_sync(0xffffffffu, H >= 0 && max(e0, max(e1, e2)) < 0x7FF);
+    const bool fixed = __all_sync(0xffffffffu, H >= 0 && in_range(z0) && in_range(z1) && in_range(z2));
     double s;
     if (fixed) {
-        long long a0 = 0, a1 = 0, a2 = 0;
+        // a component of zeros: every term shifts out
+        const int r0 = (z0 ? z0 >> 20 : 4000) + 10 - H, r1 = (z1 ? z1 >> 20 : 4000) + 10 - H,
+                  r2 = (z2 ? z2 >> 20 : 4000) + 10 - H;
+        const int rx = turned ? r1 : r0, ry = turned ? r2 : r1, rw = turned ? r0 : r2;
+        long long ax = 0, ay = 0, aw = 0;
         if (BATCH) {
 #pragma unroll
             for (int j = 0; j < NB; j++) {
-                a0 += dfixed(g[3 * j], e0, H);
-                a1 += dfixed(g[3 * j + 1], e1, H);
-                a2 += dfixed(g[3 * j + 2], e2, H);
+                add_fixed(ax, g2[j].x, rx);
+                add_fixed(ay, g2[j].y, ry);
+                add_fixed(aw, g1[j], rw);
             }
         }
-        for (int k = k0 + q + 4 * NB; k < k1; k += 4) {
-            double f0, f1, f2;
-            ld_slot24(p.fe, k, f0, f1, f2);
-            a0 += dfixed(f0, e0, H);
-            a1 += dfixed(f1, e1, H);
-            a2 += dfixed(f2, e2, H);
+        for (int k = k0 + q + 4 * NB, o = 12 * NB; k < k1; k += 4, o += 12) {
+            const double2 f = __ldg(reinterpret_cast<const double2 *>(at2 + o));
+            const double w = __ldg(at1 + o);
+            add_fixed(ax, f.x, rx);
+            add_fixed(ay, f.y, ry);
+            add_fixed(aw, w, rw);
         }
+        long long a0 = turned ? aw : ax, a1 = turned ? ax : ay, a2 = turned ? ay : aw;
 #pragma unroll
         for (int o = 1; o <= 2; o <<= 1) {
             a0 += __shfl_xor_sync(0xffffffffu, a0, o);
@@ -670,7 +684,7 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
             a2 += __shfl_xor_sync(0xffffffffu, a2, o);
         }
         if (!own) return;
-        s = pow2_scale(__ll2double_rn(pick3(q, a0, a1, a2)), max(pick3(q, e0, e1, e2), 1) - 1075 - H);
+        s = pow2_scale(__ll2double_rn(pick3(q, a0, a1, a2)), (pick3(q, z0, z1, z2) >> 20) - 1075 - H);
     } else {
         double s0 = 0.0, s1 = 0.0, s2 = 0.0;
         for (int k = k0 + q; k < k1; k += 4) {
