@@ -578,7 +578,7 @@ __device__ __forceinline__ void st_slot24(double *base, long long k, double x, d
 constexpr int kBatch = 8;
 
 template <bool BATCH>
-__device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bool valid, const NodeStep &ns)
+__device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bool valid, const NodeStep &ns, int2 slots)
 {
     const int q = threadIdx.x & 3;
     const bool odd = q & 1;
@@ -593,11 +593,7 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
         minv = p.minv[i];
         rec = p.node_bc[i];
     }
-    int k0 = 0, k1 = 0;
-    if (valid && ns.ran) {
-        k0 = p.node_ptr[i];
-        k1 = p.node_ptr[i + 1];
-    }
+    const int k0 = slots.x, k1 = slots.y;
     // The node's f_int per component as one exact integer sum, rounded once:
     // each term's 53-bit significand aligned to the largest exponent E of that
     // component among the node's terms, with H guard bits below it, summed in
@@ -742,7 +738,7 @@ __device__ __forceinline__ void node_quad_fp64(const Problem &p, long long i, bo
 __device__ __forceinline__ float *mixed_a32(const Problem &p) { return reinterpret_cast<float *>(p.ahl); }
 
 template <bool BATCH>
-__device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, bool valid, const NodeStep &ns)
+__device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, bool valid, const NodeStep &ns, int2 slots)
 {
     const int q = threadIdx.x & 3;
     const bool odd = q & 1;
@@ -757,11 +753,7 @@ __device__ __forceinline__ void node_quad_mixed(const Problem &p, long long i, b
         minv = p.minv2[i];
         rec = p.node_bc[i];
     }
-    int k0 = 0, k1 = 0;
-    if (valid && ns.ran) {
-        k0 = p.node_ptr[i];
-        k1 = p.node_ptr[i + 1];
-    }
+    const int k0 = slots.x, k1 = slots.y;
     // compensated FP32 sums (Neumaier) of the FP32 corner forces
     const float4 *fe = reinterpret_cast<const float4 *>(p.fe32);
     float h0 = 0.f, h1 = 0.f, h2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
@@ -2124,7 +2116,7 @@ __device__ __forceinline__ void dw_sum_merge(float &s, float &c, float s2, float
 }
 
 template <bool BATCH>
-__device__ __forceinline__ void node_quad_dw(const Problem &p, long long i, bool valid, const NodeStep &ns)
+__device__ __forceinline__ void node_quad_dw(const Problem &p, long long i, bool valid, const NodeStep &ns, int2 slots)
 {
     const int q = threadIdx.x & 3;
     const bool odd = q & 1;
@@ -2139,11 +2131,7 @@ __device__ __forceinline__ void node_quad_dw(const Problem &p, long long i, bool
         minv = p.minv2[i];
         rec = p.node_bc[i];
     }
-    int k0 = 0, k1 = 0;
-    if (valid && ns.ran) {
-        k0 = p.node_ptr[i];
-        k1 = p.node_ptr[i + 1];
-    }
+    const int k0 = slots.x, k1 = slots.y;
     const float2 *fe = reinterpret_cast<const float2 *>(p.fe);
     float h0 = 0.f, h1 = 0.f, h2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
     int k = k0 + q;
@@ -2403,9 +2391,23 @@ __device__ __forceinline__ void pull_element(const Problem &p, long long e)
     }
 }
 
-// Node kernel over tiles (node ranges of one solve), four lanes per node.
-template <int MODE, bool BATCH, typename SRC>
-__device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int parity)
+// The node's corner-force slots [x, y); none without forces to add
+__device__ __forceinline__ int2 node_slots(const Problem &p, long long i, bool any)
+{
+    return any ? make_int2(p.node_ptr[i], p.node_ptr[i + 1]) : make_int2(0, 0);
+}
+
+template <int MODE, bool BATCH>
+__device__ __forceinline__ void node_quad(const Problem &p, long long i, bool valid, const NodeStep &ns, int2 slots)
+{
+    if (MODE == MODE_MIXED) node_quad_mixed<BATCH>(p, i, valid, ns, slots);
+    else if (MODE == MODE_DW) node_quad_dw<BATCH>(p, i, valid, ns, slots);
+    else node_quad_fp64<BATCH>(p, i, valid, ns, slots);
+}
+
+// The pool's node kernel over tiles (node ranges of one solve), four lanes per node.
+template <int MODE>
+__device__ __forceinline__ void node_tile_loop(const PoolTiles &src, TileQueue q, int parity)
 {
     __shared__ int s_tile;
     int t = q.first(&s_tile), cur = -1;
@@ -2422,9 +2424,7 @@ __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int 
             const int per = blockDim.x >> 2;   // every lane runs the same number of passes
             for (long long b = tl.begin; b < tl.end; b += per) {
                 long long i = b + (threadIdx.x >> 2);
-                if (MODE == MODE_MIXED) node_quad_mixed<BATCH>(p, i, i < tl.end, ns);
-                else if (MODE == MODE_DW) node_quad_dw<BATCH>(p, i, i < tl.end, ns);
-                else node_quad_fp64<BATCH>(p, i, i < tl.end, ns);
+                node_quad<MODE, false>(p, i, i < tl.end, ns, node_slots(p, i, i < tl.end && ns.ran));
             }
         }
         t = q.next(claimed, &s_tile);
@@ -2433,25 +2433,55 @@ __device__ __forceinline__ void node_tile_loop(const SRC &src, TileQueue q, int 
 }
 
 // CTAs of kStepThreads an SM holds at the least: the register caps of the node
-// kernels (mixed, 6M tets: 0.120 ms with 48 registers, 0.137 with 58)
-constexpr int node_ctas(int mode, bool batch) { return batch ? (mode == MODE_MIXED ? 3 : 2) : (mode == MODE_MIXED ? 5 : 4); }
+// kernels (6M tets, mixed: 104 us with 48 registers, 109 with 40, 114 with 64;
+// FP64: 160 with 48, 163 with 64, 171 with 80)
+constexpr int node_ctas(int mode, bool batch) { return batch ? (mode == MODE_MIXED ? 3 : 2) : 5; }
 
 template <int MODE>
-__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, false)) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
+__global__ void __launch_bounds__(kStepThreads, MODE == MODE_MIXED ? 5 : 4) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
                                  int *__restrict__ sched, int parity)
 {
-    node_tile_loop<MODE, false>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+    node_tile_loop<MODE>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
 }
 
-// One solve: tiles of `size` nodes
-template <int MODE, bool BATCH>
-__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH)) solve_node_kernel(const __grid_constant__ Problem p, int size, int ntiles,
-                                                                  int *__restrict__ sched, int parity)
+// A node's next slots into L2, a line or two a lane
+template <int MODE>
+__device__ __forceinline__ void prefetch_slots(const Problem &p, int2 slots)
 {
-    if (ntiles <= (int)gridDim.x) pull_node(p, (long long)blockIdx.x * size + (threadIdx.x >> 2));
+    constexpr int bytes = MODE == MODE_MIXED ? 16 : 24;
+    const char *f = (MODE == MODE_MIXED ? (const char *)p.fe32 : (const char *)p.fe) + (long long)slots.x * bytes;
+    const int n = (slots.y - slots.x) * bytes, o = (threadIdx.x & 3) * 128;
+    if (o < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(f + o));
+    if (MODE != MODE_MIXED && o + 512 < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(f + o + 512));
+}
+
+// One solve: passes of blockDim / 4 nodes, which go to the blocks in turn (a
+// node's work hardly differs from the next one's, so claims would only add
+// their barriers), with the next pass's slot range loaded a pass ahead and its
+// slots prefetched.  Bound by the latency of each pass's loads and, in FP64, the
+// ALU pipe.  Node kernel of 6M tets: FP64 174 -> 163 us without claims, 145 with
+// the next slots ahead; mixed 121 -> 104 and 104; 1.6M tets double-word 51 -> 46.
+// Shared-memory stages of a tile's slots instead: 250, 131 and 54 us, for the
+// warps they cost.
+template <int MODE, bool BATCH>
+__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH))
+    solve_node_kernel(const __grid_constant__ Problem p, int, int ntiles, int *__restrict__, int parity)
+{
+    const long long per = blockDim.x >> 2, stride = per * gridDim.x;
+    if (ntiles <= (int)gridDim.x) pull_node(p, blockIdx.x * per + (threadIdx.x >> 2));
     pdl_wait();
     pdl_release();
-    node_tile_loop<MODE, BATCH>(SolveTiles{p, p.nn, size}, TileQueue(sched, ntiles), parity);
+    NodeStep ns;
+    node_step<MODE>(p, parity, blockIdx.x == 0 && threadIdx.x == 0, ns);
+    if (!ns.ran && !ns.run) return;
+    long long i = blockIdx.x * per + (threadIdx.x >> 2);
+    int2 k = node_slots(p, i, i < p.nn && ns.ran);
+    for (long long b = blockIdx.x * per; b < p.nn; b += stride, i += stride) {
+        const int2 now = k;
+        k = node_slots(p, i + stride, i + stride < p.nn && ns.ran);
+        node_quad<MODE, BATCH>(p, i, i < p.nn, ns, now);
+        if (!BATCH) prefetch_slots<MODE>(p, k);
+    }
 }
 
 // The fixed-point FP64 kernels' streamed element data of the pass

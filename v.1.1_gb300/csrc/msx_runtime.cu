@@ -470,12 +470,12 @@ static msx_status plan_tiled(msx_handle *h)
         }
     }
     q.elem_tile = bestp * thr;
-    // node tiles of two CTA passes (four lanes a node); one pass, with batched
-    // gathers, while all those tiles' CTAs are resident at once (115,506 tets in
-    // mixed mode: 17.6 -> 16.4 us a step)
+    // node passes of one CTA (four lanes a node), with batched gathers while all
+    // their CTAs are resident at once (115,506 tets in mixed mode: 17.6 -> 16.4 us
+    // a step)
     const int batch_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true, false, FIXED_NONE, true);
     q.node_batch = (h->P.nn + thr / 4 - 1) / (thr / 4) <= batch_grid;
-    q.node_tile = q.node_batch ? thr / 4 : 128;
+    q.node_tile = thr / 4;
     if (q.node_batch) q.node_grid = batch_grid;
     if (!h->d_counts.p) {
         MSX_CUDA(h->d_counts.alloc(kTileSched));
