@@ -2389,6 +2389,22 @@ __device__ __forceinline__ void node_quad(const Problem &p, long long i, bool va
     else node_quad_fp64<BATCH>(p, i, valid, ns, slots);
 }
 
+// The step decision by one warp for its block: about 60 instructions on the FP64
+// pipe, which kept it 69 % busy when every warp took them (mixed node kernel,
+// 1.6M tets; 116,000 tets mixed 16.3 -> 14.2 us a step).
+template <int MODE>
+__device__ __forceinline__ NodeStep block_node_step(const Problem &p, int parity, bool publish)
+{
+    __shared__ NodeStep s_ns;   // read by all before the caller's next barrier
+    if (threadIdx.x < 32) {
+        NodeStep ns;
+        node_step<MODE>(p, parity, publish && threadIdx.x == 0, ns);
+        if (threadIdx.x == 0) s_ns = ns;
+    }
+    __syncthreads();
+    return s_ns;
+}
+
 // The pool's node kernel over tiles (node ranges of one solve), four lanes per node.
 template <int MODE>
 __device__ __forceinline__ void node_tile_loop(const PoolTiles &src, TileQueue q, int parity)
@@ -2401,7 +2417,7 @@ __device__ __forceinline__ void node_tile_loop(const PoolTiles &src, TileQueue q
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (tl.solve != cur) {   // a solve's first tile (begin 0) is the first of its tiles a block meets
-            node_step<MODE>(p, parity, tl.begin == 0 && threadIdx.x == 0, ns);
+            ns = block_node_step<MODE>(p, parity, tl.begin == 0);
             cur = tl.solve;
         }
         if (ns.ran || ns.run) {
@@ -2447,8 +2463,11 @@ __device__ __forceinline__ void prefetch_slots(const Problem &p, int2 slots)
 // the next slots ahead; mixed 121 -> 104 and 104; 1.6M tets double-word 51 -> 46.
 // Shared-memory stages of a tile's slots instead: 250, 131 and 54 us, for the
 // warps they cost.
-template <int MODE, bool BATCH>
-__global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH))
+// SMALL: blocks of 128 threads, one warp a scheduler, where every warp derives
+// the step decision and no barrier is worth it (72 tets 10.4 us a step, 11.2
+// with it).
+template <int MODE, bool BATCH, bool SMALL = false>
+__global__ void __launch_bounds__(SMALL ? 128 : kStepThreads, node_ctas(MODE, BATCH))
     solve_node_kernel(const __grid_constant__ Problem p, int, int ntiles, int *__restrict__, int parity)
 {
     const long long per = blockDim.x >> 2, stride = per * gridDim.x;
@@ -2456,7 +2475,8 @@ __global__ void __launch_bounds__(kStepThreads, node_ctas(MODE, BATCH))
     pdl_wait();
     pdl_release();
     NodeStep ns;
-    node_step<MODE>(p, parity, blockIdx.x == 0 && threadIdx.x == 0, ns);
+    if (SMALL) node_step<MODE>(p, parity, blockIdx.x == 0 && threadIdx.x == 0, ns);
+    else ns = block_node_step<MODE>(p, parity, blockIdx.x == 0);
     if (!ns.ran && !ns.run) return;
     long long i = blockIdx.x * per + (threadIdx.x >> 2);
     int2 k = node_slots(p, i, i < p.nn && ns.ran);

@@ -70,7 +70,10 @@ void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int m
     const int n = (int)((p.nn + q.node_tile - 1) / q.node_tile);
     const bool b = q.node_batch;
     solve_kernel f;
-    if (mode == MODE_MIXED) f = b ? solve_node_kernel<MODE_MIXED, true> : solve_node_kernel<MODE_MIXED, false>;
+    if (b && q.threads == 128)
+        f = mode == MODE_MIXED ? solve_node_kernel<MODE_MIXED, true, true>
+                               : (mode == MODE_DW ? solve_node_kernel<MODE_DW, true, true> : solve_node_kernel<MODE_FP64, true, true>);
+    else if (mode == MODE_MIXED) f = b ? solve_node_kernel<MODE_MIXED, true> : solve_node_kernel<MODE_MIXED, false>;
     else if (mode == MODE_DW) f = b ? solve_node_kernel<MODE_DW, true> : solve_node_kernel<MODE_DW, false>;
     else f = b ? solve_node_kernel<MODE_FP64, true> : solve_node_kernel<MODE_FP64, false>;
     launch_solve(f, p, q, q.node_tile, n, q.node_grid, counts + 3, parity, s);

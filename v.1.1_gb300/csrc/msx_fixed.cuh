@@ -420,7 +420,7 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
 MSX_HD int64_t limbs_pack(Limbs x) { return (int64_t)((uint64_t)(uint32_t)x.h << 32 | (uint32_t)x.l); }
 MSX_HD Limbs limbs_unpack(int64_t x) { return {(int32_t)(x >> 32), (int32_t)x}; }
 
-// kappa as kq 2^(ks - 61) with |kappa| < 2^ks; ks < 0 where there is none
+// kappa as kq 2^(ks - 57) with |kappa| < 2^ks, in limbs; ks < 0 where there is none
 inline void fixed_kappa(double mu2, double lambda, int64_t *kq, int *ks)
 {
     const double kappa = lambda / mu2;
@@ -429,7 +429,7 @@ inline void fixed_kappa(double mu2, double lambda, int64_t *kq, int *ks)
     if (!(mu2 > 0) || !(std::fabs(kappa) < 0x1p20)) return;
     *ks = 0;
     while (std::fabs(kappa) >= std::ldexp(1.0, *ks)) ++*ks;
-    *kq = (int64_t)std::rint(std::ldexp(kappa, 61 - *ks));
+    *kq = limbs_pack(limbs((int64_t)std::rint(std::ldexp(kappa, 57 - *ks))));
 }
 
 // false: the element is left to FP64 (see fixed_setup; w g beyond 4 to 8)
@@ -508,8 +508,10 @@ MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, i
     }
     const int64_t tr = G[0] + G[3] + G[5], most = 1LL << (57 - ks);
     if (out >= (1u << 29) || tr >= most || tr <= -most) return false;
-    const int64_t ts = (int64_t)((uint64_t)tr << (3 + ks));
-    const int64_t kt = mulhi_near((int32_t)(ts >> 32), (int32_t)((uint32_t)ts >> 1), kq);
+    // rounded to nearest: a truncation is a pressure on every element of the body
+    int64_t th = 0, tm = mac_half(1 + ks);
+    mac(th, tm, limbs(tr), limbs_unpack(kq));
+    const int64_t kt = mac_sum(th, tm, 1 + ks);
     G[0] += kt;
     G[3] += kt;
     G[5] += kt;
