@@ -53,7 +53,7 @@ def peaks():
         return 6800.0, "fallback"
 
 
-def profiled(key, kernel="pool_elem_kernel<FP64>"):
+def profiled(key, kernel="solve_elem_cnh_kernel"):
     """A per-element figure of a kernel from the committed ncu captures
     (profiles/ncu_figures.json: DRAM bytes per element from one --set full
     capture on the 64^3 cube, FP64 instructions per element, the FP64 peak
@@ -151,8 +151,8 @@ def mixed_roofline(ne, nn, prof, ms_per_step):
     alg_elem, alg_step = 72.0 * ne, 72.0 * ne + 176.0 * nn
     ach = alg_elem / (prof.element_ms * 1e-3) / 1e9
     step = alg_step / (ms_per_step * 1e-3) / 1e9
-    tr = profiled("dram_bytes_per_element", "pool_elem_kernel<MIXED>")
-    return {"bound": "hbm", "kernel": "pool_elem_kernel<MIXED>", "achieved": ach, "peak": peak, "unit": "GB/s",
+    tr = profiled("dram_bytes_per_element", "solve_elem_kernel<MIXED>")
+    return {"bound": "hbm", "kernel": "solve_elem_kernel<MIXED>", "achieved": ach, "peak": peak, "unit": "GB/s",
             "frac": ach / peak, "peak_kind": peak_kind, "traffic": tr * ne if tr else None,
             "alg_bytes_per_launch": alg_elem,
             "step": {"alg_bytes": alg_step, "achieved": step, "frac": step / peak}}
@@ -165,8 +165,8 @@ def dword_roofline(ne, nn, prof, ms_per_step):
     alg_elem, alg_step = 100.0 * ne, 100.0 * ne + 176.0 * nn
     ach = alg_elem / (prof.element_ms * 1e-3) / 1e9
     step = alg_step / (ms_per_step * 1e-3) / 1e9
-    tr = profiled("dram_bytes_per_element", "pool_elem_kernel<DW>")
-    return {"bound": "hbm", "kernel": "pool_elem_kernel<DW>", "achieved": ach, "peak": peak, "unit": "GB/s",
+    tr = profiled("dram_bytes_per_element", "solve_elem_kernel<DW>")
+    return {"bound": "hbm", "kernel": "solve_elem_kernel<DW>", "achieved": ach, "peak": peak, "unit": "GB/s",
             "frac": ach / peak, "peak_kind": peak_kind, "traffic": tr * ne if tr else None,
             "alg_bytes_per_launch": alg_elem,
             "step": {"alg_bytes": alg_step, "achieved": step, "frac": step / peak},
@@ -628,7 +628,7 @@ def main():
     ops = profiled("fp64_ops_per_element")
     opk, opk_kind = fp64_peak()
     step_gbs = alg_step / (secs / args.steps) / 1e9
-    roofline = {"bound": "hbm", "kernel": "pool_elem_kernel<FP64>", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "hbm", "kernel": "solve_elem_cnh_kernel", "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                 "traffic": tr * ne if tr else None,
                 "alg_bytes_per_launch": alg_elem, "element_kernel_ms": prof.element_ms,
@@ -641,7 +641,8 @@ def main():
                     "peak_kind": opk_kind,
                     "note": "FP64 ops/element from ncu counters (profiles/ncu_figures.json); peak: DFMA "
                             "rate with eight independent chains per thread on this GPU (msx_fp64_peak)"},
-                "note": "the kernel is bound by the FP64 pipe, not by HBM; both fractions are reported"}
+                "note": "the kernel is bound by the integer pipes (corner forces in 64-bit fixed point), "
+                        "not by HBM or the FP64 pipe; both fractions are reported"}
     # a profiling run of one other precision reports that precision's kernel
     if args.only == "mixed":
         roofline = mixed_roofline(ne, nn, prof, 1e3 * secs / args.steps)

@@ -48,7 +48,9 @@ enum { MSX_BC_RAMP = 0,      /* *BOUNDARY, TYPE=DISPLACEMENT RAMP: value reached
        MSX_BC_RAMP_RATE = 3 };/* a ramp given by its rate U/(tf - t0), the value a ramped
                                  classDirichlet stores (getUU(), classNodes.cpp:66-73)     */
 
-enum { MSX_PREC_FP64 = 0,        /* plain FP64, FMA-contracted, algebraically simplified laws */
+enum { MSX_PREC_FP64 = 0,        /* plain FP64, FMA-contracted, algebraically simplified laws;
+                                    element forces of every law but Neo-Hookean in 64-bit fixed
+                                    point, at no larger error                              */
        MSX_PREC_FP64_EXACT = 1,  /* FP64 in the reference's operation order, no contraction   */
        MSX_PREC_MIXED = 2,       /* FP32 element kinematics, stress, B^T P, J-1 and ln J (trace
                                     summed exactly); nodal u, v as double-word FP32 pairs

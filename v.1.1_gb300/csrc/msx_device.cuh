@@ -1381,7 +1381,8 @@ __device__ __forceinline__ void store_fixed_forces(const Problem &p, long long e
 // additions of f_0 are left to the FP64 pipe, against 115 operations of the same
 // formulas in FP64.
 // Per warp of 32 elements on the 6M-tet cube (ncu): 115 FP64 instructions and
-// 1020 others took 1.290 ms, FP64 pipe 86 % busy.
+// 1020 others took 1.290 ms, FP64 pipe 86 % busy; now 18 and 1350 take 0.450 ms,
+// ALU pipe 49 % busy.
 template <bool FORCE_ONLY>
 __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long e, int parity, const MatParams &m,
                                                     const int *nd, float gmin)
