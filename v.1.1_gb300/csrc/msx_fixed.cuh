@@ -1,5 +1,5 @@
-// msx_fixed.cuh -- corner forces of a compressible neo-Hookean tet in 64-bit
-// fixed point.
+// msx_fixed.cuh -- corner forces of a tet in 64-bit fixed point: compressible
+// neo-Hookean (here), St-Venant-Kirchhoff and linear elastic (fixed_setup_svk).
 //
 // The FP64 pipe of this GPU issues one warp instruction per scheduler in 64-80
 // cycles, the integer pipes one in 1-2 (multiply-add of two 32-bit limbs into
@@ -415,8 +415,12 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
 //     P = (I + H) S (linear: S),  f_a' = P (w g_a),
 // where scale 2^x0 w = |det E| W mu, 1/2 <= scale < 1.  Units: du 2^-57, w g
 // 2^-111, H to P 2^-55, scale 2^-57; every one of them below 2^57.  An error of
-// one unit in H, S or P is 2^-55, against 2^-53 for F itself in FP64.  E holds
-// w g in limbs, S[0] the scale.
+// one unit in H, S or P is 2^-55, against 2^-53 for F itself in FP64; corner-force
+// error against quad precision over that of the FP64 form, 4000 tets a case of
+// cubes and boxes of 1:0.4, nu 0 to 0.4, strains 1e-9 to 0.3: 0.2 to 0.9.  With
+// products of edges instead, E_b . E_c and their metric, it is 2 to 8 on cubes
+// and grows with the square of the flatness.  E holds w g in limbs, S[0] the
+// scale.
 MSX_HD int64_t limbs_pack(Limbs x) { return (int64_t)((uint64_t)(uint32_t)x.h << 32 | (uint32_t)x.l); }
 MSX_HD Limbs limbs_unpack(int64_t x) { return {(int32_t)(x >> 32), (int32_t)x}; }
 

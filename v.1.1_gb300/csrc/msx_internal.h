@@ -29,7 +29,8 @@ struct MatParams {
     float lambda_f, mu_f, K1_f, mu2_f, lam_stvk_f, inv_c_f, rho_f;
     float2 lambda_w, mu_w, K1_w, mu2_w, lam_stvk_w, mu3_w;   // double-word copies (mu3 = mu/3)
     // compressible neo-Hookean law in fixed point (msx_fixed.cuh): the series of
-    // c2 in units of 2^-ks, and W 2^ks
+    // c2 in units of 2^-ks, and W 2^ks.  StVK and linear elastic: lambda / mu2 in
+    // kq[0] and ks (fixed_kappa)
     int64_t kq[kFixTerms];
     double ksw;
     int ks;
