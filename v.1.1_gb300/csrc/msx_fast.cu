@@ -61,8 +61,9 @@ static void launch_solve(solve_kernel f, const Problem &p, const SolveSched &q, 
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &at;
-    c.numAttrs = n <= q.pdl ? 1 : 0;
-    cudaLaunchKernelEx(&c, f, p, size, n, sched, parity);
+    Problem P = p;
+    P.dependent = c.numAttrs = n <= q.pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, f, P, size, n, sched, parity);
 }
 
 void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)

@@ -105,6 +105,7 @@ struct Problem {
     // kernel gathers a node with two loads of one sector instead of three
     // 8-byte loads from three rows.  Null in the other modes.
     double *u4;
+    int dependent;   // this launch may begin before the one that writes u4 has ended (SolveSched::pdl)
     // plain FP64 mode: the fixed-point data of msx_fixed.cuh and the packed
     // exponents fxw (a zero word: the element takes the FP64 cofactor form).
     // Compressible neo-Hookean elements: the reference edges (9*ne:
