@@ -1,0 +1,113 @@
+"""The fixed-point corner forces compiled for the host, at and beyond the ends of
+their range: whatever they accept has to be right, against the same formulas in
+extended precision."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import test_gpu_fixed_point as cnh
+import test_gpu_fixed_stress as svk
+from test_gpu_fixed_point import EPS, N, rotation, tets
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+YOUNG = 1e6
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fixed") / "fixed.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared",
+                    os.path.join(HERE, "fixed_point_host.cpp"), "-o", so], check=True)
+    return C.CDLL(so)
+
+
+def _p(a):
+    return a.ctypes.data_as(C.c_void_p)
+
+
+def lame(nu):
+    return YOUNG * nu / ((1 + nu) * (1 - 2 * nu)), YOUNG / (1 + nu)
+
+
+def forces(lib, law, X, u, conn, nu):
+    """(forces (N, 4, 3), accepted (N,)) of the host build; law: "cnh", "stvk" or "le"."""
+    lam, mu2 = lame(nu)
+    x, w = np.ascontiguousarray(X.T[conn]), np.ascontiguousarray(u.T[conn])
+    f, taken = np.zeros(x.shape), np.zeros(len(x), np.int32)
+    n = C.c_longlong(len(x))
+    if law == "cnh":
+        lib.fixed_cnh(n, _p(x), _p(w), C.c_double(lam), C.c_double(0.5 * mu2), _p(f), _p(taken))
+    else:
+        lib.fixed_svk(n, _p(x), _p(w), C.c_int(law == "le"), C.c_double(lam), C.c_double(mu2), _p(f), _p(taken))
+    return f, taken.astype(bool)
+
+
+def reference(law, X, u, conn, nu):
+    lam, mu2 = lame(nu)
+    if law == "cnh":
+        return cnh.reference(X, u, conn, lam, 0.5 * mu2)
+    return svk.reference(X, u, conn, law == "le", lam, mu2)
+
+
+def check(lib, law, X, u, conn, nu):
+    """How many are accepted; those have to be right to the GPU tests' bound."""
+    f, taken = forces(lib, law, X, u, conn, nu)
+    with np.errstate(invalid="ignore", divide="ignore"):
+        want, scale = reference(law, X, u, conn, nu)
+        err = np.abs((f - want).astype(float)).max(-1) / (64 * EPS * scale)
+    assert not (~(err[taken] <= 1.0)).any(), (int((~(err[taken] <= 1.0)).any(1).sum()), int(taken.sum()))
+    return int(taken.sum())
+
+
+STRETCHES = [1.5, 2, 4, 8, 12, 16, 18, 20, 24, 28, 31, 32, 33, 63.5, 64, 65, 100, 128, 1000, 1e6, 1e30]
+
+
+@pytest.mark.parametrize("law", ["cnh", "stvk", "le"])
+@pytest.mark.parametrize("along", ["x", "y", "z", "all"])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_stretches(lib, law, along, sign):
+    rng = np.random.default_rng(7)
+    X, conn = tets(rng, 1.0, 1.0)
+    x = X.T[conn]
+    for s in STRETCHES:
+        F = np.eye(3)
+        for i in range(3) if along == "all" else ["xyz".index(along)]:
+            F[i, i] = sign * s
+        y = np.einsum("ij,naj->nai", F, x - x[:, :1]) + x[:, :1]
+        check(lib, law, X, np.ascontiguousarray((y - x).reshape(4 * N, 3).T), conn, 0.3)
+
+
+@pytest.mark.parametrize("law", ["cnh", "stvk", "le"])
+@pytest.mark.parametrize("component", [0, 1, 2])
+@pytest.mark.parametrize("node", [0, 1, 2, 3])
+def test_one_node_moved(lib, law, component, node):
+    """Unit corner tets, one node of each displaced by just under, at and over multiples of the edge length."""
+    ref = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
+    d = np.concatenate([k * np.array([0.97, 1 - 2.0 ** -20, 1, 1 + 2.0 ** -20, 1.03])
+                        for k in (1, 2, 4, 8, 15, 16, 31, 32, 33, 48, 63.5, 64, 96, 128, 1000, 2.0 ** 20, 2.0 ** 40)])
+    d = np.concatenate([d, -d])
+    n = len(d)
+    X = np.ascontiguousarray(np.tile(ref, (n, 1)).T)
+    conn = np.arange(4 * n, dtype=np.int32).reshape(n, 4)
+    u = np.zeros((3, 4 * n))
+    u[component, node::4] = d
+    check(lib, law, X, u, conn, 0.3)
+
+
+@pytest.mark.parametrize("law", ["cnh", "stvk", "le"])
+def test_graded_edges(lib, law):
+    """Tets whose three edges differ by up to 1:12, stretched along each axis."""
+    rng = np.random.default_rng(11)
+    for grade in ([1, 1, 12], [1, 5, 12], [12, 1, 3]):
+        X, conn = tets(rng, 1.0, 1.0)
+        X = X * np.array(grade, float)[:, None]
+        x = X.T[conn]
+        for s in (1.01, 1.7, 2.5, 9, 17, 33, 65):
+            for i in range(3):
+                F = np.eye(3)
+                F[i, i] = s
+                y = np.einsum("ij,naj->nai", F, x - x[:, :1]) + x[:, :1]
+                check(lib, law, X, np.ascontiguousarray((y - x).reshape(4 * N, 3).T), conn, 0.3)

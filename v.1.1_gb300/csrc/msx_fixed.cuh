@@ -15,8 +15,8 @@
 //     f_a w_a = sum_b (S_ab w_a w_b) n_b + (c2 w_1 w_2 w_3) (n_c x n_d)
 // has one unit for the nine products of a kind.
 //
-// Sizes.  |E_b| < 2^57 w_b, components of n_b below 2^58 (a stretch of two at
-// least); cross products in units of 2^57, below 2^60; S below 2^57 and c2
+// Sizes.  |E_b| < 2^57 w_b, components of n_b below 2^58 - 2^32 (a stretch of two
+// at least); cross products in units of 2^57, below 2^60 - 2^34; S below 2^57 and c2
 // below 2^59; sums of a force in units of 2^58, below 2^61.3.  Numbers are split into a high and a signed 29-bit low limb,
 // whose products fit 64-bit accumulators.  Products of two low limbs are left
 // out; with the final shifts that drops half a unit of 2^-55 to 2^-56 of the
@@ -96,6 +96,15 @@ MSX_HD int64_t mulhi_near(int32_t h, int32_t l, int64_t b)
     const int32_t bh = (int32_t)(b >> 32), bl = (int32_t)((uint32_t)b >> 1);
     const int64_t t = mad_wide(l, bh, mad_wide(h, bl, 0));
     return mad_wide(h, bh, t >> 31);
+}
+
+MSX_HD uint32_t abs32(int32_t x)   // 2^31 for -2^31
+{
+#ifdef __CUDA_ARCH__
+    return (uint32_t)abs(x);   // one instruction; with shift and exclusive or 2 % off a step of 6M tets
+#else
+    return x < 0 ? 0u - (uint32_t)x : (uint32_t)x;
+#endif
 }
 
 MSX_HD int top_bit(int64_t x)   // floor(log2 x), x > 0
@@ -212,7 +221,9 @@ MSX_HD void fixed_unpack(uint32_t w0, uint32_t w1, FixedElem &q)
 
 // The deformed edges n_b = (E_b + u_b - u_0) / w_b in limbs, exact up to the
 // final rounding and the bits of u below the smallest w; false for a component
-// beyond 2^58, infinities and NaN.  Displacements beyond 2^62 of the smallest w
+// of 2^58 - 2^32 and more (judged before limbs(), whose high half is the value
+// modulo 2^61), a motion of 2^62 of the smallest w and more, infinities and NaN.
+// Displacements beyond 2^62 of the smallest w
 // (32 edge lengths at least) are taken in a unit 2^k times larger, whose lost
 // bits lie 2^-9 below u's own last one.  moved: an upper bound of
 // max |u_b - u_0| component by component, in units of 2^32 of the smallest w.
@@ -251,23 +262,23 @@ MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int 
         }
         if (far) return false;
     }
-    uint32_t out = 0;
-    int m = 0;
+    uint32_t m = 0, most = 0;
 #pragma unroll
     for (int b = 0; b < 3; b++) {
         const int d = MOTION ? 0 : q.lw[b] - lw;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const int64_t du = U[b + 1][i] - U[0][i];
-            const int dh = (int)(du >> 32);
-            const int da = dh ^ (dh >> 31);
+            const uint32_t da = abs32((int)(du >> 32));
             m = m > da ? m : da;
-            n[3 * b + i] = limbs(MOTION ? du : (q.E[3 * b + i] + du) >> d);
-            out |= (uint32_t)(n[3 * b + i].h + (1 << 29));
+            const int64_t x = MOTION ? du : (int64_t)((uint64_t)q.E[3 * b + i] + (uint64_t)du) >> d;
+            const uint32_t xa = abs32((int)(x >> 32));
+            most = most > xa ? most : xa;
+            n[3 * b + i] = limbs(x);
         }
     }
-    moved = m + 1;
-    return out < (1u << 30);
+    moved = m < (1u << 30) ? (int)m + 1 : 1 << 30;
+    return m < (1u << 30) && most < (1u << 26) - 1;
 }
 
 // Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of
