@@ -1243,7 +1243,7 @@ __device__ __forceinline__ float f32_trunc(double x)
 // over the sound speed.  Elements above (1 + 2^-8) times the solve's running
 // minimum cannot hold the step's minimum and skip the screen: about 200 FP32
 // instructions an element, for 12 to 30.  A reference sliver (negative Lref32)
-// and NaN never pass.  Element kernels with and without: mixed, 6M tets 0.164
+// and NaN never skip it.  Element kernels with and without: mixed, 6M tets 0.164
 // and 0.185 ms; reference order, 384 K tets 0.208 and 0.247; FP64, 6M tets 0.621
 // and 0.647; double-word, 1.57M tets 0.1165 and 0.1214.  (On a mesh of equal
 // elements everything is near the minimum and passes to the screen as before.)
@@ -1251,7 +1251,9 @@ __device__ __forceinline__ float gate_frobenius(float Lr, float hh, float inv_c)
 {
     float s;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(hh));
-    return Lr * (0.9995f - s) * inv_c;   // the margin covers sqrt.approx and the rounding of H
+    // the margin covers sqrt.approx and the rounding of H; s times |L_ref|, so that no motion makes a sliver's
+    // negative length a large gate
+    return (Lr * 0.9995f - fabsf(Lr) * s) * inv_c;
 }
 
 __device__ __forceinline__ float gate_moved(float Lr, float d, float inv_c) { return (Lr - 2.002f * d) * inv_c; }
