@@ -50,7 +50,11 @@ enum { MSX_BC_RAMP = 0,      /* *BOUNDARY, TYPE=DISPLACEMENT RAMP: value reached
 
 enum { MSX_PREC_FP64 = 0,        /* plain FP64, FMA-contracted, algebraically simplified laws;
                                     element forces of every law but Neo-Hookean in 64-bit fixed
-                                    point, at no larger error                              */
+                                    point.  Its rounding is 2^-55 of the element's largest
+                                    stress (St-Venant-Kirchhoff, linear elastic) or stiffness
+                                    (compressible Neo-Hookean), FP64's own 2^-53; only where
+                                    FP64's products happen to be exact (grids whose sides are
+                                    powers of two) can plain FP64 come closer               */
        MSX_PREC_FP64_EXACT = 1,  /* FP64 in the reference's operation order, no contraction   */
        MSX_PREC_MIXED = 2,       /* FP32 element kinematics, stress, B^T P, J-1 and ln J (trace
                                     summed exactly); nodal u, v as double-word FP32 pairs

@@ -111,3 +111,71 @@ def test_graded_edges(lib, law):
                 F[i, i] = s
                 y = np.einsum("ij,naj->nai", F, x - x[:, :1]) + x[:, :1]
                 check(lib, law, X, np.ascontiguousarray((y - x).reshape(4 * N, 3).T), conn, 0.3)
+
+
+# ------------------------------------------------------------------ accuracy against the FP64 forms
+SPLIT = np.array([(1, 3, 4, 7), (1, 2, 3, 7), (4, 1, 7, 8), (1, 5, 7, 8), (1, 5, 6, 7), (2, 1, 6, 7)]) - 1
+CORNER = np.array([(0, 0, 0), (1, 0, 0), (1, 1, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1), (1, 1, 1), (0, 1, 1)])
+SHEAR = np.zeros((3, 3))
+SHEAR[0, 2] = 1
+MOTIONS = {
+    "simple shear": SHEAR,
+    "pure shear": SHEAR + SHEAR.T,
+    "shears in three planes": np.array([[0, 1, 0.3], [0.2, 0, -0.7], [0.5, 0.4, 0]]),
+    "pulled": np.diag([-0.3, -0.3, 1]),
+    "swollen": np.eye(3),
+    "general": np.array([[0.3, 1, 0.3], [0.2, -0.4, -0.7], [0.5, 0.4, 0.6]]),
+}
+
+
+def grid(n, h, jitter):
+    """n^3 hexes of sides h, six tets each, nodes jittered by `jitter` h; X (3, nn), conn."""
+    rng = np.random.default_rng(1)
+    at = np.stack(np.meshgrid(*[np.arange(n + 1)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    X = at * np.array(h) + jitter * np.array(h) * rng.uniform(-1, 1, at.shape)
+    cell = np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), -1).reshape(-1, 1, 1, 3) + CORNER[SPLIT][None]
+    conn = ((cell[..., 0] * (n + 1) + cell[..., 1]) * (n + 1) + cell[..., 2]).reshape(-1, 4)
+    return np.ascontiguousarray(X.T), conn.astype(np.int32)
+
+
+def forces_fp64(lib, law, X, u, conn, nu):
+    lam, mu2 = lame(nu)
+    x, w = np.ascontiguousarray(X.T[conn]), np.ascontiguousarray(u.T[conn])
+    f, n = np.zeros(x.shape), C.c_longlong(len(x))
+    if law == "cnh":
+        lib.fp64_cnh(n, _p(x), _p(w), C.c_double(lam), C.c_double(0.5 * mu2), _p(f))
+    else:
+        lib.fp64_svk(n, _p(x), _p(w), C.c_int(law == "le"), C.c_double(lam), C.c_double(mu2), _p(f))
+    return f
+
+
+def rms_errors(lib, law, h, jitter, motion, strain, nu):
+    """Root mean squares of the fixed-point and of the FP64 form's corner-force errors over that of the forces."""
+    X, conn = grid(4, h, jitter)
+    u = strain * (MOTIONS[motion] @ X)
+    f, taken = forces(lib, law, X, u, conn, nu)
+    assert taken.all()
+    want = reference(law, X, u, conn, nu)[0]
+    rms = lambda e: float(np.sqrt((e ** 2).sum() / (want ** 2).sum()))
+    return rms(f - want), rms(forces_fp64(lib, law, X, u, conn, nu) - want)
+
+
+@pytest.mark.parametrize("motion", list(MOTIONS))
+@pytest.mark.parametrize("h,jitter", [((0.1,) * 3, 0.0), ((0.1,) * 3, 0.1), ((0.125,) * 3, 0.0), ((0.1, 0.1, 0.3), 0.0),
+                                      ((0.1, 0.1, 0.04), 0.0)])
+@pytest.mark.parametrize("law", ["le", "stvk"])
+def test_no_less_accurate_than_fp64(lib, law, h, jitter, motion):
+    """At or below the FP64 form's error at every strain, or below two roundings of the result (where the FP64 form's
+    own products happen to be exact); twice its error at strains whose roundings both forms share (0.1)."""
+    for nu in (0.0, 0.3, 0.49):
+        for strain in (0.1, 1e-2, 1e-3, 1e-5, 1e-7, 1e-9, 1e-12):
+            ours, theirs = rms_errors(lib, law, h, jitter, motion, strain, nu)
+            assert ours <= max((2 if strain > 0.05 else 1) * theirs, 2 * EPS), (nu, strain, ours, theirs)
+
+
+@pytest.mark.parametrize("motion", list(MOTIONS))
+def test_no_less_accurate_than_fp64_cnh(lib, motion):
+    for nu in (0.0, 0.3, 0.49):
+        for strain in (1e-2, 1e-3, 1e-5, 1e-7, 1e-9):
+            ours, theirs = rms_errors(lib, "cnh", (0.1,) * 3, 0.1, motion, strain, nu)
+            assert ours <= max(theirs, 2 * EPS), (nu, strain, ours, theirs)

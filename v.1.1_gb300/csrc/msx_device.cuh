@@ -1258,17 +1258,22 @@ __device__ __forceinline__ float gate_frobenius(float Lr, float hh, float inv_c)
 
 __device__ __forceinline__ float gate_moved(float Lr, float d, float inv_c) { return (Lr - 2.002f * d) * inv_c; }
 
-// An upper bound of max_k |x_k| of FP64 values from their high words; infinite
-// (or NaN) when it leaves FP32's range.
+// An upper bound of max_k |x_k| of FP64 values from the largest of their high
+// words m; infinite (or NaN) when it leaves FP32's range.
+__device__ __forceinline__ float abs_bound_hi(int m)
+{
+    // high word: 11 exponent bits biased by 1023, 20 of the mantissa's; modulo 2^32
+    const unsigned f = ((unsigned)(m + 1) << 3) - ((unsigned)(1023 - 127) << 23);
+    return m >= ((1023 + 100) << 20) ? INFINITY : (m <= ((1023 - 100) << 20) ? 0x1p-99f : __uint_as_float(f));
+}
+
 template <int N>
 __device__ __forceinline__ float abs_bound(const double *x)
 {
     int m = 0;
 #pragma unroll
-    for (int k = 0; k < N; k++) m = max(m, __double2hiint(x[k]) & 0x7FFFFFFF);
-    // high word: 11 exponent bits biased by 1023, 20 of the mantissa's; modulo 2^32
-    const unsigned f = ((unsigned)(m + 1) << 3) - ((unsigned)(1023 - 127) << 23);
-    return m >= ((1023 + 100) << 20) ? INFINITY : (m <= ((1023 - 100) << 20) ? 0x1p-99f : __uint_as_float(f));
+    for (int k = 0; k < N; k++) m = max(m, abs_hi(x[k]));
+    return abs_bound_hi(m);
 }
 
 // FP32 estimate of an element's CFL value: the reference edges X_b - X_0 are
@@ -1445,7 +1450,7 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
 // differences, the displacement gradient and the stress in 64-bit fixed point
 // (msx_fixed.cuh); 99 products of limb pairs in place of about 190 FP64
 // operations.  264,000 shuffled tets, StVK: 86 us in FP64, the FP64 pipe its
-// bound, 42 us now, bound by the integer pipes and the scattered slot writes.
+// bound, 44 us now, bound by the integer pipes and the scattered slot writes.
 // ACT: element birth, whose dead elements have no force.
 template <bool FORCE_ONLY, bool ACT>
 __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long e, int parity, double t,
@@ -1461,22 +1466,29 @@ __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long 
 #pragma unroll
     for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
     q.S[0] = limbs_unpack(__ldg(&p.fxD[e].x));
-    Limbs du[9];
-    int moved;
-    if (!fixed_edges<true>(q, ua, du, moved)) return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    double x[9];
+    int hi = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        x[k] = ua[k / 3 + 1][k % 3] - ua[0][k % 3];
+        hi = max(hi, abs_hi(x[k]));
+    }
     float scr = INFINITY;
-    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(q.lw[0] + 32)), m.inv_c_f) > gmin)) {
+    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound_hi(hi), m.inv_c_f) > gmin)) {
         float du32[9], g32[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-            du32[k] = (float)du[k].h * pow2f_or_inf(q.lw[0] + 29);
+            du32[k] = f32_trunc(x[k]);
             g32[k] = (float)limbs_unpack(q.E[k]).h * pow2f_or_inf(29 - 111 - q.lw[0]);
         }
         scr = cfl_screen(p, e, g32, du32, m);
     }
+    Limbs du[9];
     int64_t f[9];
-    if (!fixed_forces_svk(q, du, m.law == 3, m.kq[0], m.ks, f))
+    int s;
+    if (!fixed_motion(q, x, hi, m.law == 3, du, s) || !fixed_forces_svk(q, du, m.law == 3, m.kq[0], m.ks, f, s))
         return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    q.x0 += s;
     if (ACT && elem_dead(p, e, t))
 #pragma unroll
         for (int k = 0; k < 9; k++) f[k] = 0;

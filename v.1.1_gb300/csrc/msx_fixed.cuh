@@ -45,6 +45,7 @@ constexpr int kFixShort = 9;    // those that |1 - J| < 2^-7 needs
 // formulas in FP64, 5000 random tets a case, nu 0 to 0.49, strains to 3 %: 0.3
 // to 0.5 (0.05 undeformed) above 0.25, 0.4 to 0.8 around 0.15, 1.1 at 0.06.
 constexpr double kFixFlat = 0.12;
+constexpr int kFixMotionLeast = 64;   // exponent field of a motion that fixed_motion takes
 
 struct Limbs {
     int32_t h, l;   // h 2^29 + l, |l| <= 2^28
@@ -191,7 +192,7 @@ struct FixedElem {
     int64_t d0, rd;
     int32_t lw[3];   // log2 w_b
     int32_t x0;      // log2 of f_a's unit = x0 - lw_a
-    int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t)
+    int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t); StVK: sum_b |w g_b| <= 2^(cs + 2) / 2^57
     int32_t ds;
 };
 
@@ -227,11 +228,9 @@ MSX_HD void fixed_unpack(uint32_t w0, uint32_t w1, FixedElem &q)
 // (32 edge lengths at least) are taken in a unit 2^k times larger, whose lost
 // bits lie 2^-9 below u's own last one.  moved: an upper bound of
 // max |u_b - u_0| component by component, in units of 2^32 of the smallest w.
-// MOTION: without E_b (all w_b equal), the differences of displacement alone.
-template <bool MOTION = false>
 MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int &moved)
 {
-    const int lw = MOTION ? q.lw[0] : fixed_lw_min(q);
+    const int lw = fixed_lw_min(q);
     int emax = 0;
 #pragma unroll
     for (int a = 0; a < 4; a++)
@@ -265,13 +264,13 @@ MSX_HD bool fixed_edges(const FixedElem &q, const double (*u)[3], Limbs *n, int 
     uint32_t m = 0, most = 0;
 #pragma unroll
     for (int b = 0; b < 3; b++) {
-        const int d = MOTION ? 0 : q.lw[b] - lw;
+        const int d = q.lw[b] - lw;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const int64_t du = U[b + 1][i] - U[0][i];
             const uint32_t da = abs32((int)(du >> 32));
             m = m > da ? m : da;
-            const int64_t x = MOTION ? du : (int64_t)((uint64_t)q.E[3 * b + i] + (uint64_t)du) >> d;
+            const int64_t x = (int64_t)((uint64_t)q.E[3 * b + i] + (uint64_t)du) >> d;
             const uint32_t xa = abs32((int)(x >> 32));
             most = most > xa ? most : xa;
             n[3 * b + i] = limbs(x);
@@ -419,19 +418,28 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
 // St-Venant-Kirchhoff and linear elasticity: the displacement gradient and the
 // stress in the axes of space, as in FP64 (products of the edges would lose
 // accuracy with the square of an element's flatness).  With the shape
-// functions' gradients g_a, one unit w for all three edges and
-// du_b = (u_b - u_0) / w, f_a = f_a' |det E| W mu / w:
-//     H = sum_b du_b (w g_b),  G = H + H^T + H^T H (linear: without H^T H),
+// functions' gradients g_a, one unit w for all three edges, and a unit 2^s for
+// the strain that follows from the largest |u_b - u_0| (a state of strain 1e-9
+// has all its bits; in linear elasticity it also grows with the motion),
+// du_b = (u_b - u_0) / (w 2^s) and f_a = f_a' 2^s |det E| W mu / w:
+//     H = sum_b du_b (w g_b),  G = H + H^T + 2^s H^T H (linear: without H^T H),
 //     S = scale (G + kappa tr(G) I),  kappa = lambda / (2 mu),
-//     P = (I + H) S (linear: S),  f_a' = P (w g_a),
+//     P = S + 2^s H S (linear: S),  f_a' = P (w g_a),
 // where scale 2^x0 w = |det E| W mu, 1/2 <= scale < 1.  Units: du 2^-57, w g
-// 2^-111, H to P 2^-55, scale 2^-57; every one of them below 2^57.  An error of
-// one unit in H, S or P is 2^-55, against 2^-53 for F itself in FP64; corner-force
-// error against quad precision over that of the FP64 form, 4000 tets a case of
-// cubes and boxes of 1:0.4, nu 0 to 0.4, strains 1e-9 to 0.3: 0.2 to 0.9.  With
-// products of edges instead, E_b . E_c and their metric, it is 2 to 8 on cubes
-// and grows with the square of the flatness.  E holds w g in limbs, S[0] the
-// scale.
+// 2^-111, H to P 2^-55, scale 2^-57, du so small that |H| < 2^57 (FixedElem::cs).
+// G and what follows it take a unit 2^t larger where kappa tr(G) asks for it.
+// An error of one unit in H, S or P is 2^-55 of the largest of them, against
+// 2^-53 of 1 for F's diagonal in FP64, whatever the strain.  Corner-force error
+// against extended precision over that of the FP64 form, grids of hexes of
+// 1:1:0.4 to 1:1:3, six tets each, jittered and not, nu 0 to 0.49, strains 1e-14 to 0.3: median 0.002
+// (linear) and 0.0004; above 1 only where both are below 1.5 roundings of the
+// result (grids whose sides are powers of two, on which FP64's own products can
+// be exact) or, to 1.2, at strains of 0.3.  One StVK step of 264,000 shuffled
+// tets: 64.7 us, 63.0 with a unit set by the element alone, whose error at a
+// shear of 1e-5 on a cubic grid was 8,700 (linear) and 4.4 times FP64's.  With
+// products of edges instead, E_b . E_c and their metric, the error is 2 to 8
+// times FP64's on cubes and grows with the square of the flatness.  E holds w g
+// in limbs, S[0] the scale, both rounded from 128-bit products.
 MSX_HD int64_t limbs_pack(Limbs x) { return (int64_t)((uint64_t)(uint32_t)x.h << 32 | (uint32_t)x.l); }
 MSX_HD Limbs limbs_unpack(int64_t x) { return {(int32_t)(x >> 32), (int32_t)x}; }
 
@@ -450,8 +458,7 @@ inline void fixed_kappa(double mu2, double lambda, int64_t *kq, int *ks)
 // false: the element is left to FP64 (see fixed_setup; w g beyond 4 to 8)
 MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
 {
-    Limbs n[9], cl[9];
-    int64_t c[9];
+    int64_t n[9], c[9];
     double l2 = 0;
     for (int b = 0; b < 3; b++) {
         const double x = E[3 * b] * E[3 * b] + E[3 * b + 1] * E[3 * b + 1] + E[3 * b + 2] * E[3 * b + 2];
@@ -460,36 +467,81 @@ MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
     }
     const int lw = (((int)(double_bits(l2) >> 52) - 1023) >> 1) + 1 - 57;
     q.lw[0] = q.lw[1] = q.lw[2] = lw;
-    for (int k = 0; k < 9; k++) n[k] = limbs(fixed_from(E[k], lw));
-    for (int a = 0; a < 3; a++) {
-        fixed_cross(n + 3 * ((a + 1) % 3), n + 3 * ((a + 2) % 3), c + 3 * a);
-        for (int i = 0; i < 3; i++) cl[3 * a + i] = limbs(c[3 * a + i]);
-    }
-    q.d0 = fixed_det(n, cl);
-    if (q.d0 < (1LL << 50) || q.d0 >= (1LL << 62)) return false;
+    // edges in units of w 2^-5, cross products of w^2 2^51 and det E of w^3 2^108, all below 2^63
+    for (int k = 0; k < 9; k++) n[k] = fixed_from(E[k], lw - 5);
+    __int128 det = 0;
+    for (int a = 0; a < 3; a++)
+        for (int i = 0; i < 3; i++) {
+            const int64_t *p = n + 3 * ((a + 1) % 3), *r = n + 3 * ((a + 2) % 3);
+            const int y = (i + 1) % 3, z = (i + 2) % 3;
+            c[3 * a + i] = (int64_t)(((__int128)p[y] * r[z] - (__int128)p[z] * r[y] + ((__int128)1 << 60)) >> 61);
+            if (a == 0) det += (__int128)n[i] * c[i];
+        }
+    q.d0 = (int64_t)(det >> 62);
+    if (q.d0 < (1LL << 56)) return false;
     fixed_reciprocal(q);
-    for (int k = 0; k < 9; k++) {
-        const int64_t x = mulhi64((int64_t)((uint64_t)c[k] << 5), q.rd);   // c / d0 2^(ds + 3)
-        const int sh = q.ds - 51;
-        const int64_t g = sh > 0 ? (x + (1LL << (sh - 1))) >> sh : (int64_t)((uint64_t)x << -sh);
+    int64_t sum[3] = {0, 0, 0};
+    for (int k = 0; k < 9; k++) {   // c / det E 2^111 / w
+        const int64_t g = (int64_t)(((__int128)c[k] * q.rd + ((__int128)1 << (7 + q.ds))) >> (8 + q.ds));
         if (g >= (1LL << 57) || g <= -(1LL << 57)) return false;
+        sum[k % 3] += g < 0 ? -g : g;
         q.E[k] = limbs_pack(limbs(g));
     }
-    const double s = 0.166666666667 * ((double)q.d0 * pow2_double(-q.ds)) * mu;   // |det E| W mu = s 2^(ds + 114 + 3 lw)
-    if (ks < 0 || !(s < 1e100) || !(s > 1e-100)) return false;
-    const int x = (int)(double_bits(s) >> 52) - 1022;
-    q.S[0] = limbs((int64_t)(s * pow2_double(57 - x)));
+    // |du| < 2^(57 - cs) makes |H| < 2^57: sum_b |w g_b| <= 2^(56 + cs), component by component
     q.cs = 0;
-    q.x0 = x + q.ds + 114 + 3 * lw - 109;
+    while (sum[0] > 1LL << (56 + q.cs) || sum[1] > 1LL << (56 + q.cs) || sum[2] > 1LL << (56 + q.cs)) q.cs++;
+    // |det E| W mu = scale 2^x w^3, 1/2 <= scale < 1, to the scale's 57 bits
+    if (ks < 0 || !(mu < 1e100) || !(mu > 1e-100)) return false;
+    const int xm = (int)(double_bits(mu) >> 52) - 1022;
+    const int64_t wm = (int64_t)(((__int128)fixed_from(0.166666666667, -64) * fixed_from(mu, xm - 62)) >> 62);
+    const int64_t v = (int64_t)(((__int128)wm * (q.d0 << (62 - q.ds))) >> 62);   // W mu det E 2^(64 - xm - ds - 108)
+    const int tv = top_bit(v);   // 59 to 62
+    q.S[0] = limbs((v + (1LL << (tv - 57))) >> (tv - 56));
+    q.x0 = tv + 1 - 64 + xm + q.ds + 108 + 3 * lw - 109;
     return q.x0 - lw <= 900 && q.x0 - lw >= -900;
 }
 
-// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of 2^(x0 - lw);
-// du: fixed_edges<true>; kq, ks: fixed_kappa.  false: beyond the sizes above.
-MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, int64_t kq, int ks, int64_t *f)
+// x 2^-r rounded to nearest, 0 <= r <= 61, |x| < 2^62.9
+MSX_HD int64_t shift_round(int64_t x, int r) { return (x + (int64_t)((1ull << r) >> 1)) >> r; }
+
+MSX_HD int32_t high_word(int64_t x) { return (int32_t)(x >> 32); }
+
+// The motion x[3(b-1) + i] = u_b - u_0 in limbs and the exponent s of its unit
+// w 2^s; hi: the largest high word of |x|.  s <= 0 with H^T H, whose elements
+// larger motions leave to FP64.  false: infinities, NaN, a motion beyond 2^58
+// of w, forces near the ends of the FP64 range.
+MSX_HD bool fixed_motion(const FixedElem &q, const double *x, int hi, bool linear, Limbs *du, int &s)
+{
+    if (hi < kFixMotionLeast << 20) {   // at rest, or nearly
+        uint64_t any = 0;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            any |= double_bits(x[k]) << 1;
+            du[k] = {0, 0};
+        }
+        s = 0;
+        return any == 0;
+    }
+    const int e = (hi >> 20) - 1022;   // |x| < 2^e
+    int lu = e - 57 + (linear ? 0 : q.cs);
+    if (!linear && lu > q.lw[0]) lu = q.lw[0];
+    s = lu - q.lw[0];
+    const int unit = q.x0 + s - q.lw[0];
+#pragma unroll
+    for (int k = 0; k < 9; k++) du[k] = limbs(fixed_from(x[k], lu));
+    return hi < 0x7FF << 20 && e - lu <= 58 && unit <= 870 && unit >= -870;
+}
+
+// Corner forces f_1..f_3 (f[3(a-1) + i]) as integers in units of
+// 2^(x0 - lw + s), s as it returns; du, s: fixed_motion; kq, ks: fixed_kappa.
+// false: beyond the sizes above.  Every bound is judged on 64-bit values.
+MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, int64_t kq, int ks, int64_t *f, int &s)
 {
     Limbs g[9], H[9], S[6];
     uint32_t out = 0;
+    // the products of H, when there are any, go 2^r below G's unit; half of that unit begins their sums
+    const int r = s < -61 ? 61 : -s;
+    const int64_t half_hh = r > 36 ? 1LL << (r - 4) : 0, half_mid = r > 36 ? 0 : 1LL << (25 + r);
 #pragma unroll
     for (int k = 0; k < 9; k++) g[k] = limbs_unpack(q.E[k]);
     int64_t h[9], G[6];
@@ -502,8 +554,9 @@ MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, i
             for (int b = 0; b < 3; b++) mac(hh, mid, du[3 * b + i], g[3 * b + j]);
             h[3 * i + j] = mac_sum(hh, mid, 2);
             H[3 * i + j] = limbs(h[3 * i + j]);
-            out |= (uint32_t)(H[3 * i + j].h + (1 << 28));
+            out |= (uint32_t)(high_word(h[3 * i + j]) + (1 << 25));   // 2^57
         }
+    if (!linear && out >= (1u << 26)) return false;
     int k = 0;
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -515,28 +568,44 @@ MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, i
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = i; j < 3; j++) {
-                int64_t hh = 0, mid = mac_half(3);
+                int64_t hh = half_hh, mid = half_mid;
 #pragma unroll
-                for (int r = 0; r < 3; r++) mac(hh, mid, H[3 * r + i], H[3 * r + j]);
-                G[k++] += mac_sum(hh, mid, 3);
+                for (int b = 0; b < 3; b++) mac(hh, mid, H[3 * b + i], H[3 * b + j]);
+                G[k++] += mac_sum(hh, mid, 3) >> r;
             }
+    } else {   // |H| < 2^(57 + cs): G to 2^58, by up to 25 bits where a spin cancelled in it
+        uint32_t any = 1;
+#pragma unroll
+        for (k = 0; k < 6; k++) any |= abs32(high_word(G[k]));
+        const int d = top_bit(any) - 25, right = d > 0 ? d : 0, left = right - d;
+#pragma unroll
+        for (k = 0; k < 6; k++) G[k] = (int64_t)((uint64_t)shift_round(G[k], right) << left);
+        s += d;
     }
-    const int64_t tr = G[0] + G[3] + G[5], most = 1LL << (57 - ks);
-    if (out >= (1u << 29) || tr >= most || tr <= -most) return false;
-    // rounded to nearest: a truncation is a pressure on every element of the body
-    int64_t th = 0, tm = mac_half(1 + ks);
+    const int64_t tr = G[0] + G[3] + G[5], ta = tr < 0 ? -tr : tr;
+    if (ta >= (1LL << 60) - (1LL << 29)) return false;
+    // kappa tr < 2^(ks + 1 + top bit of tr), below 2^57 in a unit 2^t larger; rounded to
+    // nearest (a truncation is a pressure on every element of the body)
+    int t = ta ? ks + top_bit(ta) - 56 : 0;
+    t = t > 0 ? t : 0;
+    const int kk = 1 + ks - t, kd = kk < 0 ? -kk : 0;   // kk >= -2
+    int64_t th = 0, tm = 1LL << (28 - kk);
     mac(th, tm, limbs(tr), limbs_unpack(kq));
-    const int64_t kt = mac_sum(th, tm, 1 + ks);
-    G[0] += kt;
-    G[3] += kt;
-    G[5] += kt;
+    const int64_t kt = mac_sum(th, tm, kk + kd) >> kd;
+    if (t > 0) {
+        s += t;
+#pragma unroll
+        for (k = 0; k < 6; k++) G[k] = shift_round(G[k], t);
+    }
+    out = 0;
 #pragma unroll
     for (k = 0; k < 6; k++) {
-        const Limbs x = limbs(G[k]);
-        out |= (uint32_t)(x.h + (1 << 28));
+        const int64_t x = G[k] + (k == 0 || k == 3 || k == 5 ? kt : 0);
+        out |= (uint32_t)(high_word(x) + (1 << 27));   // 2^59
         int64_t hh = 0, mid = mac_half(1);
-        mac(hh, mid, x, q.S[0]);
-        S[k] = limbs(mac_sum(hh, mid, 1));
+        mac(hh, mid, limbs(x), q.S[0]);
+        G[k] = mac_sum(hh, mid, 1);
+        S[k] = limbs(G[k]);
     }
     const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
     Limbs P[9];
@@ -545,19 +614,18 @@ MSX_HD bool fixed_forces_svk(const FixedElem &q, const Limbs *du, bool linear, i
         for (k = 0; k < 9; k++) P[k] = S[mi[k]];
     } else {
 #pragma unroll
-        for (k = 0; k < 3; k++) H[4 * k].h += 1 << 26;   // I + H
-#pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                int64_t hh = 0, mid = mac_half(3);
+                int64_t hh = half_hh, mid = half_mid;
 #pragma unroll
-                for (int r = 0; r < 3; r++) mac(hh, mid, H[3 * i + r], S[mi[3 * r + j]]);
-                P[3 * i + j] = limbs(mac_sum(hh, mid, 3));
-                out |= (uint32_t)(P[3 * i + j].h + (1 << 28));
+                for (int b = 0; b < 3; b++) mac(hh, mid, H[3 * i + b], S[mi[3 * b + j]]);
+                const int64_t x = G[mi[3 * i + j]] + (mac_sum(hh, mid, 3) >> r);
+                out |= (uint32_t)(high_word(x) + (1 << 27));
+                P[3 * i + j] = limbs(x);
             }
     }
-    if (out >= (1u << 29)) return false;
+    if (out >= (1u << 28)) return false;
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
