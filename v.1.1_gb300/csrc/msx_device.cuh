@@ -1221,6 +1221,53 @@ __device__ __forceinline__ double cfl_quad(const Problem &p, long long e, bool p
     return ((dist < Lr) ? dist : Lr) / c;
 }
 
+// The same value, bit for bit, by one lane: half the instructions of four lanes
+// an element, for blocks with candidates for every lane.
+static __device__ __noinline__ double cfl_lane(const Problem &p, long long e, bool pairs)
+{
+    const long long nn = p.nn;
+    const int4 cn = p.conn[e];
+    const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
+    double x0[3], e1[3], e2[3], e3[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        double x[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            double u;
+            if (pairs) {
+                const float2 w = p.uhl[k * nn + nd[q]];
+                u = (double)w.x + (double)w.y;
+            } else {
+                u = p.u[k * nn + nd[q]];
+            }
+            x[q] = p.X[k * nn + nd[q]] + u;
+        }
+        x0[k] = x[0];
+        e1[k] = x[1] - x0[k];
+        e2[k] = x[2] - x0[k];
+        e3[k] = x[3] - x0[k];
+    }
+    const auto face = [](const double *a, const double *b, double *f) {
+        f[0] = fma(a[1], b[2], -__dmul_rn(a[2], b[1]));
+        f[1] = fma(a[2], b[0], -__dmul_rn(a[0], b[2]));
+        f[2] = fma(a[0], b[1], -__dmul_rn(a[1], b[0]));
+    };
+    const auto norm = [](const double *f) { return sqrt(fma(f[2], f[2], fma(f[0], f[0], __dmul_rn(f[1], f[1])))); };
+    double A[3], B[3], C[3], D[3];
+    face(e1, e2, A);
+    face(e1, e3, B);
+    face(e2, e3, C);
+#pragma unroll
+    for (int k = 0; k < 3; k++) D[k] = __dadd_rn(__dadd_rn(C[k], A[k]), -B[k]);
+    const double v6 = fabs(fma(e1[2], C[2], fma(e1[0], C[0], __dmul_rn(e1[1], C[1]))));
+    double s = __dadd_rn(norm(A), norm(B));
+    s = __dadd_rn(s, norm(C));
+    s = __dadd_rn(s, norm(D));
+    const double dist = __dmul_rn(2.0, v6) / s, Lr = p.Lref[e];
+    return ((dist < Lr) ? dist : Lr) / mat_of(p, e).c;
+}
+
 // x rounded toward zero to FP32 with integer operations only (the FP64->FP32
 // conversion instruction would take the FP64 pipe): relative error below
 // 2^-23 in FP32's normal range, signed zero below it, signed infinity above.
@@ -2719,12 +2766,21 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
                 const float thr = s_thr;
                 double v = INFINITY;
                 const int quads = blockDim.x >> 2;
-                for (int c0 = 0; c0 < nc; c0 += quads) {   // four lanes a candidate
-                    const int c = c0 + (threadIdx.x >> 2);
-                    const bool mine = c < nc && !(sval[c] > thr);
-                    if (!__any_sync(0xffffffffu, mine)) continue;
-                    const double d = cfl_quad(p, tl.begin + (mine ? scand[c] : 0), MODE == MODE_DW);
-                    if (mine) v = fmin(v, d);
+                // One lane a candidate above two passes of four lanes each: those double the
+                // instructions on the FP64 pipe and only halve their chain, and a mesh of equal
+                // elements lists nearly all of its elements (1M tets of an unjittered cube at
+                // rest: 323 us a step, 521 with four lanes throughout).
+                if (nc > 2 * quads) {
+                    for (int c = threadIdx.x; c < nc; c += blockDim.x)
+                        if (!(sval[c] > thr)) v = fmin(v, cfl_lane(p, tl.begin + scand[c], MODE == MODE_DW));
+                } else {
+                    for (int c0 = 0; c0 < nc; c0 += quads) {
+                        const int c = c0 + (threadIdx.x >> 2);
+                        const bool mine = c < nc && !(sval[c] > thr);
+                        if (!__any_sync(0xffffffffu, mine)) continue;
+                        const double d = cfl_quad(p, tl.begin + (mine ? scand[c] : 0), MODE == MODE_DW);
+                        if (mine) v = fmin(v, d);
+                    }
                 }
                 block_min_to(v, p.dtmin + (parity ^ 1));
             }
