@@ -1375,14 +1375,9 @@ template <bool FORCE_ONLY, bool ACT, bool VISC>
 __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
                                                     const MatParams &m, const int *nd, float gmin);
 
-// The cofactor form for an element that fixed point leaves out.
-template <bool FORCE_ONLY, bool ACT>
-static __device__ __noinline__ float elem_fp64_general(const Problem &p, long long e, int parity, double t, float gmin)
-{
-    const int4 cn = p.conn[e];
-    const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
-    return elem_cofactor_fp64<FORCE_ONLY, ACT, false>(p, e, parity, t, 0.0, mat_of(p, e), nd, gmin);
-}
+// What the fixed-point bodies return for an element they leave to FP64
+// (elem_left_out), whose forces are not written yet.
+constexpr float kLeftOut = -2.0f;
 
 // 2^k in FP32, infinite outside its normal range
 __device__ __forceinline__ float pow2f_or_inf(int k)
@@ -1463,14 +1458,14 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
     double ua[4][3];
     gather_u<FORCE_ONLY>(p, nd, ua);
     const uint2 w = __ldg(p.fxw + e);
-    if (w.x == 0) return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
+    if (w.x == 0) return kLeftOut;
     FixedElem q;
     fixed_unpack(w.x, w.y, q);
 #pragma unroll
     for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
     Limbs n[9];
     int moved;
-    if (!fixed_edges(q, ua, n, moved)) return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
+    if (!fixed_edges(q, ua, n, moved)) return kLeftOut;
     float scr = INFINITY;
     if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * ((float)moved * pow2f_or_inf(fixed_lw_min(q) + 32)), m.inv_c_f) > gmin)) {
         float e32[9];
@@ -1488,7 +1483,7 @@ __device__ __forceinline__ float elem_body_fp64_cnh(const Problem &p, long long 
     }
     int64_t f[9];
     if (!fixed_forces(q, n, m.kq, [&](double J) { return (int64_t)__double2ll_rn((m.mu - m.lambda * log(J)) * m.ksw / J); }, f))
-        return elem_fp64_general<FORCE_ONLY, false>(p, e, parity, 0.0, gmin);
+        return kLeftOut;
     store_fixed_forces<FORCE_ONLY>(p, e, parity, q, f);
     return scr;
 }
@@ -1507,7 +1502,7 @@ __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long 
     double ua[4][3];
     gather_u<FORCE_ONLY>(p, nd, ua);
     const uint2 w = __ldg(p.fxw + e);
-    if (w.x == 0) return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+    if (w.x == 0) return kLeftOut;
     FixedElem q;
     fixed_unpack(w.x, w.y, q);
 #pragma unroll
@@ -1534,7 +1529,7 @@ __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long 
     int64_t f[9];
     int s;
     if (!fixed_motion(q, x, hi, m.law == 3, du, s) || !fixed_forces_svk(q, du, m.law == 3, m.kq[0], m.ks, f, s))
-        return elem_fp64_general<FORCE_ONLY, ACT>(p, e, parity, t, gmin);
+        return kLeftOut;
     q.x0 += s;
     if (ACT && elem_dead(p, e, t))
 #pragma unroll
@@ -1608,6 +1603,79 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
     return scr;
 }
 
+// Compressible neo-Hookean elements that fixed point leaves out (set-up: flat,
+// graded, out of range; at a step: stretched past 2 to 4), in FP64 from their
+// deformed edges: about 110 FP64 operations against the cofactor form's 130.  Their
+// data lie in the fixed-point arrays, as FP64 bits for those left out at set-up
+// (a zero fxw).
+template <bool FORCE_ONLY>
+__device__ __forceinline__ float elem_edges_fp64(const Problem &p, long long e, int parity, const MatParams &m,
+                                                 const int *nd, const EdgeElem &d, float gmin)
+{
+    double ua[4][3], du[9], ed[9];
+    gather_u<FORCE_ONLY>(p, nd, ua);
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        du[k] = ua[k / 3 + 1][k % 3] - ua[0][k % 3];
+        ed[k] = d.E[k] + du[k];
+    }
+    float scr = INFINITY;
+    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound<9>(du), m.inv_c_f) > gmin)) {
+        float e32[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) e32[k] = f32_trunc(ed[k]);
+        scr = cfl_screen_edges(p, e, e32, e32 + 3, e32 + 6, m);
+    }
+    double f[9];
+    edge_forces(d, ed, __ldg(p.wJ + e), [&](double J) { return m.lambda * log_near1(J) - m.mu; }, f);
+    const int4 sl = __ldg(p.slot + e);
+    st_slot24(p.fe, sl.x, -(f[0] + f[3] + f[6]), -(f[1] + f[4] + f[7]), -(f[2] + f[5] + f[8]));
+    st_slot24(p.fe, sl.y, f[0], f[1], f[2]);
+    st_slot24(p.fe, sl.z, f[3], f[4], f[5]);
+    st_slot24(p.fe, sl.w, f[6], f[7], f[8]);
+    if (!FORCE_ONLY && e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
+    return scr;
+}
+
+// The FP64 form of an element that fixed point leaves out.
+template <bool FORCE_ONLY, bool ACT, int FIXED>
+static __device__ __noinline__ float elem_left_out(const Problem &p, long long e, int parity, double t, float gmin)
+{
+    const long long ne = p.ne;
+    const int4 cn = p.conn[e];
+    const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
+    const MatParams &m = mat_of(p, e);
+    if (FIXED == FIXED_CNH || (!FIXED && m.law == 1)) {
+        const uint2 w = __ldg(p.fxw + e);
+        FixedElem q;
+        EdgeElem d;
+        q.rd = __ldg(&p.fxD[e].y);
+        bool edges = true;
+        if (w.x == 0) {
+            d.rdet = bits_double((uint64_t)q.rd);
+#pragma unroll
+            for (int k = 0; k < 9; k++) d.E[k] = bits_double((uint64_t)__ldg(p.fxE + k * ne + e));
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                const int2 x = __ldg(p.fxS + k * ne + e);
+                d.S[k] = __hiloint2double(x.x, x.y);
+            }
+        } else {
+            fixed_unpack(w.x, w.y, q);
+#pragma unroll
+            for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                const int2 x = __ldg(p.fxS + k * ne + e);
+                q.S[k] = {x.x, x.y};
+            }
+            edges = edge_from_fixed(q, d);
+        }
+        if (edges) return elem_edges_fp64<FORCE_ONLY>(p, e, parity, m, nd, d, gmin);
+    }
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, false>(p, e, parity, t, 0.0, m, nd, gmin);
+}
+
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, int FIXED = FIXED_NONE>
 __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, int parity, double t = 0.0,
                                                 double idt = 0.0, float gmin = 0.0f, int4 cn_ahead = make_int4(0, 0, 0, 0))
@@ -1625,8 +1693,13 @@ __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, i
 // corner forces only (internal-force hook)
 static __global__ void __launch_bounds__(kElemBlock) elem_force_kernel_fp64(Problem p, int parity)
 {
-    long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < p.ne) elem_body_fp64<true>(p, e, parity);
+    __shared__ int left[kElemBlock], s_nleft;   // left out by fixed point: by consecutive threads at the end
+    if (threadIdx.x == 0) s_nleft = 0;
+    __syncthreads();
+    const long long b = (long long)blockIdx.x * blockDim.x, e = b + threadIdx.x;
+    if (e < p.ne && elem_body_fp64<true>(p, e, parity) == kLeftOut) left[atomicAdd(&s_nleft, 1)] = threadIdx.x;
+    __syncthreads();
+    if ((int)threadIdx.x < s_nleft) elem_left_out<true, false, FIXED_NONE>(p, b + left[threadIdx.x], parity, 0.0, 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -2593,7 +2666,7 @@ __device__ __forceinline__ void prefetch_pass(const Problem &p, long long b, lon
 // decides which elements are dead.
 template <int MODE, bool ACT, bool VISC, int FIXED = FIXED_NONE>
 __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
-                                               unsigned short *scand, int *ncand)
+                                               unsigned short *scand, int *ncand, int *nleft)
 {
     float v32 = INFINITY;
     const double t = ACT ? p.ctrl[parity].t : 0.0;
@@ -2614,10 +2687,42 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
                                                         : elem_body_fp64<false, ACT, VISC, FIXED>(p, e, parity, t, idt, gmin, cn));
         if (MODE == MODE_MIXED) {
             v32 = d < 0.0f ? -1.0f : fminf(v32, d);   // -1 sticks: fminf(-1, d) = -1 for d >= 0
+        } else if (MODE == MODE_FP64 && !VISC && d == kLeftOut) {
+            scand[kMaxTileElems - 1 - atomicAdd(nleft, 1)] = (unsigned short)(e - tl.begin);
         } else if (!(d > gmin)) {
             const int k = atomicAdd(ncand, 1);
             sval[k] = d;
             scand[k] = (unsigned short)(e - tl.begin);
+            if (d >= 0.0f) v32 = fminf(v32, d);
+        }
+    }
+    return v32;
+}
+
+// The nl elements of a tile that fixed point left out, in FP64 by consecutive
+// threads: one of them in a warp costs it the FP64 pipe as long as 32 do.  1M
+// tets in hexes of 1:1:0.2, compressible neo-Hookean, a third of them left out
+// and every warp with some: 331 us a step, 622 with the FP64 form inside their
+// warps (407 with all elements in FP64); 1:1:3, jittered, 202, 349 and 276.
+// Lists CFL candidates and returns the thread's minimum as tile_elements does.
+// Left-out elements lie at the end of scand, last one first; an element is in
+// one list at a time, and a pass reads its entries, the lowest that remain,
+// before it lists candidates, so these never reach an entry still to be read.
+template <bool ACT, int FIXED>
+__device__ __forceinline__ float tile_left_out(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
+                                               unsigned short *scand, int *ncand, int nl)
+{
+    float v32 = INFINITY;
+    const double t = ACT ? p.ctrl[parity].t : 0.0;
+    for (int at = nl - 1 - (int)threadIdx.x, base = 0; base < nl; base += blockDim.x, at -= blockDim.x) {
+        const int i = at >= 0 ? scand[kMaxTileElems - 1 - at] : 0;
+        __syncthreads();
+        if (at < 0) continue;
+        const float d = elem_left_out<false, ACT, FIXED>(p, tl.begin + i, parity, t, gmin);
+        if (!(d > gmin)) {
+            const int k = atomicAdd(ncand, 1);
+            sval[k] = d;
+            scand[k] = (unsigned short)i;
             if (d >= 0.0f) v32 = fminf(v32, d);
         }
     }
@@ -2688,7 +2793,7 @@ __device__ __forceinline__ void mixed_tile_loop(const SRC &src, TileQueue &q, in
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
             const float g = running_min(p, parity), gmin = g * (1.0f + 1.0f / 256.0f);
-            const float mine = tile_elements<MODE_MIXED, ACT, VISC>(p, tl, parity, gmin, nullptr, nullptr, nullptr);
+            const float mine = tile_elements<MODE_MIXED, ACT, VISC>(p, tl, parity, gmin, nullptr, nullptr, nullptr, nullptr);
             if (!(mine > gmin)) {
                 const int k = atomicAdd(&s_npend, 1);   // < kMixedPending: flushed below in time
                 s_pend[k] = make_int2(t, (int)threadIdx.x);
@@ -2732,14 +2837,14 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
 {
     __shared__ float sval[MODE == MODE_MIXED ? 1 : kMaxTileElems];
     __shared__ unsigned short scand[MODE == MODE_MIXED ? 1 : kMaxTileElems];
-    __shared__ int s_tile, s_ncand;
+    __shared__ int s_tile, s_ncand, s_nleft;
     __shared__ float s_thr;
     if constexpr (MODE == MODE_MIXED) {
         mixed_tile_loop<ACT, VISC>(src, q, parity);
         q.finish();
         return;
     }
-    if (threadIdx.x == 0) s_ncand = 0;
+    if (threadIdx.x == 0) s_ncand = s_nleft = 0;
     __syncthreads();
     int t = q.first(&s_tile);
     while (t < q.n) {
@@ -2747,9 +2852,17 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
         const Tile tl = src.tile(t);
         const Problem &p = src.problem(tl);
         if (p.ctrl[parity].ran) {
-            const float v32 = tile_elements<MODE, ACT, VISC, FIXED>(p, tl, parity, running_min(p, parity) * (1.0f + 1.0f / 256.0f),
-                                                             sval, scand, &s_ncand);
+            const float gmin = running_min(p, parity) * (1.0f + 1.0f / 256.0f);
+            float v32 = tile_elements<MODE, ACT, VISC, FIXED>(p, tl, parity, gmin, sval, scand, &s_ncand, &s_nleft);
             __syncthreads();
+            if constexpr (MODE == MODE_FP64 && !VISC) {
+                const int nl = s_nleft;
+                if (nl > 0) {   // uniform across the block
+                    v32 = fminf(v32, tile_left_out<ACT, FIXED>(p, tl, parity, gmin, sval, scand, &s_ncand, nl));
+                    __syncthreads();
+                    if (threadIdx.x == 0) s_nleft = 0;
+                }
+            }
             const int nc = s_ncand;
             if (nc > 0) {   // uniform across the block
                 const float bmin = block_min_bcast(v32);
@@ -2890,6 +3003,18 @@ __device__ __forceinline__ void write_fixed_arrays(const Problem &p, long long e
 #pragma unroll
         for (int k = 0; k < 6; k++) const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2(q.S[k].h, q.S[k].l);
         const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(q.d0, q.rd);
+    } else if (m.law == 1) {   // left to the FP64 edge form
+        EdgeElem d;
+        edge_setup(E, m.mu, d);
+#pragma unroll
+        for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = (long long)double_bits(d.E[k]);
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const uint64_t b = double_bits(d.S[k]);
+            const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2((int)(b >> 32), (int)(uint32_t)b);
+        }
+        const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(0, (long long)double_bits(d.rdet));
+        w[0] = 0;
     } else if (m.law >= 2 && fixed_setup_svk(E, 0.5 * m.mu2, m.ks, q)) {
         fixed_pack(q, w);
 #pragma unroll

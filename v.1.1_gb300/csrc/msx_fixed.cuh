@@ -108,14 +108,16 @@ MSX_HD uint32_t abs32(int32_t x)   // 2^31 for -2^31
 #endif
 }
 
-MSX_HD int top_bit(int64_t x)   // floor(log2 x), x > 0
+MSX_HD int top_bit_u(uint64_t x)   // floor(log2 x), x > 0
 {
 #ifdef __CUDA_ARCH__
-    return 63 - __clzll(x);
+    return 63 - __clzll((long long)x);
 #else
     return 63 - __builtin_clzll((unsigned long long)x);
 #endif
 }
+
+MSX_HD int top_bit(int64_t x) { return top_bit_u((uint64_t)x); }
 
 MSX_HD uint64_t double_bits(double x)
 {
@@ -125,6 +127,17 @@ MSX_HD uint64_t double_bits(double x)
     uint64_t b;
     memcpy(&b, &x, 8);
     return b;
+#endif
+}
+
+MSX_HD double bits_double(uint64_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double x;
+    memcpy(&x, &b, 8);
+    return x;
 #endif
 }
 
@@ -158,6 +171,19 @@ MSX_HD int64_t fixed_from(double x, int lw)
     const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | (uint32_t)v) << 9;   // below 2^62
     const int64_t sg = (int64_t)((int32_t)hi >> 31);
     return ((int64_t)shr64(m, lw + (1075 + 9) - ex) ^ sg) - sg;
+}
+
+// x 2^k rounded to nearest (halves away from zero), on the integer pipes (a
+// conversion takes the FP64 pipe as long as a product): the result has to be a
+// normal number or zero.
+MSX_HD double fixed_to_fp64(int64_t x, int k)
+{
+    const uint64_t m = x < 0 ? 0 - (uint64_t)x : (uint64_t)x;
+    if (m == 0) return 0.0;
+    const int lead = 63 - top_bit_u(m);
+    const uint64_t v = m << lead;
+    const uint64_t b = ((uint64_t)(1085 - lead + k) << 52) + (v >> 11) + ((v >> 10) & 1);
+    return bits_double(b | (x < 0 ? 1ull << 63 : 0));
 }
 
 // c = n_a x n_b in units of 2^57
@@ -413,6 +439,80 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
     const int lmax = q.lw[0] + (d1 > d2 ? (d1 > 0 ? d1 : 0) : (d2 > 0 ? d2 : 0));
     const int lmin = q.lw[0] + (d1 < d2 ? (d1 < 0 ? d1 : 0) : (d2 < 0 ? d2 : 0));
     return q.x0 - lmin <= 900 && q.x0 - lmax >= -900;   // forces stay normal FP64 numbers
+}
+
+// What the FP64 edge form (below) needs of an element that the fixed-point form
+// leaves out: the reference edges, S_ab = W |det E| mu g_a.g_b and 1 / det E, as
+// FP64 bits where fixed_setup refused the element and its data hold no integers.
+struct EdgeElem {
+    double E[9], S[6], rdet;
+};
+
+// e1 x e2 etc. (rows a: the cross product of the other two edges) and det e
+MSX_HD double fp64_crosses(const double *e, double *cr)
+{
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int p = 3 * ((a + 1) % 3), q = 3 * ((a + 2) % 3), y = (i + 1) % 3, z = (i + 2) % 3;
+            cr[3 * a + i] = fma(e[p + y], e[q + z], -(e[p + z] * e[q + y]));
+        }
+    return fma(e[2], cr[2], fma(e[0], cr[0], e[1] * cr[1]));
+}
+
+MSX_HD void edge_setup(const double *E, double mu, EdgeElem &d)
+{
+    double c[9];
+    const double det = fp64_crosses(E, c), w = 0.166666666667 * mu / fabs(det);
+    int k = 0;
+    for (int a = 0; a < 3; a++)
+        for (int b = a; b < 3; b++)
+            d.S[k++] = w * fma(c[3 * a + 2], c[3 * b + 2], fma(c[3 * a], c[3 * b], c[3 * a + 1] * c[3 * b + 1]));
+    for (k = 0; k < 9; k++) d.E[k] = E[k];
+    d.rdet = 1.0 / det;
+}
+
+// The same from the integers of an element inside fixed_setup's range; false
+// where S might not be a normal FP64 number.
+MSX_HD bool edge_from_fixed(const FixedElem &q, EdgeElem &d)
+{
+    const int lw = fixed_lw_min(q);
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const int s = q.lw[k / 3] - lw;
+        d.E[k] = fixed_to_fp64(q.E[k] - (s ? 1LL << (s - 1) : 0), lw);
+    }
+    bool normal = true;
+    int k = 0;
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = a; b < 3; b++) {
+            const int x = q.x0 - 58 - q.lw[a] - q.lw[b];
+            normal = normal && x >= -1000 && x <= 900;
+            d.S[k] = fixed_to_fp64(((int64_t)q.S[k].h << 29) + q.S[k].l, x);
+            k++;
+        }
+    d.rdet = fixed_to_fp64(q.rd, -(62 + q.ds) - 114 - (q.lw[0] + q.lw[1] + q.lw[2]));
+    return normal;
+}
+
+// Corner forces f_1..f_3 (f[3(a-1) + i]) in FP64 from the deformed edges e:
+// f_a = sum_b S_ab e_b + c2 (e_c x e_d); law(J) gives lambda ln J - mu; wJ is
+// W |det E|.
+template <typename LAW>
+MSX_HD void edge_forces(const EdgeElem &d, const double *e, double wJ, LAW law, double *f)
+{
+    double cr[9];
+    const double det = fp64_crosses(e, cr), c2 = law(det * d.rdet) * (wJ / det);
+    const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            f[3 * a + i] = fma(c2, cr[3 * a + i],
+                               fma(e[6 + i], d.S[mi[3 * a + 2]], fma(e[i], d.S[mi[3 * a]], e[3 + i] * d.S[mi[3 * a + 1]])));
 }
 
 // St-Venant-Kirchhoff and linear elasticity: the displacement gradient and the
