@@ -162,7 +162,8 @@ def rms_errors(lib, law, h, jitter, motion, strain, nu):
 
 @pytest.mark.parametrize("motion", list(MOTIONS))
 @pytest.mark.parametrize("h,jitter", [((0.1,) * 3, 0.0), ((0.1,) * 3, 0.1), ((0.125,) * 3, 0.0), ((0.1, 0.1, 0.3), 0.0),
-                                      ((0.1, 0.1, 0.04), 0.0)])
+                                      ((0.1, 0.1, 0.04), 0.0), ((0.1, 0.1, 0.02), 0.0), ((0.1, 0.1, 0.02), 0.1),
+                                      ((0.1, 0.1, 1.0), 0.0)])
 @pytest.mark.parametrize("law", ["le", "stvk"])
 def test_no_less_accurate_than_fp64(lib, law, h, jitter, motion):
     """At or below the FP64 form's error at every strain, or below two roundings of the result (where the FP64 form's

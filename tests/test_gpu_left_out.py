@@ -19,13 +19,16 @@ YOUNG, NU = 1e6, 0.3
 LAM, MU2 = YOUNG * NU / ((1 + NU) * (1 - 2 * NU)), YOUNG / (1 + NU)
 
 
+HEIGHT = 4e-4   # flatter than any of the forms takes
+
+
 def mesh(n, flat, far, seed):
-    """n disjoint jittered corner tets, a share `flat` of them of height 0.004, and a displacement of strain 1e-3 that
+    """n disjoint jittered corner tets, a share `flat` of them of that height, and a displacement of strain 1e-3 that
     stretches a share `far` of them sixfold along x."""
     rng = np.random.default_rng(seed)
     ref = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
     x = ref[None] + rng.uniform(-0.15, 0.15, (n, 4, 3))
-    x[rng.random(n) < flat, :, 2] *= 0.004
+    x[rng.random(n) < flat, :, 2] *= HEIGHT
     F = np.eye(3) + 1e-3 * rng.uniform(-1, 1, (n, 3, 3))
     F[rng.random(n) < far, 0] *= 6.0
     y = np.einsum("nij,naj->nai", F, x - x[:, :1]) + x[:, :1]
@@ -59,7 +62,7 @@ def test_forces_and_time_step(n, flat, far, law):
     second = S.run(1).dt
     S.close()
     want = expected_dt(X, conn, u, law)
-    tol = 64 * EPS * 2 / 0.004   # positions of size 2, heights of 0.004
+    tol = 64 * EPS * 2 / HEIGHT   # positions of size 2
     assert abs(first - want) <= tol * want and abs(second - want) <= tol * want
 
 
@@ -84,8 +87,8 @@ def test_pool_bits(law, tile):
     P.wait(t)
     pooled = P.fetch(t)
     P.close()
-    for a, b in zip(alone, pooled):
-        assert np.array_equal(a, b)
+    for a, b in zip(alone, pooled):   # the flattest tets of St-Venant-Kirchhoff overturn: NaN in both
+        assert np.array_equal(a, b, equal_nan=True)
 
 
 def test_two_laws_in_a_tile():

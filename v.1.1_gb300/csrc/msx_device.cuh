@@ -1521,7 +1521,7 @@ __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long 
 #pragma unroll
         for (int k = 0; k < 9; k++) {
             du32[k] = f32_trunc(x[k]);
-            g32[k] = (float)limbs_unpack(q.E[k]).h * pow2f_or_inf(29 - 111 - q.lw[0]);
+            g32[k] = (float)limbs_unpack(q.E[k]).h * pow2f_or_inf(29 - 111 + (q.cs >> 2) - q.lw[0]);
         }
         scr = cfl_screen(p, e, g32, du32, m);
     }
@@ -1637,15 +1637,17 @@ __device__ __forceinline__ float elem_edges_fp64(const Problem &p, long long e, 
     return scr;
 }
 
-// The FP64 form of an element that fixed point leaves out.
-template <bool FORCE_ONLY, bool ACT, int FIXED>
+// The FP64 form of an element that fixed point leaves out.  One function for all
+// kernels: which product of a b + c d is fused is the compiler's choice, and
+// would differ between instantiations.
+template <bool FORCE_ONLY, bool ACT>
 static __device__ __noinline__ float elem_left_out(const Problem &p, long long e, int parity, double t, float gmin)
 {
     const long long ne = p.ne;
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
-    if (FIXED == FIXED_CNH || (!FIXED && m.law == 1)) {
+    if (m.law == 1) {
         const uint2 w = __ldg(p.fxw + e);
         FixedElem q;
         EdgeElem d;
@@ -1699,7 +1701,7 @@ static __global__ void __launch_bounds__(kElemBlock) elem_force_kernel_fp64(Prob
     const long long b = (long long)blockIdx.x * blockDim.x, e = b + threadIdx.x;
     if (e < p.ne && elem_body_fp64<true>(p, e, parity) == kLeftOut) left[atomicAdd(&s_nleft, 1)] = threadIdx.x;
     __syncthreads();
-    if ((int)threadIdx.x < s_nleft) elem_left_out<true, false, FIXED_NONE>(p, b + left[threadIdx.x], parity, 0.0, 0.0f);
+    if ((int)threadIdx.x < s_nleft) elem_left_out<true, false>(p, b + left[threadIdx.x], parity, 0.0, 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -2708,7 +2710,7 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
 // Left-out elements lie at the end of scand, last one first; an element is in
 // one list at a time, and a pass reads its entries, the lowest that remain,
 // before it lists candidates, so these never reach an entry still to be read.
-template <bool ACT, int FIXED>
+template <bool ACT>
 __device__ __forceinline__ float tile_left_out(const Problem &p, const Tile &tl, int parity, float gmin, float *sval,
                                                unsigned short *scand, int *ncand, int nl)
 {
@@ -2718,7 +2720,7 @@ __device__ __forceinline__ float tile_left_out(const Problem &p, const Tile &tl,
         const int i = at >= 0 ? scand[kMaxTileElems - 1 - at] : 0;
         __syncthreads();
         if (at < 0) continue;
-        const float d = elem_left_out<false, ACT, FIXED>(p, tl.begin + i, parity, t, gmin);
+        const float d = elem_left_out<false, ACT>(p, tl.begin + i, parity, t, gmin);
         if (!(d > gmin)) {
             const int k = atomicAdd(ncand, 1);
             sval[k] = d;
@@ -2858,7 +2860,7 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
             if constexpr (MODE == MODE_FP64 && !VISC) {
                 const int nl = s_nleft;
                 if (nl > 0) {   // uniform across the block
-                    v32 = fminf(v32, tile_left_out<ACT, FIXED>(p, tl, parity, gmin, sval, scand, &s_ncand, nl));
+                    v32 = fminf(v32, tile_left_out<ACT>(p, tl, parity, gmin, sval, scand, &s_ncand, nl));
                     __syncthreads();
                     if (threadIdx.x == 0) s_nleft = 0;
                 }

@@ -218,7 +218,7 @@ struct FixedElem {
     int64_t d0, rd;
     int32_t lw[3];   // log2 w_b
     int32_t x0;      // log2 of f_a's unit = x0 - lw_a
-    int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t); StVK: sum_b |w g_b| <= 2^(cs + 2) / 2^57
+    int32_t cs;      // c2's series (MatParams::kq) << cs is c2 w_1 w_2 w_3 2^(57 + t); StVK: headroom hr and gradient unit gs, hr | gs << 2
     int32_t ds;
 };
 
@@ -520,13 +520,14 @@ MSX_HD void edge_forces(const EdgeElem &d, const double *e, double wJ, LAW law, 
 // accuracy with the square of an element's flatness).  With the shape
 // functions' gradients g_a, one unit w for all three edges, and a unit 2^s for
 // the strain that follows from the largest |u_b - u_0| (a state of strain 1e-9
-// has all its bits; in linear elasticity it also grows with the motion),
-// du_b = (u_b - u_0) / (w 2^s) and f_a = f_a' 2^s |det E| W mu / w:
-//     H = sum_b du_b (w g_b),  G = H + H^T + 2^s H^T H (linear: without H^T H),
+// has all its bits; in linear elasticity it also grows with the motion), a unit
+// 2^gs for flat elements' gradients, du_b = (u_b - u_0) / (w 2^(s - gs)) and
+// f_a = f_a' 2^(s + gs) |det E| W mu / w:
+//     H = sum_b du_b (w g_b / 2^gs),  G = H + H^T + 2^s H^T H (linear: without H^T H),
 //     S = scale (G + kappa tr(G) I),  kappa = lambda / (2 mu),
-//     P = S + 2^s H S (linear: S),  f_a' = P (w g_a),
-// where scale 2^x0 w = |det E| W mu, 1/2 <= scale < 1.  Units: du 2^-57, w g
-// 2^-111, H to P 2^-55, scale 2^-57, du so small that |H| < 2^57 (FixedElem::cs).
+//     P = S + 2^s H S (linear: S),  f_a' = P (w g_a / 2^gs),
+// where scale 2^(x0 - gs) w = |det E| W mu, 1/2 <= scale < 1.  Units: du 2^-57, w g
+// 2^-111, H to P 2^-55, scale 2^-57, du so small that |H| < 2^57 (by hr bits).
 // G and what follows it take a unit 2^t larger where kappa tr(G) asks for it.
 // An error of one unit in H, S or P is 2^-55 of the largest of them, against
 // 2^-53 of 1 for F's diagonal in FP64, whatever the strain.  Corner-force error
@@ -539,7 +540,10 @@ MSX_HD void edge_forces(const EdgeElem &d, const double *e, double wJ, LAW law, 
 // shear of 1e-5 on a cubic grid was 8,700 (linear) and 4.4 times FP64's.  With
 // products of edges instead, E_b . E_c and their metric, the error is 2 to 8
 // times FP64's on cubes and grows with the square of the flatness.  E holds w g
-// in limbs, S[0] the scale, both rounded from 128-bit products.
+// in limbs, S[0] the scale, both rounded from 128-bit products.  gs up to 7
+// takes hexes down to 1:1:0.02; without it (w g below 8 / |E| alone) hexes
+// flatter than 1:1:0.2 went to FP64: 1M jittered tets of 1:1:0.2, StVK, 140 us a
+// step, 348 without, 308 with all elements in FP64.
 MSX_HD int64_t limbs_pack(Limbs x) { return (int64_t)((uint64_t)(uint32_t)x.h << 32 | (uint32_t)x.l); }
 MSX_HD Limbs limbs_unpack(int64_t x) { return {(int32_t)(x >> 32), (int32_t)x}; }
 
@@ -555,7 +559,7 @@ inline void fixed_kappa(double mu2, double lambda, int64_t *kq, int *ks)
     *kq = limbs_pack(limbs((int64_t)std::rint(std::ldexp(kappa, 57 - *ks))));
 }
 
-// false: the element is left to FP64 (see fixed_setup; w g beyond 4 to 8)
+// false: the element is left to FP64 (see fixed_setup; w g beyond 2^7 times 4 to 8)
 MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
 {
     int64_t n[9], c[9];
@@ -567,7 +571,7 @@ MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
     }
     const int lw = (((int)(double_bits(l2) >> 52) - 1023) >> 1) + 1 - 57;
     q.lw[0] = q.lw[1] = q.lw[2] = lw;
-    // edges in units of w 2^-5, cross products of w^2 2^51 and det E of w^3 2^108, all below 2^63
+    // edges in units of w 2^-5 and cross products of w^2 2^51, below 2^62 and 2^63; det E of w^3 2^46
     for (int k = 0; k < 9; k++) n[k] = fixed_from(E[k], lw - 5);
     __int128 det = 0;
     for (int a = 0; a < 3; a++)
@@ -577,27 +581,39 @@ MSX_HD bool fixed_setup_svk(const double *E, double mu, int ks, FixedElem &q)
             c[3 * a + i] = (int64_t)(((__int128)p[y] * r[z] - (__int128)p[z] * r[y] + ((__int128)1 << 60)) >> 61);
             if (a == 0) det += (__int128)n[i] * c[i];
         }
-    q.d0 = (int64_t)(det >> 62);
-    if (q.d0 < (1LL << 56)) return false;
+    // det E = d0 2^dx w^3, d0 of 62 bits
+    const int64_t dh = (int64_t)(det >> 63);
+    if (dh < (1LL << 40)) return false;   // below 2^-21 |E|^3 (or not positive)
+    const int down = top_bit(dh) + 2, dx = down + 46;
+    q.d0 = (int64_t)(det >> down);
     fixed_reciprocal(q);
+    // w g = c 2^51 / (d0 2^dx) = c rd 2^-sh in units of 2^-111; 2^gs times larger where that leaves 2^57
+    const int sh = 62 + q.ds + dx - 51 - 111;
+    int gs = 0;
+    for (int k = 0; k < 9; k++) {
+        const int64_t a = mulhi64(c[k] < 0 ? -c[k] : c[k], q.rd);
+        const int over = a ? top_bit(a) + 64 - sh - 56 : 0;
+        gs = over > gs ? over : gs;
+    }
+    if (gs > 7) return false;
     int64_t sum[3] = {0, 0, 0};
-    for (int k = 0; k < 9; k++) {   // c / det E 2^111 / w
-        const int64_t g = (int64_t)(((__int128)c[k] * q.rd + ((__int128)1 << (7 + q.ds))) >> (8 + q.ds));
-        if (g >= (1LL << 57) || g <= -(1LL << 57)) return false;
+    for (int k = 0; k < 9; k++) {
+        const int64_t g = (int64_t)(((__int128)c[k] * q.rd + ((__int128)1 << (sh + gs - 1))) >> (sh + gs));
         sum[k % 3] += g < 0 ? -g : g;
         q.E[k] = limbs_pack(limbs(g));
     }
-    // |du| < 2^(57 - cs) makes |H| < 2^57: sum_b |w g_b| <= 2^(56 + cs), component by component
-    q.cs = 0;
-    while (sum[0] > 1LL << (56 + q.cs) || sum[1] > 1LL << (56 + q.cs) || sum[2] > 1LL << (56 + q.cs)) q.cs++;
+    // |du| < 2^(57 - hr) makes |H| < 2^57: sum_b |w g_b| <= 2^(56 + hr), component by component
+    int hr = 0;
+    while (sum[0] > 1LL << (56 + hr) || sum[1] > 1LL << (56 + hr) || sum[2] > 1LL << (56 + hr)) hr++;
+    q.cs = hr | gs << 2;   // at most 31
     // |det E| W mu = scale 2^x w^3, 1/2 <= scale < 1, to the scale's 57 bits
     if (ks < 0 || !(mu < 1e100) || !(mu > 1e-100)) return false;
     const int xm = (int)(double_bits(mu) >> 52) - 1022;
     const int64_t wm = (int64_t)(((__int128)fixed_from(0.166666666667, -64) * fixed_from(mu, xm - 62)) >> 62);
-    const int64_t v = (int64_t)(((__int128)wm * (q.d0 << (62 - q.ds))) >> 62);   // W mu det E 2^(64 - xm - ds - 108)
+    const int64_t v = (int64_t)(((__int128)wm * (q.d0 << (62 - q.ds))) >> 62);   // W mu det E 2^(64 - xm - ds - dx) / w^3
     const int tv = top_bit(v);   // 59 to 62
     q.S[0] = limbs((v + (1LL << (tv - 57))) >> (tv - 56));
-    q.x0 = tv + 1 - 64 + xm + q.ds + 108 + 3 * lw - 109;
+    q.x0 = tv + 1 - 64 + xm + q.ds + dx + 3 * lw - 109 + gs;
     return q.x0 - lw <= 900 && q.x0 - lw >= -900;
 }
 
@@ -606,10 +622,9 @@ MSX_HD int64_t shift_round(int64_t x, int r) { return (x + (int64_t)((1ull << r)
 
 MSX_HD int32_t high_word(int64_t x) { return (int32_t)(x >> 32); }
 
-// The motion x[3(b-1) + i] = u_b - u_0 in limbs and the exponent s of its unit
-// w 2^s; hi: the largest high word of |x|.  s <= 0 with H^T H, whose elements
+// The motion x[3(b-1) + i] = u_b - u_0 in limbs and the exponent s of H's unit; hi: the largest high word of |x|.  s <= 0 with H^T H, whose elements
 // larger motions leave to FP64.  false: infinities, NaN, a motion beyond 2^58
-// of w, forces near the ends of the FP64 range.
+// of w 2^-gs, forces near the ends of the FP64 range.
 MSX_HD bool fixed_motion(const FixedElem &q, const double *x, int hi, bool linear, Limbs *du, int &s)
 {
     if (hi < kFixMotionLeast << 20) {   // at rest, or nearly
@@ -623,9 +638,10 @@ MSX_HD bool fixed_motion(const FixedElem &q, const double *x, int hi, bool linea
         return any == 0;
     }
     const int e = (hi >> 20) - 1022;   // |x| < 2^e
-    int lu = e - 57 + (linear ? 0 : q.cs);
-    if (!linear && lu > q.lw[0]) lu = q.lw[0];
-    s = lu - q.lw[0];
+    const int gs = q.cs >> 2;
+    int lu = e - 57 + (linear ? 0 : q.cs & 3);
+    if (!linear && lu > q.lw[0] - gs) lu = q.lw[0] - gs;
+    s = lu - q.lw[0] + gs;
     const int unit = q.x0 + s - q.lw[0];
 #pragma unroll
     for (int k = 0; k < 9; k++) du[k] = limbs(fixed_from(x[k], lu));
