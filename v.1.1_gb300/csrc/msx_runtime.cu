@@ -640,11 +640,10 @@ static msx_status set_opts(msx_handle *h, const msx_solver_opts *o)
     h->max_steps = o->max_steps;
     int spg = o->steps_per_graph > 0 ? o->steps_per_graph : 64;
     spg = (spg + 1) & ~1;   // even: every replay starts on the same parity
-    if (spg != h->spg && h->graph) {
-        cudaGraphExecDestroy(h->graph);
-        h->graph = nullptr;
-    }
     h->spg = spg;
+    // the captured launches hold the Problem by value, tf and the scale factor with it: they go
+    // here, where those change, whatever the caller does next or fails at
+    drop_graphs(h);
     h->block_ready = false;
     h->block_steps = 0;
     return MSX_OK;
@@ -1513,9 +1512,7 @@ extern "C" msx_status msx_next_solver(msx_handle *h, const msx_bc *bcs, int64_t 
     if (opts && opts->precision == MSX_PREC_DOUBLE_WORD && (st = check_double_word(h)) != MSX_OK) return st;
     if ((st = set_opts(h, opts)) != MSX_OK) return st;
     if ((st = mode_buffers(h, h->precision, true)) != MSX_OK) return st;
-    if ((st = upload_bcs(h, bcs, num_bcs)) != MSX_OK) return st;
-    drop_graphs(h);
-    return MSX_OK;
+    return upload_bcs(h, bcs, num_bcs);
 }
 
 extern "C" msx_status msx_internal_force(msx_handle *h, const double *u, double *fint)
