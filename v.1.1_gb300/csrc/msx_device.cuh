@@ -1692,8 +1692,10 @@ __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, i
     return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
 }
 
-// corner forces only (internal-force hook)
-static __global__ void __launch_bounds__(kElemBlock) elem_force_kernel_fp64(Problem p, int parity)
+// corner forces only (internal-force hook); three CTAs an SM in spite of the
+// registers of the left-out elements' FP64 form (80 instead of 114: a call of
+// 1.3M tets 334 us, 341 with two, 322 with that form inside the warps)
+static __global__ void __launch_bounds__(kElemBlock, 3) elem_force_kernel_fp64(Problem p, int parity)
 {
     __shared__ int left[kElemBlock], s_nleft;   // left out by fixed point: by consecutive threads at the end
     if (threadIdx.x == 0) s_nleft = 0;
