@@ -293,6 +293,9 @@ msx_status msx_element_values(msx_handle *h, int32_t quantity, const int32_t *el
 msx_status msx_element_reduce(msx_handle *h, int32_t quantity, int32_t op, const int32_t *elems, int64_t n,
                               double *value);
 
+/* Frees the handle and its device memory: the solve's arrays and up to 64 MB
+ * of scratch, which the calls that compute and copy out (node and element values,
+ * reductions, internal force) keep between them at the size of the largest. */
 msx_status msx_destroy(msx_handle *h);
 
 /* Message of the last failing call on this host thread. */
@@ -435,6 +438,8 @@ msx_status msx_pool_fetch(msx_pool *p, int64_t ticket, double *u, double *v, dou
  * other resident solves advance too; their results are kept for poll/fetch).
  * MSX_ERR_ARG if the ticket is unknown or already fetched. */
 msx_status msx_pool_wait(msx_pool *p, int64_t ticket, msx_pool_result *result);
+/* A pool keeps up to 2 GB of fetched solves' device memory for its next
+ * admissions; all of it goes back to the device here. */
 msx_status msx_pool_destroy(msx_pool *p);
 
 typedef struct {

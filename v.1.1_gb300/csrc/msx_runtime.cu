@@ -162,7 +162,9 @@ struct msx_handle {
 static void drop_graphs(msx_handle *h);
 
 // Device scratch of one call, carved from the handle's buffer (a cudaMalloc and
-// its cudaFree cost 8-20 us a call, and the free waits for the device); a call
+// its cudaFree cost 8-20 us a call, and the free waits for the device), of the
+// size that the largest call so far needed (with twice that to be mapped, a
+// handle's first internal-force call of 1.3M tets took 474 us, 441 now); a call
 // that needs more than kScratchKept bytes has its own allocation, freed with
 // this object.  The calls of a handle come from one thread and synchronise its
 // stream before they return, so one buffer serves them all.
@@ -179,14 +181,18 @@ struct Scratch {
     bool reserve(msx_handle *h, size_t bytes)
     {
         if (bytes > kScratchKept) {
-            if (cudaMalloc((void **)&own, bytes) != cudaSuccess) return false;
+            if (cudaMalloc((void **)&own, bytes) != cudaSuccess) {
+                (void)cudaGetLastError();   // reported by the caller, not by a later call
+                return false;
+            }
             p = own;
             return true;
         }
-        if (h->scratch.n < bytes) {
+        if (h->scratch.n < bytes) {   // what the call needs, no more: it is mapped on the handle's first call
             h->scratch.release();
-            if (h->scratch.alloc(std::min(kScratchKept, std::max<size_t>(2 * bytes, 1 << 16))) != cudaSuccess) {
+            if (h->scratch.alloc(bytes) != cudaSuccess) {
                 h->scratch = DBuf<unsigned char>();
+                (void)cudaGetLastError();
                 return false;
             }
         }
