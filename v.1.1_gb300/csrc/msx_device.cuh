@@ -1371,10 +1371,6 @@ __device__ __forceinline__ float cfl_screen(const Problem &p, long long e, const
     return cfl_screen_edges(p, e, e1, e2, e3, m);
 }
 
-template <bool FORCE_ONLY, bool ACT, bool VISC>
-__device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
-                                                    const MatParams &m, const int *nd, float gmin);
-
 // What the fixed-point bodies return for an element they leave to FP64
 // (elem_left_out), whose forces are not written yet.
 constexpr float kLeftOut = -2.0f;
@@ -1545,12 +1541,8 @@ __device__ __forceinline__ float elem_body_fp64_svk(const Problem &p, long long 
 // value (see cfl_screen).
 template <bool FORCE_ONLY, bool ACT, bool VISC>
 __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long e, int parity, double t, double idt,
-                                                    const MatParams &m, const int *nd, float gmin)
+                                                    const MatParams &m, const int *nd, const double *G, float gmin)
 {
-    const long long ne = p.ne;
-    double G[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) G[k] = __ldg(p.G + k * ne + e);
     double ua[4][3], du[9];
     gather_u<FORCE_ONLY>(p, nd, ua);
 #pragma unroll
@@ -1637,6 +1629,12 @@ __device__ __forceinline__ float elem_edges_fp64(const Problem &p, long long e, 
     return scr;
 }
 
+__device__ __forceinline__ void load_G(const Problem &p, long long e, double *G)
+{
+#pragma unroll
+    for (int k = 0; k < 9; k++) G[k] = __ldg(p.G + k * p.ne + e);
+}
+
 // The FP64 form of an element that fixed point leaves out.  One function for all
 // kernels: which product of a b + c d is fused is the compiler's choice, and
 // would differ between instantiations.
@@ -1647,6 +1645,7 @@ static __device__ __noinline__ float elem_left_out(const Problem &p, long long e
     const int4 cn = p.conn[e];
     const int nd[4] = {cn.x, cn.y, cn.z, cn.w};
     const MatParams &m = mat_of(p, e);
+    double G[9];
     if (m.law == 1) {
         const uint2 w = __ldg(p.fxw + e);
         FixedElem q;
@@ -1674,8 +1673,20 @@ static __device__ __noinline__ float elem_left_out(const Problem &p, long long e
             edges = edge_from_fixed(q, d);
         }
         if (edges) return elem_edges_fp64<FORCE_ONLY>(p, e, parity, m, nd, d, gmin);
+        load_G(p, e, G);
+    } else {   // the gradients, FP64 bits or limbs of w g 2^(111 - gs)
+        const uint2 w = __ldg(p.fxw + e);
+        FixedElem q;
+        fixed_unpack(w.x, w.y, q);
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            const long long x = __ldg(p.fxE + k * ne + e);
+            const Limbs g = limbs_unpack(x);
+            G[k] = w.x == 0 ? bits_double((uint64_t)x)
+                            : fixed_to_fp64(((int64_t)g.h << 29) + g.l, (q.cs >> 2) - 111 - q.lw[0]);
+        }
     }
-    return elem_cofactor_fp64<FORCE_ONLY, ACT, false>(p, e, parity, t, 0.0, m, nd, gmin);
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, false>(p, e, parity, t, 0.0, m, nd, G, gmin);
 }
 
 template <bool FORCE_ONLY, bool ACT = false, bool VISC = false, int FIXED = FIXED_NONE>
@@ -1689,7 +1700,9 @@ __device__ __forceinline__ float elem_body_fp64(const Problem &p, long long e, i
         return elem_body_fp64_cnh<FORCE_ONLY>(p, e, parity, m, nd, gmin);
     if (FIXED == FIXED_SVK || (!VISC && p.fxE && m.law >= 2))
         return elem_body_fp64_svk<FORCE_ONLY, ACT>(p, e, parity, t, m, nd, gmin);
-    return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, gmin);
+    double G[9];
+    load_G(p, e, G);
+    return elem_cofactor_fp64<FORCE_ONLY, ACT, VISC>(p, e, parity, t, idt, m, nd, G, gmin);
 }
 
 // corner forces only (internal-force hook); three CTAs an SM in spite of the
@@ -3024,6 +3037,17 @@ __device__ __forceinline__ void write_fixed_arrays(const Problem &p, long long e
 #pragma unroll
         for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = q.E[k];
         const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(limbs_pack(q.S[0]), 0);
+    } else if (m.law >= 2) {   // left to the FP64 cofactor form: G as Problem::G holds it
+        double xyz[12], Jac[9], iJ[9];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int i = 0; i < 3; i++) xyz[i * 4 + k] = pts[k * 3 + i];
+        ref_jacobian(xyz, Jac);
+        inv3_ref(Jac, iJ);
+#pragma unroll
+        for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = (long long)double_bits(0.0 + iJ[k]);
+        w[0] = 0;
     }
     const_cast<uint2 *>(p.fxw)[e] = make_uint2(w[0], w[1]);
 }
@@ -3058,7 +3082,7 @@ __global__ void setup_elements_kernel(Problem p, const double *X, double *G, dou
 #pragma unroll
     for (int k = 0; k < 9; k++) {
         double g = 0.0 + iJ[k];
-        G[k * ne + e] = g;
+        if (G) G[k * ne + e] = g;
         if (G32) G32[k * ne + e] = (float)g;
         if (p.G32lo) const_cast<float *>(p.G32lo)[k * ne + e] = (float)(g - (double)(float)g);
     }

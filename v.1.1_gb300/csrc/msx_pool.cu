@@ -164,13 +164,12 @@ static size_t footprint(long long nn, long long ne, long long nbc, int precision
     if (fixed)   // fixed-point data: fxE, fxD, fxw, fxS
         b += align256(sizeof(double) * 9 * ne) + align256(sizeof(longlong2) * ne) + align256(sizeof(uint2) * ne);
     if (fixed == FIXED_CNH) b += align256(sizeof(int2) * 6 * ne);
-    b += align256(sizeof(int4) * ne) + align256(sizeof(double) * 9 * ne);           // conn, G
-    b += 2 * align256(sizeof(double) * ne);                                         // wJ, Lref
-    b += align256(sizeof(float) * 9 * ne) + 2 * align256(sizeof(float) * ne);        // G32, wJ32, Lref32
+    b += align256(sizeof(int4) * ne) + 2 * align256(sizeof(double) * ne) + align256(sizeof(float) * ne);   // conn, wJ, Lref, Lref32
+    if (fixed != FIXED_SVK) b += align256(sizeof(double) * 9 * ne);                  // G (fxE holds it there)
     b += 4 * align256(sizeof(double) * 3 * nn) + 2 * align256(sizeof(double) * nn);  // X, u, v, a, mass, minv
-    b += align256(sizeof(float2) * 3 * nn);                                          // uhl
-    if (pair_state(precision))                                                       // vhl, ahl, minv2
-        b += 2 * align256(sizeof(float2) * 3 * nn) + align256(sizeof(float2) * nn);
+    if (pair_state(precision))                                                       // G32, wJ32, uhl, vhl, ahl, minv2
+        b += align256(sizeof(float) * 9 * ne) + align256(sizeof(float) * ne) + 3 * align256(sizeof(float2) * 3 * nn) +
+             align256(sizeof(float2) * nn);
     if (precision == MSX_PREC_FP64) b += align256(sizeof(double) * 4 * nn);          // u4 (node-major u)
     if (precision == MSX_PREC_DOUBLE_WORD)                                           // G32lo, wJ32lo
         b += align256(sizeof(float) * 9 * ne) + align256(sizeof(float) * ne);
@@ -650,11 +649,13 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         P.mats[0] = mp;
         P.mat = nullptr;
         P.conn = (int4 *)carve(sizeof(int4) * ne);
-        P.G = (double *)carve(sizeof(double) * 9 * ne);
+        if (fixed != FIXED_SVK) P.G = (double *)carve(sizeof(double) * 9 * ne);
         P.wJ = (double *)carve(sizeof(double) * ne);
         P.Lref = (double *)carve(sizeof(double) * ne);
-        P.G32 = (float *)carve(sizeof(float) * 9 * ne);
-        P.wJ32 = (float *)carve(sizeof(float) * ne);
+        if (pair_state(prec)) {
+            P.G32 = (float *)carve(sizeof(float) * 9 * ne);
+            P.wJ32 = (float *)carve(sizeof(float) * ne);
+        }
         P.Lref32 = (float *)carve(sizeof(float) * ne);
         if (prec == MSX_PREC_DOUBLE_WORD) {
             P.G32lo = (float *)carve(sizeof(float) * 9 * ne);
@@ -668,7 +669,6 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         double *mass = (double *)carve(sizeof(double) * nn), *minv = (double *)carve(sizeof(double) * nn);
         P.mass = mass;
         P.minv = minv;
-        P.uhl = (float2 *)carve(sizeof(float2) * 3 * nn);
         if (prec == MSX_PREC_FP64) P.u4 = (double *)carve(sizeof(double) * 4 * nn);
         if (fixed) {   // written by the element set-up, as for a single solve
             P.fxE = (long long *)carve(sizeof(long long) * 9 * ne);
@@ -678,6 +678,7 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         }
         float2 *minv2 = nullptr;
         if (pair_state(prec)) {
+            P.uhl = (float2 *)carve(sizeof(float2) * 3 * nn);
             P.vhl = (float2 *)carve(sizeof(float2) * 3 * nn);
             P.ahl = (float2 *)carve(sizeof(float2) * 3 * nn);
             minv2 = (float2 *)carve(sizeof(float2) * nn);
@@ -725,9 +726,9 @@ extern "C" msx_status msx_pool_submit(msx_pool *p, const msx_mesh *mesh, const m
         PCUDA(cudaMemsetAsync(P.u, 0, sizeof(double) * 3 * nn, s));
         PCUDA(cudaMemsetAsync(P.v, 0, sizeof(double) * 3 * nn, s));
         PCUDA(cudaMemsetAsync(P.a, 0, sizeof(double) * 3 * nn, s));
-        PCUDA(cudaMemsetAsync(P.uhl, 0, sizeof(float2) * 3 * nn, s));
         if (P.u4) PCUDA(cudaMemsetAsync(P.u4, 0, sizeof(double) * 4 * nn, s));
         if (pair_state(prec)) {
+            PCUDA(cudaMemsetAsync(P.uhl, 0, sizeof(float2) * 3 * nn, s));
             PCUDA(cudaMemsetAsync(P.vhl, 0, sizeof(float2) * 3 * nn, s));
             PCUDA(cudaMemsetAsync(P.ahl, 0, sizeof(float2) * 3 * nn, s));
         }
