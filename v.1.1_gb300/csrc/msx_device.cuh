@@ -2408,8 +2408,8 @@ __device__ __forceinline__ float block_min_bcast(float v)
 // Where the tiled kernels get their work.  PoolTiles: the pool's tile list and
 // descriptors in device memory.  SolveTiles: one solve, whose Problem is a
 // kernel argument (the constant bank: no load stands before the first use of
-// its pointers) and whose tiles are equal ranges of `size` of its n elements or
-// nodes, computed instead of loaded.
+// its pointers) and whose tiles are equal ranges of `size` elements, computed
+// instead of loaded.
 struct PoolTiles {
     const Problem *descs;
     const Tile *tiles;
@@ -2419,12 +2419,11 @@ struct PoolTiles {
 
 struct SolveTiles {
     const Problem &p;
-    long long n;
     int size;
     __device__ __forceinline__ Tile tile(int t) const
     {
         const long long b = (long long)t * size, e = b + size;
-        return {0, (int)b, (int)(e < n ? e : n)};
+        return {0, (int)b, (int)(e < p.ne ? e : p.ne)};
     }
     __device__ __forceinline__ const Problem &problem(const Tile &) const { return p; }
 };
@@ -2625,10 +2624,10 @@ __device__ __forceinline__ void prefetch_slots(const Problem &p, int2 slots)
 // with it).
 template <int MODE, bool BATCH, bool SMALL = false>
 __global__ void __launch_bounds__(SMALL ? 128 : kStepThreads, node_ctas(MODE, BATCH))
-    solve_node_kernel(const __grid_constant__ Problem p, int, int ntiles, int *__restrict__, int parity)
+    solve_node_kernel(const __grid_constant__ Problem p, int parity)
 {
     const long long per = blockDim.x >> 2, stride = per * gridDim.x;
-    if (ntiles <= (int)gridDim.x) pull_node(p, blockIdx.x * per + (threadIdx.x >> 2));
+    if (p.nn <= stride) pull_node(p, blockIdx.x * per + (threadIdx.x >> 2));
     pdl_wait();
     pdl_release();
     NodeStep ns;
@@ -2923,11 +2922,12 @@ __device__ __forceinline__ void elem_tile_loop(const SRC &src, TileQueue q, int 
 // CTAs of kStepThreads an SM holds: the register caps of the element kernels
 constexpr int elem_ctas(int mode) { return mode == MODE_MIXED ? 4 : (mode == MODE_DW ? 3 : 2); }
 
-template <int MODE, bool ACT = false, bool VISC = false>
+// (no element birth, no viscosity in a pool)
+template <int MODE>
 __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     pool_elem_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles, int *__restrict__ sched, int parity)
 {
-    elem_tile_loop<MODE, ACT, VISC>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
+    elem_tile_loop<MODE, false, false>(PoolTiles{descs, tiles}, TileQueue(sched, sched[0]), parity);
 }
 
 // One solve: tiles of `size` elements
@@ -2938,7 +2938,7 @@ __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE))
     if (ntiles <= (int)gridDim.x) pull_element<MODE>(p, (long long)blockIdx.x * size + threadIdx.x);
     pdl_wait();
     pdl_release();
-    elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+    elem_tile_loop<MODE, ACT, VISC>(SolveTiles{p, size}, TileQueue(sched, ntiles), parity);
 }
 
 // One solve in FP64 whose every material is compressible neo-Hookean.  128
@@ -2951,7 +2951,7 @@ static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
     if (ntiles <= (int)gridDim.x) pull_element<MODE_FP64>(p, (long long)blockIdx.x * size + threadIdx.x);
     pdl_wait();
     pdl_release();
-    elem_tile_loop<MODE_FP64, false, false, FIXED_CNH>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+    elem_tile_loop<MODE_FP64, false, false, FIXED_CNH>(SolveTiles{p, size}, TileQueue(sched, ntiles), parity);
 }
 
 // One solve in FP64 whose every material is St-Venant-Kirchhoff or linear elastic.
@@ -2961,7 +2961,7 @@ static __global__ void __launch_bounds__(kStepThreads, elem_ctas(MODE_FP64))
     if (ntiles <= (int)gridDim.x) pull_element<MODE_FP64>(p, (long long)blockIdx.x * size + threadIdx.x);
     pdl_wait();
     pdl_release();
-    elem_tile_loop<MODE_FP64, false, false, FIXED_SVK>(SolveTiles{p, p.ne, size}, TileQueue(sched, ntiles), parity);
+    elem_tile_loop<MODE_FP64, false, false, FIXED_SVK>(SolveTiles{p, size}, TileQueue(sched, ntiles), parity);
 }
 
 // ---------------------------------------------------------------------------

@@ -46,12 +46,11 @@ void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, in
         pool_elem_kernel<MODE_FP64><<<grid, threads, 0, s>>>(descs, etiles, counts, parity);
 }
 
-// A step kernel of one solve over n tiles, with programmatic dependent launch
-// for small grids (SolveSched::pdl).
-typedef void (*solve_kernel)(const Problem, int, int, int *, int);
-
-static void launch_solve(solve_kernel f, const Problem &p, const SolveSched &q, int size, int n, int most, int *sched,
-                         int parity, cudaStream_t s)
+// A step kernel of one solve on n CTAs or the most that are resident, with
+// programmatic dependent launch for small grids (SolveSched::pdl).
+template <typename... ARGS>
+static void launch_solve(void (*f)(const Problem, ARGS...), const Problem &p, const SolveSched &q, int n, int most,
+                         cudaStream_t s, ARGS... args)
 {
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(n < most ? n : most);
@@ -63,39 +62,50 @@ static void launch_solve(solve_kernel f, const Problem &p, const SolveSched &q, 
     c.attrs = &at;
     Problem P = p;
     P.dependent = c.numAttrs = n <= q.pdl ? 1 : 0;
-    cudaLaunchKernelEx(&c, f, P, size, n, sched, parity);
+    cudaLaunchKernelEx(&c, f, P, args...);
 }
 
-void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
+typedef void (*solve_node_fn)(const Problem, int);
+typedef void (*solve_elem_fn)(const Problem, int, int, int *, int);
+
+template <int MODE>
+static solve_node_fn solve_node_variant(const SolveSched &q)
 {
-    const int n = (int)((p.nn + q.node_tile - 1) / q.node_tile);
-    const bool b = q.node_batch;
-    solve_kernel f;
-    if (b && q.threads == 128)
-        f = mode == MODE_MIXED ? solve_node_kernel<MODE_MIXED, true, true>
-                               : (mode == MODE_DW ? solve_node_kernel<MODE_DW, true, true> : solve_node_kernel<MODE_FP64, true, true>);
-    else if (mode == MODE_MIXED) f = b ? solve_node_kernel<MODE_MIXED, true> : solve_node_kernel<MODE_MIXED, false>;
-    else if (mode == MODE_DW) f = b ? solve_node_kernel<MODE_DW, true> : solve_node_kernel<MODE_DW, false>;
-    else f = b ? solve_node_kernel<MODE_FP64, true> : solve_node_kernel<MODE_FP64, false>;
-    launch_solve(f, p, q, q.node_tile, n, q.node_grid, counts + 3, parity, s);
+    if (!q.node_batch) return solve_node_kernel<MODE, false>;
+    return q.threads == 128 ? solve_node_kernel<MODE, true, true> : solve_node_kernel<MODE, true>;
+}
+
+static solve_node_fn solve_node(int mode, const SolveSched &q)
+{
+    return mode == MODE_MIXED ? solve_node_variant<MODE_MIXED>(q)
+                              : (mode == MODE_DW ? solve_node_variant<MODE_DW>(q) : solve_node_variant<MODE_FP64>(q));
 }
 
 // element birth and bulk viscosity are separate instantiations (never both: the host refuses that)
 template <int MODE>
-static solve_kernel solve_elem_variant(const Problem &p, const SolveSched &q)
+static solve_elem_fn solve_elem_variant(const Problem &p, const SolveSched &q)
 {
     if (p.act_t) return solve_elem_kernel<MODE, true>;
     if (MODE == MODE_FP64 && q.fixed) return q.fixed == FIXED_CNH ? solve_elem_cnh_kernel : solve_elem_svk_kernel;
     return p.visc ? solve_elem_kernel<MODE, false, true> : solve_elem_kernel<MODE>;
 }
 
+static solve_elem_fn solve_elem(const Problem &p, int mode, const SolveSched &q)
+{
+    return mode == MODE_MIXED ? solve_elem_variant<MODE_MIXED>(p, q)
+                              : (mode == MODE_DW ? solve_elem_variant<MODE_DW>(p, q) : solve_elem_variant<MODE_FP64>(p, q));
+}
+
+void launch_solve_node(const Problem &p, const SolveSched &q, int mode, int parity, cudaStream_t s)
+{
+    const int per = q.threads / 4;
+    launch_solve(solve_node(mode, q), p, q, (int)((p.nn + per - 1) / per), q.node_grid, s, parity);
+}
+
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s)
 {
     const int n = (int)((p.ne + q.elem_tile - 1) / q.elem_tile);
-    const solve_kernel f = mode == MODE_MIXED ? solve_elem_variant<MODE_MIXED>(p, q)
-                                              : (mode == MODE_DW ? solve_elem_variant<MODE_DW>(p, q)
-                                                                 : solve_elem_variant<MODE_FP64>(p, q));
-    launch_solve(f, p, q, q.elem_tile, n, q.elem_grid, counts, parity, s);
+    launch_solve(solve_elem(p, mode, q), p, q, n, q.elem_grid, s, (int)q.elem_tile, (int)n, counts, parity);
 }
 
 // a32: the mixed mode, whose acceleration is one FP32 per DOF (mixed_a32)
@@ -204,25 +214,26 @@ void launch_abs_range(const double *x, long long n, unsigned long long *mm, cuda
     abs_range_kernel<<<256, 256, 0, s>>>(x, n, mm);
 }
 
-int tiled_ctas_per_sm(int mode, int threads, bool node, bool pool, int fixed, bool batch)
+static int ctas_per_sm(const void *kernel, int threads)
 {
-    const void *f[3][2][2] = {
-        {{(const void *)solve_elem_kernel<MODE_FP64>, (const void *)pool_elem_kernel<MODE_FP64>},
-         {(const void *)solve_node_kernel<MODE_FP64, false>, (const void *)pool_node_kernel<MODE_FP64>}},
-        {{(const void *)solve_elem_kernel<MODE_MIXED>, (const void *)pool_elem_kernel<MODE_MIXED>},
-         {(const void *)solve_node_kernel<MODE_MIXED, false>, (const void *)pool_node_kernel<MODE_MIXED>}},
-        {{(const void *)solve_elem_kernel<MODE_DW>, (const void *)pool_elem_kernel<MODE_DW>},
-         {(const void *)solve_node_kernel<MODE_DW, false>, (const void *)pool_node_kernel<MODE_DW>}}};
     int a = 0;
-    if (fixed) f[0][0][0] = fixed == FIXED_CNH ? (const void *)solve_elem_cnh_kernel : (const void *)solve_elem_svk_kernel;
-    if (batch) {
-        f[0][1][0] = (const void *)solve_node_kernel<MODE_FP64, true>;
-        f[1][1][0] = (const void *)solve_node_kernel<MODE_MIXED, true>;
-        f[2][1][0] = (const void *)solve_node_kernel<MODE_DW, true>;
-    }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f[mode == MODE_MIXED ? 1 : (mode == MODE_DW ? 2 : 0)][node][pool],
-                                                  threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel, threads, 0);
     return a > 0 ? a : 1;
+}
+
+int solve_node_ctas(int mode, const SolveSched &q) { return ctas_per_sm((const void *)solve_node(mode, q), q.threads); }
+
+int solve_elem_ctas(const Problem &p, int mode, const SolveSched &q)
+{
+    return ctas_per_sm((const void *)solve_elem(p, mode, q), q.threads);
+}
+
+int pool_ctas_per_sm(int mode, int threads, bool node)
+{
+    const void *f[3][2] = {{(const void *)pool_elem_kernel<MODE_FP64>, (const void *)pool_node_kernel<MODE_FP64>},
+                           {(const void *)pool_elem_kernel<MODE_MIXED>, (const void *)pool_node_kernel<MODE_MIXED>},
+                           {(const void *)pool_elem_kernel<MODE_DW>, (const void *)pool_node_kernel<MODE_DW>}};
+    return ctas_per_sm(f[mode == MODE_MIXED ? 1 : (mode == MODE_DW ? 2 : 0)][node], threads);
 }
 
 }  // namespace msx

@@ -194,25 +194,26 @@ void launch_tiled_node(const Problem *descs, const Tile *ntiles, int *counts, in
                        int threads, cudaStream_t s);
 void launch_tiled_elem(const Problem *descs, const Tile *etiles, int *counts, int mode, int parity, int grid,
                        int threads, cudaStream_t s);
-// The same kernels over one solve, whose Problem goes as a kernel argument:
-// CTA size, tile sizes and the largest grids (a launch takes no more CTAs than
-// it has tiles).  Problem::act_t selects the element kernel with element birth,
-// Problem::visc the one with bulk viscosity.
 // Fixed-point forms of the plain FP64 mode (msx_fixed.cuh) by law
 enum : int { FIXED_NONE = 0, FIXED_CNH = 1, FIXED_SVK = 2 };
 __host__ __device__ inline int fixed_form(int law) { return law == 1 ? FIXED_CNH : (law >= 2 ? FIXED_SVK : FIXED_NONE); }
+// The same kernels over one solve, whose Problem goes as a kernel argument: CTA
+// size, elements of a tile and the largest grids (a launch takes no more CTAs
+// than it has tiles, or passes of threads / 4 nodes).  Problem::act_t selects
+// the element kernel with element birth, Problem::visc the one with bulk viscosity.
 struct SolveSched {
     int threads = kStepThreads;
-    int elem_tile = 0, node_tile = 0, elem_grid = 0, node_grid = 0;
-    int node_batch = 0;   // the node kernel with batched gathers (a block for every tile)
+    int elem_tile = 0, elem_grid = 0, node_grid = 0;
+    int node_batch = 0;   // the node kernel with batched gathers (a block for every pass)
     int pdl = 0;   // grids of up to this many CTAs are launched with programmatic dependent launch
     int fixed = FIXED_NONE;   // plain FP64: the fixed-point form of every element
 };
-void launch_solve_node(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
+void launch_solve_node(const Problem &p, const SolveSched &q, int mode, int parity, cudaStream_t s);
 void launch_solve_elem(const Problem &p, const SolveSched &q, int *counts, int mode, int parity, cudaStream_t s);
-// CTAs of a tiled element kernel (node kernel when `node` is true) that fit on one SM
-// of the pool, or of a single solve: of one fixed-point form (SolveSched::fixed), with batched gathers
-int tiled_ctas_per_sm(int mode, int threads, bool node = false, bool pool = false, int fixed = FIXED_NONE, bool batch = false);
+// CTAs of the kernel that such a launch, or the pool's, runs that fit on one SM
+int solve_node_ctas(int mode, const SolveSched &q);
+int solve_elem_ctas(const Problem &p, int mode, const SolveSched &q);
+int pool_ctas_per_sm(int mode, int threads, bool node = false);
 // Mixed-mode state conversions: u, v, a (FP64) -> uhl, vhl, ahl, and back
 // (hi + lo, exact unless the pair spans more than 53 bits); minv -> minv2.
 void launch_state_split(const Problem &p, bool mixed, cudaStream_t s);

@@ -239,7 +239,7 @@ static msx_status build_pool_graph(msx_pool *p, int steps)
     }
     const int mode = pool_mode(p->opts.precision);
     const int threads = p->sched.threads, grid = p->sms * p->sched.ctas_per_sm;
-    const int node_grid = p->sms * tiled_ctas_per_sm(mode, threads, true, true);
+    const int node_grid = p->sms * pool_ctas_per_sm(mode, threads, true);
     cudaGraph_t g;
     PCUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < steps; i++) {
@@ -384,7 +384,7 @@ static msx_status replay(msx_pool *p, float *ms)
 static msx_status autotune(msx_pool *p)
 {
     const int mode = pool_mode(p->opts.precision);
-    const int occ128 = tiled_ctas_per_sm(mode, 128, false, true), occ256 = tiled_ctas_per_sm(mode, 256, false, true);
+    const int occ128 = pool_ctas_per_sm(mode, 128), occ256 = pool_ctas_per_sm(mode, 256);
     const Sched cands[] = {{128, 512, occ128}, {128, 1024, occ128}, {256, 512, occ256}, {256, 1024, occ256},
                            {256, 2048, occ256}, {256, 4096, occ256}, {256, 1024, std::max(1, occ256 / 2)},
                            {128, 2048, occ128}};
@@ -485,18 +485,18 @@ extern "C" msx_status msx_pool_create(const msx_pool_opts *opts, msx_pool **out)
     p->spl = opts->steps_per_launch > 0 ? ((opts->steps_per_launch + 1) & ~1) : 32;
     const int pmode = pool_mode(opts->precision);
     p->sched.threads = kStepThreads;
-    p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, kStepThreads, false, true);
+    p->sched.ctas_per_sm = pool_ctas_per_sm(pmode, kStepThreads);
     if (opts->elems_per_block > 0) {
         p->sched.threads = opts->elems_per_block >= 256 ? 256 : 128;
         p->sched.tile_elems = opts->elems_per_block;
-        p->sched.ctas_per_sm = tiled_ctas_per_sm(pmode, p->sched.threads, false, true);
+        p->sched.ctas_per_sm = pool_ctas_per_sm(pmode, p->sched.threads);
         p->tuned = true;
     } else if (opts->tune_cache) {
         if (FILE *f = fopen(opts->tune_cache, "r")) {
             Sched s;
             if (fscanf(f, "%d %d %d", &s.threads, &s.tile_elems, &s.ctas_per_sm) == 3 && s.threads > 0 &&
                 s.threads <= kStepThreads && s.tile_elems > 0 && s.ctas_per_sm > 0 &&
-                s.ctas_per_sm <= tiled_ctas_per_sm(pmode, s.threads, false, true)) {
+                s.ctas_per_sm <= pool_ctas_per_sm(pmode, s.threads)) {
                 p->sched = s;
                 p->tuned = true;
             }

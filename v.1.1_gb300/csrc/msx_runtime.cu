@@ -144,7 +144,7 @@ struct msx_handle {
     double visc_c1 = 0, visc_cl = 0, visc_h = 0, visc_c0 = 0;
     DBuf<double> visc_f0;
     DBuf<float> visc_h0;
-    DBuf<int> d_counts;                 // tile queues of the tiled kernels
+    DBuf<int> d_counts;                 // the tiled element kernel's tile queue
     // scratch of the calls that compute and copy out (node and element values,
     // reductions, internal force), kept between calls up to kScratchKept bytes
     DBuf<unsigned char> scratch;
@@ -415,7 +415,7 @@ static bool pair_state(const msx_handle *h)
 
 static void launch_node_part(msx_handle *h, int parity)
 {
-    if (h->tiled) launch_solve_node(h->P, h->sched, h->d_counts.p, tiled_mode(h), parity, h->stream);
+    if (h->tiled) launch_solve_node(h->P, h->sched, tiled_mode(h), parity, h->stream);
     else h->node(h->P, parity, h->stream);
     if (h->nfaces) launch_face_loads(h->P, parity, pair_state(h), h->stream);
 }
@@ -453,8 +453,7 @@ static msx_status plan_tiled(msx_handle *h)
     q.fixed = h->P.fxE && !h->P.visc && !h->P.act_t ? fixed_form(h->P.mats[0].law) : FIXED_NONE;
     for (int k = 1; k < h->P.nmat; k++)
         if (fixed_form(h->P.mats[k].law) != q.fixed) q.fixed = FIXED_NONE;
-    q.elem_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, false, false, q.fixed);
-    q.node_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true);
+    q.elem_grid = sms * solve_elem_ctas(h->P, tiled_mode(h), q);
     // Element tiles of P whole CTA passes (P * threads elements).  Spread over
     // the grid, the busiest CTA runs ceil(tiles / grid) tiles; P minimises that
     // count times (P + 1/2), the half pass standing for a tile's close (the
@@ -479,10 +478,12 @@ static msx_status plan_tiled(msx_handle *h)
     // node passes of one CTA (four lanes a node), with batched gathers while all
     // their CTAs are resident at once (115,506 tets in mixed mode: 17.6 -> 16.4 us
     // a step)
-    const int batch_grid = sms * tiled_ctas_per_sm(tiled_mode(h), q.threads, true, false, FIXED_NONE, true);
-    q.node_batch = (h->P.nn + thr / 4 - 1) / (thr / 4) <= batch_grid;
-    q.node_tile = thr / 4;
-    if (q.node_batch) q.node_grid = batch_grid;
+    q.node_batch = 1;
+    q.node_grid = sms * solve_node_ctas(tiled_mode(h), q);
+    if ((h->P.nn + thr / 4 - 1) / (thr / 4) > q.node_grid) {
+        q.node_batch = 0;
+        q.node_grid = sms * solve_node_ctas(tiled_mode(h), q);
+    }
     if (!h->d_counts.p) {
         MSX_CUDA(h->d_counts.alloc(kTileSched));
         MSX_CUDA(cudaMemsetAsync(h->d_counts.p, 0, sizeof(int) * kTileSched, h->stream));
