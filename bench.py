@@ -13,7 +13,9 @@ Prints one JSON line: value = element-steps/s of the plain FP64 path with the
 mesh resident in HBM (device time of K steps), e2e = the same through the C ABI
 from host buffers (mesh upload, set-up, K steps and the read-back of u, v, a),
 plus the mixed-precision and reference-order variants, the element kernel's
-roofline and the CPU baseline.  --impl reference times the CPU implementation
+roofline and the CPU baseline.  The line holds each variant's headline figures;
+--details FILE writes the whole record (error histories, schedules, samples).
+--impl reference times the CPU implementation
 of the path (the oracle's C restatement on all host cores) on a bounded sample.
 Under torchrun each rank runs an independent replica ("replicas only").
 """
@@ -535,6 +537,27 @@ def barrier(ws):
         dist.barrier()
 
 
+# what the printed line keeps of a variant
+BRIEF = ("value", "ms_per_step", "rel_l2_u_vs_fp64", "all_ok", "lambda_per_s", "p50_ms",
+         "p99_ms", "offered_fraction_of_capacity", "saturated", "max_rel_l2_u_vs_fp64", "within_bar", "accuracy",
+         "worst_rel_l2_u", "worst_rel_vms")
+
+
+def brief(x, variant=False):
+    """The record without its notes, its variants cut to BRIEF and their figures to six digits: about three kilobytes."""
+    if isinstance(x, list):
+        return [brief(y, variant) for y in x]
+    if isinstance(x, dict):
+        out = {}
+        for k, v in x.items():
+            if k == "variants":
+                out[k] = {n: brief(y, True) for n, y in v.items()}
+            elif k in BRIEF if variant else k not in ("note", "wall_s_runs"):
+                out[k] = brief(v, variant)
+        return out
+    return float("%.6g" % x) if variant and isinstance(x, float) else x
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -547,6 +570,7 @@ def main():
     ap.add_argument("--no-pool", action="store_true", help="skip the batched and serving variants")
     ap.add_argument("--no-sweep", action="store_true", help="skip the precision sweep (6 x 5000 steps)")
     ap.add_argument("--sweep-steps", type=int, default=5000)
+    ap.add_argument("--details", default=None, help="also write the whole record to this file")
     ap.add_argument("--cube", type=int, default=N_CUBE, help="hexes per cube edge (profiling runs only)")
     ap.add_argument("--only", choices=["fp64", "mixed", "fp64_exact", "dword"], default=None,
                     help="time a single variant (profiling runs only)")
@@ -628,7 +652,7 @@ def main():
     ops = profiled("fp64_ops_per_element")
     opk, opk_kind = fp64_peak()
     step_gbs = alg_step / (secs / args.steps) / 1e9
-    roofline = {"bound": "hbm", "kernel": "solve_elem_cnh_kernel", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "integer pipes", "kernel": "solve_elem_cnh_kernel", "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                 "traffic": tr * ne if tr else None,
                 "alg_bytes_per_launch": alg_elem, "element_kernel_ms": prof.element_ms,
@@ -664,7 +688,10 @@ def main():
             "variants": variants}
     if not args.no_cpu:
         line["cpu_baseline"] = cpu_baseline(X, conn, bcs)
-    print(json.dumps(line))
+    if args.details:
+        with open(args.details, "w") as f:
+            json.dump(line, f, indent=1)
+    print(json.dumps(brief(line)))
 
 
 if __name__ == "__main__":
