@@ -532,10 +532,10 @@ MSX_HD void edge_forces(const EdgeElem &d, const double *e, double wJ, LAW law, 
 // An error of one unit in H, S or P is 2^-55 of the largest of them, against
 // 2^-53 of 1 for F's diagonal in FP64, whatever the strain.  Corner-force error
 // against extended precision over that of the FP64 form, grids of hexes of
-// 1:1:0.4 to 1:1:3, six tets each, jittered and not, nu 0 to 0.49, strains 1e-14 to 0.3: median 0.002
-// (linear) and 0.0004; above 1 only where both are below 1.5 roundings of the
-// result (grids whose sides are powers of two, on which FP64's own products can
-// be exact) or, to 1.2, at strains of 0.3.  One StVK step of 264,000 shuffled
+// 1:1:0.4 to 1:1:3, six tets each, jittered and not, nu 0 to 0.49, strains 1e-14
+// to 0.3: median 0.002 (linear) and 0.0004; above 1 only where both are below 1.5
+// roundings of the result (grids whose sides are powers of two, on which FP64's
+// own products can be exact) or, to 1.3, at strains of 0.3.  One StVK step of 264,000 shuffled
 // tets: 64.7 us, 63.0 with a unit set by the element alone, whose error at a
 // shear of 1e-5 on a cubic grid was 8,700 (linear) and 4.4 times FP64's.  With
 // products of edges instead, E_b . E_c and their metric, the error is 2 to 8
