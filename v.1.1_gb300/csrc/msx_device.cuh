@@ -3054,7 +3054,9 @@ __device__ __forceinline__ void write_fixed_arrays(const Problem &p, long long e
 
 // classLinearTetrahedra.cpp:171-268 (Jacobian, inverse, dphi), classGPs.cpp:27
 // (wJ = 0.166666666667 |J|), classLinearTetrahedra.cpp:129-140 (charLength).
-__global__ void setup_elements_kernel(Problem p, const double *X, double *G, double *wJ, double *Lref,
+// Two CTAs an SM: the fixed-point data's 128-bit products would take 133
+// registers, one CTA, and msx_create of 6M tets 5.57 ms instead of 5.13.
+__global__ void __launch_bounds__(256, 2) setup_elements_kernel(Problem p, const double *X, double *G, double *wJ, double *Lref,
                                       float *G32, float *wJ32, float *Lref32, long long e0, long long e1)
 {
     const long long e = e0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;   // elements [e0, e1)
