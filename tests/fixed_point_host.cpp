@@ -158,33 +158,4 @@ extern "C" void fp64_cnh(long long n, const double *X, const double *u, double l
     }
 }
 
-// The FP64 edge form of the elements that fixed_cnh leaves out, from FP64 data
-// (an element left out at set-up) or from the integers of one inside its range.
-extern "C" void edge_cnh(long long n, const double *X, const double *u, double lambda, double mu, int integers, double *f,
-                         int *taken)
-{
-    int64_t kq[kFixTerms];
-    int ks;
-    fixed_series(lambda, mu, kq, &ks);
-    for (long long k = 0; k < n; k++) {
-        FixedElem q;
-        EdgeElem d;
-        double E[9], ua[4][3], e[9], c[9];
-        edges(X + 12 * k, E);
-        nodes(u + 12 * k, ua);
-        if (integers) {
-            taken[k] = fixed_setup(E, kq[0], ks, q) && edge_from_fixed(q, d);
-        } else {
-            taken[k] = 1;
-            edge_setup(E, mu, d);
-        }
-        if (!taken[k]) continue;
-        for (int j = 0; j < 9; j++) e[j] = d.E[j] + (ua[j / 3 + 1][j % 3] - ua[0][j % 3]);
-        const double wJ = 0.166666666667 * std::fabs(fp64_crosses(E, c));
-        double *o = f + 12 * k;
-        edge_forces(d, e, wJ, [&](double J) { return lambda * std::log(J) - mu; }, o + 3);
-        for (int i = 0; i < 3; i++) o[i] = -(o[3 + i] + o[6 + i] + o[9 + i]);
-    }
-}
-
 extern "C" double to_fp64(long long x, int k) { return fixed_to_fp64(x, k); }

@@ -182,29 +182,6 @@ def test_no_less_accurate_than_fp64_cnh(lib, motion):
             assert ours <= max(theirs, 2 * EPS), (nu, strain, ours, theirs)
 
 
-# ------------------------------------------------------------------ the FP64 form of left-out elements
-@pytest.mark.parametrize("integers", [0, 1])
-@pytest.mark.parametrize("flat", [1.0, 0.05, 0.004, 30.0])
-def test_edge_form(lib, integers, flat):
-    """Far inside the range to far beyond: right whatever the data come from; integers exist above the flatness limit."""
-    rng = np.random.default_rng(5)
-    for scale in (1.0, 1e-9, 1e7):
-        X, conn = tets(rng, scale, flat)
-        x = X.T[conn]
-        for s in (1.0, 1.5, 5.0, 40.0):
-            y = np.einsum("nij,naj->nai", s * np.eye(3) + 1e-2 * rng.uniform(-1, 1, (N, 3, 3)), x - x[:, :1]) + x[:, :1]
-            u = np.ascontiguousarray((y - x).reshape(4 * N, 3).T)
-            lam, mu2 = lame(0.3)
-            xs, w = np.ascontiguousarray(x), np.ascontiguousarray(u.T[conn])
-            f, taken = np.zeros(x.shape), np.zeros(N, np.int32)
-            lib.edge_cnh(C.c_longlong(N), _p(xs), _p(w), C.c_double(lam), C.c_double(0.5 * mu2), C.c_int(integers), _p(f),
-                         _p(taken))
-            want, bound = cnh.reference(X, u, conn, lam, 0.5 * mu2)
-            err = np.abs((f - want).astype(float)).max(-1) / (64 * EPS * bound)
-            assert (err[taken == 1] <= 1.0).all()
-            assert taken.all() if not integers or flat == 1.0 else True
-
-
 def test_integer_to_fp64(lib):
     lib.to_fp64.restype = C.c_double
     rng = np.random.default_rng(6)

@@ -1595,49 +1595,19 @@ __device__ __forceinline__ float elem_cofactor_fp64(const Problem &p, long long 
     return scr;
 }
 
-// Compressible neo-Hookean elements that fixed point leaves out (set-up: flat,
-// graded, out of range; at a step: stretched past 2 to 4), in FP64 from their
-// deformed edges: about 110 FP64 operations against the cofactor form's 130.  Their
-// data lie in the fixed-point arrays, as FP64 bits for those left out at set-up
-// (a zero fxw).
-template <bool FORCE_ONLY>
-__device__ __forceinline__ float elem_edges_fp64(const Problem &p, long long e, int parity, const MatParams &m,
-                                                 const int *nd, const EdgeElem &d, float gmin)
-{
-    double ua[4][3], du[9], ed[9];
-    gather_u<FORCE_ONLY>(p, nd, ua);
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        du[k] = ua[k / 3 + 1][k % 3] - ua[0][k % 3];
-        ed[k] = d.E[k] + du[k];
-    }
-    float scr = INFINITY;
-    if (!FORCE_ONLY && !(gate_moved(__ldg(p.Lref32 + e), 1.7321f * abs_bound<9>(du), m.inv_c_f) > gmin)) {
-        float e32[9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) e32[k] = f32_trunc(ed[k]);
-        scr = cfl_screen_edges(p, e, e32, e32 + 3, e32 + 6, m);
-    }
-    double f[9];
-    edge_forces(d, ed, __ldg(p.wJ + e), [&](double J) { return m.lambda * log_near1(J) - m.mu; }, f);
-    const int4 sl = __ldg(p.slot + e);
-    st_slot24(p.fe, sl.x, -(f[0] + f[3] + f[6]), -(f[1] + f[4] + f[7]), -(f[2] + f[5] + f[8]));
-    st_slot24(p.fe, sl.y, f[0], f[1], f[2]);
-    st_slot24(p.fe, sl.z, f[3], f[4], f[5]);
-    st_slot24(p.fe, sl.w, f[6], f[7], f[8]);
-    if (!FORCE_ONLY && e == 0 && !isfinite(p.u[1])) atomicOr(p.flags + (parity ^ 1), 1);
-    return scr;
-}
-
 __device__ __forceinline__ void load_G(const Problem &p, long long e, double *G)
 {
 #pragma unroll
     for (int k = 0; k < 9; k++) G[k] = __ldg(p.G + k * p.ne + e);
 }
 
-// The FP64 form of an element that fixed point leaves out.  One function for all
-// kernels: which product of a b + c d is fused is the compiler's choice, and
-// would differ between instantiations.
+// An element that fixed point leaves out, in the FP64 cofactor form.  The form
+// from the deformed edges (f_a = sum_b S_ab e_b + c2 e_c x e_d, 110 operations
+// for 130) is a little faster, but compressible neo-Hookean elements are left
+// out because they are flat, and there its error is 5 to 10 times this one's
+// (hexes of 1:1:0.1, strain 1e-4: 2e-11 to 4e-11 of the forces, 4e-12 here).
+// One function for all kernels: which product of a b + c d is fused is the
+// compiler's choice, and would differ between instantiations.
 template <bool FORCE_ONLY, bool ACT>
 static __device__ __noinline__ float elem_left_out(const Problem &p, long long e, int parity, double t, float gmin)
 {
@@ -1647,32 +1617,6 @@ static __device__ __noinline__ float elem_left_out(const Problem &p, long long e
     const MatParams &m = mat_of(p, e);
     double G[9];
     if (m.law == 1) {
-        const uint2 w = __ldg(p.fxw + e);
-        FixedElem q;
-        EdgeElem d;
-        q.rd = __ldg(&p.fxD[e].y);
-        bool edges = true;
-        if (w.x == 0) {
-            d.rdet = bits_double((uint64_t)q.rd);
-#pragma unroll
-            for (int k = 0; k < 9; k++) d.E[k] = bits_double((uint64_t)__ldg(p.fxE + k * ne + e));
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                const int2 x = __ldg(p.fxS + k * ne + e);
-                d.S[k] = __hiloint2double(x.x, x.y);
-            }
-        } else {
-            fixed_unpack(w.x, w.y, q);
-#pragma unroll
-            for (int k = 0; k < 9; k++) q.E[k] = __ldg(p.fxE + k * ne + e);
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                const int2 x = __ldg(p.fxS + k * ne + e);
-                q.S[k] = {x.x, x.y};
-            }
-            edges = edge_from_fixed(q, d);
-        }
-        if (edges) return elem_edges_fp64<FORCE_ONLY>(p, e, parity, m, nd, d, gmin);
         load_G(p, e, G);
     } else {   // the gradients, FP64 bits or limbs of w g 2^(111 - gs)
         const uint2 w = __ldg(p.fxw + e);
@@ -2595,7 +2539,7 @@ constexpr int node_ctas(int mode, bool batch) { return batch ? (mode == MODE_MIX
 
 // 64 registers, four CTAs an SM: a step of 16 mixed solves of 162,000 tets 182 us,
 // 204 with 48 registers (five CTAs, best for one solve, leave the tile queue a
-// longer last round), 194 with 80; 256 solves 1.97e10, 1.90e10 and 1.93e10
+// longer last wave), 194 with 80; 256 solves 1.97e10, 1.90e10 and 1.93e10
 // element-steps/s; FP64 and double-word as with five, 3 to 4 % slower with three.
 template <int MODE>
 __global__ void __launch_bounds__(kStepThreads, 4) pool_node_kernel(const Problem *__restrict__ descs, const Tile *__restrict__ tiles,
@@ -2722,8 +2666,8 @@ __device__ __forceinline__ float tile_elements(const Problem &p, const Tile &tl,
 // The nl elements of a tile that fixed point left out, in FP64 by consecutive
 // threads: one of them in a warp costs it the FP64 pipe as long as 32 do.  1M
 // tets in hexes of 1:1:0.2, compressible neo-Hookean, a third of them left out
-// and every warp with some: 331 us a step, 622 with the FP64 form inside their
-// warps (407 with all elements in FP64); 1:1:3, jittered, 202, 349 and 276.
+// and every warp with some: 346 us a step, 622 with the FP64 form inside their
+// warps (407 with all elements in FP64); 1:1:3, jittered, 217, 349 and 276.
 // Lists CFL candidates and returns the thread's minimum as tile_elements does.
 // Left-out elements lie at the end of scand, last one first; an element is in
 // one list at a time, and a pass reads its entries, the lowest that remain,
@@ -3024,18 +2968,6 @@ __device__ __forceinline__ void write_fixed_arrays(const Problem &p, long long e
 #pragma unroll
         for (int k = 0; k < 6; k++) const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2(q.S[k].h, q.S[k].l);
         const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(q.d0, q.rd);
-    } else if (m.law == 1) {   // left to the FP64 edge form
-        EdgeElem d;
-        edge_setup(E, m.mu, d);
-#pragma unroll
-        for (int k = 0; k < 9; k++) const_cast<long long *>(p.fxE)[k * ne + e] = (long long)double_bits(d.E[k]);
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            const uint64_t b = double_bits(d.S[k]);
-            const_cast<int2 *>(p.fxS)[k * ne + e] = make_int2((int)(b >> 32), (int)(uint32_t)b);
-        }
-        const_cast<longlong2 *>(p.fxD)[e] = make_longlong2(0, (long long)double_bits(d.rdet));
-        w[0] = 0;
     } else if (m.law >= 2 && fixed_setup_svk(E, 0.5 * m.mu2, m.ks, q)) {
         fixed_pack(q, w);
 #pragma unroll

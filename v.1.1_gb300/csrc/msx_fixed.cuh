@@ -441,80 +441,6 @@ MSX_HD bool fixed_setup(const double *E, int64_t kq0, int ks, FixedElem &q)
     return q.x0 - lmin <= 900 && q.x0 - lmax >= -900;   // forces stay normal FP64 numbers
 }
 
-// What the FP64 edge form (below) needs of an element that the fixed-point form
-// leaves out: the reference edges, S_ab = W |det E| mu g_a.g_b and 1 / det E, as
-// FP64 bits where fixed_setup refused the element and its data hold no integers.
-struct EdgeElem {
-    double E[9], S[6], rdet;
-};
-
-// e1 x e2 etc. (rows a: the cross product of the other two edges) and det e
-MSX_HD double fp64_crosses(const double *e, double *cr)
-{
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int p = 3 * ((a + 1) % 3), q = 3 * ((a + 2) % 3), y = (i + 1) % 3, z = (i + 2) % 3;
-            cr[3 * a + i] = fma(e[p + y], e[q + z], -(e[p + z] * e[q + y]));
-        }
-    return fma(e[2], cr[2], fma(e[0], cr[0], e[1] * cr[1]));
-}
-
-MSX_HD void edge_setup(const double *E, double mu, EdgeElem &d)
-{
-    double c[9];
-    const double det = fp64_crosses(E, c), w = 0.166666666667 * mu / fabs(det);
-    int k = 0;
-    for (int a = 0; a < 3; a++)
-        for (int b = a; b < 3; b++)
-            d.S[k++] = w * fma(c[3 * a + 2], c[3 * b + 2], fma(c[3 * a], c[3 * b], c[3 * a + 1] * c[3 * b + 1]));
-    for (k = 0; k < 9; k++) d.E[k] = E[k];
-    d.rdet = 1.0 / det;
-}
-
-// The same from the integers of an element inside fixed_setup's range; false
-// where S might not be a normal FP64 number.
-MSX_HD bool edge_from_fixed(const FixedElem &q, EdgeElem &d)
-{
-    const int lw = fixed_lw_min(q);
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        const int s = q.lw[k / 3] - lw;
-        d.E[k] = fixed_to_fp64(q.E[k] - (s ? 1LL << (s - 1) : 0), lw);
-    }
-    bool normal = true;
-    int k = 0;
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = a; b < 3; b++) {
-            const int x = q.x0 - 58 - q.lw[a] - q.lw[b];
-            normal = normal && x >= -1000 && x <= 900;
-            d.S[k] = fixed_to_fp64(((int64_t)q.S[k].h << 29) + q.S[k].l, x);
-            k++;
-        }
-    d.rdet = fixed_to_fp64(q.rd, -(62 + q.ds) - 114 - (q.lw[0] + q.lw[1] + q.lw[2]));
-    return normal;
-}
-
-// Corner forces f_1..f_3 (f[3(a-1) + i]) in FP64 from the deformed edges e:
-// f_a = sum_b S_ab e_b + c2 (e_c x e_d); law(J) gives lambda ln J - mu; wJ is
-// W |det E|.
-template <typename LAW>
-MSX_HD void edge_forces(const EdgeElem &d, const double *e, double wJ, LAW law, double *f)
-{
-    double cr[9];
-    const double det = fp64_crosses(e, cr), c2 = law(det * d.rdet) * (wJ / det);
-    const int mi[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-            f[3 * a + i] = fma(c2, cr[3 * a + i],
-                               fma(e[6 + i], d.S[mi[3 * a + 2]], fma(e[i], d.S[mi[3 * a]], e[3 + i] * d.S[mi[3 * a + 1]])));
-}
-
 // St-Venant-Kirchhoff and linear elasticity: the displacement gradient and the
 // stress in the axes of space, as in FP64 (products of the edges would lose
 // accuracy with the square of an element's flatness).  With the shape

@@ -107,12 +107,11 @@ struct Problem {
     double *u4;
     int dependent;   // this launch may begin before the one that writes u4 has ended (SolveSched::pdl)
     // plain FP64 mode: the fixed-point data of msx_fixed.cuh and the packed
-    // exponents fxw; a zero word: the element is left to FP64, and the arrays
-    // hold FP64 bits.  Compressible neo-Hookean elements: the reference edges
+    // exponents fxw; a zero word: the element is left to FP64.  Compressible neo-Hookean elements: the reference edges
     // (9*ne: fxE[(3(b-1) + i)*ne + e], b = 1..3), S's limbs (6*ne: fxS[k*ne + e])
-    // and (d0, rd); left out: EdgeElem's E, S and, in fxD.y, 1 / det E.
+    // and (d0, rd).
     // St-Venant-Kirchhoff and linear elastic ones: the limbs of w g (fxE, the
-    // same order) and the scale's (fxD.x); left out: G.  Null in the other modes;
+    // same order) and the scale's (fxD.x); left out: G's FP64 bits in fxE.  Null in the other modes;
     // fxS only with a compressible neo-Hookean material.
     const long long *fxE;
     const int2 *fxS;
